@@ -182,6 +182,29 @@ void collect(cz_ctx *c)
     }
 }
 
+// The field descriptors and, behind them, the fields' tensor maps to the
+// device in one copy; `extra` bytes of pinned scratch stay free after them.
+size_t maps_at(size_t nfields) { return (sizeof(CzField) * nfields + 127) / 128 * 128; }
+size_t fields_bytes(size_t nfields) { return maps_at(nfields) + sizeof(CUtensorMap) * nfields; }
+const CUtensorMap *maps_of(cz_ctx *c, size_t nfields)
+{
+    return reinterpret_cast<const CUtensorMap *>(P<uint8_t>(c->fields) + maps_at(nfields));
+}
+int put_fields(cz_ctx *c, const std::vector<CzField> &fields, size_t extra, cudaStream_t st)
+{
+    const size_t n = fields.size(), bytes = fields_bytes(n);
+    CZ_TRY(grow(c, c->fields, bytes));
+    CZ_TRY(grow_pin(c, std::max<size_t>(4096, bytes + extra)));
+    memcpy(c->pin, fields.data(), sizeof(CzField) * n);
+    for (size_t i = 0; i < n; ++i) {
+        CUtensorMap m;
+        if (!cz_field_map(fields[i], &m)) return fail(c, CZ_E_CUDA, "no tensor map for a field");
+        memcpy(static_cast<char *>(c->pin) + maps_at(n) + sizeof(m) * i, &m, sizeof(m));
+    }
+    CZ_CUDA(c, cudaMemcpyAsync(c->fields.p, c->pin, bytes, cudaMemcpyHostToDevice, st));
+    return CZ_OK;
+}
+
 // The compress pipeline in three steps:
 //   prepare  grows the context's buffers for the workload and uploads the
 //            field descriptors (may allocate and copy);
@@ -212,7 +235,6 @@ int prepare(cz_ctx *c, const std::vector<CzField> &fields, long long nblocks, co
     job.lz_slot = ((zlib ? seq_bound_ll(chunk_max) : lz4_bound_ll(chunk_max)) + 15) / 16 * 16;
     job.z_slot = zlib ? (zlib_bound_ll(chunk_max) + 16 + 15) / 16 * 16 : 0;
     const int nchunks = job.nchunks;
-    CZ_TRY(grow(c, c->fields, sizeof(CzField) * fields.size()));
     CZ_TRY(grow(c, c->stage, (size_t)nblocks * kSlotBytes));
     CZ_TRY(grow(c, c->rec_bytes, sizeof(int) * nblocks));
     CZ_TRY(grow(c, c->in_off, sizeof(long long) * nchunks));
@@ -240,11 +262,8 @@ int prepare(cz_ctx *c, const std::vector<CzField> &fields, long long nblocks, co
     CZ_TRY(grow(c, c->out_data, out_cap));
     const int grid = (int)std::min<long long>(nblocks, c->sms);
     if (refit_iters > 0) CZ_TRY(grow(c, c->refit, sizeof(float) * cz_refit_scratch_floats(grid)));
-    CZ_TRY(grow_pin(c, std::max<size_t>(4096, sizeof(CzField) * fields.size() + 64)));
-    memcpy(c->pin, fields.data(), sizeof(CzField) * fields.size());
     // finish() reuses the pinned staging only after this copy (stream order)
-    CZ_CUDA(c, cudaMemcpyAsync(c->fields.p, c->pin, sizeof(CzField) * fields.size(), cudaMemcpyHostToDevice, st));
-    return CZ_OK;
+    return put_fields(c, fields, 0, st);
 }
 
 int enqueue(cz_ctx *c, const Job &job, cudaStream_t st, bool marks)
@@ -263,7 +282,8 @@ int enqueue(cz_ctx *c, const Job &job, cudaStream_t st, bool marks)
     else
         CZ_CUDA(c, cz_launch_encode(p->wtype, P<CzField>(c->fields), job.nfields, nblocks, p->zerobits,
                                     p->shuffle ? 1 : 0, P<uint8_t>(c->stage), P<int>(c->rec_bytes),
-                                    P<unsigned long long>(c->queue), grid, st, job.enc_variant));
+                                    P<unsigned long long>(c->queue), grid, st, maps_of(c, job.nfields), nullptr,
+                                    P<int>(c->flag) + 1, job.enc_variant));
     if (marks) CZ_TRY(mark(c, 1, st));
     CZ_CUDA(c, cz_launch_chunk_setup(bpc, nblocks, nchunks, P<int>(c->rec_bytes), P<long long>(c->in_off),
                                      P<int>(c->in_len), bpc > 1 ? P<long long>(c->blk_dst) : nullptr,
@@ -319,8 +339,9 @@ int finish(cz_ctx *c, const Job &job, cudaStream_t st, cz_stream *out)
     const int nchunks = job.nchunks;
     CZ_CUDA(c, cudaMemcpyAsync(&h[0], P<long long>(c->out_off) + nchunks, 8, cudaMemcpyDeviceToHost, st));
     CZ_CUDA(c, cudaMemcpyAsync(&h[1], P<long long>(c->raw_off) + nchunks, 8, cudaMemcpyDeviceToHost, st));
-    CZ_CUDA(c, cudaMemcpyAsync(&h[2], c->flag.p, 4, cudaMemcpyDeviceToHost, st));
+    CZ_CUDA(c, cudaMemcpyAsync(&h[2], c->flag.p, 8, cudaMemcpyDeviceToHost, st));
     CZ_CUDA(c, cudaStreamSynchronize(st));
+    if (reinterpret_cast<int *>(&h[2])[1] != 0) return fail(c, CZ_E_CUDA, "wavelet kernel: a tile copy did not complete");
     if (reinterpret_cast<int *>(&h[2])[0] != 0)
         return fail(c, CZ_E_CUDA, "lossless encoder output exceeded its bound");
     c->nblocks = job.nblocks;
@@ -359,7 +380,6 @@ int decompress_fields(cz_ctx *c, const std::vector<CzField> &fields, long long n
     const int per_chunk = h_block_chunk ? maxsub : bpc;
     if (diff_ref) CZ_TRY(grow(c, c->diff, sizeof(double) * (8 * (size_t)nblocks + 8)));
     const long long dcap = ((long long)per_chunk * (4 + kMaxRecord) + 15) / 16 * 16;
-    CZ_TRY(grow(c, c->fields, sizeof(CzField) * fields.size()));
     CZ_TRY(grow(c, c->in_len, sizeof(int) * nchunks));
     CZ_TRY(grow(c, c->dec_off, sizeof(long long) * nchunks));
     CZ_TRY(grow(c, c->dec_cap, sizeof(int) * nchunks));
@@ -369,12 +389,10 @@ int decompress_fields(cz_ctx *c, const std::vector<CzField> &fields, long long n
     CZ_TRY(grow(c, c->queue, 64));
     CZ_TRY(grow(c, c->flag, 64));
     if (encoder != CZ_ENCODER_NONE) CZ_TRY(grow(c, c->dec, (size_t)nchunks * dcap));
-    // pinned scratch: [fields | flag (64 B) | block map]
-    const size_t pin_fields = (sizeof(CzField) * fields.size() + 63) / 64 * 64;
+    // pinned scratch: [fields and tensor maps | flag (64 B) | block map]
+    const size_t pin_fields = fields_bytes(fields.size());
     const size_t map_bytes = h_block_chunk ? sizeof(int) * 2 * nblocks : 0;
-    CZ_TRY(grow_pin(c, std::max<size_t>(4096, pin_fields + 64 + map_bytes)));
-    memcpy(c->pin, fields.data(), sizeof(CzField) * fields.size());
-    CZ_CUDA(c, cudaMemcpyAsync(c->fields.p, c->pin, sizeof(CzField) * fields.size(), cudaMemcpyHostToDevice, st));
+    CZ_TRY(put_fields(c, fields, 64 + map_bytes, st));
     CZ_CUDA(c, cudaMemsetAsync(c->queue.p, 0, 64, st));
     CZ_CUDA(c, cudaMemsetAsync(c->flag.p, 0, 64, st));
     const int raw = encoder == CZ_ENCODER_NONE;
@@ -430,7 +448,7 @@ int decompress_fields(cz_ctx *c, const std::vector<CzField> &fields, long long n
     double *per_block = diff_ref ? P<double>(c->diff) : nullptr;
     CZ_CUDA(c, cz_launch_decode(wtype, P<CzField>(c->fields), (int)fields.size(), nblocks, shuffle ? 1 : 0, base,
                                 P<long long>(c->rec_off), P<int>(c->status), P<unsigned long long>(c->queue), grid,
-                                st, diff_ref, per_block, planes));
+                                st, maps_of(c, fields.size()), diff_ref, per_block, planes));
     if (diff_ref) CZ_CUDA(c, cz_launch_diff_total(per_block, nblocks, per_block + 8 * nblocks, st));
     CZ_TRY(mark(c, 3, st));
     CZ_CUDA(c, cz_launch_status_reduce(P<int>(c->status), nblocks, P<int>(c->flag), st));
@@ -1223,7 +1241,8 @@ int cz_compress_to_image(cz_ctx *c, const float *h_field, int nx, int ny, int nz
         uint8_t *stage = P<uint8_t>(c->stage) + f0 * kSlotBytes;
         CZ_CUDA(c, cudaStreamWaitEvent(cs, c->ev_h2d[i], 0));
         CZ_CUDA(c, cz_launch_encode(p->wtype, P<CzField>(c->fields) + i, 1, n, p->zerobits, p->shuffle ? 1 : 0, stage,
-                                    P<int>(c->rec_bytes) + f0, queues + i, std::min(n, c->sms), cs));
+                                    P<int>(c->rec_bytes) + f0, queues + i, std::min(n, c->sms), cs,
+                                    maps_of(c, nslab) + i, nullptr, P<int>(c->flag) + 1));
         CZ_CUDA(c, cz_launch_chunk_setup(1, n, n, P<int>(c->rec_bytes) + f0, P<long long>(c->in_off) + f0,
                                          P<int>(c->in_len) + f0, nullptr, P<long long>(c->lz_off) + f0, job.lz_slot,
                                          cs));
@@ -1258,12 +1277,13 @@ int cz_compress_to_image(cz_ctx *c, const float *h_field, int nx, int ny, int nz
     CZ_CUDA(c, cudaStreamWaitEvent(st, c->ev_join, 0));
     // sizes and offsets back, then the host-side tail
     std::vector<long long> off(job.nchunks + 1);
-    int flag = 0;
+    int flag[2] = {0, 0};
     CZ_CUDA(c, cudaMemcpyAsync(off.data(), c->out_off.p, sizeof(long long) * (job.nchunks + 1), cudaMemcpyDeviceToHost,
                                st));
-    CZ_CUDA(c, cudaMemcpyAsync(&flag, c->flag.p, 4, cudaMemcpyDeviceToHost, st));
+    CZ_CUDA(c, cudaMemcpyAsync(flag, c->flag.p, 8, cudaMemcpyDeviceToHost, st));
     CZ_CUDA(c, cudaStreamSynchronize(st));
-    if (flag != 0) return fail(c, CZ_E_CUDA, "LZ4 encoder output exceeded its bound");
+    if (flag[1] != 0) return fail(c, CZ_E_CUDA, "wavelet kernel: a tile copy did not complete");
+    if (flag[0] != 0) return fail(c, CZ_E_CUDA, "LZ4 encoder output exceeded its bound");
     const long long payload = off[job.nchunks];
     const long long need = czf::image_bytes(payload, job.nchunks, nblocks, hdr);
     if (need > cap) return fail(c, CZ_E_SPACE, "image buffer too small");

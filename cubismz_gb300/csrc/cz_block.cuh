@@ -62,19 +62,6 @@ __device__ __forceinline__ size_t row_offset(const BlockRef &r, int y, int z)
     return ((size_t)(r.bz * 32 + z) * f.ny + (size_t)(r.by * 32 + y)) * f.nx + (size_t)r.bx * 32;
 }
 
-// Rows (y, z) and (y, z+16) of a block, y = tid&31, z = tid>>5: the two x
-// lines this thread transforms first.
-__device__ __forceinline__ void load_rows(const BlockRef &r, float4 (&pf)[16])
-{
-    const int y = threadIdx.x & 31, z = threadIdx.x >> 5;
-    const float4 *r0 = reinterpret_cast<const float4 *>(r.f->data + row_offset(r, y, z));
-    const float4 *r1 = reinterpret_cast<const float4 *>(r.f->data + row_offset(r, y, z + 16));
-#pragma unroll
-    for (int k = 0; k < 8; ++k) pf[k] = __ldg(r0 + k);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) pf[8 + k] = __ldg(r1 + k);
-}
-
 template <int N>
 __device__ __forceinline__ unsigned keep_bits(const float (&v)[N], float eps)
 {
@@ -275,10 +262,7 @@ __device__ __forceinline__ void run_geom(int r, int &base, int &stride)
 // Needs s.off from scan_segments and S, the survivor total.
 //   emit: every lane copies its run's survivors from the block into the
 //         warp's stage, then the warp hands them out in stream order,
-//         put(k, value) with k consecutive across the warp;
-//   load: the warp fetches the group's values in stream order,
-//         get(k) with k consecutive across the warp, into the stage; every
-//         lane then places its run's survivors in the block.
+//         put(k, value) with k consecutive across the warp.
 template <class Put>
 __device__ __forceinline__ void emit_survivors(const Shared &s, int S, Put &&put)
 {
@@ -304,58 +288,8 @@ __device__ __forceinline__ void emit_survivors(const Shared &s, int S, Put &&put
         __syncwarp();
     }
 }
-template <class Get>
-__device__ __forceinline__ void load_survivors(const Shared &s, int S, Get &&get)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float *stg = s.stage + warp * kStagePerWarp;
-    if (threadIdx.x < 64) {
-        const int t = threadIdx.x;
-        s.sb[pidx(t & 3, (t >> 2) & 3, t >> 4)] = get(t);
-    }
-    for (int r0 = kSegBase8 + 32 * warp; r0 < kSegs; r0 += 32 * kNW) {
-        const int r = r0 + lane;
-        const unsigned m = r < kSegs ? run_mask(s, r) : 0u;
-        const int o = r < kSegs ? s.off[r] : S;
-        const int first = __shfl_sync(0xffffffffu, o, 0);
-        const int total = __shfl_sync(0xffffffffu, o + __popc(m), 31) - first;
-        if (total > 0) {
-            for (int b = lane; b < total; b += 32) stg[b] = get(first + b);
-            __syncwarp();
-        }
-        int base = 0, stride = 0;
-        if (r < kSegs) run_geom(r, base, stride);
-        int i = o - first;
-        // every place of the run: its survivor or zero (the runs and the
-        // coarse corner cover the whole block, so no separate zeroing)
-        const int len = r < kSegBase16 ? 4 : (r < kSegBase32 ? 8 : 16);
-        if (r < kSegs)
-            for (int e = 0; e < len; ++e) s.sb[base + e * stride] = ((m >> e) & 1u) ? stg[i++] : 0.f;
-        __syncwarp();
-    }
-}
 
 // ------------------------------------------------------------------ decode
-// Run masks from the positional mask words (the inverse of emit32/16/8).
-__device__ __forceinline__ void runs_from_mask(const Shared &s)
-{
-    for (int i = threadIdx.x; i < kSeg32; i += kNT) {
-        const int c = (i >> 8) + 1, sub = i & 255;
-        const int x = 16 * ((c >> 1) & 1) + (sub & 15), y = 16 * (c >> 2) + (sub >> 4);
-        s.seg32[i] = (uint16_t)(s.mask32[x + 32 * y] >> (16 * (c & 1)));
-    }
-    for (int i = threadIdx.x; i < kSeg16; i += kNT) {
-        const int c = (i >> 6) + 1, sub = i & 63;
-        const int x = 8 * (c >> 2) + (sub >> 3), z = 8 * ((c >> 1) & 1) + (sub & 7);
-        s.seg16[i] = (uint8_t)(s.mask32[z + 32 * x] >> (8 * (c & 1)));
-    }
-    for (int i = threadIdx.x; i < kSeg8; i += kNT) {
-        const int c = (i >> 4) + 1, sub = i & 15;
-        const int y = 4 * ((c >> 1) & 1) + (sub & 3), z = 4 * (c >> 2) + (sub >> 2);
-        s.seg8[i] = (uint8_t)((s.mask32[y + 32 * z] >> (4 * (c & 1))) & 0xF);
-    }
-}
-
 // n bytes from p into L2, one 128-byte line per thread and step, by
 // threads t of nt (a hint: nothing is read into registers)
 __device__ __forceinline__ void prefetch_l2_span(const uint8_t *p, int n, int t, int nt)
@@ -402,7 +336,6 @@ struct Payload {
 __device__ __forceinline__ void emit_record(const Shared &s, long long g, uint32_t zmask, int shuffle, uint8_t *stage,
                                             int *rec_bytes)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // ---- offsets of every run, record header and mask
     const int S = scan_segments(s);
     const int nb = kMaskBytes + 4 * S;

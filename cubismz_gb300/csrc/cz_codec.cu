@@ -14,127 +14,448 @@
 // One CTA of 512 threads per SM, persistent; blocks come from a device work
 // queue, so one launch serves one field or a batch of uneven fields.
 //
-// Block layout in shared memory: coefficient (x,y,z) at x + 33y + 1057z. Lines
-// along any axis are read with immediate offsets and hit 32 distinct banks
-// (lane strides 33 and 1057 are 1 mod 32).
-//
-// Thresholding is fused into the last sweep of each level: the thread that
-// finishes a line holds exactly one run of the reference's survivor order
-// per octant (16 coefficients along z at level 32, 8 along y at level 16, 4
-// along x at level 8, cz_layout.cuh) and the matching bits of one mask word,
-// so it records a keep mask per run and its mask bits. One scan over the run
-// counts gives every run's output offset; one pass then writes the survivors.
-//
-// Encode pipeline per block: the x sweep takes its lines from registers that
-// were loaded while the previous block was finishing (levels 16/8, scan and
-// emission), so HBM reads overlap compute.
+// What bounds these kernels is not memory (a block is 128 KB in, under 60 KB
+// out) but one block's serial chain: nine sweeps, each needing the whole
+// result of the one before, with the SM to itself (a block fills more than
+// half of shared memory). So the chain is cut to five block-wide barriers:
+//   * planes -- the x and y sweeps of level 32 only mix values of one z plane,
+//     so a warp takes a plane through both on its own. Planes move between
+//     the field and a ring of 4 KB slots by TMA (128-byte swizzle: the x
+//     lines, one per lane, are read and written as 16-byte words without
+//     bank conflicts); a consumed slot is refilled at once, which brings in
+//     the next block while this one finishes.
+//   * slabs -- the block lies as [y][z][x], so the z lines of one y are 4 KB
+//     that belong to one warp. It transforms them, thresholds them (a lane's
+//     line holds two runs of the survivor order) and packs the survivors of
+//     each octant into a quarter of the same slab, so that they leave the SM
+//     in stream order without a second pass over the block. The corner's z
+//     lines continue through level 16 in registers, as the corner's y lines
+//     later do through level 8.
+//   * corner -- levels 16 and 8 (an eighth of the block) stay in the first
+//     quarters of slabs 0..15 and are thresholded 8 positions per thread.
+// The decoder runs the same steps backwards. Measured at 512^3 (wtype 1,
+// threshold 1e-3 of the range): encode 0.664 -> 0.429 ms, decode 0.730 ->
+// 0.646 ms against one thread-block-wide pass per sweep with row loads into
+// registers (fourteen barriers a block, 16-byte loads and stores that touch
+// 32 rows each).
 #include "cz_block.cuh"
+#include "cz_tma.cuh"
 
 namespace cz {
 
-// SPLIT: the next block's rows are loaded by the warps level 16 leaves idle
-// during level 16 and by the others after it; otherwise every thread loads
-// its rows after level 32 (one of the autotuner's shapes).
-template <int KIND, bool SPLIT>
-__device__ __forceinline__ void encode_body(const CzField *fields, int nfields, long long total_blocks, int zerobits,
-                                            int shuffle, uint8_t *stage, int *rec_bytes, unsigned long long *queue)
+// ------------------------------------------------------- shared memory map
+constexpr int kMain = 0;                           // [y][z][x], 128 KB; slab y at 4096 y
+constexpr int kPlane = 4096;                       // bytes of a z plane and of a slab
+constexpr int kRing = kMain + 32 * kPlane;         // plane slots
+constexpr int kSlots = 22;                         // what fits beside the block
+constexpr int kStores = 16;                        // decode: one slot per warp
+constexpr int kMaskAt = kRing + kSlots * kPlane;   // 4096 B, u32 words
+constexpr int kSegCnt = kMaskAt + kMaskBytes;      // int x 112: survivors per (octant, slab) of level 32
+constexpr int kWarpCnt = kSegCnt + 112 * 4;        // int x 16: survivors per warp of the corner
+constexpr int kBlkAt = kWarpCnt + 64;              // Blk x 4
+constexpr int kBarAt = kBlkAt + 4 * 32;            // mbarrier per slot
+constexpr int kFailAt = kBarAt + 8 * kSlots;
+constexpr int kCodecSmem = kFailAt + 16;
+constexpr int kMaskOdd = kRing + (kStores + 1) * kPlane;  // decode: the mask of every second block
+constexpr int kRecAt = kRing + (kStores + 2) * kPlane;    // decode: Rec x 2
+static_assert(kCodecSmem <= 232448, "shared memory of one CTA");
+static_assert(kBarAt % 8 == 0 && kBlkAt % 8 == 0, "alignment");
+
+// One block of the CTA's sequence; g < 0: no more.
+struct Blk {
+    long long g;
+    int field, x, y, z;  // first sample
+    float eps;
+    int pad;
+};
+static_assert(sizeof(Blk) == 32, "Blk");
+
+__device__ __forceinline__ void take_ticket(Blk *b, const CzField *fields, int nfields, long long total,
+                                            unsigned long long *queue)
 {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const Shared s = carve(smem);
-    __shared__ long long s_ticket;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t zmask = zerobits > 0 ? ~((1u << zerobits) - 1u) : 0xffffffffu;
-
-    if (threadIdx.x == 0) s_ticket = (long long)atomicAdd(queue, 1ull);
-    __syncthreads();
-    long long g = s_ticket;
-    float4 pf[16];
-    if (g < total_blocks) load_rows(locate(fields, nfields, g), pf);
-
-    while (g < total_blocks) {
-        const BlockRef ref = locate(fields, nfields, g);
-        const float eps = ref.f->eps;
-        __syncthreads();  // the previous block's emission is done with smem
-        if (threadIdx.x == 0) s_ticket = (long long)atomicAdd(queue, 1ull);
-        // ---- level 32, x lines straight from the prefetched rows
-        {
-            const int y = threadIdx.x & 31, z = threadIdx.x >> 5;
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                float v[32];
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    v[4 * k + 0] = pf[8 * r + k].x;
-                    v[4 * k + 1] = pf[8 * r + k].y;
-                    v[4 * k + 2] = pf[8 * r + k].z;
-                    v[4 * k + 3] = pf[8 * r + k].w;
-                }
-                line_fwd<32, KIND>(v);
-                st_line<32, 0>(s.sb, pidx(0, y, z + 16 * r), v);
-            }
-        }
-        __syncthreads();
-        const long long gn = s_ticket;
-        sweep<32, 1, true, KIND>(s.sb);
-        __syncthreads();
-        // ---- level 32, z lines + run masks
-        for (int l = threadIdx.x; l < 1024; l += kNT) {
-            const int x = l & 31, y = l >> 5;
-            const int base = pidx(x, y, 0);
-            float v[32];
-            ld_line<32, 2>(s.sb, base, v);
-            line_fwd<32, KIND>(v);
-            st_line<32, 2>(s.sb, base, v);
-            emit32(s, x, y, keep_bits<32>(v, eps));
-        }
-        __syncthreads();
-        // the next block's rows load while this one finishes: the warps
-        // that level 16 leaves idle (threads >= 256) now, the others once
-        // level 16 is done
-        if ((!SPLIT || threadIdx.x >= 256) && gn < total_blocks) load_rows(locate(fields, nfields, gn), pf);
-        // ---- level 16 (z, x, y) on the [0,16)^3 corner
-        sweep<16, 2, true, KIND>(s.sb);
-        __syncthreads();
-        sweep<16, 0, true, KIND>(s.sb);
-        __syncthreads();
-        if (threadIdx.x < 256) {
-            const int x = threadIdx.x & 15, z = threadIdx.x >> 4;
-            const int base = pidx(x, 0, z);
-            float v[16];
-            ld_line<16, 1>(s.sb, base, v);
-            line_fwd<16, KIND>(v);
-            st_line<16, 1>(s.sb, base, v);
-            emit16(s, x, z, keep_bits<16>(v, eps));
-        }
-        __syncthreads();
-        if (SPLIT && threadIdx.x < 256 && gn < total_blocks) load_rows(locate(fields, nfields, gn), pf);
-        // ---- level 8 (y, z, x) on the [0,8)^3 corner
-        sweep<8, 1, true, KIND>(s.sb);
-        __syncthreads();
-        sweep<8, 2, true, KIND>(s.sb);
-        __syncthreads();
-        if (threadIdx.x < 64) {
-            const int y = threadIdx.x & 7, z = threadIdx.x >> 3;
-            const int base = pidx(0, y, z);
-            float v[8];
-            ld_line<8, 0>(s.sb, base, v);
-            line_fwd<8, KIND>(v);
-            st_line<8, 0>(s.sb, base, v);
-            emit8(s, y, z, keep_bits<8>(v, eps));
-        }
-        __syncthreads();
-        emit_record(s, g, zmask, shuffle, stage, rec_bytes);
-        g = gn;
+    const long long g = (long long)atomicAdd(queue, 1ull);
+    b->g = -1;
+    if (g < total) {
+        const BlockRef r = locate(fields, nfields, g);
+        b->field = (int)(r.f - fields);
+        b->x = 32 * r.bx;
+        b->y = 32 * r.by;
+        b->z = 32 * r.bz;
+        b->eps = r.f->eps;
+        b->g = g;
     }
 }
 
-// One CTA per SM with the whole register file.
-template <int KIND, bool SPLIT>
-__global__ void __launch_bounds__(kNT, 1)
-encode_kernel(const CzField *fields, int nfields, long long total_blocks, int zerobits, int shuffle,
-              uint8_t *stage, int *rec_bytes, unsigned long long *queue)
+// Named barrier of the first n threads (whole warps).
+template <int ID, int N>
+__device__ __forceinline__ void bar_first()
 {
-    encode_body<KIND, SPLIT>(fields, nfields, total_blocks, zerobits, shuffle, stage, rec_bytes, queue);
+    asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(N) : "memory");
+}
+
+// Survivor q of a 1 KB quarter (byte address p = base + 4 q) sits at
+// quarter(p): 16 lanes that write 16 consecutive survivors each (a dense
+// region) then hit 16 different banks, and 32 lanes that read consecutive
+// survivors 32.
+__device__ __forceinline__ uint32_t quarter(uint32_t p) { return p ^ ((p >> 4) & 0x3cu); }
+
+// Corner coefficient (x, y, z), all < 16, of the block.
+__device__ __forceinline__ int corner(int x, int y, int z) { return kMain + y * kPlane + z * 64 + ((x ^ z) & 15) * 4; }
+
+__device__ __forceinline__ float &at(unsigned char *sm, uint32_t byte) { return *reinterpret_cast<float *>(sm + byte); }
+
+// x line of a plane slot (row = lane), 16-byte words behind the TMA's
+// 128-byte swizzle (word c of row r at c ^ (r & 7)).
+__device__ __forceinline__ void ld_row(const unsigned char *slot, int row, float (&v)[32])
+{
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const float4 q = *reinterpret_cast<const float4 *>(slot + row * 128 + ((c ^ (row & 7)) << 4));
+        v[4 * c] = q.x;
+        v[4 * c + 1] = q.y;
+        v[4 * c + 2] = q.z;
+        v[4 * c + 3] = q.w;
+    }
+}
+__device__ __forceinline__ void st_row(unsigned char *slot, int row, const float (&v)[32])
+{
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+        *reinterpret_cast<float4 *>(slot + row * 128 + ((c ^ (row & 7)) << 4)) =
+            make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+}
+// y line of a plane slot (column x).
+__device__ __forceinline__ uint32_t col_at(int x, int y)
+{
+    return (uint32_t)(y * 128 + (((x >> 2) ^ (y & 7)) << 4) + (x & 3) * 4);
+}
+
+// The 8 positions of the corner that thread t holds in stream order (stream
+// indices 8t .. 8t+7, FullWaveletTransform.h:63-93): the coarse 4^3 (t < 8),
+// two runs of 4 along x of level 8 (t < 64), one run of 8 along y of level
+// 16. f(e, x, y, z) for e = 0..7.
+template <class F>
+__device__ __forceinline__ void corner_run(int t, F &&f)
+{
+    if (t < 8) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f(e, e & 3, 2 * (t & 1) + (e >> 2), t >> 1);
+    } else if (t < 64) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int q = 2 * (t - 8) + (e >> 2), c = (q >> 4) + 1;
+            f(e, 4 * (c & 1) + (e & 3), 4 * ((c >> 1) & 1) + (q & 3), 4 * (c >> 2) + ((q >> 2) & 3));
+        }
+    } else {
+        const int q = t - 64, c = (q >> 6) + 1;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f(e, 8 * (c >> 2) + ((q >> 3) & 7), 8 * (c & 1) + e, 8 * ((c >> 1) & 1) + (q & 7));
+    }
+}
+
+// Inclusive sums within each half warp.
+__device__ __forceinline__ int half_scan(int c, int lane)
+{
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, c, o, 16);
+        if ((lane & 15) >= o) c += t;
+    }
+    return c;
+}
+__device__ __forceinline__ int warp_scan(int c, int lane)
+{
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, c, o);
+        if (lane >= o) c += t;
+    }
+    return c;
+}
+
+// Stream offsets once every count is in shared memory: where the warp's
+// part of the corner starts, the corner's total, and the survivors before
+// each of the 112 level-32 segments (order: octant code, then y).
+struct Offsets {
+    int mine, corner, total, seg;  // seg: exclusive sum of segment 4 lane + (warp & 3)
+    __device__ __forceinline__ int of(int code, int warp) const
+    {
+        return corner + __shfl_sync(0xffffffffu, seg, (code - 1) * 4 + (warp >> 2));
+    }
+};
+__device__ __forceinline__ Offsets stream_offsets(const unsigned char *sm, int warp, int lane)
+{
+    const int *wc = reinterpret_cast<const int *>(sm + kWarpCnt);
+    const int n = lane < kNW ? wc[lane] : 0, in = warp_scan(n, lane);
+    Offsets o;
+    o.mine = __shfl_sync(0xffffffffu, in - n, warp);
+    o.corner = __shfl_sync(0xffffffffu, in, 31);
+    int4 c = make_int4(0, 0, 0, 0);
+    if (lane < 28) c = reinterpret_cast<const int4 *>(sm + kSegCnt)[lane];
+    const int s = c.x + c.y + c.z + c.w, si = warp_scan(s, lane), k = warp & 3;
+    o.total = o.corner + __shfl_sync(0xffffffffu, si, 31);
+    o.seg = si - s + (k > 0 ? c.x : 0) + (k > 1 ? c.y : 0) + (k > 2 ? c.z : 0);
+    return o;
+}
+
+// ------------------------------------------------------------------ encode
+// Survivors j of a lane's line whose keep bit is set, in order, to the
+// quarter at shared address p. Predicated: as branches the 64 tests of a
+// line took 15 instructions each.
+template <int J0>
+__device__ __forceinline__ void pack16(uint32_t p, unsigned bits, const float (&v)[32])
+{
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+        asm volatile("{\n .reg .pred q;\n .reg .b32 t;\n setp.ne.u32 q, %1, 0;\n"
+                     " shr.u32 t, %0, 4;\n and.b32 t, t, 60;\n xor.b32 t, t, %0;\n"
+                     " @q st.shared.f32 [t], %2;\n @q add.u32 %0, %0, 4;\n}"
+                     : "+r"(p)
+                     : "r"(bits & (1u << j)), "f"(v[J0 + j])
+                     : "memory");
+}
+
+// n survivors of the quarter at p to stream positions k0 ..: zero bits, byte
+// planes S apart when shuffling.
+__device__ __forceinline__ void emit_quarter(unsigned char *sm, uint32_t p, int n, uint8_t *pay, int k0, int S,
+                                             uint32_t zmask, int shuffle, int lane)
+{
+    if (shuffle) {
+        uint8_t *d0 = pay + k0, *d1 = d0 + S, *d2 = d1 + S, *d3 = d2 + S;
+        for (int b = lane; b < n; b += 32) {
+            const uint32_t u = __float_as_uint(at(sm, quarter(p + 4 * b))) & zmask;
+            d0[b] = (uint8_t)u;
+            d1[b] = (uint8_t)(u >> 8);
+            d2[b] = (uint8_t)(u >> 16);
+            d3[b] = (uint8_t)(u >> 24);
+        }
+    } else {
+        uint32_t *d = reinterpret_cast<uint32_t *>(pay) + k0;
+        for (int b = lane; b < n; b += 32) d[b] = __float_as_uint(at(sm, quarter(p + 4 * b))) & zmask;
+    }
+}
+
+// AHEAD: the planes of the next block that do not fit the ring are brought
+// into L2 while this block is finished (the autotuner times both).
+template <int KIND, bool AHEAD>
+__global__ void __launch_bounds__(kNT, 1)
+encode_kernel(const CzField *fields, int nfields, long long total_blocks, int zerobits, int shuffle, uint8_t *stage,
+              int *rec_bytes, unsigned long long *queue, const __grid_constant__ CUtensorMap map0,
+              const CUtensorMap *maps, int *err)
+{
+    extern __shared__ __align__(1024) unsigned char sm[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t zmask = zerobits > 0 ? ~((1u << zerobits) - 1u) : 0xffffffffu;
+    uint32_t *mask32 = reinterpret_cast<uint32_t *>(sm + kMaskAt);
+    int *seg_cnt = reinterpret_cast<int *>(sm + kSegCnt), *warp_cnt = reinterpret_cast<int *>(sm + kWarpCnt);
+    Blk *blk = reinterpret_cast<Blk *>(sm + kBlkAt);
+    volatile int *fail = reinterpret_cast<volatile int *>(sm + kFailAt);
+    const uint32_t bars = smem_u32(sm + kBarAt), ring = smem_u32(sm + kRing);
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kSlots; ++s) mbar_init(bars + 8 * s, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        *fail = 0;
+        take_ticket(blk, fields, nfields, total_blocks, queue);
+        take_ticket(blk + 1, fields, nfields, total_blocks, queue);
+    }
+    __syncthreads();
+    // plane n of the CTA's sequence (plane n & 31 of its block n >> 5) into
+    // its slot, by one lane
+    auto bring = [&](uint32_t n) {
+        const Blk &b = blk[(n >> 5) & 3];
+        if (b.g < 0) return;
+        const uint32_t s = n % kSlots;
+        tma_load_3d(ring + s * kPlane, maps ? maps + b.field : &map0, b.x, b.y, b.z + (int)(n & 31), bars + 8 * s,
+                    kPlane);
+    };
+    if (lane == 0) {
+        bring(warp);
+        if (warp + 16 < kSlots) bring(warp + 16);
+    }
+
+    uint32_t it = 0;
+    for (;; ++it) {
+        const Blk &cur = blk[it & 3];
+        const long long g = cur.g;
+        if (g < 0) break;
+        const float eps = cur.eps;
+        // ---- level 32, x then y: planes z = warp and warp + 16
+#pragma unroll 1
+        for (int r = 0; r < 2; ++r) {
+            const int z = warp + 16 * r;
+            const uint32_t n = 32 * it + z, s = n % kSlots;
+            unsigned char *slot = sm + kRing + s * kPlane;
+            // after one wait ran out the others poll only briefly: the
+            // launch ends, and its error is reported
+            if (!mbar_wait(bars + 8 * s, (n / kSlots) & 1, *fail ? 64 : kWaitLimit)) *fail = 1;
+            float v[32];
+            ld_row(slot, lane, v);
+            line_fwd<32, KIND>(v);
+            st_row(slot, lane, v);
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = at(slot, col_at(lane, j));
+            __syncwarp();
+            if (lane == 0) {
+                fence_async_smem();
+                bring(n + kSlots);
+            }
+            line_fwd<32, KIND>(v);
+            if (r == 0) __syncthreads();  // the previous block has left the slabs
+#pragma unroll
+            for (int j = 0; j < 32; ++j) at(sm, kMain + j * kPlane + z * 128 + lane * 4) = v[j];
+        }
+        __syncthreads();
+        // ---- level 32, z: slabs y = warp and warp + 16
+#pragma unroll 1
+        for (int r = 0; r < 2; ++r) {
+            const int y = warp + 16 * r;
+            const uint32_t slab = kMain + y * kPlane;
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = at(sm, slab + j * 128 + lane * 4);
+            __syncwarp();
+            line_fwd<32, KIND>(v);
+            const bool in_corner = r == 0 && lane < 16;
+            unsigned kb = keep_bits<32>(v, eps);
+            if (in_corner) kb &= 0xffff0000u;
+            mask32[lane + 32 * y] = kb;  // positional word y*32+x, bits z
+            // quarters: code & 3 = (z >= 16) | (x >= 16) << 1
+            const int c = __popc(kb & 0xffffu) | __popc(kb >> 16) << 16;
+            const int in = half_scan(c, lane), ex = in - c;
+            const int xh = lane >> 4, code = (xh << 1) | (r << 2);
+            if ((lane & 15) == 15) {
+                if (code) seg_cnt[(code - 1) * 16 + warp] = in & 0xffff;
+                seg_cnt[code * 16 + warp] = in >> 16;
+            }
+            const uint32_t q = smem_u32(sm) + slab + xh * 2048;
+            pack16<0>(q + (ex & 0xffff) * 4, kb & 0xffffu, v);
+            pack16<16>(q + 1024 + (ex >> 16) * 4, kb >> 16, v);
+            if (r == 0) {  // the corner's z lines go on through level 16
+                float u[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) u[j] = v[j];
+                line_fwd<16, KIND>(u);
+                if (lane < 16) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) at(sm, corner(lane, y, j)) = u[j];
+                }
+            }
+        }
+        __syncthreads();
+        if (warp == kNW - 1 && lane == 0) take_ticket(blk + ((it + 2) & 3), fields, nfields, total_blocks, queue);
+        if (AHEAD && warp == kNW - 2 && lane >= kSlots) {
+            const Blk &b = blk[(it + 1) & 3];
+            if (b.g >= 0) tma_prefetch_3d(maps ? maps + b.field : &map0, b.x, b.y, b.z + lane);
+        }
+        if (warp < 8) {
+            // ---- level 16, x (lines (y, z)) and y (lines (x, z)), level 8, y
+            float u[16];
+            {
+                const int z = lane & 15, y = 2 * warp + (lane >> 4);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) u[j] = at(sm, corner(j, y, z));
+                line_fwd<16, KIND>(u);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) at(sm, corner(j, y, z)) = u[j];
+            }
+            bar_first<1, 256>();
+            {
+                const int z = lane & 15, x = 2 * warp + (lane >> 4);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) u[j] = at(sm, corner(x, j, z));
+                line_fwd<16, KIND>(u);
+                const unsigned kb = keep_bits<16>(u, eps);
+                // positional word x*32+z, bits y; the 8^3 corner's low byte comes later
+                if (x < 8 && z < 8) reinterpret_cast<uint8_t *>(mask32)[4 * (z + 32 * x) + 1] = (uint8_t)(kb >> 8);
+                else reinterpret_cast<uint16_t *>(mask32)[2 * (z + 32 * x)] = (uint16_t)kb;
+                if (warp < 4) {
+                    float w[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) w[j] = u[j];
+                    line_fwd<8, KIND>(w);
+                    if (z < 8) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) u[j] = w[j];
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j) at(sm, corner(x, j, z)) = u[j];
+            }
+            if (warp < 4) bar_first<2, 128>();
+            if (warp < 2) {
+                // ---- level 8, z then x
+                float w[8];
+                {
+                    const int x = lane & 7, y = 4 * warp + (lane >> 3);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) w[j] = at(sm, corner(x, y, j));
+                    line_fwd<8, KIND>(w);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) at(sm, corner(x, y, j)) = w[j];
+                }
+                bar_first<3, 64>();
+                const int y = lane & 7, z = 4 * warp + (lane >> 3);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) w[j] = at(sm, corner(j, y, z));
+                line_fwd<8, KIND>(w);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) at(sm, corner(j, y, z)) = w[j];
+                unsigned kb = keep_bits<8>(w, eps);
+                if (y < 4 && z < 4) kb |= 0xFu;  // the coarse 4^3 is always kept (FullWaveletTransform.h:165-168)
+                reinterpret_cast<uint8_t *>(mask32)[4 * (y + 32 * z)] = (uint8_t)kb;
+            }
+        }
+        __syncthreads();
+        // ---- the corner's survivors, 8 stream positions per thread
+        float u[8];
+        corner_run((int)threadIdx.x, [&](int e, int x, int y, int z) { u[e] = at(sm, corner(x, y, z)); });
+        unsigned kc = keep_bits<8>(u, eps);
+        if (threadIdx.x < 8) kc = 0xffu;
+        const int nc = __popc(kc), inc = warp_scan(nc, lane);
+        if (lane == 31) warp_cnt[warp] = inc;
+        __syncthreads();
+        const Offsets of = stream_offsets(sm, warp, lane);
+        const int S = of.total, nb = kMaskBytes + 4 * S;
+        uint8_t *rec = stage + (size_t)g * kSlotBytes, *pay = rec + 4 + kMaskBytes;
+        if (threadIdx.x == 0) {
+            *reinterpret_cast<int *>(rec) = nb;
+            rec_bytes[g] = nb;
+        }
+        for (int i = threadIdx.x; i < kMaskBytes / 4; i += kNT) reinterpret_cast<uint32_t *>(rec + 4)[i] = mask32[i];
+        {
+            // the corner has been read: its first quarters take its survivors
+            const uint32_t q = kMain + warp * kPlane;
+            uint32_t p = q + 4 * (inc - nc);
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                if (kc & (1u << e)) {
+                    at(sm, quarter(p)) = u[e];
+                    p += 4;
+                }
+            const int n = __shfl_sync(0xffffffffu, inc, 31);
+            __syncwarp();
+            emit_quarter(sm, q, n, pay, of.mine, S, zmask, shuffle, lane);
+        }
+#pragma unroll 1
+        for (int code = 1; code < 8; ++code) {
+            const int y = warp + 16 * (code >> 2), n = seg_cnt[(code - 1) * 16 + warp];
+            emit_quarter(sm, kMain + y * kPlane + (code & 3) * 1024, n, pay, of.of(code, warp), S, zmask, shuffle,
+                         lane);
+        }
+    }
+    // every plane brought in was waited for; a launch that gave up waiting
+    // lets its copies land (bounded) before it leaves
+    __syncthreads();
+    if (*fail && threadIdx.x == 0) {
+        if (err) atomicExch(err, 1);
+        for (uint32_t s = 0; s < kSlots && s < 32 * it; ++s) {
+            const uint32_t last = (32 * it - 1 - s) / kSlots;  // the slot's last use
+            mbar_wait(bars + 8 * s, last & 1);
+        }
+    }
+    __syncthreads();
 }
 
 // Error statistics of a decoded block against a reference field (the
@@ -198,132 +519,256 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
+// ------------------------------------------------------------------ decode
+// The record of a block (n is its number in the CTA's sequence).
+struct Rec {
+    const uint8_t *rec, *q12;  // record; byte planes 1 and 2 left in the LZ4 input (or null)
+    int nb, ok;                // record bytes; whether they can be a record's
+};
+
+// n survivors from stream position k0 on into the quarter at p.
+__device__ __forceinline__ void load_quarter(unsigned char *sm, uint32_t p, int n, const Payload &pl, int k0, int lane)
+{
+    for (int b = lane; b < n; b += 32) at(sm, quarter(p + 4 * b)) = pl.get(k0 + b);
+}
+// A lane's run from its quarter at shared address p: survivor or zero at
+// each place.
+template <int J0>
+__device__ __forceinline__ void unpack16(uint32_t p, unsigned bits, float (&v)[32])
+{
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+        float x = 0.f;
+        asm volatile("{\n .reg .pred q;\n .reg .b32 t;\n setp.ne.u32 q, %2, 0;\n"
+                     " shr.u32 t, %0, 4;\n and.b32 t, t, 60;\n xor.b32 t, t, %0;\n"
+                     " @q ld.shared.f32 %1, [t];\n @q add.u32 %0, %0, 4;\n}"
+                     : "+r"(p), "+f"(x)
+                     : "r"(bits & (1u << j))
+                     : "memory");
+        v[J0 + j] = x;
+    }
+}
+
 template <int KIND, bool DIFF>
 __global__ void __launch_bounds__(kNT, 1)
 decode_kernel(const CzField *fields, int nfields, long long total_blocks, int shuffle, const uint8_t *base,
               const long long *rec_off, int *status, unsigned long long *queue, const float *diff_ref,
-              double *diff_out, CzPlanes planes)
+              double *diff_out, CzPlanes planes, const CUtensorMap *maps)
 {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const Shared s = carve(smem);
-    __shared__ long long s_ticket, s_next;
-    __shared__ int s_bad;
-    // the next block's record, found by the last warp (s_pf_n < 0: none)
-    __shared__ const uint8_t *s_pf_slot, *s_pf_q12;
-    __shared__ int s_pf_n;
-    constexpr int kPfWarp = kNT / 32 - 1;
-    const int warp = threadIdx.x >> 5;
-    // byte planes 1 and 2 of block b's record in the LZ4 input (or null)
-    auto planes12 = [&](long long b, int nb) -> const uint8_t * {
-        if (!planes.hole || !shuffle) return nullptr;
-        const int c4 = (nb - kMaskBytes) / 4;
-        const int4 h = planes.hole[b];
-        return h.z > 0 && h.z == 2 * c4 && h.x == 4 + kMaskBytes + c4 ? planes.src + planes.src_off[b] + h.y
-                                                                       : nullptr;
-    };
-
-    // tickets are taken one block ahead, so that the next block's record
-    // can be brought into L2 while this one is transformed
-    if (threadIdx.x == 0) s_next = (long long)atomicAdd(queue, 1ull);
-    for (;;) {
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            s_ticket = s_next;
-            s_next = s_next < total_blocks ? (long long)atomicAdd(queue, 1ull) : total_blocks;
-            s_bad = 0;
-        }
-        __syncthreads();
-        const long long g = s_ticket;
-        if (g >= total_blocks) break;
-        const long long gn = s_next;
-        const long long ron = warp == kPfWarp && gn < total_blocks ? rec_off[gn] : -1;  // used after the load
-        const BlockRef ref = locate(fields, nfields, g);
-        const long long ro = rec_off[g];
-        const uint8_t *slot = base + (ro < 0 ? 0 : ro);
-        const int nb = ro < 0 ? -1 : *reinterpret_cast<const int *>(slot);
+    extern __shared__ __align__(1024) unsigned char sm[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int *seg_cnt = reinterpret_cast<int *>(sm + kSegCnt), *warp_cnt = reinterpret_cast<int *>(sm + kWarpCnt);
+    Blk *blk = reinterpret_cast<Blk *>(sm + kBlkAt);
+    Rec *recs = reinterpret_cast<Rec *>(sm + kRecAt);
+    volatile int *bad = reinterpret_cast<volatile int *>(sm + kFailAt);  // per parity of the block's number
+    unsigned char *slot = sm + kRing + warp * kPlane;  // this warp's plane
+    // Record of block n of the CTA's sequence, by threads t of nt: where it
+    // is, its mask (deserialize_bitset, WaveletCompressor.cpp:124-150) into
+    // shared memory, its payload into L2.
+    auto fetch = [&](uint32_t n, int t, int nt) {
+        const long long g = blk[n & 3].g, ro = g >= 0 ? rec_off[g] : -1;
+        const uint8_t *rec = base + (ro < 0 ? 0 : ro);
+        const int nb = ro < 0 ? -1 : *reinterpret_cast<const int *>(rec);
         const bool size_ok = nb >= kMaskBytes && nb <= kMaxRecord + 4;
-        // the payload into L2 while the mask is read and scanned (a no-op
-        // when the previous block's pass already brought it)
-        const uint8_t *q12 = size_ok ? planes12(g, nb) : nullptr;
-        if (size_ok) prefetch_record(slot, nb, q12, threadIdx.x, kNT);
-        // deserialize_bitset (WaveletCompressor.cpp:124-150)
-        for (int i = threadIdx.x; i < kMaskBytes / 4; i += kNT)
-            s.mask32[i] = size_ok ? reinterpret_cast<const uint32_t *>(slot + 4)[i] : 0u;
-        __syncthreads();
-        runs_from_mask(s);
-        // the base case consumes exactly the 64 coarse survivors (:178-189)
-        if (threadIdx.x < 16) {
-            const int y = threadIdx.x & 3, z = threadIdx.x >> 2;
-            if ((s.mask32[y + 32 * z] & 0xFu) != 0xFu) s_bad = 1;
+        uint32_t *m = reinterpret_cast<uint32_t *>(sm + (n & 1 ? kMaskOdd : kMaskAt));
+        for (int i = t; i < kMaskBytes / 4; i += nt)
+            m[i] = size_ok ? reinterpret_cast<const uint32_t *>(rec + 4)[i] : 0u;
+        // byte planes 1 and 2 where the LZ4 stage left them in its input
+        const uint8_t *q12 = nullptr;
+        if (size_ok && planes.hole && shuffle) {
+            const int c4 = (nb - kMaskBytes) / 4;
+            const int4 h = planes.hole[g];
+            if (h.z > 0 && h.z == 2 * c4 && h.x == 4 + kMaskBytes + c4) q12 = planes.src + planes.src_off[g] + h.y;
         }
+        if (size_ok) prefetch_record(rec, nb, q12, t, nt);
+        if (t == 0) recs[n & 1] = Rec{rec, q12, nb, size_ok};
+    };
+    if (threadIdx.x == 0) {
+        take_ticket(blk, fields, nfields, total_blocks, queue);
+        take_ticket(blk + 1, fields, nfields, total_blocks, queue);
+        bad[0] = bad[1] = 0;
+    }
+    __syncthreads();
+    if (blk[0].g >= 0) fetch(0, threadIdx.x, kNT);
+    __syncthreads();
+    for (uint32_t it = 0;; ++it) {
+        const Blk &cur = blk[it & 3];
+        const long long g = cur.g;
+        if (g < 0) break;
+        const uint32_t *mask32 = reinterpret_cast<const uint32_t *>(sm + (it & 1 ? kMaskOdd : kMaskAt));
+        const uint8_t *rec = recs[it & 1].rec, *q12 = recs[it & 1].q12;
+        const int nb = recs[it & 1].nb;
+        const bool size_ok = recs[it & 1].ok != 0;
+        // ---- survivor counts: level 32 per (octant, slab), the corner per warp
+        unsigned kz[2];
+        int ex[2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            kz[r] = mask32[lane + 32 * (warp + 16 * r)];
+            if (r == 0 && lane < 16) kz[r] &= 0xffff0000u;
+            const int c = __popc(kz[r] & 0xffffu) | __popc(kz[r] >> 16) << 16;
+            const int in = half_scan(c, lane);
+            ex[r] = in - c;
+            const int code = ((lane >> 4) << 1) | (r << 2);
+            if ((lane & 15) == 15) {
+                if (code) seg_cnt[(code - 1) * 16 + warp] = in & 0xffff;
+                seg_cnt[code * 16 + warp] = in >> 16;
+            }
+        }
+        unsigned kc = 0;
+        corner_run((int)threadIdx.x, [&](int e, int x, int y, int z) {
+            const int b = threadIdx.x < 64 ? 32 * (y + 32 * z) + x : 32 * (z + 32 * x) + y;
+            kc |= ((mask32[b >> 5] >> (b & 31)) & 1u) << e;
+        });
+        // the base case consumes exactly the 64 coarse survivors (:178-189)
+        if (threadIdx.x < 8 && kc != 0xffu) bad[it & 1] = 1;
+        const int nc = __popc(kc), inc = warp_scan(nc, lane);
+        if (lane == 31) warp_cnt[warp] = inc;
         __syncthreads();
-        const int expected = scan_segments(s);
-        const int payload = nb - kMaskBytes;
+        const Offsets of = stream_offsets(sm, warp, lane);
+        const int expected = of.total, payload = nb - kMaskBytes;
         int nel = payload / 4;
         if (nel - expected == 1) nel--;  // :247-250
-        const bool ok = size_ok && nel == expected && !s_bad;
-        if (threadIdx.x == 0) status[g] = ok ? 0 : -1;
-        // ---- load (FullWaveletTransform.h:99-150): every survivor at its
-        // place, read in stream order (consecutive across each warp), and
-        // zeros at every other place (the runs cover the block); a bad
-        // record leaves the block all zeros
+        const bool ok = size_ok && nel == expected && !bad[it & 1];
+        if (threadIdx.x == 0) {
+            status[g] = ok ? 0 : -1;
+            bad[(it + 1) & 1] = 0;
+        }
+        // ---- load (FullWaveletTransform.h:99-150): the survivors of every
+        // quarter in stream order; a bad record decodes as an empty one
         if (ok) {
             Payload pl;
-            pl.p = slot + 4 + kMaskBytes;
+            pl.p = rec + 4 + kMaskBytes;
             pl.c = payload / 4;
             pl.q = q12 ? q12 : pl.p + pl.c;  // planes 1 and 2
             pl.shuffle = shuffle != 0;
-            load_survivors(s, expected, [&](int k) { return pl.get(k); });
+            if (lane == 0) tma_store_wait_read();  // the slot holds the warp's corner survivors next
+            __syncwarp();
+            load_quarter(sm, kRing + warp * kPlane, __shfl_sync(0xffffffffu, inc, 31), pl, of.mine, lane);
+#pragma unroll 1
+            for (int code = 1; code < 8; ++code)
+                load_quarter(sm, kMain + (warp + 16 * (code >> 2)) * kPlane + (code & 3) * 1024,
+                             seg_cnt[(code - 1) * 16 + warp], pl, of.of(code, warp), lane);
         } else {
-            for (int i = threadIdx.x; i < kBS3; i += kNT) s.sb[pidx(i & 31, (i >> 5) & 31, i >> 10)] = 0.f;
+            kc = kz[0] = kz[1] = 0;
+        }
+        __syncwarp();
+        {
+            uint32_t p = kRing + warp * kPlane + 4 * (inc - nc);
+            corner_run((int)threadIdx.x, [&](int e, int x, int y, int z) {
+                float c = 0.f;
+                if (kc & (1u << e)) {
+                    c = at(sm, quarter(p));
+                    p += 4;
+                }
+                at(sm, corner(x, y, z)) = c;
+            });
         }
         __syncthreads();
-        // the last warp finds the next record while level 8 runs on the
-        // first two warps
-        if (warp == kPfWarp) {
-            const int nbn = ron >= 0 ? *reinterpret_cast<const int *>(base + ron) : -1;
-            const bool okn = nbn >= kMaskBytes && nbn <= kMaxRecord + 4;
-            const uint8_t *qn = okn ? planes12(gn, nbn) : nullptr;
-            if ((threadIdx.x & 31) == 0) {
-                s_pf_slot = base + (ron < 0 ? 0 : ron);
-                s_pf_q12 = qn;
-                s_pf_n = okn ? nbn : -1;
-            }
-        }
-        // ---- iwt: level 8 (x, z, y), level 16 (y, x, z), level 32 (z, y, x)
-        sweep<8, 0, false, KIND>(s.sb);
-        __syncthreads();
-        sweep<8, 2, false, KIND>(s.sb);
-        __syncthreads();
-        sweep<8, 1, false, KIND>(s.sb);
-        __syncthreads();
-        // threads 256-511, idle during level 16, bring the next record into L2
-        if (threadIdx.x >= 256 && s_pf_n > 0) prefetch_record(s_pf_slot, s_pf_n, s_pf_q12, threadIdx.x - 256, kNT - 256);
-        sweep<16, 1, false, KIND>(s.sb);
-        __syncthreads();
-        sweep<16, 0, false, KIND>(s.sb);
-        __syncthreads();
-        sweep<16, 2, false, KIND>(s.sb);
-        __syncthreads();
-        sweep<32, 2, false, KIND>(s.sb);
-        __syncthreads();
-        sweep<32, 1, false, KIND>(s.sb);
-        __syncthreads();
-        // x lines: inverse, then straight to the field (copy_to, WaveletCompressor.h:73-82)
-        float *out = const_cast<float *>(ref.f->data);
-        DiffAcc acc;
-        for (int l = threadIdx.x; l < 1024; l += kNT) {
-            const int y = l & 31, z = l >> 5;
-            float v[32];
-            ld_line<32, 0>(s.sb, pidx(0, y, z), v);
-            line_inv<32, KIND>(v);
-            const size_t ro = row_offset(ref, y, z);
-            float4 *dst = reinterpret_cast<float4 *>(out + ro);
+        if (warp < 8) {
+            // ---- level 8: x, z, then y with level 16's y and x
+            float u[16];
+            if (warp < 2) {
+                float w[8];
+                {
+                    const int y = lane & 7, z = 4 * warp + (lane >> 3);
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-                __stcs(dst + k, make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]));
+                    for (int j = 0; j < 8; ++j) w[j] = at(sm, corner(j, y, z));
+                    line_inv<8, KIND>(w);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) at(sm, corner(j, y, z)) = w[j];
+                }
+                bar_first<3, 64>();
+                const int x = lane & 7, y = 4 * warp + (lane >> 3);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) w[j] = at(sm, corner(x, y, j));
+                line_inv<8, KIND>(w);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) at(sm, corner(x, y, j)) = w[j];
+            }
+            if (warp < 4) bar_first<2, 128>();
+            {
+                const int z = lane & 15, x = 2 * warp + (lane >> 4);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) u[j] = at(sm, corner(x, j, z));
+                if (warp < 4) {
+                    float w[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) w[j] = u[j];
+                    line_inv<8, KIND>(w);
+                    if (z < 8) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) u[j] = w[j];
+                    }
+                }
+                line_inv<16, KIND>(u);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) at(sm, corner(x, j, z)) = u[j];
+            }
+            bar_first<1, 256>();
+            const int z = lane & 15, y = 2 * warp + (lane >> 4);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) u[j] = at(sm, corner(j, y, z));
+            line_inv<16, KIND>(u);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) at(sm, corner(j, y, z)) = u[j];
+        } else if (warp == kNW - 1) {  // idle meanwhile: the ticket after next
+            if (lane == 0) take_ticket(blk + ((it + 2) & 3), fields, nfields, total_blocks, queue);
+        } else if (blk[(it + 1) & 3].g >= 0) {  // ... and the next record
+            fetch(it + 1, threadIdx.x - 256, kNT - 256 - 32);
+        }
+        __syncthreads();
+        // ---- level 16, z, and level 32, z: slabs y = warp and warp + 16
+#pragma unroll 1
+        for (int r = 0; r < 2; ++r) {
+            const int y = warp + 16 * r;
+            const uint32_t slab = kMain + y * kPlane, q = smem_u32(sm) + slab + (lane >> 4) * 2048;
+            const unsigned kb = r ? kz[1] : kz[0];
+            const int e = r ? ex[1] : ex[0];
+            float v[32];
+            unpack16<0>(q + (e & 0xffff) * 4, kb & 0xffffu, v);
+            unpack16<16>(q + 1024 + (e >> 16) * 4, kb >> 16, v);
+            if (r == 0) {
+                float u[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) u[j] = at(sm, corner(lane & 15, y, j));
+                line_inv<16, KIND>(u);
+                if (lane < 16) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] = u[j];
+                }
+            }
+            __syncwarp();
+            line_inv<32, KIND>(v);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) at(sm, slab + j * 128 + lane * 4) = v[j];
+        }
+        __syncthreads();
+        // ---- level 32, y then x: planes z = warp and warp + 16, then straight
+        // to the field (copy_to, WaveletCompressor.h:73-82)
+        DiffAcc acc;
+#pragma unroll 1
+        for (int r = 0; r < 2; ++r) {
+            const int z = warp + 16 * r;
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = at(sm, kMain + j * kPlane + z * 128 + lane * 4);
+            line_inv<32, KIND>(v);
+            if (lane == 0) tma_store_wait_read();
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) at(slot, col_at(lane, j)) = v[j];
+            __syncwarp();
+            ld_row(slot, lane, v);
+            line_inv<32, KIND>(v);
+            st_row(slot, lane, v);
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) tma_store_3d(maps + cur.field, cur.x, cur.y, cur.z + z, smem_u32(slot));
             if (DIFF) {
-                const float4 *rr = reinterpret_cast<const float4 *>(diff_ref + ro);
+                const CzField &f = fields[cur.field];
+                const float4 *rr = reinterpret_cast<const float4 *>(
+                    diff_ref + ((size_t)(cur.z + z) * f.ny + (size_t)(cur.y + lane)) * f.nx + (size_t)cur.x);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
                     const float4 q = __ldcs(rr + k);
@@ -336,8 +781,7 @@ decode_kernel(const CzField *fields, int nfields, long long total_blocks, int sh
         }
         if (DIFF) {
             // block totals in binary64: maxima exact, sums of the compensated partials
-            __shared__ double red[kNW][8];
-            const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+            double(*red)[8] = reinterpret_cast<double(*)[8]>(sm + kRing + kStores * kPlane);
             double t[8];
             t[0] = warp_max(fabs((double)acc.es + acc.ee));
             t[1] = warp_max(acc.ninf);
@@ -360,6 +804,7 @@ decode_kernel(const CzField *fields, int nfields, long long total_blocks, int sh
             }
         }
     }
+    if (lane == 0) tma_store_wait_all();
 }
 
 // Totals over blocks, in block order: {e_inf, n_inf, e_1, e_2, n_1, n_2, min, max}.
@@ -405,64 +850,81 @@ diff_total_kernel(const double *per_block, long long nblocks, double *total)
 
 using namespace cz;
 
-extern "C" int cz_codec_smem_bytes(void) { return kSmBytes; }
+bool cz_field_map(const CzField &f, CUtensorMap *map)
+{
+    CzEncodeTiled enc = cz_encode_tiled();
+    if (!enc) return false;
+    // one z plane of a block per box
+    const cuuint64_t dim[3] = {(cuuint64_t)f.nx, (cuuint64_t)f.ny, (cuuint64_t)f.nz};
+    const cuuint64_t stride[2] = {(cuuint64_t)f.nx * 4, (cuuint64_t)f.nx * f.ny * 4};
+    const cuuint32_t box[3] = {32, 32, 1}, es[3] = {1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(f.data), dim, stride, box, es,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 template <int KIND>
 static cudaError_t launch_encode(const CzField *fields, int nfields, long long total_blocks, int zerobits,
                                  int shuffle, uint8_t *stage, int *rec_bytes, unsigned long long *queue, int grid,
-                                 cudaStream_t st, int variant)
+                                 cudaStream_t st, const CUtensorMap *maps, const CUtensorMap &map0, int *err,
+                                 int variant)
 {
     auto k = variant == 1 ? encode_kernel<KIND, false> : encode_kernel<KIND, true>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmBytes);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCodecSmem);
     if (e != cudaSuccess) return e;
-    k<<<grid, kNT, kSmBytes, st>>>(fields, nfields, total_blocks, zerobits, shuffle, stage, rec_bytes, queue);
+    k<<<grid, kNT, kCodecSmem, st>>>(fields, nfields, total_blocks, zerobits, shuffle, stage, rec_bytes, queue, map0,
+                                     maps, err);
     return cudaGetLastError();
 }
 
 template <int KIND>
 static cudaError_t launch_decode(const CzField *fields, int nfields, long long total_blocks, int shuffle,
                                  const uint8_t *base, const long long *rec_off, int *status,
-                                 unsigned long long *queue, int grid, cudaStream_t st, const float *diff_ref,
-                                 double *diff_out, CzPlanes planes)
+                                 unsigned long long *queue, int grid, cudaStream_t st, const CUtensorMap *maps,
+                                 const float *diff_ref, double *diff_out, CzPlanes planes)
 {
     auto k = diff_ref ? decode_kernel<KIND, true> : decode_kernel<KIND, false>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmBytes);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCodecSmem);
     if (e != cudaSuccess) return e;
-    k<<<grid, kNT, kSmBytes, st>>>(fields, nfields, total_blocks, shuffle, base, rec_off, status, queue, diff_ref,
-                                   diff_out, planes);
+    k<<<grid, kNT, kCodecSmem, st>>>(fields, nfields, total_blocks, shuffle, base, rec_off, status, queue, diff_ref,
+                                     diff_out, planes, maps);
     return cudaGetLastError();
 }
 
 cudaError_t cz_launch_encode(int wtype, const CzField *fields, int nfields, long long total_blocks, int zerobits,
                              int shuffle, uint8_t *stage, int *rec_bytes, unsigned long long *queue, int grid,
-                             cudaStream_t st, int variant)
+                             cudaStream_t st, const CUtensorMap *maps, const CUtensorMap *map0, int *err, int variant)
 {
+    if (!maps && !map0) return cudaErrorInvalidValue;
+    CUtensorMap own = {};
+    if (map0) own = *map0;
     switch (wkind(wtype)) {
     case 1:
         return launch_encode<1>(fields, nfields, total_blocks, zerobits, shuffle, stage, rec_bytes, queue, grid, st,
-                                variant);
+                                maps, own, err, variant);
     case 2:
         return launch_encode<2>(fields, nfields, total_blocks, zerobits, shuffle, stage, rec_bytes, queue, grid, st,
-                                variant);
+                                maps, own, err, variant);
     default:
         return launch_encode<3>(fields, nfields, total_blocks, zerobits, shuffle, stage, rec_bytes, queue, grid, st,
-                                variant);
+                                maps, own, err, variant);
     }
 }
 
 cudaError_t cz_launch_decode(int wtype, const CzField *fields, int nfields, long long total_blocks, int shuffle,
                              const uint8_t *base, const long long *rec_off, int *status, unsigned long long *queue,
-                             int grid, cudaStream_t st, const float *diff_ref, double *diff_out, CzPlanes planes)
+                             int grid, cudaStream_t st, const CUtensorMap *maps, const float *diff_ref,
+                             double *diff_out, CzPlanes planes)
 {
     switch (wkind(wtype)) {
     case 1:
-        return launch_decode<1>(fields, nfields, total_blocks, shuffle, base, rec_off, status, queue, grid, st,
+        return launch_decode<1>(fields, nfields, total_blocks, shuffle, base, rec_off, status, queue, grid, st, maps,
                                 diff_ref, diff_out, planes);
     case 2:
-        return launch_decode<2>(fields, nfields, total_blocks, shuffle, base, rec_off, status, queue, grid, st,
+        return launch_decode<2>(fields, nfields, total_blocks, shuffle, base, rec_off, status, queue, grid, st, maps,
                                 diff_ref, diff_out, planes);
     default:
-        return launch_decode<3>(fields, nfields, total_blocks, shuffle, base, rec_off, status, queue, grid, st,
+        return launch_decode<3>(fields, nfields, total_blocks, shuffle, base, rec_off, status, queue, grid, st, maps,
                                 diff_ref, diff_out, planes);
     }
 }

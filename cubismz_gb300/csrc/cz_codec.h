@@ -1,5 +1,6 @@
 // cz_codec.h -- internal interface between the C-ABI layer and the kernels.
 #pragma once
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -14,17 +15,25 @@ struct CzField {
     long long block0;
 };
 
-extern "C" int cz_codec_smem_bytes(void);
+// Tensor map of a field's z planes (32 x 32 boxes, 128-byte swizzle) for the
+// codec kernels' tile copies; false if the driver cannot make it. The field
+// must be 16-byte aligned.
+bool cz_field_map(const CzField &f, CUtensorMap *map);
 
-// variant 0: the next block's rows load in two halves, by the warps each
-// level leaves idle; 1: all at once after level 32 (same records)
+// maps: the fields' tensor maps in device memory (64-byte aligned), or
+// nullptr with map0 (host) for a single field. err (optional, device): set
+// to 1 if a tile copy did not complete in time.
+// variant 0: the part of the next block that shared memory does not hold yet
+// is brought into L2 ahead; 1: it is not (same records)
 cudaError_t cz_launch_encode(int wtype, const CzField *fields, int nfields, long long total_blocks, int zerobits,
                              int shuffle, uint8_t *stage, int *rec_bytes, unsigned long long *queue, int grid,
-                             cudaStream_t st, int variant = 0);
+                             cudaStream_t st, const CUtensorMap *maps, const CUtensorMap *map0, int *err,
+                             int variant = 0);
 // Record of block g at base + rec_off[g] ([int32 nbytes][record]); a
 // negative rec_off marks a block whose record is missing (status -1).
 // diff_ref (optional, a field of the same geometry as fields[0]): per-block
-// error statistics into diff_out[8*g] (cz2diff's quantities).
+// error statistics into diff_out[8*g] (cz2diff's quantities). maps as for
+// cz_launch_encode (device memory).
 // Byte planes 1 and 2 of one-record chunks left in the LZ4 input by
 // cz_launch_lz4_decode (hole per chunk = per block, chunk c at src +
 // src_off[c]); hole == nullptr: every record is whole.
@@ -35,8 +44,8 @@ struct CzPlanes {
 };
 cudaError_t cz_launch_decode(int wtype, const CzField *fields, int nfields, long long total_blocks, int shuffle,
                              const uint8_t *base, const long long *rec_off, int *status, unsigned long long *queue,
-                             int grid, cudaStream_t st, const float *diff_ref = nullptr, double *diff_out = nullptr,
-                             CzPlanes planes = CzPlanes());
+                             int grid, cudaStream_t st, const CUtensorMap *maps, const float *diff_ref = nullptr,
+                             double *diff_out = nullptr, CzPlanes planes = CzPlanes());
 cudaError_t cz_launch_diff_total(const double *per_block, long long nblocks, double *total, cudaStream_t st);
 
 // Linear inverse transform and its adjoint on stacked 32^3 blocks; block

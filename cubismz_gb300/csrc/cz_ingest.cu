@@ -20,11 +20,10 @@
 // destination. Each wait on an mbarrier is bounded; past the bound the
 // CTA records an error, drains its copies in flight (bounded too) and
 // returns, and the call reports the error.
-#include <cuda.h>
-
 #include <algorithm>
 
 #include "cz_codec.h"
+#include "cz_tma.cuh"
 
 namespace cz {
 
@@ -76,34 +75,6 @@ constexpr int kStages = 4;
 constexpr int kPlanes = 4;                                   // y planes per tile
 constexpr int kTileBytes = kPlanes * 32 * 128;               // 16 KB
 constexpr int kTmaSmem = kStages * kTileBytes + 1024;        // + alignment slack
-constexpr long long kWaitLimit = 1ll << 22;  // try_wait polls before giving up
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p)
-{
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
-{
-    for (long long i = 0; i < kWaitLimit; ++i) {
-        uint32_t ok;
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                     : "=r"(ok)
-                     : "r"(bar), "r"(parity)
-                     : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, uint32_t bar,
-                                            uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-            dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
-        : "memory");
-}
 
 // Tile t of the source: planes y0..y0+3, 32 rows each (along the
 // destination's fastest axis, r) of BC elements (along the source's fastest
@@ -192,33 +163,13 @@ using namespace cz;
 
 namespace {
 
-using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-// Looked up once; the initialisation of a function-local static is
-// thread-safe, so contexts on several host threads may reach it together.
-EncodeTiled encode_tiled()
-{
-    static const EncodeTiled fn = []() -> EncodeTiled {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        const bool ok = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault,
-                                                         &q) == cudaSuccess &&
-                        q == cudaDriverEntryPointSuccess;
-        cudaGetLastError();
-        return ok ? reinterpret_cast<EncodeTiled>(p) : nullptr;
-    }();
-    return fn;
-}
-
 // The TMA transpose of a 3-D array (d0 fastest, then d1, d2) whose tiles are
 // 128 bytes along d0 and 32 rows along d2; false if the map cannot be made
 // (the caller then takes the plain kernel).
 bool launch_tma(const void *in, int bytes, long long d0, long long d1, long long d2, float *out, long long sc,
                 long long sy, int *err, cudaStream_t st)
 {
-    EncodeTiled enc = encode_tiled();
+    CzEncodeTiled enc = cz_encode_tiled();
     if (!enc) return false;
     const int bc = 128 / bytes;
     if (d0 % bc || d2 % 32 || reinterpret_cast<uintptr_t>(in) % 16) return false;

@@ -11,31 +11,51 @@
 namespace cz {
 
 // ---------------------------------------------------------------- wtype 1/2
+// Predictions of a line's odd samples from its H scalings e
+// (WaveletsOnInterval.h:33-51), stencil by stencil.
+CZ_RARE void interp_rare(const float *e, float *o, int H)
+{
+    o[0] = st4_main<W1F>(e[0], e[1], e[2], e[3]);
+#pragma unroll 1
+    for (int i = 1; i < H - 2; ++i) o[i] = st4_main<W1M>(e[i - 1], e[i], e[i + 1], e[i + 2]);
+    o[H - 2] = st4_main<W1O>(e[H - 4], e[H - 3], e[H - 2], e[H - 1]);
+    o[H - 1] = st4_lastany(e[H - 4], e[H - 3], e[H - 2], e[H - 1]);
+}
+template <int H>
+CZ_HD void interp_predict(const float (&e)[H], float (&o)[H])
+{
+    uint32_t amax;
+    bool narrow;
+    if (line_grid<H>(e, amax, narrow)) {
+        const float C = split_const<kGridBits>(amax);
+        Pair p[H];
+#pragma unroll
+        for (int i = 0; i < H; ++i) p[i] = split_pair(e[i], C);
+        o[0] = st4_pair<W1F>(p[0], p[1], p[2], p[3]);
+#pragma unroll
+        for (int i = 1; i < H - 2; ++i) o[i] = st4_pair<W1M>(p[i - 1], p[i], p[i + 1], p[i + 2]);
+        o[H - 2] = st4_pair<W1O>(p[H - 4], p[H - 3], p[H - 2], p[H - 1]);
+        o[H - 1] = interp_last(e[H - 4], e[H - 3], e[H - 2], e[H - 1], amax, narrow);
+    } else {
+        float te[H], to[H];  // the call's arrays live in memory, e and o in registers
+#pragma unroll
+        for (int i = 0; i < H; ++i) te[i] = e[i];
+        interp_rare(te, to, H);
+#pragma unroll
+        for (int i = 0; i < H; ++i) o[i] = to[i];
+    }
+}
+
 template <int N>
 CZ_HD void fwd_interp(float (&x)[N], bool lifting)
 {
     constexpr int H = N / 2;
-    float e[H], h[H], l[H], d[H];
-    uint32_t amax;
+    float e[H], d[H];
 #pragma unroll
     for (int i = 0; i < H; ++i) e[i] = x[2 * i];
-    if (line_split<H>(e, h, l, amax)) {
-        d[0] = CZ_SUB(x[1], st4_fast<W1F>(h[0], h[1], h[2], h[3], l[0], l[1], l[2], l[3]));
+    interp_predict<H>(e, d);
 #pragma unroll
-        for (int i = 1; i < H - 2; ++i)
-            d[i] = CZ_SUB(x[2 * i + 1], st4_fast<W1M>(h[i - 1], h[i], h[i + 1], h[i + 2], l[i - 1], l[i], l[i + 1],
-                                                      l[i + 2]));
-        d[H - 2] = CZ_SUB(x[N - 3], st4_fast<W1O>(h[H - 4], h[H - 3], h[H - 2], h[H - 1], l[H - 4], l[H - 3],
-                                                  l[H - 2], l[H - 1]));
-        d[H - 1] = CZ_SUB(x[N - 1], interp_last(e[H - 4], e[H - 3], e[H - 2], e[H - 1], amax));
-    } else {
-        d[0] = CZ_SUB(x[1], st4_main<W1F>(e[0], e[1], e[2], e[3]));
-#pragma unroll
-        for (int i = 1; i < H - 2; ++i)
-            d[i] = CZ_SUB(x[2 * i + 1], st4_main<W1M>(e[i - 1], e[i], e[i + 1], e[i + 2]));
-        d[H - 2] = CZ_SUB(x[N - 3], st4_main<W1O>(e[H - 4], e[H - 3], e[H - 2], e[H - 1]));
-        d[H - 1] = CZ_SUB(x[N - 1], st4_lastany(e[H - 4], e[H - 3], e[H - 2], e[H - 1]));
-    }
+    for (int i = 0; i < H; ++i) d[i] = CZ_SUB(x[2 * i + 1], d[i]);
     // scalings[i] += 0.5*details[i] in binary64, rounded to binary32 (:124-126):
     // a single fma is the correctly rounded value of the same exact sum.
 #pragma unroll
@@ -48,27 +68,13 @@ template <int N>
 CZ_HD void inv_interp(float (&x)[N], bool lifting)
 {
     constexpr int H = N / 2;
-    float s[H], d[H], h[H], l[H], o[H];
-    uint32_t amax;
+    float s[H], d[H], o[H];
 #pragma unroll
     for (int i = 0; i < H; ++i) {
         d[i] = x[H + i];
         s[i] = lifting ? CZ_FMA(-0.5f, d[i], x[i]) : x[i];  // :137-139
     }
-    if (line_split<H>(s, h, l, amax)) {
-        o[0] = st4_fast<W1F>(h[0], h[1], h[2], h[3], l[0], l[1], l[2], l[3]);
-#pragma unroll
-        for (int i = 1; i < H - 2; ++i)
-            o[i] = st4_fast<W1M>(h[i - 1], h[i], h[i + 1], h[i + 2], l[i - 1], l[i], l[i + 1], l[i + 2]);
-        o[H - 2] = st4_fast<W1O>(h[H - 4], h[H - 3], h[H - 2], h[H - 1], l[H - 4], l[H - 3], l[H - 2], l[H - 1]);
-        o[H - 1] = interp_last(s[H - 4], s[H - 3], s[H - 2], s[H - 1], amax);
-    } else {
-        o[0] = st4_main<W1F>(s[0], s[1], s[2], s[3]);
-#pragma unroll
-        for (int i = 1; i < H - 2; ++i) o[i] = st4_main<W1M>(s[i - 1], s[i], s[i + 1], s[i + 2]);
-        o[H - 2] = st4_main<W1O>(s[H - 4], s[H - 3], s[H - 2], s[H - 1]);
-        o[H - 1] = st4_lastany(s[H - 4], s[H - 3], s[H - 2], s[H - 1]);
-    }
+    interp_predict<H>(s, o);
     // :141-151: even samples are the scalings, odd samples interp + detail
 #pragma unroll
     for (int i = 0; i < H; ++i) {
@@ -78,37 +84,61 @@ CZ_HD void inv_interp(float (&x)[N], bool lifting)
 }
 
 // ---------------------------------------------------------------- wtype 3
+// Predictions of a line's even and odd samples from its H scalings s
+// (WaveletsOnInterval.h:55-83).
+CZ_RARE void avg_rare(const float *s, float *p0, float *p1, int H)
+{
+    p0[0] = st3_any<P0F>(s[0], s[1], s[2]);
+    p1[0] = st3_any<P1F>(s[0], s[1], s[2]);
+#pragma unroll 1
+    for (int i = 1; i < H - 1; ++i) {
+        p0[i] = st3_any<P0M>(s[i - 1], s[i], s[i + 1]);
+        p1[i] = st3_any<P1M>(s[i - 1], s[i], s[i + 1]);
+    }
+    p0[H - 1] = st3_any<P0L>(s[H - 3], s[H - 2], s[H - 1]);
+    p1[H - 1] = st3_any<P1L>(s[H - 3], s[H - 2], s[H - 1]);
+}
+template <int H>
+CZ_HD void avg_predict(const float (&s)[H], float (&p0)[H], float (&p1)[H])
+{
+    uint32_t amax;
+    bool narrow;
+    if (line_grid<H>(s, amax, narrow)) {
+        const float C = split_const<kGridBits>(amax);
+        Pair p[H];
+#pragma unroll
+        for (int i = 0; i < H; ++i) p[i] = split_pair(s[i], C);
+        p0[0] = st3_pair<P0F>(p[0], p[1], p[2]);
+        p1[0] = st3_pair<P1F>(p[0], p[1], p[2]);
+#pragma unroll
+        for (int i = 1; i < H - 1; ++i) {
+            p0[i] = st3_pair<P0M>(p[i - 1], p[i], p[i + 1]);
+            p1[i] = st3_pair<P1M>(p[i - 1], p[i], p[i + 1]);
+        }
+        p0[H - 1] = st3_pair<P0L>(p[H - 3], p[H - 2], p[H - 1]);
+        p1[H - 1] = st3_pair<P1L>(p[H - 3], p[H - 2], p[H - 1]);
+    } else {
+        float t[H], t0[H], t1[H];
+#pragma unroll
+        for (int i = 0; i < H; ++i) t[i] = s[i];
+        avg_rare(t, t0, t1, H);
+#pragma unroll
+        for (int i = 0; i < H; ++i) {
+            p0[i] = t0[i];
+            p1[i] = t1[i];
+        }
+    }
+}
+
 template <int N>
 CZ_HD void fwd_avg(float (&x)[N])
 {
     constexpr int H = N / 2;
-    float s[H], h[H], l[H], d[H];
-    uint32_t amax;
+    float s[H], d[H], p0[H], p1[H];
     // scalings = 0.5*(x0+x1): binary32 add, exact halving (:159-160)
 #pragma unroll
     for (int i = 0; i < H; ++i) s[i] = CZ_MUL(0.5f, CZ_ADD(x[2 * i], x[2 * i + 1]));
-    float p0[H], p1[H];
-    if (line_split<H>(s, h, l, amax)) {
-        p0[0] = st3_fast<P0F>(h[0], h[1], h[2], l[0], l[1], l[2]);
-        p1[0] = st3_fast<P1F>(h[0], h[1], h[2], l[0], l[1], l[2]);
-#pragma unroll
-        for (int i = 1; i < H - 1; ++i) {
-            p0[i] = st3_fast<P0M>(h[i - 1], h[i], h[i + 1], l[i - 1], l[i], l[i + 1]);
-            p1[i] = st3_fast<P1M>(h[i - 1], h[i], h[i + 1], l[i - 1], l[i], l[i + 1]);
-        }
-        p0[H - 1] = st3_fast<P0L>(h[H - 3], h[H - 2], h[H - 1], l[H - 3], l[H - 2], l[H - 1]);
-        p1[H - 1] = st3_fast<P1L>(h[H - 3], h[H - 2], h[H - 1], l[H - 3], l[H - 2], l[H - 1]);
-    } else {
-        p0[0] = st3_any<P0F>(s[0], s[1], s[2]);
-        p1[0] = st3_any<P1F>(s[0], s[1], s[2]);
-#pragma unroll
-        for (int i = 1; i < H - 1; ++i) {
-            p0[i] = st3_any<P0M>(s[i - 1], s[i], s[i + 1]);
-            p1[i] = st3_any<P1M>(s[i - 1], s[i], s[i + 1]);
-        }
-        p0[H - 1] = st3_any<P0L>(s[H - 3], s[H - 2], s[H - 1]);
-        p1[H - 1] = st3_any<P1L>(s[H - 3], s[H - 2], s[H - 1]);
-    }
+    avg_predict<H>(s, p0, p1);
     // details = 0.5*((x1-x0) - (p1-p0)), every step in binary32 (:164-176)
 #pragma unroll
     for (int i = 0; i < H; ++i)
@@ -124,34 +154,13 @@ template <int N>
 CZ_HD void inv_avg(float (&x)[N])
 {
     constexpr int H = N / 2;
-    float s[H], d[H], h[H], l[H], p0[H], p1[H];
-    uint32_t amax;
+    float s[H], d[H], p0[H], p1[H];
 #pragma unroll
     for (int i = 0; i < H; ++i) {
         s[i] = x[i];
         d[i] = x[H + i];
     }
-    if (line_split<H>(s, h, l, amax)) {
-        p0[0] = st3_fast<P0F>(h[0], h[1], h[2], l[0], l[1], l[2]);
-        p1[0] = st3_fast<P1F>(h[0], h[1], h[2], l[0], l[1], l[2]);
-#pragma unroll
-        for (int i = 1; i < H - 1; ++i) {
-            p0[i] = st3_fast<P0M>(h[i - 1], h[i], h[i + 1], l[i - 1], l[i], l[i + 1]);
-            p1[i] = st3_fast<P1M>(h[i - 1], h[i], h[i + 1], l[i - 1], l[i], l[i + 1]);
-        }
-        p0[H - 1] = st3_fast<P0L>(h[H - 3], h[H - 2], h[H - 1], l[H - 3], l[H - 2], l[H - 1]);
-        p1[H - 1] = st3_fast<P1L>(h[H - 3], h[H - 2], h[H - 1], l[H - 3], l[H - 2], l[H - 1]);
-    } else {
-        p0[0] = st3_any<P0F>(s[0], s[1], s[2]);
-        p1[0] = st3_any<P1F>(s[0], s[1], s[2]);
-#pragma unroll
-        for (int i = 1; i < H - 1; ++i) {
-            p0[i] = st3_any<P0M>(s[i - 1], s[i], s[i + 1]);
-            p1[i] = st3_any<P1M>(s[i - 1], s[i], s[i + 1]);
-        }
-        p0[H - 1] = st3_any<P0L>(s[H - 3], s[H - 2], s[H - 1]);
-        p1[H - 1] = st3_any<P1L>(s[H - 3], s[H - 2], s[H - 1]);
-    }
+    avg_predict<H>(s, p0, p1);
     // :187-197
 #pragma unroll
     for (int i = 0; i < H; ++i) {

@@ -35,7 +35,7 @@ using cz::kSlotBytes;
 constexpr int kMaxBlocks = CZ_NOALLOC_MAX_BLOCKS;
 constexpr size_t kHdrBytes = 1024;  // descriptor, queue counter, record sizes
 constexpr size_t kScratchBytes = kHdrBytes + (size_t)kMaxBlocks * kSlotBytes;
-static_assert(sizeof(CzField) + 16 + 4 * kMaxBlocks <= kHdrBytes, "scratch header too small");
+static_assert(sizeof(CzField) <= 256 && 512 + 4 * kMaxBlocks <= 768, "scratch header too small");
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -47,6 +47,7 @@ struct Layout {
     CzField *field;
     unsigned long long *queue;
     int *rec_bytes;
+    int *err;
     uint8_t *stage;
 };
 
@@ -56,6 +57,7 @@ __host__ __device__ inline Layout layout(unsigned char *base)
     l.field = reinterpret_cast<CzField *>(base);
     l.queue = reinterpret_cast<unsigned long long *>(base + 256);
     l.rec_bytes = reinterpret_cast<int *>(base + 512);
+    l.err = reinterpret_cast<int *>(base + 768);
     l.stage = base + kHdrBytes;
     return l;
 }
@@ -66,6 +68,7 @@ __global__ void noalloc_init(unsigned char *base, const float *d_blocks, int nbl
 {
     const Layout l = layout(base);
     *l.queue = 0ull;
+    *l.err = 0;
     CzField f;
     f.data = d_blocks;
     f.nx = 32;
@@ -76,7 +79,8 @@ __global__ void noalloc_init(unsigned char *base, const float *d_blocks, int nbl
     *l.field = f;
 }
 
-// Staging slot [int32 nbytes][record] -> caller's record buffer and size.
+// Staging slot [int32 nbytes][record] -> caller's record buffer and size
+// (-1 for every block when the kernel's tile copies did not complete).
 __global__ void noalloc_copy_out(unsigned char *base, int nblocks, uint8_t *d_records, int *d_nbytes)
 {
     const Layout l = layout(base);
@@ -86,7 +90,7 @@ __global__ void noalloc_copy_out(unsigned char *base, int nblocks, uint8_t *d_re
     const uint32_t *src = reinterpret_cast<const uint32_t *>(l.stage + (size_t)g * kSlotBytes + 4);
     uint32_t *dst = reinterpret_cast<uint32_t *>(d_records + (size_t)g * CZ_MAX_RECORD);
     for (int i = threadIdx.x; i < nb / 4; i += blockDim.x) dst[i] = src[i];
-    if (threadIdx.x == 0) d_nbytes[g] = nb;
+    if (threadIdx.x == 0) d_nbytes[g] = *l.err ? -1 : nb;
 }
 
 // Device address of the scratch array for the current device.
@@ -118,7 +122,7 @@ extern "C" int cz_blocks_compress_noalloc(const float *d_blocks, int nblocks, fl
 {
     if (!d_blocks || !d_records || !d_nbytes) return CZ_E_ARG;
     if (nblocks < 1 || nblocks > kMaxBlocks) return CZ_E_ARG;  // beyond the static scratch
-    // the encode kernel reads blocks as float4 rows and the copy-out writes
+    // the encode kernel reads blocks as 16-byte aligned tiles and the copy-out writes
     // records and sizes as 32-bit words: misaligned pointers are rejected
     // here instead of faulting on the device
     if ((reinterpret_cast<uintptr_t>(d_blocks) & 15u) || (reinterpret_cast<uintptr_t>(d_records) & 3u) ||
@@ -137,8 +141,10 @@ extern "C" int cz_blocks_compress_noalloc(const float *d_blocks, int nblocks, fl
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int grid = nblocks < sms ? nblocks : sms;
+    CUtensorMap map;
+    if (!cz_field_map(CzField{d_blocks, 32, 32, 32 * nblocks, eps, 0}, &map)) return CZ_E_CUDA;
     if (cz_launch_encode(wtype, l.field, 1, nblocks, zerobits, shuffle ? 1 : 0, l.stage, l.rec_bytes, l.queue, grid,
-                         st) != cudaSuccess) {
+                         st, nullptr, &map, l.err) != cudaSuccess) {
         cudaGetLastError();
         return CZ_E_CUDA;
     }

@@ -559,7 +559,7 @@ cudaError_t cz_launch_refit(int wtype, const CzField *fields, int nfields, long 
                             float *scratch, int grid, cudaStream_t st)
 {
     if (total_blocks <= 0) return cudaSuccess;
-    const int smem = cz_codec_smem_bytes();
+    const int smem = kSmBytes;
     cudaError_t e;
     switch (wkind(wtype)) {
     case 1:
