@@ -270,6 +270,17 @@ CZ_HD Pair pfma(Pair x, Pair y, Pair z)
 #endif
     return p;
 }
+CZ_HD Pair padd(Pair x, Pair y)
+{
+    Pair p;
+#if defined(__CUDA_ARCH__)
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(p.v) : "l"(x.v), "l"(y.v));
+#else
+    p.a = CZ_ADD(x.a, y.a);
+    p.b = CZ_ADD(x.b, y.b);
+#endif
+    return p;
+}
 CZ_HD float psum(Pair x)
 {
 #if defined(__CUDA_ARCH__)
@@ -291,6 +302,29 @@ CZ_HD float st4_pair(Pair p0, Pair p1, Pair p2, Pair p3)
 {
     constexpr float k0 = S::c[0], k1 = S::c[1], k2 = S::c[2], k3 = S::c[3];
     return psum(pfma(pair(k3, k3), p3, pfma(pair(k2, k2), p2, pfma(pair(k1, k1), p1, pmul(pair(k0, k0), p0)))));
+}
+CZ_HD void unpair(Pair x, float &a, float &b)
+{
+#if defined(__CUDA_ARCH__)
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
+#else
+    a = x.a;
+    b = x.b;
+#endif
+}
+// 16 times the W1M stencil, RN32 of 9 (p1 + p2) - (p0 + p3), from the pair
+// sums u_i = p_i + p_{i+1} as 10 u_1 - (u_0 + u_2). Scaling by a power of two
+// commutes with the rounding (line_grid keeps a line's sums clear of the
+// subnormals), so the caller's fma with 1/16 gives the bits of the stencil's
+// own rounding followed by the add. Every step is exact (sums below
+// 22 * 2^19), zeros come out +0 as from the chain, and a stencil takes 8
+// cycles of the fma pipe instead of 10.
+CZ_HD float w1m_16(Pair u0, Pair u1, Pair u2)
+{
+    float uh, ul, wh, wl;
+    unpair(u1, uh, ul);
+    unpair(padd(u0, u2), wh, wl);
+    return CZ_ADD(CZ_FMA(10.f, uh, -wh), CZ_FMA(10.f, ul, -wl));
 }
 template <class S>
 CZ_HD float st3_pair(Pair p0, Pair p1, Pair p2)

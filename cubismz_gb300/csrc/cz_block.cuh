@@ -320,13 +320,6 @@ struct Payload {
     const uint8_t *q;  // byte planes 1 and 2 (p + c, or where the LZ4 stage left them)
     int c;             // byte-plane stride (reshuffle3's n/4, WaveletCompressor.cpp:80)
     bool shuffle;
-    __device__ __forceinline__ float get(int k) const
-    {
-        if (shuffle)
-            return __uint_as_float((uint32_t)p[k] | ((uint32_t)q[k] << 8) | ((uint32_t)q[c + k] << 16) |
-                                   ((uint32_t)p[3 * c + k] << 24));
-        return __uint_as_float(reinterpret_cast<const uint32_t *>(p)[k]);
-    }
 };
 
 // Record emission for block g once its coefficients sit in s.sb and its run

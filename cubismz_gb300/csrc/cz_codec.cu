@@ -34,8 +34,8 @@
 //   * corner -- levels 16 and 8 (an eighth of the block) stay in the first
 //     quarters of slabs 0..15 and are thresholded 8 positions per thread.
 // The decoder runs the same steps backwards. Measured at 512^3 (wtype 1,
-// threshold 1e-3 of the range): encode 0.664 -> 0.429 ms, decode 0.730 ->
-// 0.646 ms against one thread-block-wide pass per sweep with row loads into
+// threshold 1e-3 of the range): encode 0.664 -> 0.424 ms, decode 0.730 ->
+// 0.421 ms against one thread-block-wide pass per sweep with row loads into
 // registers (fourteen barriers a block, 16-byte loads and stores that touch
 // 32 rows each).
 #include "cz_block.cuh"
@@ -57,7 +57,7 @@ constexpr int kBarAt = kBlkAt + 4 * 32;            // mbarrier per slot
 constexpr int kFailAt = kBarAt + 8 * kSlots;
 constexpr int kCodecSmem = kFailAt + 16;
 constexpr int kMaskOdd = kRing + (kStores + 1) * kPlane;  // decode: the mask of every second block
-constexpr int kRecAt = kRing + (kStores + 2) * kPlane;    // decode: Rec x 2
+constexpr int kRecAt = kRing + (kStores + 2) * kPlane;    // decode: Rec x 4
 static_assert(kCodecSmem <= 232448, "shared memory of one CTA");
 static_assert(kBarAt % 8 == 0 && kBlkAt % 8 == 0, "alignment");
 
@@ -70,10 +70,8 @@ struct Blk {
 };
 static_assert(sizeof(Blk) == 32, "Blk");
 
-__device__ __forceinline__ void take_ticket(Blk *b, const CzField *fields, int nfields, long long total,
-                                            unsigned long long *queue)
+__device__ __forceinline__ void set_block(Blk *b, long long g, const CzField *fields, int nfields, long long total)
 {
-    const long long g = (long long)atomicAdd(queue, 1ull);
     b->g = -1;
     if (g < total) {
         const BlockRef r = locate(fields, nfields, g);
@@ -84,6 +82,20 @@ __device__ __forceinline__ void take_ticket(Blk *b, const CzField *fields, int n
         b->eps = r.f->eps;
         b->g = g;
     }
+}
+
+__device__ __forceinline__ void take_ticket(Blk *b, const CzField *fields, int nfields, long long total,
+                                            unsigned long long *queue)
+{
+    set_block(b, (long long)atomicAdd(queue, 1ull), fields, nfields, total);
+}
+// The CTA's second block is taken with the first one: not when every block
+// can have a CTA of its own.
+__device__ __forceinline__ void take_second(Blk *b, const CzField *fields, int nfields, long long total,
+                                            unsigned long long *queue)
+{
+    if (total > gridDim.x) take_ticket(b, fields, nfields, total, queue);
+    else b->g = -1;
 }
 
 // Named barrier of the first n threads (whole warps).
@@ -199,6 +211,18 @@ __device__ __forceinline__ Offsets stream_offsets(const unsigned char *sm, int w
 }
 
 // ------------------------------------------------------------------ encode
+// Bit j: |v[j]| > eps (FullWaveletTransform.h:84), eps not -0, as the sign of
+// eps - |v[j]| (rounding keeps a difference's sign; a NaN's is clear): one
+// ALU instruction per value, where a compare and an OR take two.
+template <int N>
+__device__ __forceinline__ unsigned keep_line(const float (&v)[N], float eps)
+{
+    unsigned b = 0;
+#pragma unroll
+    for (int j = N - 1; j >= 0; --j) b = __funnelshift_l(__float_as_uint(__fadd_rn(eps, -fabsf(v[j]))), b, 1);
+    return b;
+}
+
 // Survivors j of a lane's line whose keep bit is set, in order, to the
 // quarter at shared address p. Predicated: as branches the 64 tests of a
 // line took 15 instructions each.
@@ -257,7 +281,6 @@ encode_kernel(const CzField *fields, int nfields, long long total_blocks, int ze
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         *fail = 0;
         take_ticket(blk, fields, nfields, total_blocks, queue);
-        take_ticket(blk + 1, fields, nfields, total_blocks, queue);
     }
     __syncthreads();
     // plane n of the CTA's sequence (plane n & 31 of its block n >> 5) into
@@ -273,13 +296,15 @@ encode_kernel(const CzField *fields, int nfields, long long total_blocks, int ze
         bring(warp);
         if (warp + 16 < kSlots) bring(warp + 16);
     }
+    if (threadIdx.x == 0) take_second(blk + 1, fields, nfields, total_blocks, queue);
+    __syncthreads();
 
     uint32_t it = 0;
     for (;; ++it) {
         const Blk &cur = blk[it & 3];
         const long long g = cur.g;
         if (g < 0) break;
-        const float eps = cur.eps;
+        const float eps = cur.eps + 0.f;  // a threshold of -0 as 0
         // ---- level 32, x then y: planes z = warp and warp + 16
 #pragma unroll 1
         for (int r = 0; r < 2; ++r) {
@@ -318,7 +343,7 @@ encode_kernel(const CzField *fields, int nfields, long long total_blocks, int ze
             __syncwarp();
             line_fwd<32, KIND>(v);
             const bool in_corner = r == 0 && lane < 16;
-            unsigned kb = keep_bits<32>(v, eps);
+            unsigned kb = keep_line(v, eps);
             if (in_corner) kb &= 0xffff0000u;
             mask32[lane + 32 * y] = kb;  // positional word y*32+x, bits z
             // quarters: code & 3 = (z >= 16) | (x >= 16) << 1
@@ -366,7 +391,7 @@ encode_kernel(const CzField *fields, int nfields, long long total_blocks, int ze
 #pragma unroll
                 for (int j = 0; j < 16; ++j) u[j] = at(sm, corner(x, j, z));
                 line_fwd<16, KIND>(u);
-                const unsigned kb = keep_bits<16>(u, eps);
+                const unsigned kb = keep_line(u, eps);
                 // positional word x*32+z, bits y; the 8^3 corner's low byte comes later
                 if (x < 8 && z < 8) reinterpret_cast<uint8_t *>(mask32)[4 * (z + 32 * x) + 1] = (uint8_t)(kb >> 8);
                 else reinterpret_cast<uint16_t *>(mask32)[2 * (z + 32 * x)] = (uint16_t)kb;
@@ -402,7 +427,7 @@ encode_kernel(const CzField *fields, int nfields, long long total_blocks, int ze
                 line_fwd<8, KIND>(w);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) at(sm, corner(j, y, z)) = w[j];
-                unsigned kb = keep_bits<8>(w, eps);
+                unsigned kb = keep_line(w, eps);
                 if (y < 4 && z < 4) kb |= 0xFu;  // the coarse 4^3 is always kept (FullWaveletTransform.h:165-168)
                 reinterpret_cast<uint8_t *>(mask32)[4 * (y + 32 * z)] = (uint8_t)kb;
             }
@@ -411,7 +436,7 @@ encode_kernel(const CzField *fields, int nfields, long long total_blocks, int ze
         // ---- the corner's survivors, 8 stream positions per thread
         float u[8];
         corner_run((int)threadIdx.x, [&](int e, int x, int y, int z) { u[e] = at(sm, corner(x, y, z)); });
-        unsigned kc = keep_bits<8>(u, eps);
+        unsigned kc = keep_line(u, eps);
         if (threadIdx.x < 8) kc = 0xffu;
         const int nc = __popc(kc), inc = warp_scan(nc, lane);
         if (lane == 31) warp_cnt[warp] = inc;
@@ -520,17 +545,51 @@ __device__ __forceinline__ double warp_sum(double v)
 }
 
 // ------------------------------------------------------------------ decode
-// The record of a block (n is its number in the CTA's sequence).
+// Where a block's record is.
 struct Rec {
     const uint8_t *rec, *q12;  // record; byte planes 1 and 2 left in the LZ4 input (or null)
     int nb, ok;                // record bytes; whether they can be a record's
 };
 
-// n survivors from stream position k0 on into the quarter at p.
-__device__ __forceinline__ void load_quarter(unsigned char *sm, uint32_t p, int n, const Payload &pl, int k0, int lane)
+// Four bytes of each plane of a shuffled payload, as read: survivors k + j ..
+// k + j + 3 (j < n wanted, j a multiple of 4) from two aligned words per
+// plane; every load is of a word that holds a wanted byte. The words' place
+// within the aligned ones depends on k and the plane alone.
+struct Raw {
+    uint32_t lo[4], hi[4];
+};
+__device__ __forceinline__ const uint8_t *plane_at(const Payload &pl, int i, int k)
 {
-    for (int b = lane; b < n; b += 32) at(sm, quarter(p + 4 * b)) = pl.get(k0 + b);
+    return (i == 0 ? pl.p : i == 1 ? pl.q : i == 2 ? pl.q + pl.c : pl.p + 3 * pl.c) + k;
 }
+__device__ __forceinline__ void planes_load(const Payload &pl, int k, int j, int n, Raw &r)
+{
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uintptr_t a = reinterpret_cast<uintptr_t>(plane_at(pl, i, k));
+        const int off = (int)(a & 3);
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3) + ((unsigned)j >> 2);
+        r.lo[i] = j < n ? __ldg(w) : 0u;
+        r.hi[i] = off && j + 4 - off < n ? __ldg(w + 1) : 0u;
+    }
+}
+// ... and into the quarter whose first survivor is k's, at p.
+__device__ __forceinline__ void planes_store(unsigned char *sm, uint32_t p, const Payload &pl, int k, int j, int n,
+                                             const Raw &r)
+{
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        w[i] = __funnelshift_r(r.lo[i], r.hi[i], 8 * (uint32_t)(reinterpret_cast<uintptr_t>(plane_at(pl, i, k)) & 3));
+    const uint32_t a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[0], w[1], 0x7362);
+    const uint32_t c = __byte_perm(w[2], w[3], 0x5140), d = __byte_perm(w[2], w[3], 0x7362);
+    const uint32_t at0 = quarter(p + 4 * j);  // the four share the swizzle
+    if (j < n) at(sm, at0) = __uint_as_float(__byte_perm(a, c, 0x5410));
+    if (j + 1 < n) at(sm, at0 ^ 4) = __uint_as_float(__byte_perm(a, c, 0x7632));
+    if (j + 2 < n) at(sm, at0 ^ 8) = __uint_as_float(__byte_perm(b, d, 0x5410));
+    if (j + 3 < n) at(sm, at0 ^ 12) = __uint_as_float(__byte_perm(b, d, 0x7632));
+}
+
 // A lane's run from its quarter at shared address p: survivor or zero at
 // each place.
 template <int J0>
@@ -562,43 +621,76 @@ decode_kernel(const CzField *fields, int nfields, long long total_blocks, int sh
     Rec *recs = reinterpret_cast<Rec *>(sm + kRecAt);
     volatile int *bad = reinterpret_cast<volatile int *>(sm + kFailAt);  // per parity of the block's number
     unsigned char *slot = sm + kRing + warp * kPlane;  // this warp's plane
-    // Record of block n of the CTA's sequence, by threads t of nt: where it
-    // is, its mask (deserialize_bitset, WaveletCompressor.cpp:124-150) into
-    // shared memory, its payload into L2.
-    auto fetch = [&](uint32_t n, int t, int nt) {
-        const long long g = blk[n & 3].g, ro = g >= 0 ? rec_off[g] : -1;
-        const uint8_t *rec = base + (ro < 0 ? 0 : ro);
-        const int nb = ro < 0 ? -1 : *reinterpret_cast<const int *>(rec);
-        const bool size_ok = nb >= kMaskBytes && nb <= kMaxRecord + 4;
-        uint32_t *m = reinterpret_cast<uint32_t *>(sm + (n & 1 ? kMaskOdd : kMaskAt));
-        for (int i = t; i < kMaskBytes / 4; i += nt)
-            m[i] = size_ok ? reinterpret_cast<const uint32_t *>(rec + 4)[i] : 0u;
+    // Record of block n of the CTA's sequence in two steps, so that none of
+    // the dependent loads (offset, byte count, mask) waits on its own: where
+    // it is ...
+    auto find = [&](uint32_t n, long long ro, int nb, const int4 &hole, long long src_off) {
+        const uint8_t *rec = base + (ro < 0 ? 0 : ro), *q12 = nullptr;
+        const bool ok = nb >= kMaskBytes && nb <= kMaxRecord + 4;
         // byte planes 1 and 2 where the LZ4 stage left them in its input
-        const uint8_t *q12 = nullptr;
-        if (size_ok && planes.hole && shuffle) {
-            const int c4 = (nb - kMaskBytes) / 4;
-            const int4 h = planes.hole[g];
-            if (h.z > 0 && h.z == 2 * c4 && h.x == 4 + kMaskBytes + c4) q12 = planes.src + planes.src_off[g] + h.y;
-        }
-        if (size_ok) prefetch_record(rec, nb, q12, t, nt);
-        if (t == 0) recs[n & 1] = Rec{rec, q12, nb, size_ok};
+        const int c4 = (nb - kMaskBytes) / 4;
+        if (ok && hole.z > 0 && hole.z == 2 * c4 && hole.x == 4 + kMaskBytes + c4) q12 = planes.src + src_off + hole.y;
+        recs[n & 3] = Rec{rec, q12, nb, ok};
     };
-    if (threadIdx.x == 0) {
-        take_ticket(blk, fields, nfields, total_blocks, queue);
-        take_ticket(blk + 1, fields, nfields, total_blocks, queue);
+    const bool holes = planes.hole != nullptr && shuffle;
+    // ... then, by threads t of nt, its mask (deserialize_bitset,
+    // WaveletCompressor.cpp:124-150) into shared memory, its payload into L2.
+    auto fetch = [&](uint32_t n, int t, int nt) {
+        const Rec r = recs[n & 3];
+        uint32_t *m = reinterpret_cast<uint32_t *>(sm + (n & 1 ? kMaskOdd : kMaskAt));
+#pragma unroll 5
+        for (int i = t; i < kMaskBytes / 4; i += nt)
+            m[i] = r.ok ? __ldg(reinterpret_cast<const uint32_t *>(r.rec + 4) + i) : 0u;
+        if (r.ok) prefetch_record(r.rec, r.nb, r.q12, t, nt);
+    };
+    // the block after next, by the last warp's first lane: its ticket, record
+    // offset, byte count and planes, each loaded in one phase of the block
+    // and used in a later one
+    const bool scout = threadIdx.x == 32 * (kNW - 1);
+    unsigned long long s_ticket = 0;
+    long long s_off = -1, s_src = 0;
+    int s_nb = -1;
+    int4 s_hole = make_int4(0, 0, 0, 0);
+    auto scout_off = [&](uint32_t n) {
+        const long long g = blk[n & 3].g;
+        s_off = g >= 0 ? rec_off[g] : -1;
+    };
+    auto scout_rec = [&](uint32_t n) {
+        const long long g = blk[n & 3].g;
+        s_nb = s_off >= 0 ? *reinterpret_cast<const int *>(base + s_off) : -1;
+        if (g >= 0 && holes) {
+            s_hole = planes.hole[g];
+            s_src = planes.src_off[g];
+        }
+    };
+    if (scout) {
         bad[0] = bad[1] = 0;
+        take_ticket(blk, fields, nfields, total_blocks, queue);
+        scout_off(0);
+        scout_rec(0);
+        find(0, s_off, s_nb, s_hole, s_src);
     }
     __syncthreads();
-    if (blk[0].g >= 0) fetch(0, threadIdx.x, kNT);
+    if (blk[0].g < 0) return;
+    if (scout) {
+        take_second(blk + 1, fields, nfields, total_blocks, queue);
+        scout_off(1);
+        scout_rec(1);
+        find(1, s_off, s_nb, s_hole, s_src);
+    } else if (warp < kNW - 1) {
+        fetch(0, threadIdx.x, kNT - 32);
+    }
     __syncthreads();
     for (uint32_t it = 0;; ++it) {
         const Blk &cur = blk[it & 3];
         const long long g = cur.g;
         if (g < 0) break;
         const uint32_t *mask32 = reinterpret_cast<const uint32_t *>(sm + (it & 1 ? kMaskOdd : kMaskAt));
-        const uint8_t *rec = recs[it & 1].rec, *q12 = recs[it & 1].q12;
-        const int nb = recs[it & 1].nb;
-        const bool size_ok = recs[it & 1].ok != 0;
+        const uint8_t *rec = recs[it & 3].rec, *q12 = recs[it & 3].q12;
+        const int nb = recs[it & 3].nb;
+        const bool more = blk[(it + 1) & 3].g >= 0;
+        if (scout && more) s_ticket = atomicAdd(queue, 1ull);
+        const bool size_ok = recs[it & 3].ok != 0;
         // ---- survivor counts: level 32 per (octant, slab), the corner per warp
         unsigned kz[2];
         int ex[2];
@@ -644,11 +736,50 @@ decode_kernel(const CzField *fields, int nfields, long long total_blocks, int sh
             pl.shuffle = shuffle != 0;
             if (lane == 0) tma_store_wait_read();  // the slot holds the warp's corner survivors next
             __syncwarp();
-            load_quarter(sm, kRing + warp * kPlane, __shfl_sync(0xffffffffu, inc, 31), pl, of.mine, lane);
+            // list 0: the warp's part of the corner; 1-7: an octant's quarter
+            auto list = [&](int code, uint32_t &p, int &n, int &k0) {
+                p = code ? kMain + (warp + 16 * (code >> 2)) * kPlane + (code & 3) * 1024 : kRing + warp * kPlane;
+                n = code ? seg_cnt[(code - 1) * 16 + warp] : warp_cnt[warp];
+                const int seg = of.of(code ? code : 1, warp);
+                k0 = code ? seg : of.mine;
+            };
+            uint32_t p;
+            int n, k0;
+            list(0, p, n, k0);
+            if (pl.shuffle) {
+                // 128 survivors a step, the next list's first step in flight
+                // while this one's are placed
+                Raw now;
+                planes_load(pl, k0, 4 * lane, n, now);
 #pragma unroll 1
-            for (int code = 1; code < 8; ++code)
-                load_quarter(sm, kMain + (warp + 16 * (code >> 2)) * kPlane + (code & 3) * 1024,
-                             seg_cnt[(code - 1) * 16 + warp], pl, of.of(code, warp), lane);
+                for (int code = 0; code < 8; ++code) {
+                    uint32_t pn = 0;
+                    int nn = 0, kn = 0;
+                    if (code < 7) list(code + 1, pn, nn, kn);
+                    Raw ahead;
+                    planes_load(pl, kn, 4 * lane, nn, ahead);
+                    if (n > 128) {
+                        Raw more4;
+                        planes_load(pl, k0, 128 + 4 * lane, n, more4);
+                        planes_store(sm, p, pl, k0, 4 * lane, n, now);
+                        planes_store(sm, p, pl, k0, 128 + 4 * lane, n, more4);
+                    } else {
+                        planes_store(sm, p, pl, k0, 4 * lane, n, now);
+                    }
+                    now = ahead;
+                    p = pn;
+                    n = nn;
+                    k0 = kn;
+                }
+            } else {
+                const float *src = reinterpret_cast<const float *>(pl.p);
+#pragma unroll 1
+                for (int code = 0; code < 8; ++code) {
+                    if (code) list(code, p, n, k0);
+#pragma unroll 4
+                    for (int b = lane; b < n; b += 32) at(sm, quarter(p + 4 * b)) = __ldg(src + k0 + b);
+                }
+            }
         } else {
             kc = kz[0] = kz[1] = 0;
         }
@@ -712,12 +843,15 @@ decode_kernel(const CzField *fields, int nfields, long long total_blocks, int sh
             line_inv<16, KIND>(u);
 #pragma unroll
             for (int j = 0; j < 16; ++j) at(sm, corner(j, y, z)) = u[j];
-        } else if (warp == kNW - 1) {  // idle meanwhile: the ticket after next
-            if (lane == 0) take_ticket(blk + ((it + 2) & 3), fields, nfields, total_blocks, queue);
-        } else if (blk[(it + 1) & 3].g >= 0) {  // ... and the next record
+        } else if (scout) {  // idle meanwhile
+            blk[(it + 2) & 3].g = -1;
+            if (more) set_block(blk + ((it + 2) & 3), (long long)s_ticket, fields, nfields, total_blocks);
+            scout_off(it + 2);
+        } else if (more && warp < kNW - 1) {
             fetch(it + 1, threadIdx.x - 256, kNT - 256 - 32);
         }
         __syncthreads();
+        if (scout) scout_rec(it + 2);
         // ---- level 16, z, and level 32, z: slabs y = warp and warp + 16
 #pragma unroll 1
         for (int r = 0; r < 2; ++r) {
@@ -744,6 +878,7 @@ decode_kernel(const CzField *fields, int nfields, long long total_blocks, int sh
             for (int j = 0; j < 32; ++j) at(sm, slab + j * 128 + lane * 4) = v[j];
         }
         __syncthreads();
+        if (scout) find(it + 2, s_off, s_nb, s_hole, s_src);
         // ---- level 32, y then x: planes z = warp and warp + 16, then straight
         // to the field (copy_to, WaveletCompressor.h:73-82)
         DiffAcc acc;

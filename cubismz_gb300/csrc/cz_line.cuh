@@ -21,8 +21,10 @@ CZ_RARE void interp_rare(const float *e, float *o, int H)
     o[H - 2] = st4_main<W1O>(e[H - 4], e[H - 3], e[H - 2], e[H - 1]);
     o[H - 1] = st4_lastany(e[H - 4], e[H - 3], e[H - 2], e[H - 1]);
 }
+// o[i] = base[i] + sign * prediction i, each rounded as the reference rounds
+// (the prediction, then the sum).
 template <int H>
-CZ_HD void interp_predict(const float (&e)[H], float (&o)[H])
+CZ_HD void interp_predict(const float (&e)[H], float sign, const float (&base)[H], float (&o)[H])
 {
     uint32_t amax;
     bool narrow;
@@ -31,18 +33,21 @@ CZ_HD void interp_predict(const float (&e)[H], float (&o)[H])
         Pair p[H];
 #pragma unroll
         for (int i = 0; i < H; ++i) p[i] = split_pair(e[i], C);
-        o[0] = st4_pair<W1F>(p[0], p[1], p[2], p[3]);
+        o[0] = CZ_FMA(sign, st4_pair<W1F>(p[0], p[1], p[2], p[3]), base[0]);
+        Pair u[H - 1];
 #pragma unroll
-        for (int i = 1; i < H - 2; ++i) o[i] = st4_pair<W1M>(p[i - 1], p[i], p[i + 1], p[i + 2]);
-        o[H - 2] = st4_pair<W1O>(p[H - 4], p[H - 3], p[H - 2], p[H - 1]);
-        o[H - 1] = interp_last(e[H - 4], e[H - 3], e[H - 2], e[H - 1], amax, narrow);
+        for (int i = 0; i < H - 1; ++i) u[i] = padd(p[i], p[i + 1]);
+#pragma unroll
+        for (int i = 1; i < H - 2; ++i) o[i] = CZ_FMA(0.0625f * sign, w1m_16(u[i - 1], u[i], u[i + 1]), base[i]);
+        o[H - 2] = CZ_FMA(sign, st4_pair<W1O>(p[H - 4], p[H - 3], p[H - 2], p[H - 1]), base[H - 2]);
+        o[H - 1] = CZ_FMA(sign, interp_last(e[H - 4], e[H - 3], e[H - 2], e[H - 1], amax, narrow), base[H - 1]);
     } else {
         float te[H], to[H];  // the call's arrays live in memory, e and o in registers
 #pragma unroll
         for (int i = 0; i < H; ++i) te[i] = e[i];
         interp_rare(te, to, H);
 #pragma unroll
-        for (int i = 0; i < H; ++i) o[i] = to[i];
+        for (int i = 0; i < H; ++i) o[i] = CZ_FMA(sign, to[i], base[i]);
     }
 }
 
@@ -50,12 +55,13 @@ template <int N>
 CZ_HD void fwd_interp(float (&x)[N], bool lifting)
 {
     constexpr int H = N / 2;
-    float e[H], d[H];
+    float e[H], b[H], d[H];
 #pragma unroll
-    for (int i = 0; i < H; ++i) e[i] = x[2 * i];
-    interp_predict<H>(e, d);
-#pragma unroll
-    for (int i = 0; i < H; ++i) d[i] = CZ_SUB(x[2 * i + 1], d[i]);
+    for (int i = 0; i < H; ++i) {
+        e[i] = x[2 * i];
+        b[i] = x[2 * i + 1];
+    }
+    interp_predict<H>(e, -1.f, b, d);
     // scalings[i] += 0.5*details[i] in binary64, rounded to binary32 (:124-126):
     // a single fma is the correctly rounded value of the same exact sum.
 #pragma unroll
@@ -74,12 +80,12 @@ CZ_HD void inv_interp(float (&x)[N], bool lifting)
         d[i] = x[H + i];
         s[i] = lifting ? CZ_FMA(-0.5f, d[i], x[i]) : x[i];  // :137-139
     }
-    interp_predict<H>(s, o);
+    interp_predict<H>(s, 1.f, d, o);
     // :141-151: even samples are the scalings, odd samples interp + detail
 #pragma unroll
     for (int i = 0; i < H; ++i) {
         x[2 * i] = s[i];
-        x[2 * i + 1] = CZ_ADD(o[i], d[i]);
+        x[2 * i + 1] = o[i];
     }
 }
 
@@ -112,8 +118,11 @@ CZ_HD void avg_predict(const float (&s)[H], float (&p0)[H], float (&p1)[H])
         p1[0] = st3_pair<P1F>(p[0], p[1], p[2]);
 #pragma unroll
         for (int i = 1; i < H - 1; ++i) {
-            p0[i] = st3_pair<P0M>(p[i - 1], p[i], p[i + 1]);
-            p1[i] = st3_pair<P1M>(p[i - 1], p[i], p[i + 1]);
+            // p[i] +- (p[i-1] - p[i+1]) / 8: the difference is shared (exact,
+            // and +0 where it vanishes)
+            const Pair t = pfma(pair(-1.f, -1.f), p[i + 1], p[i - 1]);
+            p0[i] = psum(pfma(pair(0.125f, 0.125f), t, p[i]));
+            p1[i] = psum(pfma(pair(-0.125f, -0.125f), t, p[i]));
         }
         p0[H - 1] = st3_pair<P0L>(p[H - 3], p[H - 2], p[H - 1]);
         p1[H - 1] = st3_pair<P1L>(p[H - 3], p[H - 2], p[H - 1]);
