@@ -413,13 +413,12 @@ int decompress_fields(cz_ctx *c, const std::vector<CzField> &fields, long long n
         base = P<uint8_t>(c->dec);
         dlen = P<int>(c->dec_len);
     } else if (!raw) {
-        const int lzgrid = std::max(1, std::min((nchunks + 3) / 4, c->sms * 8));
         if (planes_in_input) {
             CZ_TRY(grow(c, c->lz_hole, sizeof(int4) * (size_t)nchunks));
             planes = CzPlanes{P<int4>(c->lz_hole), d_data, d_off};
         }
         CZ_CUDA(c, cz_launch_lz4_decode(d_data, d_off, P<int>(c->in_len), nchunks, P<uint8_t>(c->dec),
-                                        P<long long>(c->dec_off), P<int>(c->dec_cap), P<int>(c->dec_len), lzgrid, st,
+                                        P<long long>(c->dec_off), P<int>(c->dec_cap), P<int>(c->dec_len), st,
                                         planes_in_input ? P<int4>(c->lz_hole) : nullptr));
         base = P<uint8_t>(c->dec);
         dlen = P<int>(c->dec_len);
@@ -1049,7 +1048,7 @@ int cz_lz4_decompress(cz_ctx *c, const uint8_t *src, int isize, uint8_t *dst, in
     int *dlen = reinterpret_cast<int *>(meta + 16);
     int *dcap = reinterpret_cast<int *>(meta + 20);
     int *dres = reinterpret_cast<int *>(meta + 24);
-    CZ_CUDA(c, cz_launch_lz4_decode(d, doff, dlen, 1, dout, doff + 1, dcap, dres, 1, nullptr));
+    CZ_CUDA(c, cz_launch_lz4_decode(d, doff, dlen, 1, dout, doff + 1, dcap, dres, nullptr));
     int n = 0;
     CZ_CUDA(c, cudaMemcpy(&n, dres, 4, cudaMemcpyDeviceToHost));
     *out = n;

@@ -103,7 +103,7 @@ cudaError_t cz_launch_deflate(const uint8_t *in, const long long *in_off, const 
 // then leaves that span of its output unwritten and the record's reader
 // takes it from the input (CzPlanes); length 0 otherwise.
 cudaError_t cz_launch_lz4_decode(const uint8_t *in, const long long *in_off, const int *in_len, int nchunks,
-                                 uint8_t *out, const long long *out_off, const int *out_cap, int *out_len, int grid,
+                                 uint8_t *out, const long long *out_off, const int *out_cap, int *out_len,
                                  cudaStream_t st, int4 *hole = nullptr);
 
 // Stream assembly helpers (cz_lz4.cu, cz_stream.cu)

@@ -33,16 +33,17 @@
 // encoder (cz_zlib.cu).
 // Decoder: the same acceptance tests and error convention as
 // LZ4_uncompress_unknownOutputSize (-(input position) on malformed input; an
-// empty input yields 0). Windows of 128 input bytes are parsed
-// speculatively (every lane decodes tokens at 4 candidate positions; jump
-// tables by pointer doubling find the real sequences), output is staged in a
-// 4 KB per-warp ring and flushed with word stores; overlapping matches
-// repeat their first `offset` bytes, the byte-serial copy semantics. Short
-// matches are copied by their own lanes in rounds (sources before the
-// window first, then those whose sources the earlier rounds completed);
-// long ones by the whole warp. For one-record chunks of shuffled records a
-// literal run that covers byte planes 1 and 2 whole stays in the input
-// (hole), where later matches and the decode kernel read it.
+// empty input yields 0). Two kernels, chosen by the number of chunks: one
+// CTA per chunk for few, one warp per chunk for many. Both parse windows of
+// 128 input bytes speculatively (every lane decodes tokens at 4 candidate
+// positions; jump tables by pointer doubling find the real sequences) and
+// stage output in a ring in shared memory that is flushed with word stores;
+// overlapping matches repeat their first `offset` bytes, the byte-serial copy
+// semantics. For one-record chunks of shuffled records a literal run that
+// covers byte planes 1 and 2 whole stays in the input (hole), where later
+// matches and the decode kernel read it.
+#include <algorithm>
+
 #include "cz_codec.h"
 #include "cz_deflate.cuh"
 
@@ -613,20 +614,562 @@ lz4_encode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
 }
 
 // ------------------------------------------------------------------ decode
-// Length continuation bytes from ip while they are 255 and ip < lim;
-// returns their sum and leaves ip after the last byte read.
-__device__ __forceinline__ long long get_len(const uint8_t *src, int &ip, int lim)
+// n bytes from s to d by the CTA: bytes until d is 16-byte aligned, then
+// 16-byte stores (each built from five 4-byte loads with funnel shifts), then
+// the tail. Wide stores matter when the destination is host memory written
+// over the CPU-GPU link. Reads up to 4 bytes past s + n.
+__device__ __forceinline__ void cta_copy(uint8_t *__restrict__ d, const uint8_t *__restrict__ s, int n)
+{
+    if (n <= 0) return;
+    int h = (int)((16 - (reinterpret_cast<uintptr_t>(d) & 15)) & 15);
+    if (h > n) h = n;
+    if ((int)threadIdx.x < h) d[threadIdx.x] = s[threadIdx.x];
+    const uint8_t *s2 = s + h;
+    uint4 *dw = reinterpret_cast<uint4 *>(d + h);
+    const int m = n - h, nwd = m >> 4;
+    const uint32_t sa = (uint32_t)(reinterpret_cast<uintptr_t>(s2) & 3);
+    const uint32_t *sw = reinterpret_cast<const uint32_t *>(s2 - sa);
+    for (int i = threadIdx.x; i < nwd; i += blockDim.x) {
+        const uint32_t *q = sw + 4 * i;
+        const uint32_t a0 = q[0], a1 = q[1], a2 = q[2], a3 = q[3], a4 = sa ? q[4] : 0u;
+        uint4 v;
+        if (sa) {
+            v.x = __funnelshift_r(a0, a1, 8 * sa);
+            v.y = __funnelshift_r(a1, a2, 8 * sa);
+            v.z = __funnelshift_r(a2, a3, 8 * sa);
+            v.w = __funnelshift_r(a3, a4, 8 * sa);
+        } else {
+            v = make_uint4(a0, a1, a2, a3);
+        }
+        dw[i] = v;
+    }
+    const int t = m & 15;
+    if ((int)threadIdx.x < t) d[h + 16 * nwd + threadIdx.x] = s2[16 * nwd + threadIdx.x];
+}
+
+// One CTA per chunk, for few chunks. The chunk is one serial chain of sequences, each of a few
+// bytes; what bounds a decoder is that chain and, with many chunks, issue.
+// Both want many sequences per step, so a step takes kDecIn input bytes:
+//   * every warp decodes the tokens at all 128 positions of its window as if
+//     a sequence started there (4 per lane) and makes jump tables by pointer
+//     doubling in shared memory: T_b, 2^b steps along the next-token chain,
+//     positions past the window absorbing. T_6 is then the window's exit for
+//     every entry, so the chain through the step's windows costs one lookup
+//     each, and lane k finds the window's k-th sequence in six;
+//   * thread t takes the step's t-th sequence; scans give output positions,
+//     and the reference's acceptance tests run per sequence, the first that
+//     does not pass ends the step;
+//   * the output is made in a ring in shared memory, a word per thread and
+//     turn (its sequence by binary search over the output positions):
+//     literals and match bytes whose source lies before the step are written
+//     at once, other match bytes leave their distance, and are then chased
+//     along the distances to a written byte, every hop adding the distance
+//     that the byte met holds by then, so that chains of copies of copies
+//     shorten for all at once (pointer jumping) without a barrier per round.
+// Sequences with length fields of more than kFastExt bytes, or too long for
+// the ring, are decoded serially, their copies by the whole CTA.
+// A step of 1 KB of input (about 180 sequences) takes 10 k cycles on an SM of
+// its own; one-record chunks on an idle GPU 0.18 ms instead of 0.61 with one
+// warp each (64 chunks of a 128^3 field), 15-record chunks 2.33 instead of
+// 9.0 ms (35 chunks of a 256^3 field).
+constexpr int kDecWarps = 8, kDecThreads = 32 * kDecWarps;
+constexpr int kWin = 128, kLevels = 7, kFastExt = 8;
+constexpr int kDecIn = kWin * kDecWarps;     // input positions per step
+constexpr int kDecStage = kDecIn + 64;       // input bytes held in shared memory
+constexpr int kMaxSeqWin = (kWin + 2) / 3;   // a sequence takes at least 3 input bytes
+// A step adds at most kStage bytes, so at least kRing - kStage - 4 bytes of
+// history stay readable while it is written. Of the match sources in
+// block-record chunks 90% lie within 3 KB and 99% within 12 KB, but a single
+// source in global memory costs its whole step an L2 round trip: with 16 KB
+// instead of 32 a launch of 2048 chunks took 0.627 ms instead of 0.514.
+constexpr int kRing = 32768, kMask = kRing - 1, kStage = 4096;
+constexpr uint32_t kEnd = 0xffffu;  // next position of a sequence that ends the chain (last, or serial)
+
+// Sum of the length continuation bytes from ip while they are 255 and
+// ip < lim; leaves ip after the last byte read. Called by whole warps.
+__device__ __forceinline__ long long get_len(const uint8_t *src, int &ip, int lim, int lane)
 {
     long long sum = 0;
     while (ip < lim) {
-        const int s = src[ip++];
-        sum += s;
-        if (s != 255) break;
+        const int b = ip + lane < lim ? (int)__ldg(src + ip + lane) : -1;
+        const unsigned stop = __ballot_sync(0xffffffffu, b != 255);
+        const int k = stop ? __ffs(stop) - 1 : 32;  // bytes of 255 first
+        sum += 255ll * k;
+        ip += k;
+        if (k < 32) {
+            const int last = __shfl_sync(0xffffffffu, b, k);
+            if (last >= 0) {
+                sum += last;
+                ++ip;
+            }
+            break;
+        }
     }
     return sum;
 }
 
-// Parallel parse. The decoder reads a window of kWin input bytes starting
+// Byte k of a match at output ms comes from ms - off + (k mod off): the
+// byte-serial copy repeats the first `off` bytes when off < length.
+__device__ __forceinline__ int msrc(int k, int off, int ml) { return off >= ml ? k : k % off; }
+
+// Byte planes 1 and 2 of a record chunk that the decoder left in its input
+// (a literal run it did not copy): output [out, out + len) is input
+// [in, in + len); len 0: none.
+struct LzHole {
+    int out = 0, len = 0, in = 0;
+};
+
+// Output byte x from global memory: from the input inside the hole, else
+// from the output (via L2).
+__device__ __forceinline__ uint8_t old_byte(const uint8_t *src, const uint8_t *dst, const LzHole &h, int x)
+{
+    return (unsigned)(x - h.out) < (unsigned)h.len ? __ldg(src + h.in + (x - h.out)) : __ldcg(dst + x);
+}
+
+// n bytes of the ring starting at ring offset r (r + n <= kRing) to d (any
+// alignment): 4-byte stores once d is aligned. By threads t of nt.
+__device__ __forceinline__ void flush(uint8_t *d, const uint8_t *ring, int r, int n, int t, int nt)
+{
+    int h = (int)((4 - (reinterpret_cast<uintptr_t>(d) & 3)) & 3);
+    if (h > n) h = n;
+    if (t < h) d[t] = ring[r + t];
+    const int nw = (n - h) >> 2, b = r + h, sh = 8 * (b & 3);
+    const uint32_t *sw = reinterpret_cast<const uint32_t *>(ring) + (b >> 2);
+    uint32_t *dw = reinterpret_cast<uint32_t *>(d + h);
+    for (int i = t; i < nw; i += nt) dw[i] = sh ? __funnelshift_r(sw[i], sw[i + 1], sh) : sw[i];
+    const int e = (n - h) & 3;
+    if (t < e) d[h + 4 * nw + t] = ring[b + 4 * nw + t];
+}
+
+// A decoded token.
+struct LzSeq {
+    int lit_at, lit, ml, next;  // literals' input position and count, match length, position after the sequence
+    bool term, slow;            // ends the input; length field too long for the parallel parse
+};
+
+struct LzDecShared {
+    uint8_t ring[kRing + 16];              // recent output (16 bytes of slack)
+    uint16_t dist[kStage + 8];             // per output byte of the step (from its first word): distance to its source in the step, or 0
+    uint16_t jump[kDecWarps][kLevels][kWin];  // T_b, positions relative to the step
+    int4 seq[kDecThreads + 1];             // per sequence: output start, literals' end, input - output position of the literals, distance
+    uint32_t in[kDecStage / 4 + 1];        // the step's input
+    uint16_t first[kDecThreads];           // output start per sequence
+    uint16_t slot[kDecWarps][kMaxSeqWin + 1];  // positions of each window's sequences
+    int count[kDecWarps], bytes[kDecWarps];    // sequences and output bytes per warp
+    int stop[kDecWarps], epos[kDecWarps], stop_at[kDecWarps], stop_pos[kDecWarps];  // first sequence not taken
+    int exit;                              // the chain's position after the step
+};
+
+__global__ void __launch_bounds__(kDecThreads, 3)
+lz4_decode_wide_kernel(const uint8_t *__restrict__ in, const long long *in_off, const int *in_len, int nchunks,
+                  uint8_t *__restrict__ out, const long long *out_off, const int *out_cap, int *out_len,
+                  int4 *hole)
+{
+    extern __shared__ __align__(16) unsigned char lz_dec_smem[];
+    LzDecShared &s = *reinterpret_cast<LzDecShared *>(lz_dec_smem);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint8_t *ring = s.ring;
+    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
+        const uint8_t *src = in + in_off[c];
+        const int iend = in_len[c];
+        uint8_t *dst = out + out_off[c];
+        const int oend = out_cap[c];
+        int s0 = 0, op = 0, err = 0, ring_lo = 0;  // output before ring_lo is not in the ring
+        bool done = false;
+        LzHole hl;
+        if (hole && tid == 0) hole[c] = make_int4(0, 0, 0, 0);  // written for every chunk
+        __syncthreads();  // the previous chunk has left shared memory
+        // a literal run of n bytes from input i to output o, except the
+        // record's byte planes 1 and 2 when it covers them whole (hole
+        // given, record chunks: the record's byte count is output bytes 0-3)
+        auto lit_run = [&](int o, int i, int n) {
+            int a = 0, b = 0;
+            if (hole && hl.len == 0 && o >= 4) {
+                const int nb = (int)__ldcg(dst) | (int)__ldcg(dst + 1) << 8 | (int)__ldcg(dst + 2) << 16 |
+                               (int)__ldcg(dst + 3) << 24;
+                if (nb >= 4096 && nb <= 4096 + 4 * 32768 && ((nb - 4096) & 3) == 0) {
+                    const int S = (nb - 4096) >> 2;
+                    a = 4 + 4096 + S;
+                    b = a + 2 * S;
+                    if (!(o <= a && o + n >= b && b - a >= kMinHole)) a = b = 0;
+                }
+            }
+            if (b > a) {
+                cta_copy(dst + o, src + i, a - o);
+                cta_copy(dst + b, src + i + (b - o), o + n - b);
+                hl.out = a;
+                hl.len = b - a;
+                hl.in = i + (a - o);
+                if (tid == 0) hole[c] = make_int4(hl.out, hl.in, hl.len, 0);
+            } else {
+                cta_copy(dst + o, src + i, n);
+            }
+        };
+        if (iend <= 0) {
+            if (tid == 0) out_len[c] = 0;  // lz4.c:836: error exit at position 0
+            continue;
+        }
+        // word i of the input around position p (whole aligned words; none
+        // that lies past the input)
+        auto in_word = [&](int p, int i) -> uint32_t {
+            const uint8_t *a = reinterpret_cast<const uint8_t *>(reinterpret_cast<uintptr_t>(src + p) & ~(uintptr_t)3) +
+                               4 * i;
+            return a < src + iend ? __ldg(reinterpret_cast<const uint32_t *>(a)) : 0u;
+        };
+        int ahead_at = -1;  // position the words loaded ahead belong to
+        uint32_t ahead = 0, ahead2 = 0;
+        constexpr int kExtra = kDecStage / 4 + 1 - kDecThreads;  // words beyond one per thread
+        while (!done && !err) {
+            // ---- the step's input; positions count from the aligned base
+            const int base = s0 - (int)(reinterpret_cast<uintptr_t>(src + s0) & 3);
+            if (ahead_at != s0) {
+                ahead = in_word(s0, tid);
+                ahead2 = tid < kExtra ? in_word(s0, kDecThreads + tid) : 0u;
+            }
+            s.in[tid] = ahead;
+            if (tid < kExtra) s.in[kDecThreads + tid] = ahead2;
+            __syncthreads();
+            const uint8_t *ib = reinterpret_cast<const uint8_t *>(s.in);
+            auto byte_at = [&](int p) -> int { return p - base < kDecStage ? (int)ib[p - base] : (int)__ldg(src + p); };
+            // the token at p (< iend) as a sequence (lz4.c:846-882)
+            auto decode = [&](int p, int tok) {
+                LzSeq q;
+                q.lit = tok >> 4;
+                q.ml = tok & 15;
+                q.lit_at = p + 1;
+                q.next = 0;
+                q.slow = q.term = false;
+                if (q.lit == 15 && q.lit_at < iend) {
+                    int e = byte_at(q.lit_at++);
+                    q.lit += e;
+                    if (e == 255) {  // rare
+                        int k = 1;
+                        for (; k < kFastExt && e == 255 && q.lit_at < iend; ++k) {
+                            e = byte_at(q.lit_at++);
+                            q.lit += e;
+                        }
+                        q.slow = e == 255 && q.lit_at < iend;
+                    }
+                }
+                if (!q.slow && q.lit > iend - q.lit_at - (2 + 1 + kLastLiterals)) q.term = true;  // lz4.c:851
+                if (!q.slow && !q.term) {
+                    q.next = q.lit_at + q.lit + 2;
+                    const int lim = iend - (kLastLiterals + 1);
+                    if (q.ml == 15 && q.next < lim) {
+                        int e = byte_at(q.next++);
+                        q.ml += e;
+                        if (e == 255) {
+                            int k = 1;
+                            for (; k < kFastExt && e == 255 && q.next < lim; ++k) {
+                                e = byte_at(q.next++);
+                                q.ml += e;
+                            }
+                            q.slow = e == 255 && q.next < lim;
+                        }
+                    }
+                }
+                q.ml += kMinMatch;
+                return q;
+            };
+            // ---- jump tables of this warp's window
+            const int w0 = warp * kWin;  // relative to base
+            uint16_t(*T)[kWin] = s.jump[warp];
+            uint32_t t0[4];
+            {
+                const uint32_t word = s.in[(w0 >> 2) + lane];
+                const int p0 = base + w0 + 4 * lane;
+                unsigned ext = 0;  // candidates with a length continuation
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int p = p0 + j, tok = (int)((word >> (8 * j)) & 0xff), lit = tok >> 4;
+                    const bool in = p >= s0 && p < iend;
+                    const bool plain = lit != 15 && (tok & 15) != 15;
+                    if (in && !plain) ext |= 1u << j;
+                    t0[j] = in && plain && lit <= iend - p - (1 + 2 + 1 + kLastLiterals) ? (uint32_t)(p - base + 3 + lit)
+                                                                                        : kEnd;
+                }
+                while (ext) {
+                    const int j = __ffs(ext) - 1;
+                    ext &= ext - 1;
+                    const LzSeq q = decode(p0 + j, (int)((word >> (8 * j)) & 0xff));
+                    const uint32_t v = q.slow || q.term ? kEnd : (uint32_t)(q.next - base);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (i == j) t0[i] = v;
+                }
+                reinterpret_cast<uint2 *>(T[0])[lane] = make_uint2(t0[0] | t0[1] << 16, t0[2] | t0[3] << 16);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int b = 1; b < kLevels; ++b) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (t0[j] - (uint32_t)w0 < (uint32_t)kWin) t0[j] = T[b - 1][t0[j] - w0];
+                reinterpret_cast<uint2 *>(T[b])[lane] = make_uint2(t0[0] | t0[1] << 16, t0[2] | t0[3] << 16);
+                __syncwarp();
+            }
+            __syncthreads();
+            // ---- the chain through the windows, then this window's sequences
+            uint32_t e = (uint32_t)(s0 - base);
+            for (int w = 0; w < warp; ++w)
+                if (e - (uint32_t)(w * kWin) < (uint32_t)kWin) e = s.jump[w][kLevels - 1][e - w * kWin];
+            int cnt = 0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int k = lane + 32 * h;
+                uint32_t pos = e;
+#pragma unroll
+                for (int b = 0; b < kLevels - 1; ++b)
+                    if ((k >> b) & 1)
+                        if (pos - (uint32_t)w0 < (uint32_t)kWin) pos = T[b][pos - w0];
+                const bool member = k < kMaxSeqWin && pos - (uint32_t)w0 < (uint32_t)kWin;
+                if (member) s.slot[warp][k] = (uint16_t)pos;
+                cnt += __popc(__ballot_sync(0xffffffffu, member));
+            }
+            if (lane == 0) s.count[warp] = cnt;
+            if (warp == kDecWarps - 1 && lane == 0)
+                s.exit = (int)(e - (uint32_t)w0 < (uint32_t)kWin ? T[kLevels - 1][e - w0] : e);
+            __syncthreads();
+            // ---- thread t takes sequence t
+            int nseq = 0, mw = 0, mk = tid, over = -1;  // over: position of sequence kDecThreads, if there is one
+#pragma unroll
+            for (int w = 0; w < kDecWarps; ++w) {
+                const int n = s.count[w];
+                if (tid >= nseq) {
+                    mw = w;
+                    mk = tid - nseq;
+                }
+                if (kDecThreads - nseq >= 0 && kDecThreads - nseq < n) over = s.slot[w][kDecThreads - nseq];
+                nseq += n;
+            }
+            const int nthis = min(nseq, kDecThreads);
+            const bool member = tid < nthis;
+            const int after = over >= 0 ? over : s.exit;  // kEnd: the last sequence is terminal or slow
+            // the next step's input, loaded ahead
+            ahead_at = after != (int)kEnd ? base + after : -1;
+            if (ahead_at >= 0) {
+                ahead = in_word(ahead_at, tid);
+                ahead2 = tid < kExtra ? in_word(ahead_at, kDecThreads + tid) : 0u;
+            }
+            int pos = 0, off = 0, stop = 0, epos = 0;  // stop 1: end of input, 2: malformed, 3: decode serially, 4: no room
+            LzSeq q;
+            q.lit_at = q.lit = q.ml = q.next = 0;
+            q.term = q.slow = false;
+            if (member) {
+                pos = s.slot[mw][mk];
+                q = decode(base + pos, (int)ib[pos]);
+                if (!q.term && !q.slow) off = byte_at(q.lit_at + q.lit) | byte_at(q.lit_at + q.lit + 1) << 8;
+            }
+            const int len = member && !q.slow ? q.lit + (q.term ? 0 : q.ml) : 0;
+            int incl = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+            if (lane == 31) s.bytes[warp] = incl;
+            __syncthreads();
+            int before = 0, total = 0;
+#pragma unroll
+            for (int w = 0; w < kDecWarps; ++w) {
+                const int n = s.bytes[w];
+                before += w < warp ? n : 0;
+                total += n;
+            }
+            incl += before;  // output bytes of the step up to this sequence's end
+            const int at = incl - len, opl = op + at, ms = opl + q.lit;
+            // ---- acceptance tests (lz4.c:851-858, :868, :888-890)
+            if (member) {
+                if (q.slow) {
+                    stop = 3;
+                } else if (incl > kStage) {
+                    stop = 4;
+                } else if (q.term || q.lit > oend - opl - kMfLimit) {
+                    if (q.lit > oend - opl || q.lit != iend - q.lit_at) {
+                        stop = 2;
+                        epos = q.lit_at;
+                    } else {
+                        stop = 1;
+                    }
+                } else if (off == 0 || off > ms) {
+                    stop = 2;
+                    epos = q.lit_at + q.lit + 2;
+                } else if (q.ml > oend - ms - kLastLiterals) {
+                    stop = 2;
+                    epos = q.next;
+                }
+            }
+            {
+                const unsigned sb = __ballot_sync(0xffffffffu, stop != 0);
+                const int k = sb ? __ffs(sb) - 1 : 0;
+                const int why = __shfl_sync(0xffffffffu, stop, k), ep = __shfl_sync(0xffffffffu, epos, k);
+                const int sat = __shfl_sync(0xffffffffu, at + (stop == 1 ? q.lit : 0), k),
+                          sp = __shfl_sync(0xffffffffu, pos, k);
+                if (lane == 0) {
+                    s.stop[warp] = sb ? (32 * warp + k) << 3 | why : 0x7fffffff;
+                    s.epos[warp] = ep;
+                    s.stop_at[warp] = sat;
+                    s.stop_pos[warp] = sp;
+                }
+            }
+            s.first[tid] = (uint16_t)(member ? min(at, kStage) : kStage);
+            s.seq[tid] = make_int4(at, at + q.lit, q.lit_at - at, off);
+            __syncthreads();
+            // the output ends where the first sequence that is not taken
+            // starts (or ends, when it is the input's last literals)
+            int ks = 0x7fffffff, kepos = 0, nout = total, kpos = 0;
+#pragma unroll
+            for (int w = kDecWarps - 1; w >= 0; --w)
+                if (s.stop[w] < ks) {
+                    ks = s.stop[w];
+                    kepos = s.epos[w];
+                    nout = s.stop_at[w];
+                    kpos = s.stop_pos[w];
+                }
+            const int kstop = ks == 0x7fffffff ? 0 : ks & 7, kthread = ks >> 3;
+            // ---- the output words: literals, history, distances
+            const int lead = op & 3;  // bytes of the first word written by earlier steps
+            const int lo = max(ring_lo, op + kStage + 4 - kRing);  // not overwritten by this step
+            const int ngroup = nout > 0 ? (lead + nout + 3) >> 2 : 0;
+            for (int g = tid; g < ngroup; g += kDecThreads) {
+                const int i0 = 4 * g - lead;  // step-relative position of the word's first byte
+                // the sequence that holds byte max(i0, 0): its warp, then within it
+                int k = 0, sum = 0;
+#pragma unroll
+                for (int w = 0; w < kDecWarps - 1; ++w) {
+                    sum += s.bytes[w];
+                    if (sum <= i0) k = 32 * (w + 1);
+                }
+#pragma unroll
+                for (int step = 16; step; step >>= 1)
+                    if ((int)s.first[k + step] <= i0) k += step;
+                const int4 A = s.seq[k], B = s.seq[k + 1];
+                const int nextb = k + 1 < nthis ? B.x : 0x7fffffff;
+                uint32_t word = i0 < 0 ? *reinterpret_cast<const uint32_t *>(ring + ((op + i0) & kMask)) : 0u;
+                uint32_t d[4], v[4];
+                unsigned far = 0;  // bytes that lie in global memory (rare)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int i = i0 + j;
+                    const bool second = i >= nextb;
+                    const int lend = second ? B.y : A.y, lsrc = second ? B.z : A.z, f = second ? B.w : A.w;
+                    const bool lit = i < lend, live = i >= 0 && i < nout, here = live && (lit || f > i);
+                    const int x = op + i - f, p = i + lsrc - base;
+                    d[j] = live && !here ? (uint32_t)f : 0u;
+                    const bool near = lit ? p < kDecStage : x >= lo;
+                    v[j] = 0;
+                    if (here && near) v[j] = lit ? ib[p] : ring[x & kMask];
+                    if (here && !near) far |= 1u << j;
+                    if (here) word &= ~(0xffu << (8 * j));
+                }
+                while (far) {
+                    const int j = __ffs(far) - 1, i = i0 + j;
+                    far &= far - 1;
+                    const bool second = i >= nextb;
+                    const int lend = second ? B.y : A.y, lsrc = second ? B.z : A.z, f = second ? B.w : A.w;
+                    const uint32_t b = i < lend ? __ldg(src + i + lsrc) : old_byte(src, dst, hl, op + i - f);
+                    word |= b << (8 * j);
+                }
+                word |= v[0] | v[1] << 8 | v[2] << 16 | v[3] << 24;
+                *reinterpret_cast<uint32_t *>(ring + ((op + i0) & kMask)) = word;
+                reinterpret_cast<uint2 *>(s.dist)[g] = make_uint2(d[0] | d[1] << 16, d[2] | d[3] << 16);
+            }
+            __syncthreads();
+            // ---- the bytes that copy bytes of this step: along the distances to
+            // a written byte (a byte's own distance only ever grows towards it)
+            for (int g = tid; g < ngroup; g += kDecThreads) {
+                const uint2 dw = reinterpret_cast<const uint2 *>(s.dist)[g];
+                if ((dw.x | dw.y) == 0u) continue;
+                volatile uint16_t *dist = s.dist;
+                const int i = 4 * g;  // counted from the first word
+                const uint32_t e0 = dw.x & 0xffffu, e1 = dw.x >> 16, e2 = dw.y & 0xffffu, e3 = dw.y >> 16;
+                // the four bytes hop together; a byte that has arrived meets 0
+                // (one without a distance meets itself)
+                int x0 = i - (int)e0, x1 = i + 1 - (int)e1, x2 = i + 2 - (int)e2, x3 = i + 3 - (int)e3;
+                for (;;) {
+                    const uint32_t a0 = dist[x0], a1 = dist[x1], a2 = dist[x2], a3 = dist[x3];
+                    if (!(a0 | a1 | a2 | a3)) break;
+                    x0 -= (int)a0;
+                    x1 -= (int)a1;
+                    x2 -= (int)a2;
+                    x3 -= (int)a3;
+                    if (a0) dist[i] = (uint16_t)(i - x0);
+                    if (a1) dist[i + 1] = (uint16_t)(i + 1 - x1);
+                    if (a2) dist[i + 2] = (uint16_t)(i + 2 - x2);
+                    if (a3) dist[i + 3] = (uint16_t)(i + 3 - x3);
+                }
+                const int o = op - lead;
+                const uint8_t v0 = ring[(o + x0) & kMask], v1 = ring[(o + x1) & kMask], v2 = ring[(o + x2) & kMask],
+                              v3 = ring[(o + x3) & kMask];
+                if (e0) ring[(o + i) & kMask] = v0;
+                if (e1) ring[(o + i + 1) & kMask] = v1;
+                if (e2) ring[(o + i + 2) & kMask] = v2;
+                if (e3) ring[(o + i + 3) & kMask] = v3;
+            }
+            __syncthreads();
+            {
+                const int r = op & kMask, n1 = min(nout, kRing - r);
+                flush(dst + op, ring, r, n1, tid, kDecThreads);
+                if (nout > n1) flush(dst + op + n1, ring, 0, nout - n1, tid, kDecThreads);
+            }
+            // ---- advance
+            op += nout;
+            if (kstop == 0) {
+                s0 = base + after;
+            } else if (kstop == 1) {
+                done = true;
+            } else if (kstop == 2) {
+                err = kepos;
+            } else if (kstop == 4 && kthread > 0) {
+                s0 = base + kpos;
+            } else {
+                // a sequence with long length fields or a long output, decoded serially
+                int ip = base + kpos;
+                __syncthreads();  // the flushed output
+                const int token = __ldg(src + ip);
+                ++ip;
+                long long ll = token >> 4;
+                if (ll == 15) ll += get_len(src, ip, iend, lane);
+                if (ll > (long long)(oend - op - kMfLimit) || ll > (long long)(iend - ip - (2 + 1 + kLastLiterals))) {
+                    if (ll > (long long)(oend - op) || ll != (long long)(iend - ip)) {
+                        err = ip;
+                    } else {
+                        lit_run(op, ip, (int)ll);
+                        op += (int)ll;
+                        done = true;
+                    }
+                } else {
+                    lit_run(op, ip, (int)ll);
+                    op += (int)ll;
+                    ip += (int)ll;
+                    const int o = (int)__ldg(src + ip) | ((int)__ldg(src + ip + 1) << 8);
+                    ip += 2;
+                    if (o == 0 || o > op) {
+                        err = ip;
+                    } else {
+                        long long m = token & 15;
+                        if (m == 15) m += get_len(src, ip, iend - (kLastLiterals + 1), lane);
+                        m += kMinMatch;
+                        if (m > (long long)(oend - op - kLastLiterals)) {
+                            err = ip;
+                        } else {
+                            __syncthreads();
+                            for (int k = tid; k < (int)m; k += kDecThreads)
+                                dst[op + k] = old_byte(src, dst, hl, op - o + msrc(k, o, (int)m));
+                            op += (int)m;
+                            s0 = ip;
+                            ring_lo = op;  // written around the ring
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        if (tid == 0) out_len[c] = err ? -err : op;
+    }
+}
+
+// One warp per chunk, for many chunks. The decoder reads a window of kWin input bytes starting
 // at the current sequence. Every lane decodes the token at 4 candidate
 // positions as if a sequence started there (literal length, offset, match
 // length, position of the next token); only the candidates reachable from
@@ -635,12 +1178,12 @@ __device__ __forceinline__ long long get_len(const uint8_t *src, int &ip, int li
 // memory) let lane k find the k-th sequence directly. Candidates whose
 // length fields run longer than kFastExt continuation bytes are flagged
 // and decoded serially when the chain reaches them.
-constexpr int kWin = 128, kFastExt = 8, kExit = kWin;
-// Output ring per warp: the last kRing bytes of output. A window adds at
-// most kStage bytes, so at least kRing - kStage bytes of history stay
+constexpr int kExit = kWin;
+// Output ring per warp: the last kRing1 bytes of output. A window adds at
+// most kStage1 bytes, so at least kRing1 - kStage1 bytes of history stay
 // readable while it is written (about 99% of match sources in block-record
 // chunks lie within 3 KB).
-constexpr int kRing = 4096, kMask = kRing - 1, kStage = 1024;
+constexpr int kRing1 = 4096, kMask1 = kRing1 - 1, kStage1 = 1024;
 constexpr int kTermIn = 1 << 16, kSlow = 1 << 17;  // flags above the 16-bit offset
 
 // Continuation bytes like get_len, at most kFastExt of them: false if the
@@ -666,25 +1209,7 @@ __device__ __forceinline__ void copy_lit(uint8_t *ring, int o, const uint8_t *s,
     for (int j = 0; j < 8; ++j) b[j] = j < n ? __ldg(s + j) : (uint8_t)0;
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-        if (j < n) ring[(o + j) & kMask] = b[j];
-}
-
-// Byte k of a match at output ms comes from ms - off + (k mod off): the
-// byte-serial copy repeats the first `off` bytes when off < length.
-__device__ __forceinline__ int msrc(int k, int off, int ml) { return off >= ml ? k : k % off; }
-
-// Byte planes 1 and 2 of a record chunk that the decoder left in its input
-// (a literal run it did not copy): output [out, out + len) is input
-// [in, in + len); len 0: none.
-struct LzHole {
-    int out = 0, len = 0, in = 0;
-};
-
-// Output byte x from global memory: from the input inside the hole, else
-// from the output (via L2).
-__device__ __forceinline__ uint8_t old_byte(const uint8_t *src, const uint8_t *dst, const LzHole &h, int x)
-{
-    return (unsigned)(x - h.out) < (unsigned)h.len ? __ldg(src + h.in + (x - h.out)) : __ldcg(dst + x);
+        if (j < n) ring[(o + j) & kMask1] = b[j];
 }
 
 // Output byte x, x < the window's start: from the ring when it is still
@@ -692,7 +1217,7 @@ __device__ __forceinline__ uint8_t old_byte(const uint8_t *src, const uint8_t *d
 __device__ __forceinline__ uint8_t out_byte(const uint8_t *ring, const uint8_t *src, const uint8_t *dst,
                                             const LzHole &h, int x, int lo)
 {
-    return x >= lo ? ring[x & kMask] : old_byte(src, dst, h, x);
+    return x >= lo ? ring[x & kMask1] : old_byte(src, dst, h, x);
 }
 
 // ml <= 8 bytes of a match at ms whose sources lie before the window and
@@ -703,12 +1228,12 @@ __device__ __forceinline__ void copy_match(uint8_t *ring, int ms, int off, int m
     int r = 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        b[j] = j < ml ? ring[(ms - off + r) & kMask] : (uint8_t)0;
+        b[j] = j < ml ? ring[(ms - off + r) & kMask1] : (uint8_t)0;
         r = r + 1 == off ? 0 : r + 1;
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-        if (j < ml) ring[(ms + j) & kMask] = b[j];
+        if (j < ml) ring[(ms + j) & kMask1] = b[j];
 }
 
 // ml <= 8 bytes of a match at ms whose sources all lie before lo (in global
@@ -725,22 +1250,7 @@ __device__ __forceinline__ void copy_match_old(uint8_t *ring, int ms, int off, i
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j)
-        if (j < ml) ring[(ms + j) & kMask] = b[j];
-}
-
-// n bytes of the ring starting at ring offset r (r + n <= kRing) to d (any
-// alignment): 4-byte stores once d is aligned.
-__device__ __forceinline__ void flush(uint8_t *d, const uint8_t *ring, int r, int n, int lane)
-{
-    int h = (int)((4 - (reinterpret_cast<uintptr_t>(d) & 3)) & 3);
-    if (h > n) h = n;
-    if (lane < h) d[lane] = ring[r + lane];
-    const int nw = (n - h) >> 2, b = r + h, sh = 8 * (b & 3);
-    const uint32_t *sw = reinterpret_cast<const uint32_t *>(ring) + (b >> 2);
-    uint32_t *dw = reinterpret_cast<uint32_t *>(d + h);
-    for (int i = lane; i < nw; i += 32) dw[i] = sh ? __funnelshift_r(sw[i], sw[i + 1], sh) : sw[i];
-    const int t = (n - h) & 3;
-    if (lane < t) d[h + 4 * nw + lane] = ring[b + 4 * nw + lane];
+        if (j < ml) ring[(ms + j) & kMask1] = b[j];
 }
 
 __global__ void __launch_bounds__(128)
@@ -751,7 +1261,7 @@ lz4_decode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
     __shared__ int4 cand_all[4][kWin];           // (literal start, literal length, match length, flags)
     __shared__ int next_all[4][kWin];            // input position after the candidate's sequence
     __shared__ __align__(16) uint8_t jump_all[4][5][kWin + 4];  // T_b; kExit: leaves the window
-    __shared__ __align__(16) uint8_t ring_all[4][kRing + 16];  // recent output (16 bytes of slack)
+    __shared__ __align__(16) uint8_t ring_all[4][kRing1 + 16];  // recent output (16 bytes of slack)
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     int4 *cand = cand_all[wib];
     int *nextp = next_all[wib];
@@ -933,7 +1443,7 @@ lz4_decode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
             const int kepos = __shfl_sync(0xffffffffu, epos, ks & 31);
             // the window's output is staged in shared memory: sequences that
             // do not fit go to the serial path
-            const unsigned fb = __ballot_sync(0xffffffffu, member && incl > kStage);
+            const unsigned fb = __ballot_sync(0xffffffffu, member && incl > kStage1);
             if (fb && __ffs(fb) - 1 <= ks) {
                 ks = __ffs(fb) - 1;
                 kstop = 3;
@@ -950,7 +1460,7 @@ lz4_decode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
                 const int o0 = __shfl_sync(0xffffffffu, opl, who);
                 const int x0 = __shfl_sync(0xffffffffu, q.x, who);
                 const int n0 = __shfl_sync(0xffffffffu, q.y, who);
-                for (int k = lane; k < n0; k += 32) ring[(o0 + k) & kMask] = __ldg(src + x0 + k);
+                for (int k = lane; k < n0; k += 32) ring[(o0 + k) & kMask1] = __ldg(src + x0 + k);
             }
             // matches whose sources lie before the window and are still in
             // the ring are copied by their lane; then, in rounds, every
@@ -958,7 +1468,7 @@ lz4_decode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
             // match still to do (so that all of it is written) is copied by
             // its lane, and when there is none, that first match replays
             // with the whole warp (long matches, sources in global memory)
-            const int lo = max(ring_lo, op + kStage - kRing);  // not overwritten by this window
+            const int lo = max(ring_lo, op + kStage1 - kRing1);  // not overwritten by this window
             const bool fast_ring = mat && q.z <= 8 && ms - off + min(q.z, off) <= op && ms - off >= lo;
             const bool fast_old = mat && q.z <= 8 && ms - off + min(q.z, off) <= lo;
             const bool fast = fast_ring || fast_old;
@@ -985,7 +1495,7 @@ lz4_decode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
                     const int l0 = __shfl_sync(0xffffffffu, q.z, who);
                     for (int k = lane; k < l0; k += 32) {
                         const int x = m0 - o0 + msrc(k, o0, l0);
-                        ring[(m0 + k) & kMask] = out_byte(ring, src, dst, hl, x, lo);
+                        ring[(m0 + k) & kMask1] = out_byte(ring, src, dst, hl, x, lo);
                     }
                 }
                 __syncwarp();
@@ -993,9 +1503,9 @@ lz4_decode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
             const int nout = kstop == 1 ? __shfl_sync(0xffffffffu, opl + q.y, ks & 31) - op
                                         : (ks > 0 ? __shfl_sync(0xffffffffu, incl, ks - 1) : 0);
             {
-                const int r = op & kMask, n1 = min(nout, kRing - r);
-                flush(dst + op, ring, r, n1, lane);
-                if (nout > n1) flush(dst + op + n1, ring, 0, nout - n1, lane);
+                const int r = op & kMask1, n1 = min(nout, kRing1 - r);
+                flush(dst + op, ring, r, n1, lane, 32);
+                if (nout > n1) flush(dst + op + n1, ring, 0, nout - n1, lane, 32);
             }
             __syncwarp();
             // ---- advance
@@ -1009,7 +1519,7 @@ lz4_decode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
                 int ip = __shfl_sync(0xffffffffu, s0 + pos, ks & 31);
                 const int token = src[ip++];
                 long long ll = token >> 4;
-                if (ll == 15) ll += get_len(src, ip, iend);
+                if (ll == 15) ll += get_len(src, ip, iend, lane);
                 if (ll > (long long)(oend - op - kMfLimit) || ll > (long long)(iend - ip - (2 + 1 + kLastLiterals))) {
                     if (ll > (long long)(oend - op) || ll != (long long)(iend - ip)) {
                         err = ip;
@@ -1028,7 +1538,7 @@ lz4_decode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
                         err = ip;
                     } else {
                         long long m = token & 15;
-                        if (m == 15) m += get_len(src, ip, iend - (kLastLiterals + 1));
+                        if (m == 15) m += get_len(src, ip, iend - (kLastLiterals + 1), lane);
                         m += kMinMatch;
                         if (m > (long long)(oend - op - kLastLiterals)) {
                             err = ip;
@@ -1051,39 +1561,6 @@ lz4_decode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
         if (lane == 0) out_len[c] = err ? -err : op;
         __syncwarp();
     }
-}
-
-// n bytes from s to d by the CTA: bytes until d is 16-byte aligned, then
-// 16-byte stores (each built from five 4-byte loads with funnel shifts), then
-// the tail. Wide stores matter when the destination is host memory written
-// over the CPU-GPU link. Reads up to 4 bytes past s + n.
-__device__ __forceinline__ void cta_copy(uint8_t *__restrict__ d, const uint8_t *__restrict__ s, int n)
-{
-    if (n <= 0) return;
-    int h = (int)((16 - (reinterpret_cast<uintptr_t>(d) & 15)) & 15);
-    if (h > n) h = n;
-    if ((int)threadIdx.x < h) d[threadIdx.x] = s[threadIdx.x];
-    const uint8_t *s2 = s + h;
-    uint4 *dw = reinterpret_cast<uint4 *>(d + h);
-    const int m = n - h, nwd = m >> 4;
-    const uint32_t sa = (uint32_t)(reinterpret_cast<uintptr_t>(s2) & 3);
-    const uint32_t *sw = reinterpret_cast<const uint32_t *>(s2 - sa);
-    for (int i = threadIdx.x; i < nwd; i += blockDim.x) {
-        const uint32_t *q = sw + 4 * i;
-        const uint32_t a0 = q[0], a1 = q[1], a2 = q[2], a3 = q[3], a4 = sa ? q[4] : 0u;
-        uint4 v;
-        if (sa) {
-            v.x = __funnelshift_r(a0, a1, 8 * sa);
-            v.y = __funnelshift_r(a1, a2, 8 * sa);
-            v.z = __funnelshift_r(a2, a3, 8 * sa);
-            v.w = __funnelshift_r(a3, a4, 8 * sa);
-        } else {
-            v = make_uint4(a0, a1, a2, a3);
-        }
-        dw[i] = v;
-    }
-    const int t = m & 15;
-    if ((int)threadIdx.x < t) d[h + 16 * nwd + threadIdx.x] = s2[16 * nwd + threadIdx.x];
 }
 
 // One CTA per chunk: the chunk's bytes to dst + dst_off[c]. With `hole`
@@ -1112,6 +1589,15 @@ __global__ void gather_kernel(const uint8_t *__restrict__ src, const long long *
 }  // namespace cz
 
 using namespace cz;
+
+static int sm_count()
+{
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
+                                                   cudaSuccess)
+        sms = 1;
+    return sms;
+}
 
 // kLzWarps chunks per CTA; 16 (512 threads, ~123 KB of shared memory)
 // takes an SM, so that CTAs of this kernel and the wavelet kernel, which
@@ -1154,14 +1640,7 @@ static cudaError_t launch_enc_e(const uint8_t *in, const long long *in_off, cons
 // that every CTA width writes the same bytes: 768 positions when all chunks
 // fit on the SMs at once with 4 chunks per CTA (7 CTAs of 4 warps per SM),
 // else 512.
-static int window_for(int nchunks)
-{
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
-                                                   cudaSuccess)
-        sms = 1;
-    return (long long)nchunks <= 28LL * sms ? kWinLarge : kWinSmall;
-}
+static int window_for(int nchunks) { return (long long)nchunks <= 28LL * sm_count() ? kWinLarge : kWinSmall; }
 
 template <int W, bool SEQ>
 static cudaError_t launch_enc(const uint8_t *in, const long long *in_off, const int *in_len, int nchunks,
@@ -1200,12 +1679,31 @@ cudaError_t cz_launch_lz77_parse(const uint8_t *in, const long long *in_off, con
     return launch_enc<4, true>(in, in_off, in_len, nchunks, seq, seq_off, seq_bytes, records, grid, st, nullptr, effort);
 }
 
+// A CTA per chunk finishes a chunk 3 to 4 times sooner than a warp, but
+// executes about 1.5 times the instructions: it is the faster one until the
+// warps of one-warp chunks fill the SMs. Measured (ms, CTA / warp per chunk):
+// 512 chunks of a 256^3 field 0.36 / 0.59, 1 024 of 256x256x512 0.38 / 0.46,
+// 1 728 of 384^3 0.71 / 0.56, 2 048 of 256x512x512 0.51 / 0.39; 274 chunks
+// of 15 records 2.03 / 7.24, 1 024 of 4 records 1.58 / 2.13.
+constexpr int kWideChunksPerSm = 8;
+
 cudaError_t cz_launch_lz4_decode(const uint8_t *in, const long long *in_off, const int *in_len, int nchunks,
-                                 uint8_t *out, const long long *out_off, const int *out_cap, int *out_len, int grid,
+                                 uint8_t *out, const long long *out_off, const int *out_cap, int *out_len,
                                  cudaStream_t st, int4 *hole)
 {
     if (nchunks <= 0) return cudaSuccess;
-    lz4_decode_kernel<<<grid, 128, 0, st>>>(in, in_off, in_len, nchunks, out, out_off, out_cap, out_len, hole);
+    const int sms = sm_count();
+    if (nchunks <= kWideChunksPerSm * sms) {
+        const int sm = (int)sizeof(LzDecShared);
+        const cudaError_t e =
+            cudaFuncSetAttribute(lz4_decode_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+        if (e != cudaSuccess) return e;
+        lz4_decode_wide_kernel<<<std::min(nchunks, 3 * sms), kDecThreads, sm, st>>>(in, in_off, in_len, nchunks, out,
+                                                                                   out_off, out_cap, out_len, hole);
+    } else {
+        lz4_decode_kernel<<<std::min((nchunks + 3) / 4, 8 * sms), 128, 0, st>>>(in, in_off, in_len, nchunks, out, out_off,
+                                                                               out_cap, out_len, hole);
+    }
     return cudaGetLastError();
 }
 
