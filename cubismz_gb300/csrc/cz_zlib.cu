@@ -16,16 +16,22 @@
 // and OR-writes into a per-warp ring of words that is flushed to the output
 // with word stores. zlib header 78 9C, Adler-32 by a warp reduction.
 //
-// Decoder (inflate_kernel): one warp per chunk. Lane 0 reads the header and
-// the blocks (stored, fixed Huffman, dynamic Huffman) and decodes symbols
-// with 10-bit lookup tables (longer codes by the canonical walk); literals
-// go straight to the output, matches into a batch. The warp then writes all
-// of the batch's match bytes in parallel, each following its source back
-// through earlier matches of the batch to a byte written before. The Adler-32
-// of the output is a warp reduction, checked against the trailer. Malformed
-// input (bad header, code lengths, symbols, distances past the start, output
-// past the capacity, truncated input or a wrong checksum) gives a negative
-// length; every read and write is bounds checked.
+// Decoder (inflate_kernel): two warps per chunk, because a DEFLATE stream is
+// one serial chain of bits and that chain is what bounds it. Lane 0 of the
+// first warp does nothing but decode: headers, and symbols from lookup tables
+// (which the whole warp builds) into records of up to six literals and a
+// match, without a look at positions, limits or bytes. The second warp takes
+// 32 records at a time: a scan gives their output positions, every test is
+// made there, literals and matches go to a ring in shared memory (a match per
+// lane as soon as its source is written) that is flushed with word stores.
+// Stored blocks are copied by the warp. The Adler-32 of the output is a sum
+// over both warps, checked against the trailer. Malformed input (bad header,
+// code lengths, symbols, distances past the start, output past the capacity,
+// truncated input or a wrong checksum) gives a negative length; every read and
+// write is bounds checked. Zlib stage of
+// 512 one-record chunks (256^3): 10.2 -> 3.6 ms; a record of the queue takes
+// about 360 cycles, 70 dependent instructions of one lane.
+#include "cz_bytes.cuh"
 #include "cz_codec.h"
 #include "cz_deflate.cuh"
 
@@ -33,7 +39,10 @@ namespace cz {
 
 using namespace zl;
 
-constexpr int kZBatch = 128;  // matches per batch
+constexpr int kZBatch = 128;  // records per batch
+// The ring holds what 32 records can add (six literals and a match of 258
+// bytes each) and at least 7 KB of history; older sources come from the output.
+constexpr int kZRing = 16384, kZRingM = kZRing - 1, kZGroup = 32 * (6 + 258);
 
 // n bytes from s to d by the warp (4-byte stores once d is aligned); every
 // load is of an aligned word holding at least one byte of the run.
@@ -54,109 +63,317 @@ __device__ __forceinline__ void run_copy(uint8_t *d, const uint8_t *s, int n, in
     if (lane < t) d[4 * nw + lane] = s[4 * nw + lane];
 }
 
-__global__ void __launch_bounds__(32)
+// Adler-32 sums of n bytes at d (4-byte aligned) by threads t of nt: the sum
+// of the bytes and of (n - i) times byte i. CG: read past L1 (bytes the
+// kernel wrote).
+template <bool CG>
+__device__ __forceinline__ void adler_sums(const uint8_t *d, int n, int t, int nt, unsigned long long &sa,
+                                           unsigned long long &sb)
+{
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(d);
+    sa = sb = 0;
+    const int nw = n >> 2;
+#pragma unroll 8
+    for (int i = t; i < nw; i += nt) {
+        const uint32_t v = CG ? __ldcg(w + i) : w[i];
+        const unsigned s = __dp4a(v, 0x01010101u, 0u);
+        sa += s;
+        sb += (unsigned long long)(unsigned)(n - 4 * i) * s - __dp4a(v, 0x03020100u, 0u);
+    }
+    const int i = 4 * nw + t;
+    if (i < n) {
+        const unsigned v = CG ? __ldcg(d + i) : d[i];
+        sa += v;
+        sb += (unsigned long long)(n - i) * v;
+    }
+}
+__device__ __forceinline__ unsigned adler_of(unsigned long long sa, unsigned long long sb, int n)
+{
+    return ((unsigned)(((unsigned long long)n + sb) % 65521ull) << 16) | (unsigned)((1 + sa) % 65521ull);
+}
+
+// zl::build by the warp. cnt: 2 x 16 words of scratch.
+__device__ bool warp_build(Huff &h, const unsigned char *len, int n, bool lit, unsigned *cnt, int lane)
+{
+    if (lane < 16) cnt[lane] = 0;
+    __syncwarp();
+    for (int s = lane; s < n; s += 32)
+        if (len[s]) atomicAdd(&cnt[len[s]], 1u);
+    __syncwarp();
+    if (lane < 16) h.count[lane] = (unsigned short)cnt[lane];
+    __syncwarp();
+    if (!lengths_ok(h.count, false)) return false;
+    // first code and symbol offset of every length (lane l: length l)
+    unsigned first = 0, offs = 0, code = 0, sum = 0;
+    for (int l = 1; l <= kMaxBits; ++l) {
+        code = (code + (l > 1 ? cnt[l - 1] : 0u)) << 1;
+        if (lane == l) {
+            first = code;
+            offs = sum;
+        }
+        sum += cnt[l];
+    }
+    __syncwarp();
+    if (lane < 16) cnt[16 + lane] = offs;  // next place per length
+    if (lane >= 1 && lane <= kMaxBits) {
+        h.lim[lane] = (unsigned short)((first + cnt[lane]) << (kMaxBits - lane));
+        h.shift[lane] = (short)((int)offs - (int)first);
+    }
+    __syncwarp();
+    for (int s0 = 0; s0 < n; s0 += 32) {  // symbols in order
+        const int s = s0 + lane, l = s < n ? len[s] : 0;
+        const unsigned same = __match_any_sync(0xffffffffu, l);
+        const int rank = __popc(same & ((1u << lane) - 1u));
+        const unsigned at = cnt[16 + l];
+        if (l) h.sym[at + rank] = (unsigned short)s;
+        __syncwarp();
+        if (l && rank == 0) cnt[16 + l] = at + __popc(same);
+        __syncwarp();
+    }
+    // the table by index: a code of length l is the smallest l whose codes
+    // end above the index's first l bits (canonical codes grow with length)
+    unsigned lim[kFastBits + 1], shift[kFastBits + 1];  // per length: end of its codes on kFastBits bits; symbol - code
+#pragma unroll
+    for (int l = 1; l <= kFastBits; ++l) {
+        const unsigned f = __shfl_sync(0xffffffffu, first, l);
+        lim[l] = (f + cnt[l]) << (kFastBits - l);
+        shift[l] = __shfl_sync(0xffffffffu, offs, l) - f;
+    }
+#pragma unroll 1
+    for (int i = lane; i < 1 << kFastBits; i += 32) {
+        const unsigned v = __brev((unsigned)i) >> (32 - kFastBits);
+        int l = 0;
+        unsigned at = 0;
+#pragma unroll
+        for (int k = kFastBits; k >= 1; --k)
+            if (v < lim[k]) {
+                l = k;
+                at = (v >> (kFastBits - k)) + shift[k];
+            }
+        unsigned e = 0;
+        if (l) {
+            const int s = h.sym[at];
+            e = lit ? lit_entry(s, l) : dist_entry(s, l);
+        }
+        h.fast[i] = e;
+    }
+    __syncwarp();
+    if (lit) {
+        // a combined entry keeps its first literal, so any order will do
+        for (int i = lane; i < 1 << kFastBits; i += 32) h.fast[i] = pair_entry(h.fast, i);
+        __syncwarp();
+    }
+    return true;
+}
+
+template <int ID>
+__device__ __forceinline__ void bar_arrive64()
+{
+    asm volatile("bar.arrive %0, 64;" ::"n"(ID) : "memory");
+}
+template <int ID>
+__device__ __forceinline__ void bar_sync64()
+{
+    asm volatile("bar.sync %0, 64;" ::"n"(ID) : "memory");
+}
+
+__global__ void __launch_bounds__(64, 7)
 inflate_kernel(const uint8_t *__restrict__ in, const long long *in_off, const int *in_len, int nchunks,
                uint8_t *__restrict__ out, const long long *out_off, const int *out_cap, int *out_len)
 {
     __shared__ Huff lit, dist;
     __shared__ unsigned char lens[320];
-    __shared__ int batch[kZBatch][3];  // matches: output position, length, distance
-    __shared__ int mpre[kZBatch + 1];  // exclusive prefix of the match lengths
-    __shared__ int s_state[4];         // matches in the batch, error, done, Adler-32 of the trailer
-    __shared__ long long s_run[3];     // a stored block: input position, output position, length
-    const int lane = threadIdx.x;
+    __shared__ unsigned scratch[32];
+    __shared__ uint4 queue[2][kZBatch];  // records
+    __shared__ int s_state[2][4];        // per batch: records, last one of the chunk, a stored block's input position and bytes
+    __shared__ int s_end[4];             // error of the decoder and of the writer, Adler-32 of the trailer, output size
+    __shared__ unsigned long long s_sum[2];
+    __shared__ __align__(16) uint8_t ring[kZRing + 16];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
         const uint8_t *src = in + in_off[c];
         uint8_t *dst = out + out_off[c];
-        const long long oend = out_cap[c];
-        Inflater z;  // lane 0's decoder state, kept in registers across batches
-        if (lane == 0) z.start(src, in_len[c]);
-        for (;;) {
-            if (lane == 0) {
-                s_state[0] = z.step(dst, oend, batch, kZBatch, lit, dist, lens);
-                s_state[1] = z.err;
-                s_state[2] = z.done();
-                s_run[0] = z.run_src;
-                s_run[1] = z.run_dst;
-                s_run[2] = z.err ? 0 : z.run_n;
+        const int oend = out_cap[c];
+        // barriers 1, 2: batch k is full; 3, 4: batch k is free again
+        if (warp == 0) {
+            Inflater z;  // lane 0's decoder state, kept in registers
+            if (lane == 0) z.start(src, in_len[c]);
+            uint32_t it = 0;
+            for (int last = 0; !last; ++it) {
+                const int k = it & 1;
+                if (it >= 2) {
+                    if (k) bar_sync64<4>();
+                    else bar_sync64<3>();
+                }
+                int n = 0, want = 0;
+                if (lane == 0) z.run_n = 0;
+                do {
+                    want = 0;
+                    if (lane == 0) {
+                        while (!z.err && n < kZBatch) {
+                            if (!z.in_block) {
+                                if (z.final_block || z.block_header(lit.fast, lens)) break;
+                                if (z.btype != 0) {
+                                    want = z.nlen | z.ndist << 16;
+                                    break;
+                                }
+                                (void)z.stored_run();
+                                break;
+                            }
+                            while (n < kZBatch && z.in_block && !z.err) {
+                                const Record r = z.record(lit, dist);
+                                queue[k][n++] = make_uint4(r.e[0], r.e[1], r.e[2], r.m);
+                            }
+                            if (!z.err && z.b.over()) z.err = 14;
+                        }
+                    }
+                    __syncwarp();
+                    want = __shfl_sync(0xffffffffu, want, 0);
+                    if (want) {
+                        const int nlen = want & 0xffff, ndist = want >> 16;
+                        const bool ok = warp_build(lit, lens, nlen, true, scratch, lane);
+                        const bool ok2 = ok && warp_build(dist, lens + nlen, ndist, false, scratch, lane);
+                        if (lane == 0 && !ok2) z.err = ok ? 10 : 9;
+                        __syncwarp();
+                    }
+                } while (want);
+                if (lane == 0) {
+                    last = z.err || z.done();
+                    if (last) {
+                        if (!z.err) s_end[2] = (int)z.trailer();
+                        s_end[0] = z.err;
+                    }
+                    s_state[k][0] = n;
+                    s_state[k][1] = last;
+                    s_state[k][2] = (int)z.run_src;
+                    s_state[k][3] = (int)z.run_n;
+                }
+                last = __shfl_sync(0xffffffffu, last, 0);
+                if (k) bar_arrive64<2>();
+                else bar_arrive64<1>();
             }
-            __syncwarp();
-            if (s_run[2] > 0) run_copy(dst + s_run[1], src + s_run[0], (int)s_run[2], lane);
-            // the batch's match bytes, all in parallel: byte k of a match at p
-            // with distance d is out[p - d + (k mod d)]; where that lies in an
-            // earlier match of the batch (or this one) the source is followed
-            // back until it is a byte written before the replay (a literal of
-            // the batch or earlier output)
-            const int n = s_state[0];
-            {
-                int incl = 0;
-                for (int i0 = 0; i0 < n; i0 += 32) {  // exclusive prefix of the match lengths (warp-uniform loop)
-                    const int i = i0 + lane;
-                    const int v = i < n ? batch[i][1] : 0;
-                    int x = v;
+            // every batch is written before the chunk ends
+            for (uint32_t j = it < 2 ? 0 : it - 2; j < it; ++j) {
+                if (j & 1) bar_sync64<4>();
+                else bar_sync64<3>();
+            }
+        } else {
+            int op = 0, ring_lo = 0, err = 0;  // output before ring_lo is not in the ring
+            for (uint32_t it = 0, last = 0; !last; ++it) {
+                const int kb = it & 1;
+                if (kb) bar_sync64<2>();
+                else bar_sync64<1>();
+                const int n = s_state[kb][0];
+                last = (uint32_t)s_state[kb][1];
+                for (int i0 = 0; i0 < n && !err; i0 += 32) {
+                    const uint4 r = i0 + lane < n ? queue[kb][i0 + lane] : make_uint4(0, 0, 0, 0);
+                    const int c0 = literals(r.x), c1 = literals(r.y), c2 = literals(r.z);
+                    const int nl = c0 + c1 + c2 + (int)(r.w >> 31);
+                    const int len = r.w >> 31 ? 0 : (int)(r.w & 511u), d = len ? (int)(r.w >> 9) : 1;
+                    int incl = nl + len;
 #pragma unroll
                     for (int o = 1; o < 32; o <<= 1) {
-                        const int t = __shfl_up_sync(0xffffffffu, x, o);
-                        if (lane >= o) x += t;
+                        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= o) incl += t;
                     }
-                    if (i < n) mpre[i] = incl + x - v;
-                    incl += __shfl_sync(0xffffffffu, x, 31);
-                }
-                if (lane == 0) mpre[n] = incl;
-            }
-            __syncwarp();
-            const int mtotal = mpre[n];
-            for (int t = lane; t < mtotal; t += 32) {
-                int i = 0;  // match holding byte t of the batch's match bytes
+                    const int total = __shfl_sync(0xffffffffu, incl, 31);
+                    const int at = op + incl - nl - len, p = at + nl;  // the record's literals, its match
+                    const int bad = p > oend ? 15 : len && d > p ? 19 : p + len > oend ? 20 : 0;
+                    const unsigned bb = __ballot_sync(0xffffffffu, bad != 0);
+                    if (bb) {
+                        err = __shfl_sync(0xffffffffu, bad, __ffs(bb) - 1);
+                        break;
+                    }
+                    const int a1 = at + c0, a2 = a1 + c1;
+                    if (c0 > 0) ring[at & kZRingM] = (uint8_t)(r.x >> 8);
+                    if (c0 > 1) ring[(at + 1) & kZRingM] = (uint8_t)(r.x >> 16);
+                    if (c1 > 0) ring[a1 & kZRingM] = (uint8_t)(r.y >> 8);
+                    if (c1 > 1) ring[(a1 + 1) & kZRingM] = (uint8_t)(r.y >> 16);
+                    if (c2 > 0) ring[a2 & kZRingM] = (uint8_t)(r.z >> 8);
+                    if (c2 > 1) ring[(a2 + 1) & kZRingM] = (uint8_t)(r.z >> 16);
+                    if (r.w >> 31) ring[(p - 1) & kZRingM] = (uint8_t)r.w;
+                    __syncwarp();
+                    // matches in rounds: every one whose source ends before the
+                    // output of the first one still to do (so that all of it is
+                    // written) is copied by its lane, long ones by the warp; the
+                    // first one itself always is. Byte k is out[p - d + (k mod d)].
+                    const int lo = max(ring_lo, op + kZGroup - kZRing);  // not overwritten by this group
+                    auto from = [&](int x) -> uint8_t { return x >= lo ? ring[x & kZRingM] : __ldcg(dst + x); };
+                    const int send = p - d + min(len, d);
+                    unsigned todo = __ballot_sync(0xffffffffu, len > 0);
+                    while (todo) {
+                        const int m0 = __shfl_sync(0xffffffffu, p, __ffs(todo) - 1);
+                        const bool go = (todo >> lane & 1u) && send <= m0;
+                        if (go && len <= 32) {
+                            int x = p - d;
+                            for (int k = 0; k < len; k += 4) {
+                                uint8_t v[4];
 #pragma unroll
-                for (int step = 64; step; step >>= 1)
-                    if (i + step < n && mpre[i + step] <= t) i += step;
-                const int y = batch[i][0] + t - mpre[i];
-                int x = y;
-                for (int hop = 0; hop <= n; ++hop) {
-                    int j = 0;  // last match starting at or before x
+                                for (int j = 0; j < 4; ++j) {
+                                    v[j] = k + j < len ? from(x) : (uint8_t)0;
+                                    if (++x == p) x = p - d;
+                                }
 #pragma unroll
-                    for (int step = 64; step; step >>= 1)
-                        if (j + step < n && batch[j + step][0] <= x) j += step;
-                    const int pj = batch[j][0], lj = batch[j][1], dj = batch[j][2];
-                    if (x < pj || x >= pj + lj) break;
-                    x = pj - dj + (dj >= lj ? x - pj : (x - pj) % dj);
+                                for (int j = 0; j < 4; ++j)
+                                    if (k + j < len) ring[(p + k + j) & kZRingM] = v[j];
+                            }
+                        }
+                        for (unsigned lng = __ballot_sync(0xffffffffu, go && len > 32); lng; lng &= lng - 1) {
+                            const int who = __ffs(lng) - 1;
+                            const int pp = __shfl_sync(0xffffffffu, p, who), ll = __shfl_sync(0xffffffffu, len, who);
+                            const int dd = __shfl_sync(0xffffffffu, d, who);
+                            for (int k = lane; k < ll; k += 32)
+                                ring[(pp + k) & kZRingM] = from(pp - dd + (dd >= ll ? k : k % dd));
+                        }
+                        todo &= ~__ballot_sync(0xffffffffu, go);
+                        __syncwarp();
+                    }
+                    const int r0 = op & kZRingM, n1 = min(total, kZRing - r0);
+                    flush(dst + op, ring, r0, n1, lane, 32);
+                    if (total > n1) flush(dst + op + n1, ring, 0, total - n1, lane, 32);
+                    op += total;
+                    __syncwarp();
                 }
-                dst[y] = __ldcg(dst + x);
+                const int rn = s_state[kb][3];
+                if (rn > 0 && !err) {
+                    if (rn > oend - op) {
+                        err = 12;
+                    } else {
+                        run_copy(dst + op, src + s_state[kb][2], rn, lane);
+                        op += rn;
+                        ring_lo = op;  // written around the ring
+                    }
+                }
+                if (last && lane == 0) {
+                    s_end[1] = err;
+                    s_end[3] = op;
+                }
+                if (kb) bar_arrive64<4>();
+                else bar_arrive64<3>();
             }
-            __syncwarp();
-            const int e = s_state[1], dn = s_state[2];
-            __syncwarp();
-            if (e || dn) break;
         }
+        __syncthreads();
         // Adler-32 of the output (A = 1 + sum d_i, B = n + sum (n - i) d_i,
         // mod 65521) against the trailer
-        if (lane == 0) {
-            if (!z.err) s_state[3] = (int)z.trailer();
-            s_state[1] = z.err;
-            s_state[0] = (int)z.op;
-        }
-        __syncwarp();
-        int e = s_state[1];
-        const long long total = s_state[0];
+        int e = s_end[0] ? s_end[0] : s_end[1];
+        const int total = s_end[3];
         if (!e) {
-            unsigned long long sa = 0, sb = 0;
-            for (long long i = lane; i < total; i += 32) {
-                const unsigned v = __ldcg(dst + i);
-                sa += v;
-                sb += (unsigned long long)(total - i) * v;
-            }
+            unsigned long long sa, sb;
+            adler_sums<true>(dst, total, threadIdx.x, 64, sa, sb);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 sa += __shfl_xor_sync(0xffffffffu, sa, o);
                 sb += __shfl_xor_sync(0xffffffffu, sb, o);
             }
-            const unsigned A = (unsigned)((1 + sa) % 65521ull);
-            const unsigned B = (unsigned)(((unsigned long long)total + sb) % 65521ull);
-            if (((B << 16) | A) != (unsigned)s_state[3]) e = 22;
+            if (threadIdx.x == 32) {
+                s_sum[0] = sa;
+                s_sum[1] = sb;
+            }
+            __syncthreads();
+            if (threadIdx.x == 0 && adler_of(sa + s_sum[0], sb + s_sum[1], total) != (unsigned)s_end[2]) e = 22;
         }
-        if (lane == 0) out_len[c] = e ? -e : (int)total;
-        __syncwarp();
+        if (threadIdx.x == 0) out_len[c] = e ? -e : total;
+        __syncthreads();
     }
 }
 
@@ -498,20 +715,15 @@ deflate_kernel(const uint8_t *__restrict__ in, const long long *in_off, const in
             __syncwarp();
             continue;
         }
-        // Adler-32 of the input
-        unsigned long long sa = 0, sbs = 0;
-        for (int i = lane; i < L; i += 32) {
-            const unsigned v = src[i];
-            sa += v;
-            sbs += (unsigned long long)(L - i) * v;
-        }
+        // Adler-32 of the input (chunks start on 4-byte boundaries)
+        unsigned long long sa, sbs;
+        adler_sums<false>(src, L, lane, 32, sa, sbs);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             sa += __shfl_xor_sync(0xffffffffu, sa, o);
             sbs += __shfl_xor_sync(0xffffffffu, sbs, o);
         }
-        const unsigned adler =
-            ((unsigned)(((unsigned long long)L + sbs) % 65521ull) << 16) | (unsigned)((1 + sa) % 65521ull);
+        const unsigned adler = adler_of(sa, sbs, L);
         Ring rg{s.u.ring, reinterpret_cast<uint32_t *>(dst), 16, 0, (int)(out_slot / 4)};
         zl::Bounds bnd;
         bnd.init(src, L, records != 0);
@@ -647,6 +859,6 @@ cudaError_t cz_launch_inflate(const uint8_t *in, const long long *in_off, const 
                               const long long *out_off, const int *out_cap, int *out_len, int grid, cudaStream_t st)
 {
     if (nchunks <= 0) return cudaSuccess;
-    inflate_kernel<<<grid, 32, 0, st>>>(in, in_off, in_len, nchunks, out, out_off, out_cap, out_len);
+    inflate_kernel<<<grid, 64, 0, st>>>(in, in_off, in_len, nchunks, out, out_off, out_cap, out_len);
     return cudaGetLastError();
 }
