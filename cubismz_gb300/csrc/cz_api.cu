@@ -318,7 +318,7 @@ int enqueue(cz_ctx *c, const Job &job, cudaStream_t st, bool marks)
                                      P<long long>(c->lz_off), P<int>(c->lz_len), nchunks, p->shuffle ? 1 : 0,
                                      P<uint8_t>(c->zout),
                                      job.z_slot, P<long long>(c->zoff), P<int>(c->zlen),
-                                     std::max(1, std::min((nchunks + 3) / 4, c->sms * 5)), st));
+                                     std::min(nchunks, c->sms * 4), st));
         CZ_CUDA(c, cz_launch_neg_reduce(P<int>(c->zlen), nchunks, P<int>(c->flag), st));
         gsrc = P<uint8_t>(c->zout);
         gsrc_off = P<long long>(c->zoff);

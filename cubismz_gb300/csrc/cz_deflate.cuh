@@ -1,5 +1,5 @@
 // cz_deflate.cuh -- the serial parts of DEFLATE encoding (RFC 1951), shared
-// by the GPU encoder (cz_zlib.cu, run by one lane per chunk) and the host
+// by the GPU encoder (cz_zlib.cu, by one lane where it does not share them out) and the host
 // test harness: symbol mapping of lengths and distances, Huffman code
 // lengths limited to a maximum length, canonical codes, the run-length
 // coding of the code lengths, the dynamic block header and the exact size of
@@ -215,23 +215,11 @@ CZ_HD long long data_bits(const uint32_t *lf, const uint32_t *df, const uint8_t 
     return b;
 }
 
-// After llen/dlen are set: hlit, hdist, the run-length entries and the
-// code-length code (built serially: 19 symbols). Returns the header bits
-// (block type included), or -1 if the code-length code cannot be built.
-CZ_HD long long dynamic_header(Codes &c)
+// The code-length code from the frequencies cf of its 19 symbols (changed):
+// clen, ccode, hclen. Returns the header bits before the run-length entries
+// (block type included), or -1 if the code cannot be built.
+CZ_HD long long code_length_code(Codes &c, uint32_t *cf)
 {
-    int hl = kLitSyms, hd = kDistSyms;
-    while (hl > 257 && c.llen[hl - 1] == 0) --hl;
-    while (hd > 1 && c.dlen[hd - 1] == 0) --hd;
-    c.hlit = hl;
-    c.hdist = hd;
-    uint8_t all[kLitSyms + kDistSyms];
-    for (int s = 0; s < hl; ++s) all[s] = c.llen[s];
-    for (int s = 0; s < hd; ++s) all[hl + s] = c.dlen[s];
-    c.nrle = rle_lengths(all, hl + hd, c.rle);
-    uint32_t cf[kClSyms];
-    for (int s = 0; s < kClSyms; ++s) cf[s] = 0;
-    for (int i = 0; i < c.nrle; ++i) cf[c.rle[i] & 31]++;
     // symbols by (frequency, symbol), at least two of them
     int sym[kClSyms], m = 0;
     for (int s = 0; s < kClSyms; ++s)
@@ -261,7 +249,28 @@ CZ_HD long long dynamic_header(Codes &c)
     int hc = kClSyms;
     while (hc > 4 && c.clen[cl_order(hc - 1)] == 0) --hc;
     c.hclen = hc;
-    long long bits = 3 + 5 + 5 + 4 + 3 * hc;
+    return 3 + 5 + 5 + 4 + 3 * hc;
+}
+
+// After llen/dlen are set: hlit, hdist, the run-length entries and the
+// code-length code (built serially: 19 symbols). Returns the header bits
+// (block type included), or -1 if the code-length code cannot be built.
+CZ_HD long long dynamic_header(Codes &c)
+{
+    int hl = kLitSyms, hd = kDistSyms;
+    while (hl > 257 && c.llen[hl - 1] == 0) --hl;
+    while (hd > 1 && c.dlen[hd - 1] == 0) --hd;
+    c.hlit = hl;
+    c.hdist = hd;
+    uint8_t all[kLitSyms + kDistSyms];
+    for (int s = 0; s < hl; ++s) all[s] = c.llen[s];
+    for (int s = 0; s < hd; ++s) all[hl + s] = c.dlen[s];
+    c.nrle = rle_lengths(all, hl + hd, c.rle);
+    uint32_t cf[kClSyms];
+    for (int s = 0; s < kClSyms; ++s) cf[s] = 0;
+    for (int i = 0; i < c.nrle; ++i) cf[c.rle[i] & 31]++;
+    long long bits = code_length_code(c, cf);
+    if (bits < 0) return -1;
     for (int i = 0; i < c.nrle; ++i) {
         const int s = c.rle[i] & 31;
         bits += c.clen[s] + rle_extra_bits(s);

@@ -3,18 +3,17 @@
 // CompressionEncoders.h:116-190) and decoder (inflateInit/inflate,
 // CompressionEncoders.h:48-88).
 //
-// Encoder (deflate_kernel): one warp per chunk, fed by the LZ77 parse of the
-// LZ4 encoder run with a 32 KiB window (cz_lz4.cu, SEQ mode). A chunk of
-// shuffled block records gets a DEFLATE block per record mask and byte
-// plane (other chunks one per 64 KiB): per block, the warp counts the
-// symbols of the items that start in it (literal bytes with one
-// shared-memory add per distinct byte of 32; matches of more than 258 bytes
-// in pieces), sorts the used symbols (bitonic, by frequency), one lane
-// builds the length-limited codes (cz_deflate.cuh), and the exact sizes of
-// the stored, fixed and dynamic codings pick the smallest; then 32 items per
-// step (a literal or a match piece each), a warp scan of their bit counts,
-// and OR-writes into a per-warp ring of words that is flushed to the output
-// with word stores. zlib header 78 9C, Adler-32 by a warp reduction.
+// Encoder (deflate_kernel): one CTA per chunk, a warp per DEFLATE block, fed by
+// the LZ77 parse of the LZ4 encoder run with a 32 KiB window (cz_lz4.cu, SEQ
+// mode). A chunk of shuffled block records gets a DEFLATE block per record mask
+// and byte plane (other chunks one per 64 KiB): per block, the warp counts the
+// symbols of the items that start in it (literal bytes; matches of more than
+// 258 bytes in pieces), sorts the used symbols (bitonic, by frequency), builds
+// the length-limited codes (cz_deflate.cuh), and the exact sizes of the
+// stored, fixed and dynamic codings pick the smallest; then 32 sequences per
+// step, a warp scan of their bit counts, and OR-writes into a per-warp ring of
+// words that is flushed to the output with word stores. zlib header 78 9C,
+// Adler-32 by a reduction.
 //
 // Decoder (inflate_kernel): two warps per chunk, because a DEFLATE stream is
 // one serial chain of bits and that chain is what bounds it. Lane 0 of the
@@ -378,8 +377,8 @@ inflate_kernel(const uint8_t *__restrict__ in, const long long *in_off, const in
 }
 
 // ---------------------------------------------------------------- encoder
-constexpr int kZWarps = 4;     // chunks per CTA
-constexpr int kRingW = 512;    // bit-ring words per warp
+constexpr int kZWarps = 5;     // warps per chunk: a record's mask and byte planes are five blocks
+constexpr int kRingW = 1024;   // bit-ring words per warp: 32 short sequences fit (see block_items)
 constexpr int kRingM = kRingW - 1;
 
 struct DeflateWarp {
@@ -394,14 +393,78 @@ struct DeflateWarp {
             uint8_t l[288];
         } b;
     } u;
-    int beg[32], end[32], litpos[32], nlit[32], mstart[32], mlen[32], dist[32], k0[32];
-    int state[4];
+    uint32_t cnt[32];  // scratch of the code construction
 };
+
+// zl::huff_lengths of the n sorted weights in s.u.b.w into s.u.b.l, by the
+// warp: lane 0 only merges (both queues' heads in registers) and takes the
+// depths of the internal nodes; leaves, counts and lengths are shared out.
+__device__ bool warp_huff_lengths(DeflateWarp &s, int n, int maxbits, int lane)
+{
+    auto &b = s.u.b;
+    if (lane < 16) s.cnt[lane] = 0;
+    if (lane == 0) {
+        constexpr uint32_t kNone = 0xffffffffu;
+        int i = 0, j = 0;
+        uint32_t wi = b.w[0], wj = kNone;  // next leaf, next internal node (block counts stay below 2^22)
+        for (int k = 0; k < n - 1; ++k) {
+            uint32_t sum = 0;
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                if (wi <= wj) {  // a leaf goes first among equals, as there is one
+                    b.par[i++] = (uint16_t)(n + k);
+                    sum += wi;
+                    wi = i < n ? b.w[i] : kNone;
+                } else {
+                    b.par[n + j++] = (uint16_t)(n + k);
+                    sum += wj;
+                    wj = j < k ? b.iw[j] : kNone;
+                }
+            }
+            b.iw[k] = sum;
+            if (j == k) wj = sum;
+        }
+        b.dep[2 * n - 2] = 0;
+        for (int x = 2 * n - 3; x >= n; --x) b.dep[x] = (uint16_t)(b.dep[b.par[x]] + 1);  // parents come later
+    }
+    __syncwarp();
+    for (int x = lane; x < n; x += 32) atomicAdd(&s.cnt[min((int)b.dep[b.par[x]] + 1, maxbits)], 1u);
+    __syncwarp();
+    int ok = 1;
+    if (lane == 0) {
+        uint32_t kraft = 0, total = 0;
+        for (int l = 1; l <= maxbits; ++l) kraft += s.cnt[l] << (maxbits - l);
+        while (kraft > (1u << maxbits)) {
+            int l = maxbits - 1;
+            while (l > 0 && s.cnt[l] == 0) --l;
+            if (l == 0 || s.cnt[maxbits] == 0) {
+                ok = 0;
+                break;
+            }
+            s.cnt[maxbits]--;
+            s.cnt[l]--;
+            s.cnt[l + 1] += 2;
+            --kraft;
+        }
+        for (int l = 1; l <= maxbits; ++l) total += s.cnt[l];
+        ok = ok && kraft == (1u << maxbits) && (int)total == n;
+    }
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    __syncwarp();
+    if (!ok) return false;
+    for (int x = lane; x < n; x += 32) {  // longest first
+        int l = maxbits, end = (int)s.cnt[maxbits];
+        while (x >= end) end += (int)s.cnt[--l];
+        b.l[x] = (uint8_t)l;
+    }
+    __syncwarp();
+    return true;
+}
 
 // Code lengths for freq[0..n) into len: the warp sorts the used symbols by
 // (frequency, symbol) -- a bitonic sort of keys weight << 9 | symbol over 512
-// slots (block counts stay below 2^22) -- and lane 0 runs huff_lengths.
-// False if it fails.
+// slots, 32 for the distance code (block counts stay below 2^22). False if it
+// fails.
 __device__ bool warp_code(DeflateWarp &s, const uint32_t *freq, int n, uint8_t *len, int lane)
 {
     auto &b = s.u.b;
@@ -411,7 +474,8 @@ __device__ bool warp_code(DeflateWarp &s, const uint32_t *freq, int n, uint8_t *
     for (int o = 16; o; o >>= 1) used += __shfl_xor_sync(0xffffffffu, used, o);
     // at least two codes: the lowest unused symbols get weight one (never sent)
     int need = used < 2 ? 2 - used : 0;
-    for (int x0 = 0; x0 < 512; x0 += 32) {
+    const int slots = n <= 32 ? 32 : 512;
+    for (int x0 = 0; x0 < slots; x0 += 32) {
         const int x = x0 + lane;
         uint32_t f = x < n ? freq[x] : 0u;
         const bool zero = x < n && f == 0u;
@@ -422,10 +486,11 @@ __device__ bool warp_code(DeflateWarp &s, const uint32_t *freq, int n, uint8_t *
     }
     used = max(used, 2);
     __syncwarp();
-    // bitonic sort, ascending, 256 compare-exchanges per pass
-    for (int k = 2; k <= 512; k <<= 1) {
+    // bitonic sort, ascending, slots / 2 compare-exchanges per pass
+    for (int k = 2; k <= slots; k <<= 1) {
         for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = lane; i < 256; i += 32) {
+#pragma unroll 4
+            for (int i = lane; i < slots / 2; i += 32) {
                 const int lo = ((i & ~(j - 1)) << 1) | (i & (j - 1)), hi = lo + j;
                 const uint32_t a = b.key[lo], c = b.key[hi];
                 const bool up = (lo & k) == 0;
@@ -444,15 +509,123 @@ __device__ bool warp_code(DeflateWarp &s, const uint32_t *freq, int n, uint8_t *
         b.w[r] = kk >> 9;
     }
     __syncwarp();
-    int ok = 1;
-    if (lane == 0) {
-        ok = zl::huff_lengths(b.w, used, zl::kMaxLit, b.l, b.iw, b.par, b.dep) ? 1 : 0;
-        if (ok)
-            for (int i = 0; i < used; ++i) len[b.sym[i]] = b.l[i];
-    }
-    ok = __shfl_sync(0xffffffffu, ok, 0);
+    const bool ok = warp_huff_lengths(s, used, zl::kMaxLit, lane);
+    if (ok)
+        for (int i = lane; i < used; i += 32) len[b.sym[i]] = b.l[i];
     __syncwarp();
-    return ok != 0;
+    return ok;
+}
+
+// zl::canon_codes by the warp: codes in symbol order per length.
+__device__ void warp_canon_codes(DeflateWarp &s, const uint8_t *len, int n, uint16_t *code, int lane)
+{
+    if (lane < 16) s.cnt[lane] = 0;
+    __syncwarp();
+    for (int x = lane; x < n; x += 32)
+        if (len[x]) atomicAdd(&s.cnt[len[x]], 1u);
+    __syncwarp();
+    uint32_t first = 0, c = 0;
+    for (int l = 1; l < 16; ++l) {
+        c = (c + (l > 1 ? s.cnt[l - 1] : 0u)) << 1;
+        if (lane == l) first = c;
+    }
+    __syncwarp();
+    if (lane < 16) s.cnt[lane] = first;  // next code per length
+    __syncwarp();
+    for (int x0 = 0; x0 < n; x0 += 32) {
+        const int x = x0 + lane, l = x < n ? len[x] : 0;
+        const unsigned same = __match_any_sync(0xffffffffu, l);
+        const int rank = __popc(same & ((1u << lane) - 1u));
+        const uint32_t at = s.cnt[l];
+        if (x < n) code[x] = l ? (uint16_t)(__brev(at + rank) >> (32 - l)) : (uint16_t)0;
+        __syncwarp();
+        if (l && rank == 0) s.cnt[l] = at + __popc(same);
+        __syncwarp();
+    }
+}
+
+// zl::dynamic_header by the warp, which has llen and dlen: the number of
+// entries that a run of equal lengths takes has a closed form, so every lane
+// codes the runs that start at its symbols; the code-length code's own lengths
+// are lane 0's. Every lane gets the result.
+__device__ long long warp_dynamic_header(DeflateWarp &s, int lane)
+{
+    Codes &c = s.codes;
+    auto &b = s.u.b;
+    uint16_t *len16 = b.dep;  // the lengths, literals' then distances' (the code construction is done)
+    int hl = kLitSyms, hd = kDistSyms;
+    {
+        int top = 256;
+        for (int x = 257 + lane; x < kLitSyms; x += 32)
+            if (c.llen[x]) top = x;
+        hl = max(257, __reduce_max_sync(0xffffffffu, top) + 1);
+        hd = max(1, __reduce_max_sync(0xffffffffu, lane < kDistSyms && c.dlen[lane] ? lane + 1 : 0));
+    }
+    const int n = hl + hd;
+    for (int x = lane; x < n; x += 32) len16[x] = x < hl ? c.llen[x] : c.dlen[x - hl];
+    if (lane < kClSyms) s.cnt[lane] = 0;
+    __syncwarp();
+    // run lengths: the next position where the length changes
+    int out = 0;  // entries so far
+    for (int x0 = 0; x0 < n; x0 += 32) {
+        const int x = x0 + lane;
+        const int v = x < n ? len16[x] : -1;
+        const bool start = x < n && (x == 0 || len16[x - 1] != v);
+        int run = 0, m = 0;
+        if (start) {
+            run = 1;
+            while (x + run < n && len16[x + run] == v) ++run;
+            // zeros: pieces of 138 (18), then 11-137 (18), 3-10 (17) or single
+            // ones; others: one as it is, pieces of 6 (16), then 3-5 (16) or single
+            const int rep = v ? run - 1 : run, q = v ? 6 : 138, rest = rep % q;
+            m = (v ? 1 : 0) + rep / q + (rest >= 3 ? 1 : rest);
+        }
+        int inc = m;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        if (start) {
+            int at = out + inc - m;
+            auto put = [&](int e) {
+                c.rle[at++] = (uint16_t)e;
+                atomicAdd(&s.cnt[e & 31], 1u);
+            };
+            if (v) put(v);
+            const int rep = v ? run - 1 : run, q = v ? 6 : 138, rest = rep % q;
+            for (int k = 0; k < rep / q; ++k) put(v ? 16 | 3 << 8 : 18 | 127 << 8);
+            if (v) {
+                if (rest >= 3) put(16 | (rest - 3) << 8);
+                else
+                    for (int k = 0; k < rest; ++k) put(v);
+            } else if (rest >= 11) {
+                put(18 | (rest - 11) << 8);
+            } else if (rest >= 3) {
+                put(17 | (rest - 3) << 8);
+            } else {
+                for (int k = 0; k < rest; ++k) put(0);
+            }
+        }
+        out += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    __syncwarp();
+    long long bits = -1;
+    if (lane == 0) {
+        c.hlit = hl;
+        c.hdist = hd;
+        c.nrle = out;
+        bits = zl::code_length_code(c, s.cnt);
+    }
+    __syncwarp();
+    int sum = 0;
+    for (int i = lane; i < out; i += 32) {
+        const int x = c.rle[i] & 31;
+        sum += c.clen[x] + zl::rle_extra_bits(x);
+    }
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    bits = __shfl_sync(0xffffffffu, bits, 0);
+    return bits < 0 ? -1 : bits + sum;
 }
 
 // zl::data_bits (with the dynamic lengths) and zl::fixed_block_bits of the
@@ -510,56 +683,81 @@ __device__ __forceinline__ void ring_or(uint32_t *ring, int b, unsigned long lon
     if (x2) atomicOr(ring + ((wi + 2) & kRingM), x2);
 }
 
-// The ring of one chunk's output: words [flushed, bp/32] are live; older
+// The ring of one block's output: words [flushed, bp/32] are live; older
 // words are in the output, their slots zero. Flushes keep a step of at most
-// 32 items (48 bits each) clear of the live words.
+// 32 items (48 bits each) clear of the live words. A first word that the
+// block before shares (shared_word) goes to *head instead of the output.
 struct Ring {
     uint32_t *ring, *dstw;
-    int bp, flushed, wlimit;
+    int bp, flushed, wlimit, shared_word;
+    uint32_t *head;
     __device__ void flush_to(int to, int lane)
     {
         for (int w = flushed + lane; w < to; w += 32) {
-            if (w < wlimit) dstw[w] = ring[w & kRingM];
+            if (w == shared_word) *head = ring[w & kRingM];
+            else if (w < wlimit) dstw[w] = ring[w & kRingM];
             ring[w & kRingM] = 0;
         }
         flushed = to;
         __syncwarp();
     }
-    __device__ void make_room(int lane, int words = 52)
+    __device__ void make_room(int lane, int words = 64)
     {
         if ((bp >> 5) + words >= flushed + kRingW) flush_to(bp >> 5, lane);
     }
 };
-
-// Index j of the batch entry whose [beg, end) holds item t (t < end[31]).
-__device__ __forceinline__ int find_item(const int *end, int t)
-{
-    int j = 0;
-#pragma unroll
-    for (int step = 16; step; step >>= 1)
-        if (end[j + step - 1] <= t) j += step;
-    return j;
-}
 
 // Sequence cursor: record index and the input position of its literals.
 struct Cursor {
     int i, pos;
 };
 
+// Four bytes at any address as a little-endian word; reads whole aligned
+// words (inputs carry tail room).
+__device__ __forceinline__ uint32_t bytes4(const uint8_t *p)
+{
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
+    return __funnelshift_r(__ldg(w), __ldg(w + 1), 8 * (uint32_t)(a & 3));
+}
+
+// The codes of the first min(n, 4) bytes of w, one after the other.
+__device__ __forceinline__ void pack4(const zl::Codes &cd, uint32_t w, int n, unsigned long long &v, int &bits)
+{
+    v = 0;
+    bits = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t x = (w >> (8 * j)) & 0xffu;
+        if (j < n) {
+            v |= (unsigned long long)cd.lcode[x] << bits;
+            bits += cd.llen[x];
+        }
+    }
+}
+
 // The items (literal bytes and match pieces) of the parse that start in
-// [lo, hi), from cursor cur, 32 sequences per batch and 32 items per step.
-// MODE 0 counts symbols into s.lf/s.df and returns the end of the bytes the
-// items cover; MODE 1 writes their codes into the ring. `next` is set to
-// the first sequence that reaches past that end.
+// [lo, hi), from cursor cur, 32 sequences per batch, one per lane. Literal
+// runs of more than kShortLit bytes and matches of more than kShortPieces
+// pieces are shared out over the warp, 128 bytes or 32 pieces a step; the
+// other lanes take their own sequence whole, so that a batch costs one scan.
+// MODE 0 counts symbols into s.lf/s.df; MODE 1 writes their codes into the
+// ring; MODE 2 looks at no item. Returns the end of the bytes the items
+// cover; `next` is set to the first sequence that reaches past that end.
+constexpr int kShortLit = 32, kShortPieces = 4;
+constexpr int kShortWords = 32 * (15 * kShortLit + 48 * kShortPieces) / 32 + 2;  // most ring words of a batch of short ones
+static_assert(kShortWords + 1 < kRingW, "ring");
+
 template <int MODE>
 __device__ int block_items(DeflateWarp &s, const unsigned long long *seq, int nseq, Cursor cur, int lo, int hi,
                            const uint8_t *src, Ring *rg, Cursor *next, int lane)
 {
     int cov = lo;
     int i0 = cur.i, pos = cur.pos;
+    unsigned long long r = i0 + lane < nseq ? seq[i0 + lane] : 0ull;
     for (;;) {
         const int i = i0 + lane;
-        const unsigned long long r = i < nseq ? seq[i] : 0ull;
+        const unsigned long long ahead = i + 32 < nseq ? seq[i + 32] : 0ull;  // the next batch
         const int lit = zl::seq_lit(r), m = zl::seq_mlen(r), d = zl::seq_dist(r);
         const int span = lit + m;
         int incl = span;
@@ -573,87 +771,175 @@ __device__ int block_items(DeflateWarp &s, const unsigned long long *seq, int ns
         // literal sub-range [a, b) and pieces [k0, k1) that start in [lo, hi)
         const int a = min(max(lo - ls, 0), lit), b = min(max(hi - ls, 0), lit);
         const int k0 = m ? zl::pieces_before(m, lo - ms) : 0, k1 = m ? zl::pieces_before(m, hi - ms) : 0;
-        const int nl = b - a, np = k1 - k0, items = nl + np;
+        int nl = b - a, np = k1 - k0;
         int c = 0;
         if (np > 0) c = ms + zl::piece_start(m, k1 - 1) + zl::piece_len(m, k1 - 1);
         else if (nl > 0) c = ls + b;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) c = max(c, __shfl_xor_sync(0xffffffffu, c, o));
+        c = __reduce_max_sync(0xffffffffu, c);
         cov = max(cov, c);
-        int ii = items;
+        const uint8_t *lp = src + ls + a;
+        if (MODE == 0) {
+            // order does not matter: long ones by the warp, then every lane's own
+            for (unsigned lng = __ballot_sync(0xffffffffu, nl > kShortLit); lng; lng &= lng - 1) {
+                const int who = __ffs(lng) - 1;
+                const int p0 = __shfl_sync(0xffffffffu, ls + a, who), n = __shfl_sync(0xffffffffu, nl, who);
+#pragma unroll 2
+                for (int k = 4 * lane; k < n; k += 128) {
+                    const uint32_t w = bytes4(src + p0 + k);
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, ii, o);
-            if (lane >= o) ii += t;
-        }
-        s.end[lane] = ii;
-        s.beg[lane] = ii - items;
-        s.litpos[lane] = ls + a;
-        s.nlit[lane] = nl;
-        s.mstart[lane] = ms;
-        s.mlen[lane] = m;
-        s.dist[lane] = d;
-        s.k0[lane] = k0;
-        const int total = __shfl_sync(0xffffffffu, ii, 31);
-        __syncwarp();
-        // kU steps of 32 items at a time: their literal bytes are loaded
-        // together, then the steps are counted or written in order
-        constexpr int kU = 4;
-        for (int t0 = 0; t0 < total; t0 += 32 * kU) {
-            if (MODE == 1) rg->make_room(lane, 48 * kU + 4);
-            int byte[kU], nb[kU];  // byte >= 256: not a literal (inactive lanes never group)
-            unsigned long long v[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                const int t = t0 + 32 * u + lane;
-                byte[u] = 256 + lane;
-                nb[u] = 0;
-                v[u] = 0;
-                if (t < total) {
-                    const int j = find_item(s.end, t);
-                    const int k = t - s.beg[j];
-                    if (k < s.nlit[j]) {
-                        byte[u] = src[s.litpos[j] + k];
-                    } else {
-                        const int mj = s.mlen[j], pk = s.k0[j] + k - s.nlit[j];
-                        const int pl = zl::piece_len(mj, pk);
-                        if (MODE == 0) {
-                            atomicAdd(&s.lf[257 + zl::len_sym(pl)], 1u);
-                            atomicAdd(&s.df[zl::dist_sym(s.dist[j])], 1u);
-                        } else {
-                            nb[u] = zl::match_bits(s.codes, pl, s.dist[j], v[u]);
-                        }
-                    }
+                    for (int j = 0; j < 4; ++j)
+                        if (k + j < n) atomicAdd(&s.lf[(w >> (8 * j)) & 0xffu], 1u);
                 }
             }
+            for (unsigned lng = __ballot_sync(0xffffffffu, np > kShortPieces); lng; lng &= lng - 1) {
+                const int who = __ffs(lng) - 1;
+                const int mm = __shfl_sync(0xffffffffu, m, who), dd = __shfl_sync(0xffffffffu, d, who);
+                const int e = __shfl_sync(0xffffffffu, k1, who);
+                for (int k = __shfl_sync(0xffffffffu, k0, who) + lane; k < e; k += 32) {
+                    atomicAdd(&s.lf[257 + zl::len_sym(zl::piece_len(mm, k))], 1u);
+                    atomicAdd(&s.df[zl::dist_sym(dd)], 1u);
+                }
+            }
+            if (nl <= kShortLit)
+                for (int k = 0; k < nl; k += 4) {
+                    const uint32_t w = bytes4(lp + k);
 #pragma unroll
-            for (int u = 0; u < kU; ++u) {
-                if (MODE == 0) {
-                    const unsigned grp = __match_any_sync(0xffffffffu, byte[u]);
-                    if (byte[u] < 256 && lane == __ffs(grp) - 1) atomicAdd(&s.lf[byte[u]], (unsigned)__popc(grp));
-                } else {
-                    if (byte[u] < 256) {
-                        v[u] = s.codes.lcode[byte[u]];
-                        nb[u] = s.codes.llen[byte[u]];
+                    for (int j = 0; j < 4; ++j)
+                        if (k + j < nl) atomicAdd(&s.lf[(w >> (8 * j)) & 0xffu], 1u);
+                }
+            if (np > 0 && np <= kShortPieces) {
+                for (int k = k0; k < k1; ++k) atomicAdd(&s.lf[257 + zl::len_sym(zl::piece_len(m, k))], 1u);
+                atomicAdd(&s.df[zl::dist_sym(d)], (uint32_t)np);
+            }
+        } else if (MODE == 1) {
+            const zl::Codes &cd = s.codes;
+            // lanes [from, to) in turn: short ones together up to the next
+            // long one, its literals or pieces, then on from there
+            unsigned long_lit = __ballot_sync(0xffffffffu, nl > kShortLit);
+            unsigned long_rep = __ballot_sync(0xffffffffu, np > kShortPieces);
+            unsigned todo = __ballot_sync(0xffffffffu, nl + np > 0);
+            while (todo) {
+                const unsigned stops = (long_lit | long_rep) & todo;
+                const int to = stops ? __ffs(stops) - 1 : 32;
+                const unsigned below = to == 32 ? todo : todo & ((1u << to) - 1u);
+                if (below) {
+                    const bool mine = below >> lane & 1u;
+                    // the first four literals and the first piece are
+                    // looked up once (most sequences have no more)
+                    unsigned long long v0 = 0, v1 = 0;
+                    int n0 = 0, n1 = 0, bits = 0;
+                    if (mine) {
+                        if (nl > 0) pack4(cd, bytes4(lp), nl, v0, n0);
+                        if (np > 0) n1 = zl::match_bits(cd, zl::piece_len(m, k0), d, v1);
+                        bits = n0 + n1;
+                        for (int k = 4; k < nl; k += 4) {
+                            const uint32_t w = bytes4(lp + k);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (k + j < nl) bits += cd.llen[(w >> (8 * j)) & 0xffu];
+                        }
+                        unsigned long long v;
+                        for (int k = k0 + 1; k < k1; ++k) bits += zl::match_bits(cd, zl::piece_len(m, k), d, v);
                     }
-                    int bi = nb[u];
+                    int bi = bits;
 #pragma unroll
                     for (int o = 1; o < 32; o <<= 1) {
-                        const int w = __shfl_up_sync(0xffffffffu, bi, o);
-                        if (lane >= o) bi += w;
+                        const int t = __shfl_up_sync(0xffffffffu, bi, o);
+                        if (lane >= o) bi += t;
                     }
-                    if (nb[u]) ring_or(rg->ring, rg->bp + bi - nb[u], v[u]);
+                    rg->make_room(lane, kShortWords);
+                    if (mine) {
+                        int at = rg->bp + bi - bits;
+                        ring_or(rg->ring, at, v0);
+                        at += n0;
+                        for (int k = 4; k < nl; k += 4) {
+                            unsigned long long v;
+                            int n;
+                            pack4(cd, bytes4(lp + k), nl - k, v, n);
+                            ring_or(rg->ring, at, v);
+                            at += n;
+                        }
+                        ring_or(rg->ring, at, v1);
+                        at += n1;
+                        for (int k = k0 + 1; k < k1; ++k) {
+                            unsigned long long v;
+                            const int n = zl::match_bits(cd, zl::piece_len(m, k), d, v);
+                            ring_or(rg->ring, at, v);
+                            at += n;
+                        }
+                    }
                     rg->bp += __shfl_sync(0xffffffffu, bi, 31);
+                    __syncwarp();  // the next flush reads these words
+                    todo &= ~below;
+                }
+                if (to == 32) continue;
+                if (long_lit >> to & 1u) {
+                    const int p0 = __shfl_sync(0xffffffffu, ls + a, to), n = __shfl_sync(0xffffffffu, nl, to);
+                    for (int t0 = 0; t0 < n; t0 += 128) {
+                        const int k = t0 + 4 * lane;
+                        const uint32_t w = k < n ? bytes4(src + p0 + k) : 0u;
+                        unsigned long long v;
+                        int nb;
+                        pack4(cd, w, n - k, v, nb);
+                        int bi = nb;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const int t = __shfl_up_sync(0xffffffffu, bi, o);
+                            if (lane >= o) bi += t;
+                        }
+                        rg->make_room(lane, 64);
+                        if (nb) ring_or(rg->ring, rg->bp + bi - nb, v);
+                        rg->bp += __shfl_sync(0xffffffffu, bi, 31);
+                        __syncwarp();
+                    }
+                    long_lit &= ~(1u << to);
+                    if (lane == to) nl = 0;
+                    // its match: with the next short ones, or below
+                }
+                if (long_rep >> to & 1u) {
+                    // the literals before it are written (a short run first)
+                    const int n = __shfl_sync(0xffffffffu, nl, to);
+                    if (n > 0) {
+                        const int p0 = __shfl_sync(0xffffffffu, ls + a, to);
+                        const uint32_t x = lane < n ? src[p0 + lane] : 0u;
+                        const int nb = lane < n ? cd.llen[x] : 0;
+                        int bi = nb;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const int t = __shfl_up_sync(0xffffffffu, bi, o);
+                            if (lane >= o) bi += t;
+                        }
+                        rg->make_room(lane, 64);
+                        if (nb) ring_or(rg->ring, rg->bp + bi - nb, cd.lcode[x]);
+                        rg->bp += __shfl_sync(0xffffffffu, bi, 31);
+                        __syncwarp();
+                    }
+                    const int mm = __shfl_sync(0xffffffffu, m, to), dd = __shfl_sync(0xffffffffu, d, to);
+                    const int e = __shfl_sync(0xffffffffu, k1, to);
+                    for (int t0 = __shfl_sync(0xffffffffu, k0, to); t0 < e; t0 += 32) {
+                        unsigned long long v = 0;
+                        const int k = t0 + lane, nb = k < e ? zl::match_bits(cd, zl::piece_len(mm, k), dd, v) : 0;
+                        int bi = nb;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const int t = __shfl_up_sync(0xffffffffu, bi, o);
+                            if (lane >= o) bi += t;
+                        }
+                        rg->make_room(lane, 64);
+                        if (nb) ring_or(rg->ring, rg->bp + bi - nb, v);
+                        rg->bp += __shfl_sync(0xffffffffu, bi, 31);
+                        __syncwarp();
+                    }
+                    long_rep &= ~(1u << to);
+                    todo &= ~(1u << to);
                 }
             }
-            if (MODE == 1) __syncwarp();  // the next flush reads these words
         }
         __syncwarp();
         const bool last = pos + span_total >= hi || i0 + 32 >= nseq;
         if (last) {
             // the next block starts at the first sequence reaching past cov
-            const int cv = __shfl_sync(0xffffffffu, cov, 0);
-            const unsigned beyond = __ballot_sync(0xffffffffu, i < nseq && ls + span > cv);
+            const unsigned beyond = __ballot_sync(0xffffffffu, i < nseq && ls + span > cov);
             if (beyond) {
                 const int f = __ffs(beyond) - 1;
                 next->i = i0 + f;
@@ -662,10 +948,11 @@ __device__ int block_items(DeflateWarp &s, const unsigned long long *seq, int ns
                 next->i = min(i0 + 32, nseq);
                 next->pos = pos + span_total;
             }
-            return cv;
+            return cov;
         }
         pos += span_total;
         i0 += 32;
+        r = ahead;
     }
 }
 
@@ -675,9 +962,15 @@ __device__ bool parse_ok(const unsigned long long *seq, int nseq, int L, int lan
 {
     int pos = 0;
     bool ok = true;
+    constexpr int kA = 8;  // batches loaded ahead
+    unsigned long long q[kA];
+#pragma unroll
+    for (int u = 0; u < kA; ++u) q[u] = 32 * u + lane < nseq ? seq[32 * u + lane] : 0ull;
     for (int i0 = 0; i0 < nseq; i0 += 32) {
-        const int i = i0 + lane;
-        const unsigned long long r = i < nseq ? seq[i] : 0ull;
+        const unsigned long long r = q[0];
+#pragma unroll
+        for (int u = 0; u + 1 < kA; ++u) q[u] = q[u + 1];
+        q[kA - 1] = i0 + 32 * kA + lane < nseq ? seq[i0 + 32 * kA + lane] : 0ull;
         const int lit = zl::seq_lit(r), m = zl::seq_mlen(r), d = zl::seq_dist(r);
         int incl = lit + m;
 #pragma unroll
@@ -693,143 +986,253 @@ __device__ bool parse_ok(const unsigned long long *seq, int nseq, int L, int lan
     return __all_sync(0xffffffffu, ok) && pos == L;
 }
 
-__global__ void __launch_bounds__(kZWarps * 32)
+// One CTA per chunk. A chunk's DEFLATE blocks (five per block record) depend
+// on one another only through where they start in the input (a match may reach
+// past a block's end) and in the output: warp 0 finds the former from the
+// parse alone for the next kZWarps blocks, every warp then counts one block's
+// symbols and builds its codes, one thread picks the codings and adds up the
+// bits, and every warp writes its block at its place. The word two blocks
+// share is put together at the end. With a warp per chunk doing the blocks in
+// turn, 512 chunks (256^3) left three warps to an SM: the
+// DEFLATE stage took 3.0 ms, with a CTA each 0.8 ms.
+struct DeflateBlock {
+    int lo, hi, cov;
+    Cursor cur;
+    long long dyn, fix;  // bits of the dynamic coding (-1: none) and of the fixed one
+    int mode, start, bits;
+    uint32_t head, tail;  // its bits of a first and a last word that it shares
+};
+
+__global__ void __launch_bounds__(kZWarps * 32, 4)
 deflate_kernel(const uint8_t *__restrict__ in, const long long *in_off, const int *in_len,
                const uint8_t *__restrict__ sq, const long long *seq_off, const int *seq_bytes, int nchunks,
                int records, uint8_t *__restrict__ out, long long out_slot, long long *out_off, int *out_len)
 {
-    __shared__ DeflateWarp sw[kZWarps];
-    const int lane = threadIdx.x & 31;
-    DeflateWarp &s = sw[threadIdx.x >> 5];
-    const int gw = blockIdx.x * kZWarps + (threadIdx.x >> 5), nw = gridDim.x * kZWarps;
-    for (int c = gw; c < nchunks; c += nw) {
+    extern __shared__ __align__(16) unsigned char deflate_smem[];
+    DeflateWarp *sw = reinterpret_cast<DeflateWarp *>(deflate_smem);
+    __shared__ DeflateBlock blk[kZWarps];
+    __shared__ int s_n, s_ok, s_err;
+    __shared__ unsigned long long s_sum[kZWarps][2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    DeflateWarp &s = sw[warp];
+    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
         const uint8_t *src = in + in_off[c];
         const int L = in_len[c];
         const int sb = seq_bytes[c];
         const unsigned long long *seq = reinterpret_cast<const unsigned long long *>(sq + seq_off[c]);
         const int nseq = sb >= 8 && (sb & 7) == 0 ? sb / 8 : 0;
         uint8_t *dst = out + (long long)c * out_slot;
-        if (lane == 0) out_off[c] = (long long)c * out_slot;
-        if (nseq == 0 || !parse_ok(seq, nseq, L, lane)) {
-            if (lane == 0) out_len[c] = -1;
-            __syncwarp();
+        uint32_t *dstw = reinterpret_cast<uint32_t *>(dst);
+        const int wlimit = (int)(out_slot / 4);
+        if (threadIdx.x == 0) {
+            out_off[c] = (long long)c * out_slot;
+            s_err = 0;
+        }
+        if (warp == 0) {
+            const bool ok = nseq > 0 && parse_ok(seq, nseq, L, lane);
+            if (lane == 0) s_ok = ok;
+        } else {
+            // Adler-32 of the input (chunks start on 4-byte boundaries)
+            unsigned long long sa, sbs;
+            adler_sums<false>(src, L, threadIdx.x - 32, 32 * (kZWarps - 1), sa, sbs);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                sa += __shfl_xor_sync(0xffffffffu, sa, o);
+                sbs += __shfl_xor_sync(0xffffffffu, sbs, o);
+            }
+            if (lane == 0) {
+                s_sum[warp][0] = sa;
+                s_sum[warp][1] = sbs;
+            }
+        }
+        __syncthreads();
+        if (!s_ok) {
+            if (threadIdx.x == 0) out_len[c] = -1;
+            __syncthreads();
             continue;
         }
-        // Adler-32 of the input (chunks start on 4-byte boundaries)
-        unsigned long long sa, sbs;
-        adler_sums<false>(src, L, lane, 32, sa, sbs);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            sa += __shfl_xor_sync(0xffffffffu, sa, o);
-            sbs += __shfl_xor_sync(0xffffffffu, sbs, o);
-        }
-        const unsigned adler = adler_of(sa, sbs, L);
-        Ring rg{s.u.ring, reinterpret_cast<uint32_t *>(dst), 16, 0, (int)(out_slot / 4)};
-        zl::Bounds bnd;
+        zl::Bounds bnd;  // warp 0's
         bnd.init(src, L, records != 0);
         Cursor cur{0, 0};
-        int lo = 0, err = 0, nblk = 0;
-        bool first = true;
-        for (;;) {
-            const int hi = bnd.next(lo);
-            // ---- pass 1: symbol counts of the items starting in [lo, hi)
-            for (int x = lane; x < 288; x += 32) s.lf[x] = x == 256 ? 1u : 0u;
-            s.df[lane] = 0;
-            __syncwarp();
-            Cursor nxt;
-            const int cov = block_items<0>(s, seq, nseq, cur, lo, hi, src, nullptr, &nxt, lane);
-            const bool final = cov >= L;
-            // ---- codes; the block coding with the fewest bits
-            // (the code construction borrows the ring: flush it first)
-            if (!first) rg.flush_to(rg.bp >> 5, lane);
-            const uint32_t keep = first ? 0x9c78u : s.u.ring[rg.flushed & kRingM];  // zlib header / partial word
-            __syncwarp();  // read before the code construction overwrites the ring
-            bool ok = warp_code(s, s.lf, zl::kLitSyms, s.codes.llen, lane);
-            ok = warp_code(s, s.df, zl::kDistSyms, s.codes.dlen, lane) && ok;
-            long long dbits, fbits;
-            warp_block_bits(s, s.codes.llen, s.codes.dlen, lane, dbits, fbits);
-            if (lane == 0) {
-                Codes &cd = s.codes;
-                for (int x = zl::kLitSyms; x < 288; ++x) cd.llen[x] = 0;
-                for (int x = zl::kDistSyms; x < 32; ++x) cd.dlen[x] = 0;
-                long long dyn = -1;
-                if (ok) {
-                    zl::canon_codes(cd.llen, 288, cd.lcode);
-                    zl::canon_codes(cd.dlen, 32, cd.dcode);
-                    const long long hb = zl::dynamic_header(cd);
-                    if (hb >= 0) dyn = hb + dbits;
+        int lo = 0, nblk = 0;
+        int bp = 16;               // thread 0's: bits written, and those of the last, partial word
+        uint32_t carry = 0x9c78u;  // (the zlib header at first)
+        bool final = false;
+        while (!final) {
+            // ---- the next blocks
+            if (warp == 0) {
+                int n = 0, err = 0;
+                bool end = false;
+                while (n < kZWarps && !end) {
+                    const int hi = bnd.next(lo);
+                    Cursor nxt;
+                    const int cov = block_items<2>(s, seq, nseq, cur, lo, hi, src, nullptr, &nxt, lane);
+                    if (lane == 0) {
+                        blk[n].lo = lo;
+                        blk[n].hi = hi;
+                        blk[n].cov = cov;
+                        blk[n].cur = cur;
+                    }
+                    ++n;
+                    end = cov >= L;
+                    if (!end && cov <= lo) err = 3;             // every block makes progress
+                    if (++nblk > L / zl::kMinBlock + 2) err = 4;
+                    if (err) break;
+                    cur = nxt;
+                    lo = cov;
                 }
-                const long long fix = fbits;
-                const long long sto = cov - lo <= zl::kStoredMax ? zl::stored_block_bits(rg.bp, cov - lo) : -1;
-                int mode = 2;
-                long long best = dyn;
-                if (dyn < 0 || fix <= dyn) {
-                    mode = 1;
-                    best = fix;
-                }
-                if (sto >= 0 && sto <= best) {
-                    mode = 0;
-                    best = sto;
-                }
-                if (mode == 1) zl::fixed_codes(cd);
-                s.state[0] = mode;
-                s.state[2] = (int)best;
-            }
-            __syncwarp();
-            for (int w = lane; w < kRingW; w += 32) s.u.ring[w] = 0;
-            __syncwarp();
-            if (lane == 0) s.u.ring[rg.flushed & kRingM] = keep;
-            __syncwarp();
-            const int mode = s.state[0], bp0 = rg.bp;
-            // ---- pass 2: the block
-            if (mode == 0) {
                 if (lane == 0) {
-                    RingW wr{s.u.ring, rg.bp};
-                    wr.put(final ? 1u : 0u, 3);
-                    wr.bp = (wr.bp + 7) & ~7;
-                    const unsigned n = (unsigned)(cov - lo);
-                    wr.put(n | (~n & 0xffffu) << 16, 32);
-                    s.state[1] = wr.bp;
+                    s_n = n;
+                    if (err) s_err = err;
+                }
+            }
+            __syncthreads();
+            const int n = s_n;
+            if (s_err) break;
+            final = blk[n - 1].cov >= L;
+            DeflateBlock &b = blk[warp];
+            // ---- symbol counts of the items starting in [lo, hi), codes, sizes
+            if (warp < n) {
+                for (int x = lane; x < 288; x += 32) s.lf[x] = x == 256 ? 1u : 0u;
+                s.df[lane] = 0;
+                __syncwarp();
+                Cursor nxt;
+                block_items<0>(s, seq, nseq, b.cur, b.lo, b.hi, src, nullptr, &nxt, lane);
+                bool ok = warp_code(s, s.lf, zl::kLitSyms, s.codes.llen, lane);
+                ok = warp_code(s, s.df, zl::kDistSyms, s.codes.dlen, lane) && ok;
+                long long dbits, fbits;
+                warp_block_bits(s, s.codes.llen, s.codes.dlen, lane, dbits, fbits);
+                Codes &cd = s.codes;
+                if (lane < 288 - zl::kLitSyms) cd.llen[zl::kLitSyms + lane] = 0;
+                if (lane < 32 - zl::kDistSyms) cd.dlen[zl::kDistSyms + lane] = 0;
+                __syncwarp();
+                if (ok) {
+                    warp_canon_codes(s, cd.llen, 288, cd.lcode, lane);
+                    warp_canon_codes(s, cd.dlen, 32, cd.dcode, lane);
+                }
+                const long long hb = ok ? warp_dynamic_header(s, lane) : -1;
+                if (lane == 0) {
+                    b.dyn = hb >= 0 ? hb + dbits : -1;
+                    b.fix = fbits;
+                }
+            }
+            __syncthreads();
+            // ---- every block's coding, the one with the fewest bits, and place
+            if (threadIdx.x == 0) {
+                int at = bp;
+                for (int w = 0; w < n; ++w) {
+                    DeflateBlock &q = blk[w];
+                    const long long sto =
+                        q.cov - q.lo <= zl::kStoredMax ? zl::stored_block_bits(at, q.cov - q.lo) : -1;
+                    int mode = 2;
+                    long long best = q.dyn;
+                    if (q.dyn < 0 || q.fix <= q.dyn) {
+                        mode = 1;
+                        best = q.fix;
+                    }
+                    if (sto >= 0 && sto <= best) {
+                        mode = 0;
+                        best = sto;
+                    }
+                    q.mode = mode;
+                    q.start = at;
+                    q.bits = (int)best;
+                    q.head = q.tail = 0;
+                    at += (int)best;
+                }
+            }
+            __syncthreads();
+            // ---- the blocks
+            if (warp < n) {
+                const bool last = b.cov >= L;
+                for (int w = lane; w < kRingW; w += 32) s.u.ring[w] = 0;
+                if (b.mode == 1 && lane == 0) zl::fixed_codes(s.codes);
+                __syncwarp();
+                Ring rg{s.u.ring, dstw, b.start, b.start >> 5, wlimit, b.start & 31 ? b.start >> 5 : -1, &b.head};
+                RingW wr{s.u.ring, rg.bp};
+                if (lane == 0) {
+                    if (b.mode == 0) {
+                        wr.put(last ? 1u : 0u, 3);
+                        wr.bp = (wr.bp + 7) & ~7;
+                        const unsigned m = (unsigned)(b.cov - b.lo);
+                        wr.put(m | (~m & 0xffffu) << 16, 32);
+                    } else if (b.mode == 1) {
+                        wr.put((last ? 1u : 0u) | 1u << 1, 3);
+                    } else {
+                        zl::put_dynamic_header(wr, s.codes, last);
+                    }
                 }
                 __syncwarp();
-                rg.bp = s.state[1];
-                for (int t0 = 0; t0 < cov - lo; t0 += 32) {
+                rg.bp = __shfl_sync(0xffffffffu, wr.bp, 0);
+                if (b.mode == 0) {
+                    // bytes to the word boundary, whole words, the last bytes
+                    const int m = b.cov - b.lo, h = min(m, (32 - (rg.bp & 31)) / 8 & 3), nw = (m - h) >> 2;
+                    const uint8_t *q = src + b.lo;
+                    if (lane < h) ring_or(rg.ring, rg.bp + 8 * lane, q[lane]);
+                    rg.bp += 8 * h;
+                    __syncwarp();
+                    if (nw > 0) {  // at a word boundary
+                        rg.flush_to(rg.bp >> 5, lane);
+                        const uintptr_t a = reinterpret_cast<uintptr_t>(q + h);
+                        const uint32_t *sw32 = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
+                        const uint32_t sh = 8 * (uint32_t)(a & 3);
+                        const int w0 = rg.bp >> 5;
+#pragma unroll 4
+                        for (int i = lane; i < nw; i += 32)
+                            if (w0 + i < wlimit)
+                                dstw[w0 + i] = sh ? __funnelshift_r(sw32[i], sw32[i + 1], sh) : sw32[i];
+                        rg.bp += 32 * nw;
+                        rg.flushed = rg.bp >> 5;
+                    }
+                    const int t = m - h - 4 * nw;
+                    if (lane < t) ring_or(rg.ring, rg.bp + 8 * lane, q[h + 4 * nw + lane]);
+                    rg.bp += 8 * t;
+                    __syncwarp();
+                } else {
+                    Cursor dummy;
+                    block_items<1>(s, seq, nseq, b.cur, b.lo, b.hi, src, &rg, &dummy, lane);
                     rg.make_room(lane);
-                    const int t = t0 + lane;
-                    if (t < cov - lo) ring_or(rg.ring, rg.bp + 8 * lane, src[lo + t]);
-                    rg.bp += 8 * min(32, cov - lo - t0);
+                    if (lane == 0) ring_or(rg.ring, rg.bp, s.codes.lcode[256]);
+                    rg.bp += s.codes.llen[256];
                     __syncwarp();
                 }
-            } else {
+                rg.flush_to(rg.bp >> 5, lane);
                 if (lane == 0) {
-                    RingW wr{s.u.ring, rg.bp};
-                    if (mode == 1) wr.put((final ? 1u : 0u) | 1u << 1, 3);
-                    else zl::put_dynamic_header(wr, s.codes, final);
-                    s.state[1] = wr.bp;
+                    b.tail = rg.bp & 31 ? s.u.ring[(rg.bp >> 5) & kRingM] : 0u;
+                    if (rg.bp - b.start != b.bits) s_err = 2;  // written bits must be the counted ones
                 }
-                __syncwarp();
-                rg.bp = s.state[1];
-                Cursor dummy;
-                block_items<1>(s, seq, nseq, cur, lo, hi, src, &rg, &dummy, lane);
-                rg.make_room(lane);
-                if (lane == 0) ring_or(rg.ring, rg.bp, s.codes.lcode[256]);
-                rg.bp += s.codes.llen[256];
-                __syncwarp();
             }
-            first = false;
-            if (rg.bp - bp0 != s.state[2]) err = 2;  // written bits must be the counted ones
-            if (!final && cov <= lo) err = 3;         // every block makes progress
-            if (++nblk > L / zl::kMinBlock + 2) err = 4;
-            cur = nxt;
-            lo = cov;
-            if (final || err) break;
+            __syncthreads();
+            if (s_err) break;
+            // ---- the words that blocks share
+            if (threadIdx.x == 0) {
+                for (int w = 0; w < n; ++w) {
+                    const DeflateBlock &q = blk[w];
+                    const int e = q.start + q.bits;
+                    if (e >> 5 == q.start >> 5) {
+                        carry |= q.tail;
+                    } else {
+                        if (q.start & 31 && q.start >> 5 < wlimit) dstw[q.start >> 5] = carry | q.head;
+                        carry = q.tail;
+                    }
+                    bp = e;
+                }
+            }
+            __syncthreads();  // blk is free
         }
-        rg.flush_to((rg.bp + 31) >> 5, lane);
-        const int nbytes = (rg.bp + 7) >> 3;
-        if (lane == 0) {
-            if (err || nbytes + 4 > out_slot) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const int nbytes = (bp + 7) >> 3;
+            if (s_err || nbytes + 4 > out_slot) {
                 out_len[c] = -2;
             } else {
+                if (bp & 31) dstw[bp >> 5] = carry;
+                unsigned long long sa = 0, sbs = 0;
+                for (int w = 1; w < kZWarps; ++w) {
+                    sa += s_sum[w][0];
+                    sbs += s_sum[w][1];
+                }
+                const unsigned adler = adler_of(sa, sbs, L);
                 dst[nbytes] = (uint8_t)(adler >> 24);
                 dst[nbytes + 1] = (uint8_t)(adler >> 16);
                 dst[nbytes + 2] = (uint8_t)(adler >> 8);
@@ -837,7 +1240,7 @@ deflate_kernel(const uint8_t *__restrict__ in, const long long *in_off, const in
                 out_len[c] = nbytes + 4;
             }
         }
-        __syncwarp();
+        __syncthreads();
     }
 }
 
@@ -850,8 +1253,11 @@ cudaError_t cz_launch_deflate(const uint8_t *in, const long long *in_off, const 
                               long long out_slot, long long *out_off, int *out_len, int grid, cudaStream_t st)
 {
     if (nchunks <= 0) return cudaSuccess;
-    deflate_kernel<<<grid, kZWarps * 32, 0, st>>>(in, in_off, in_len, seq, seq_off, seq_bytes, nchunks, records,
-                                                  out, out_slot, out_off, out_len);
+    const int sm = (int)sizeof(DeflateWarp) * kZWarps;
+    const cudaError_t e = cudaFuncSetAttribute(deflate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    if (e != cudaSuccess) return e;
+    deflate_kernel<<<grid, kZWarps * 32, sm, st>>>(in, in_off, in_len, seq, seq_off, seq_bytes, nchunks, records, out,
+                                                   out_slot, out_off, out_len);
     return cudaGetLastError();
 }
 
