@@ -2,19 +2,23 @@
 // buffer management and the compress/decompress pipelines.
 //
 // Compress pipeline (one stream, no host round trip until the final size):
-//   encode_kernel        fwt + threshold + mask + survivors -> block slots
-//   chunk_setup          chunk geometry (blocks_per_chunk records per chunk)
-//   pack_records         (blocks_per_chunk > 1) records back to back per chunk
+//   encode_kernel        fwt + threshold + mask + survivors -> block slots; with
+//                        one record per chunk also the chunk geometry
+//   chunk_setup, pack_records  (blocks_per_chunk > 1) chunk geometry, records back
+//                        to back per chunk
 //   lz4_encode_kernel    (encoder lz4) one warp per chunk
-//   lz77 parse, deflate  (encoder zlib) one warp per chunk each
-//   scan                 chunk offsets (replaces the writer's offset allocation)
-//   gather               chunk payloads back to back
-// Decompress pipeline: decode_setup, lz4_decode_kernel or inflate_kernel,
-// record location, decode_kernel (load + iwt, optionally cz2diff's error
-// sums) straight into the output field. cz_compress_to_image pipelines the
+//   lz77 parse, deflate  (encoder zlib) a warp, then a CTA per chunk
+//   scan, gather         chunk offsets (replaces the writer's offset allocation),
+//                        chunk payloads back to back; one launch up to 1024 chunks
+// Decompress pipeline: lz4_decode or inflate_kernel, record location (more
+// than one record per chunk, or a block map), decode_kernel (load + iwt,
+// optionally cz2diff's error sums) straight into the output field.
+// A pipeline's counters, flags and totals share one buffer (Ctl), cleared by
+// one memset and read back by one copy. cz_compress_to_image pipelines the
 // compress steps over z-slabs behind the host-to-device copies.
 #include <cuda_runtime.h>
 
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -28,6 +32,16 @@
 using namespace cz;
 
 namespace {
+
+constexpr int kSlabs = 16;  // of the pipelined host-buffer path
+
+// What a pipeline's kernels count and report.
+struct Ctl {
+    int flag[2];                     // lossless stage or record (-1); tile copy did not complete (1)
+    long long out_bytes, raw_bytes;  // the stream's and the records' sizes
+    long long pad;
+    unsigned long long queue[kSlabs];
+};
 
 struct DevBuf {
     void *p = nullptr;
@@ -49,7 +63,7 @@ struct cz_ctx {
     int sms = 1;
     std::string err;
     DevBuf fields, stage, rec_bytes, chunk_in, in_off, in_len, blk_dst, lz_off, lz_out, lz_len, out_off, out_data,
-        queue, status, flag, rec_off, dec, dec_off, dec_cap, dec_len, raw_off, chunk_rec, block_chunk, block_subid,
+        ctl, rec_off, dec, dec_off, dec_cap, dec_len, chunk_rec, block_chunk, block_subid,
         tmp_field, tmp_in, refit, diff, zout, zoff, zlen, ierr, lz_hole;
     void *pin = nullptr;  // small pinned host scratch
     size_t pin_cap = 0;
@@ -242,9 +256,7 @@ int prepare(cz_ctx *c, const std::vector<CzField> &fields, long long nblocks, co
     CZ_TRY(grow(c, c->lz_off, sizeof(long long) * nchunks));
     CZ_TRY(grow(c, c->lz_len, sizeof(int) * nchunks));
     CZ_TRY(grow(c, c->out_off, sizeof(long long) * (nchunks + 1)));
-    CZ_TRY(grow(c, c->raw_off, sizeof(long long) * (nchunks + 1)));
-    CZ_TRY(grow(c, c->queue, 64));
-    CZ_TRY(grow(c, c->flag, 64));
+    CZ_TRY(grow(c, c->ctl, sizeof(Ctl)));
     if (bpc > 1) {
         CZ_TRY(grow(c, c->blk_dst, sizeof(long long) * nblocks));
         CZ_TRY(grow(c, c->chunk_in, (size_t)nchunks * bpc * kSlotBytes));
@@ -271,30 +283,31 @@ int enqueue(cz_ctx *c, const Job &job, cudaStream_t st, bool marks)
     const cz_params *p = &job.p;
     const long long nblocks = job.nblocks;
     const int nchunks = job.nchunks, bpc = job.bpc;
-    CZ_CUDA(c, cudaMemsetAsync(c->queue.p, 0, 64, st));
-    CZ_CUDA(c, cudaMemsetAsync(c->flag.p, 0, 64, st));
+    Ctl *ctl = P<Ctl>(c->ctl);
+    CZ_CUDA(c, cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
     const int grid = (int)std::min<long long>(nblocks, c->sms);
+    CzChunks chunks;
+    chunks.raw_total = reinterpret_cast<unsigned long long *>(&ctl->raw_bytes);
+    if (bpc == 1) chunks.at(P<long long>(c->in_off), P<int>(c->in_len), P<long long>(c->lz_off), job.lz_slot);
     if (marks) CZ_TRY(mark(c, 0, st));
     if (job.refit_iters > 0)
         CZ_CUDA(c, cz_launch_refit(p->wtype, P<CzField>(c->fields), job.nfields, nblocks, p->zerobits,
                                    p->shuffle ? 1 : 0, job.refit_iters, P<uint8_t>(c->stage), P<int>(c->rec_bytes),
-                                   P<unsigned long long>(c->queue), P<float>(c->refit), grid, st));
+                                   ctl->queue, P<float>(c->refit), grid, st, chunks));
     else
         CZ_CUDA(c, cz_launch_encode(p->wtype, P<CzField>(c->fields), job.nfields, nblocks, p->zerobits,
-                                    p->shuffle ? 1 : 0, P<uint8_t>(c->stage), P<int>(c->rec_bytes),
-                                    P<unsigned long long>(c->queue), grid, st, maps_of(c, job.nfields), nullptr,
-                                    P<int>(c->flag) + 1, job.enc_variant));
+                                    p->shuffle ? 1 : 0, P<uint8_t>(c->stage), P<int>(c->rec_bytes), ctl->queue, grid,
+                                    st, maps_of(c, job.nfields), nullptr, &ctl->flag[1], job.enc_variant, chunks));
     if (marks) CZ_TRY(mark(c, 1, st));
-    CZ_CUDA(c, cz_launch_chunk_setup(bpc, nblocks, nchunks, P<int>(c->rec_bytes), P<long long>(c->in_off),
-                                     P<int>(c->in_len), bpc > 1 ? P<long long>(c->blk_dst) : nullptr,
-                                     P<long long>(c->lz_off), job.lz_slot, st));
     const uint8_t *chunk_src = P<uint8_t>(c->stage);
     if (bpc > 1) {
+        CZ_CUDA(c, cz_launch_chunk_setup(bpc, nblocks, nchunks, P<int>(c->rec_bytes), P<long long>(c->in_off),
+                                         P<int>(c->in_len), P<long long>(c->blk_dst), P<long long>(c->lz_off),
+                                         job.lz_slot, st));
         CZ_CUDA(c, cz_launch_pack_records(P<uint8_t>(c->stage), P<int>(c->rec_bytes), nblocks,
                                           P<long long>(c->blk_dst), P<uint8_t>(c->chunk_in), st));
         chunk_src = P<uint8_t>(c->chunk_in);
     }
-    CZ_CUDA(c, cz_launch_scan(P<int>(c->in_len), nchunks, P<long long>(c->raw_off), st));
     const uint8_t *gsrc = chunk_src;
     const long long *gsrc_off = P<long long>(c->in_off);
     const int *glen = P<int>(c->in_len);
@@ -305,7 +318,6 @@ int enqueue(cz_ctx *c, const Job &job, cudaStream_t st, bool marks)
         CZ_CUDA(c, cz_launch_lz4_encode(chunk_src, P<long long>(c->in_off), P<int>(c->in_len), nchunks,
                                         P<uint8_t>(c->lz_out), P<long long>(c->lz_off), P<int>(c->lz_len),
                                         p->shuffle ? 1 : 0, per, lzgrid, st, P<int4>(c->lz_hole), c->lz_effort));
-        CZ_CUDA(c, cz_launch_neg_reduce(P<int>(c->lz_len), nchunks, P<int>(c->flag), st));
         gsrc = P<uint8_t>(c->lz_out);
         gsrc_off = P<long long>(c->lz_off);
         glen = P<int>(c->lz_len);
@@ -319,15 +331,14 @@ int enqueue(cz_ctx *c, const Job &job, cudaStream_t st, bool marks)
                                      P<uint8_t>(c->zout),
                                      job.z_slot, P<long long>(c->zoff), P<int>(c->zlen),
                                      std::min(nchunks, c->sms * 4), st));
-        CZ_CUDA(c, cz_launch_neg_reduce(P<int>(c->zlen), nchunks, P<int>(c->flag), st));
         gsrc = P<uint8_t>(c->zout);
         gsrc_off = P<long long>(c->zoff);
         glen = P<int>(c->zlen);
     }
     if (marks) CZ_TRY(mark(c, 2, st));
-    CZ_CUDA(c, cz_launch_scan(glen, nchunks, P<long long>(c->out_off), st));
     const bool holes = p->encoder == CZ_ENCODER_LZ4;
-    CZ_CUDA(c, cz_launch_gather(gsrc, gsrc_off, glen, nchunks, P<uint8_t>(c->out_data), P<long long>(c->out_off), st,
+    CZ_CUDA(c, cz_launch_gather(gsrc, gsrc_off, glen, nchunks, P<uint8_t>(c->out_data), P<long long>(c->out_off),
+                                true, &ctl->flag[0], &ctl->out_bytes, st,
                                 holes ? P<int4>(c->lz_hole) : nullptr, chunk_src, P<long long>(c->in_off)));
     if (marks) CZ_TRY(mark(c, 3, st));
     return CZ_OK;
@@ -335,24 +346,22 @@ int enqueue(cz_ctx *c, const Job &job, cudaStream_t st, bool marks)
 
 int finish(cz_ctx *c, const Job &job, cudaStream_t st, cz_stream *out)
 {
-    long long *h = reinterpret_cast<long long *>(c->pin);
+    const Ctl *h = reinterpret_cast<const Ctl *>(c->pin);
     const int nchunks = job.nchunks;
-    CZ_CUDA(c, cudaMemcpyAsync(&h[0], P<long long>(c->out_off) + nchunks, 8, cudaMemcpyDeviceToHost, st));
-    CZ_CUDA(c, cudaMemcpyAsync(&h[1], P<long long>(c->raw_off) + nchunks, 8, cudaMemcpyDeviceToHost, st));
-    CZ_CUDA(c, cudaMemcpyAsync(&h[2], c->flag.p, 8, cudaMemcpyDeviceToHost, st));
+    CZ_CUDA(c, cudaMemcpyAsync(c->pin, c->ctl.p, offsetof(Ctl, queue), cudaMemcpyDeviceToHost, st));
     CZ_CUDA(c, cudaStreamSynchronize(st));
-    if (reinterpret_cast<int *>(&h[2])[1] != 0) return fail(c, CZ_E_CUDA, "wavelet kernel: a tile copy did not complete");
-    if (reinterpret_cast<int *>(&h[2])[0] != 0)
+    if (h->flag[1] != 0) return fail(c, CZ_E_CUDA, "wavelet kernel: a tile copy did not complete");
+    if (h->flag[0] != 0)
         return fail(c, CZ_E_CUDA, "lossless encoder output exceeded its bound");
     c->nblocks = job.nblocks;
     c->nchunks = nchunks;
     c->bpc = job.bpc;
     out->data = P<uint8_t>(c->out_data);
-    out->data_bytes = h[0];
+    out->data_bytes = h->out_bytes;
     out->chunk_offsets = P<long long>(c->out_off);
     out->nchunks = nchunks;
     out->nblocks = job.nblocks;
-    out->raw_bytes = h[1];
+    out->raw_bytes = h->raw_bytes;
     return CZ_OK;
 }
 
@@ -380,48 +389,60 @@ int decompress_fields(cz_ctx *c, const std::vector<CzField> &fields, long long n
     const int per_chunk = h_block_chunk ? maxsub : bpc;
     if (diff_ref) CZ_TRY(grow(c, c->diff, sizeof(double) * (8 * (size_t)nblocks + 8)));
     const long long dcap = ((long long)per_chunk * (4 + kMaxRecord) + 15) / 16 * 16;
-    CZ_TRY(grow(c, c->in_len, sizeof(int) * nchunks));
-    CZ_TRY(grow(c, c->dec_off, sizeof(long long) * nchunks));
-    CZ_TRY(grow(c, c->dec_cap, sizeof(int) * nchunks));
+    // one record per chunk, blocks in chunk order: the kernels find chunks
+    // and records from the offset table and the decoded lengths alone
+    const bool own = bpc == 1 && !h_block_chunk;
     CZ_TRY(grow(c, c->dec_len, sizeof(int) * nchunks));
-    CZ_TRY(grow(c, c->rec_off, sizeof(long long) * nblocks));
-    CZ_TRY(grow(c, c->status, sizeof(int) * nblocks));
-    CZ_TRY(grow(c, c->queue, 64));
-    CZ_TRY(grow(c, c->flag, 64));
+    if (!own) {
+        CZ_TRY(grow(c, c->in_len, sizeof(int) * nchunks));
+        CZ_TRY(grow(c, c->dec_off, sizeof(long long) * nchunks));
+        CZ_TRY(grow(c, c->dec_cap, sizeof(int) * nchunks));
+        CZ_TRY(grow(c, c->rec_off, sizeof(long long) * nblocks));
+    }
+    CZ_TRY(grow(c, c->ctl, sizeof(Ctl)));
     if (encoder != CZ_ENCODER_NONE) CZ_TRY(grow(c, c->dec, (size_t)nchunks * dcap));
     // pinned scratch: [fields and tensor maps | flag (64 B) | block map]
     const size_t pin_fields = fields_bytes(fields.size());
     const size_t map_bytes = h_block_chunk ? sizeof(int) * 2 * nblocks : 0;
     CZ_TRY(put_fields(c, fields, 64 + map_bytes, st));
-    CZ_CUDA(c, cudaMemsetAsync(c->queue.p, 0, 64, st));
-    CZ_CUDA(c, cudaMemsetAsync(c->flag.p, 0, 64, st));
+    Ctl *ctl = P<Ctl>(c->ctl);
+    CZ_CUDA(c, cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
     const int raw = encoder == CZ_ENCODER_NONE;
     CZ_TRY(mark(c, 0, st));
-    CZ_CUDA(c, cz_launch_decode_setup(nchunks, d_off, P<int>(c->in_len), P<long long>(c->dec_off), P<int>(c->dec_cap),
-                                      dcap, raw, st));
-    const uint8_t *base = d_data;
-    const int *dlen = P<int>(c->in_len);
+    const int *in_len = nullptr, *dec_cap = nullptr;
+    const long long *dec_off = nullptr;
+    if (!own) {
+        CZ_CUDA(c, cz_launch_decode_setup(nchunks, d_off, P<int>(c->in_len), P<long long>(c->dec_off),
+                                          P<int>(c->dec_cap), dcap, raw, st));
+        in_len = P<int>(c->in_len);
+        dec_off = P<long long>(c->dec_off);
+        dec_cap = P<int>(c->dec_cap);
+    }
+    CzRecords recs;
+    recs.base = d_data;
+    recs.off = d_off;
+    const int *dlen = in_len;
     // one shuffled record per chunk, blocks in chunk order: the LZ4 decoder
     // may leave the records' byte planes 1 and 2 in its input, where the
     // decode kernel reads them
-    const bool planes_in_input = bpc == 1 && shuffle && !h_block_chunk && (long long)nchunks == nblocks;
+    const bool planes_in_input = own && shuffle;
     CzPlanes planes;
+    if (!raw) {
+        recs.base = P<uint8_t>(c->dec);
+        recs.dec_len = dlen = P<int>(c->dec_len);
+        recs.cap = dcap;
+    }
     if (encoder == CZ_ENCODER_ZLIB) {
-        CZ_CUDA(c, cz_launch_inflate(d_data, d_off, P<int>(c->in_len), nchunks, P<uint8_t>(c->dec),
-                                     P<long long>(c->dec_off), P<int>(c->dec_cap), P<int>(c->dec_len),
-                                     std::min(nchunks, c->sms * 32), st));
-        base = P<uint8_t>(c->dec);
-        dlen = P<int>(c->dec_len);
+        CZ_CUDA(c, cz_launch_inflate(d_data, d_off, in_len, nchunks, P<uint8_t>(c->dec), dec_off, dec_cap,
+                                     P<int>(c->dec_len), std::min(nchunks, c->sms * 32), st, dcap));
     } else if (!raw) {
         if (planes_in_input) {
             CZ_TRY(grow(c, c->lz_hole, sizeof(int4) * (size_t)nchunks));
             planes = CzPlanes{P<int4>(c->lz_hole), d_data, d_off};
         }
-        CZ_CUDA(c, cz_launch_lz4_decode(d_data, d_off, P<int>(c->in_len), nchunks, P<uint8_t>(c->dec),
-                                        P<long long>(c->dec_off), P<int>(c->dec_cap), P<int>(c->dec_len), st,
-                                        planes_in_input ? P<int4>(c->lz_hole) : nullptr));
-        base = P<uint8_t>(c->dec);
-        dlen = P<int>(c->dec_len);
+        CZ_CUDA(c, cz_launch_lz4_decode(d_data, d_off, in_len, nchunks, P<uint8_t>(c->dec), dec_off, dec_cap,
+                                        P<int>(c->dec_len), st, planes_in_input ? P<int4>(c->lz_hole) : nullptr,
+                                        dcap));
     }
     CZ_TRY(mark(c, 1, st));
     if (h_block_chunk) {
@@ -433,26 +454,25 @@ int decompress_fields(cz_ctx *c, const std::vector<CzField> &fields, long long n
         memcpy(hp + nblocks, h_block_subid, sizeof(int) * nblocks);
         CZ_CUDA(c, cudaMemcpyAsync(c->block_chunk.p, hp, sizeof(int) * nblocks, cudaMemcpyHostToDevice, st));
         CZ_CUDA(c, cudaMemcpyAsync(c->block_subid.p, hp + nblocks, sizeof(int) * nblocks, cudaMemcpyHostToDevice, st));
-        const long long *cbase = raw ? d_off : P<long long>(c->dec_off);
-        CZ_CUDA(c, cz_launch_chunk_records(nchunks, maxsub, cbase, dlen, base, P<long long>(c->chunk_rec), st));
+        const long long *cbase = raw ? d_off : dec_off;
+        CZ_CUDA(c, cz_launch_chunk_records(nchunks, maxsub, cbase, dlen, recs.base, P<long long>(c->chunk_rec), st));
         CZ_CUDA(c, cz_launch_map_blocks(nblocks, nchunks, maxsub, P<int>(c->block_chunk), P<int>(c->block_subid),
                                         P<long long>(c->chunk_rec), P<long long>(c->rec_off), st));
-    } else {
-        const long long *cbase = raw ? d_off : P<long long>(c->dec_off);
-        CZ_CUDA(c, cz_launch_locate_records(bpc, nblocks, nchunks, cbase, dlen, P<long long>(c->rec_off),
-                                            P<int>(c->status), base, st));
+    } else if (!own) {
+        CZ_CUDA(c, cz_launch_locate_records(bpc, nblocks, nchunks, raw ? d_off : dec_off, dlen,
+                                            P<long long>(c->rec_off), recs.base, st));
     }
+    if (!own) recs.rec_off = P<long long>(c->rec_off);
     const int grid = (int)std::min<long long>(nblocks, c->sms);
     CZ_TRY(mark(c, 2, st));
     double *per_block = diff_ref ? P<double>(c->diff) : nullptr;
-    CZ_CUDA(c, cz_launch_decode(wtype, P<CzField>(c->fields), (int)fields.size(), nblocks, shuffle ? 1 : 0, base,
-                                P<long long>(c->rec_off), P<int>(c->status), P<unsigned long long>(c->queue), grid,
-                                st, maps_of(c, fields.size()), diff_ref, per_block, planes));
+    CZ_CUDA(c, cz_launch_decode(wtype, P<CzField>(c->fields), (int)fields.size(), nblocks, shuffle ? 1 : 0, recs,
+                                &ctl->flag[0], ctl->queue, grid, st, maps_of(c, fields.size()), diff_ref, per_block,
+                                planes));
     if (diff_ref) CZ_CUDA(c, cz_launch_diff_total(per_block, nblocks, per_block + 8 * nblocks, st));
     CZ_TRY(mark(c, 3, st));
-    CZ_CUDA(c, cz_launch_status_reduce(P<int>(c->status), nblocks, P<int>(c->flag), st));
     int *hflag = reinterpret_cast<int *>(reinterpret_cast<char *>(c->pin) + pin_fields);
-    CZ_CUDA(c, cudaMemcpyAsync(hflag, c->flag.p, 4, cudaMemcpyDeviceToHost, st));
+    CZ_CUDA(c, cudaMemcpyAsync(hflag, ctl, 4, cudaMemcpyDeviceToHost, st));
     if (diff_ref) CZ_CUDA(c, cudaMemcpyAsync(h_stats, per_block + 8 * nblocks, 64, cudaMemcpyDeviceToHost, st));
     CZ_CUDA(c, cudaStreamSynchronize(st));
     collect(c);
@@ -491,8 +511,8 @@ int cz_destroy(cz_ctx *c)
     cudaSetDevice(c->device);
     DevBuf *all[] = {&c->ierr, &c->zout, &c->zoff, &c->zlen, &c->diff, &c->refit, &c->fields,  &c->stage,   &c->rec_bytes, &c->chunk_in,  &c->in_off,      &c->in_len,
                      &c->blk_dst, &c->lz_off,  &c->lz_out,    &c->lz_len,    &c->out_off,     &c->out_data,
-                     &c->queue,   &c->status,  &c->flag,      &c->rec_off,   &c->dec,         &c->dec_off,
-                     &c->dec_cap, &c->dec_len, &c->raw_off,   &c->chunk_rec, &c->block_chunk, &c->block_subid,
+                     &c->ctl,     &c->rec_off,   &c->dec,         &c->dec_off,
+                     &c->dec_cap, &c->dec_len, &c->chunk_rec, &c->block_chunk, &c->block_subid,
                      &c->tmp_field, &c->tmp_in, &c->lz_hole};
     for (DevBuf *b : all)
         if (b->p) cudaFree(b->p);
@@ -845,7 +865,7 @@ int cz_plan_create(cz_ctx *c, int nfields, const float *const *d_fields, const i
         pl->job.enc_variant = vpick;
         pl->c->timing = false;
     }
-    // one graph: memsets, wavelet kernel, chunk setup, scans, LZ4, gather
+    // one graph: memset, wavelet kernel, lossless stage, scan, gather
     if (cudaStreamBeginCapture(pl->st, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
         cudaGetLastError();
         return bail(CZ_E_CUDA, "stream capture");
@@ -926,11 +946,10 @@ int cz_block_compress(cz_ctx *c, const float *in, float eps, int wtype, int zero
     cz_params p = {eps, wtype, zerobits, shuffle, CZ_ENCODER_NONE, 1};
     cz_stream s;
     CZ_TRY(cz_field_compress(c, P<float>(c->tmp_field), 32, 32, 32, &p, nullptr, &s));
-    int nb = 0;
-    CZ_CUDA(c, cudaMemcpy(&nb, s.data, 4, cudaMemcpyDeviceToHost));
+    const long long nb = s.data_bytes - 4;  // the stream is the one record behind its size
     if (nb < kMaskBytes || nb > kMaxRecord) return fail(c, CZ_E_CUDA, "record size out of range");
     CZ_CUDA(c, cudaMemcpy(out, s.data + 4, nb, cudaMemcpyDeviceToHost));
-    *nbytes = nb;
+    *nbytes = (int)nb;
     return CZ_OK;
 }
 
@@ -942,13 +961,14 @@ int cz_block_decompress(cz_ctx *c, const uint8_t *in, int nbytes, int wtype, int
     CZ_TRY(grow(c, c->tmp_field, sizeof(float) * kBS3));
     const size_t need = 16 + (size_t)kSlotBytes;
     CZ_TRY(grow(c, c->tmp_in, need));
-    CZ_TRY(grow_pin(c, std::max<size_t>(4096, need)));
-    uint8_t *h = reinterpret_cast<uint8_t *>(c->pin);
+    // behind the part of the pinned scratch that the field's decompression uses
+    CZ_TRY(grow_pin(c, 4096 + need));
+    uint8_t *h = reinterpret_cast<uint8_t *>(c->pin) + 4096;
     long long off[2] = {16, 16 + 4 + (long long)nbytes};
     memcpy(h, off, 16);
     memcpy(h + 16, &nbytes, 4);
     memcpy(h + 20, in, nbytes);
-    CZ_CUDA(c, cudaMemcpy(c->tmp_in.p, h, 20 + nbytes, cudaMemcpyHostToDevice));
+    CZ_CUDA(c, cudaMemcpyAsync(c->tmp_in.p, h, 20 + nbytes, cudaMemcpyHostToDevice, nullptr));
     cz_params p = {0.f, wtype, 0, shuffle, CZ_ENCODER_NONE, 1};
     // offsets live at the start of tmp_in, the chunk right after them
     CZ_TRY(cz_field_decompress(c, P<uint8_t>(c->tmp_in), P<long long>(c->tmp_in), 1, 32, 32, 32, &p, nullptr,
@@ -1127,8 +1147,6 @@ int cz_file_image(cz_ctx *c, const cz_stream *s, int nx, int ny, int nz, const c
 
 namespace {
 
-constexpr int kSlabs = 16;
-
 // Streams of the pipelined path: the wavelet kernels on the highest
 // priority (their CTAs are scheduled before pending LZ4 CTAs), the LZ4
 // stages on the lowest.
@@ -1207,7 +1225,6 @@ int cz_compress_to_image(cz_ctx *c, const float *h_field, int nx, int ny, int nz
     }
     Job job;
     CZ_TRY(prepare(c, slabs, nblocks, p, 0, st, job));
-    CZ_TRY(grow(c, c->queue, 8 * kSlabs + 64));
     // the payload goes straight to the image when the device can write it
     const std::string hdr = czf::header_text(bx, by, bz, p->eps, p->wtype, p->encoder);
     const long long mini = czf::mini_header_bytes();
@@ -1219,8 +1236,8 @@ int cz_compress_to_image(cz_ctx *c, const float *h_field, int nx, int ny, int nz
         direct = static_cast<uint8_t *>(pa.devicePointer) + mini;
     cudaGetLastError();
     uint8_t *dst = direct ? direct : P<uint8_t>(c->out_data);
-    CZ_CUDA(c, cudaMemsetAsync(c->queue.p, 0, 8 * kSlabs, st));
-    CZ_CUDA(c, cudaMemsetAsync(c->flag.p, 0, 64, st));
+    Ctl *ctl = P<Ctl>(c->ctl);
+    CZ_CUDA(c, cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
     CZ_CUDA(c, cudaMemsetAsync(c->out_off.p, 0, 8, st));
     CZ_CUDA(c, cudaEventRecord(c->ev_join, st));
     CZ_CUDA(c, cudaStreamWaitEvent(c->s_gather, c->ev_join, 0));
@@ -1233,18 +1250,16 @@ int cz_compress_to_image(cz_ctx *c, const float *h_field, int nx, int ny, int nz
                                    cudaMemcpyHostToDevice, c->s_copy));
         CZ_CUDA(c, cudaEventRecord(c->ev_h2d[i], c->s_copy));
     }
-    unsigned long long *queues = P<unsigned long long>(c->queue);
     for (int i = 0; i < nslab; ++i) {
         const long long f0 = first[i];
         const int n = (int)(first[i + 1] - f0);
         uint8_t *stage = P<uint8_t>(c->stage) + f0 * kSlotBytes;
         CZ_CUDA(c, cudaStreamWaitEvent(cs, c->ev_h2d[i], 0));
+        CzChunks chunks;
+        chunks.at(P<long long>(c->in_off) + f0, P<int>(c->in_len) + f0, P<long long>(c->lz_off) + f0, job.lz_slot);
         CZ_CUDA(c, cz_launch_encode(p->wtype, P<CzField>(c->fields) + i, 1, n, p->zerobits, p->shuffle ? 1 : 0, stage,
-                                    P<int>(c->rec_bytes) + f0, queues + i, std::min(n, c->sms), cs,
-                                    maps_of(c, nslab) + i, nullptr, P<int>(c->flag) + 1));
-        CZ_CUDA(c, cz_launch_chunk_setup(1, n, n, P<int>(c->rec_bytes) + f0, P<long long>(c->in_off) + f0,
-                                         P<int>(c->in_len) + f0, nullptr, P<long long>(c->lz_off) + f0, job.lz_slot,
-                                         cs));
+                                    P<int>(c->rec_bytes) + f0, &ctl->queue[i], std::min(n, c->sms), cs,
+                                    maps_of(c, nslab) + i, nullptr, &ctl->flag[1], 0, chunks));
         CZ_CUDA(c, cudaEventRecord(c->ev_enc[i], cs));
         const uint8_t *src = stage;
         const long long *src_off = P<long long>(c->in_off) + f0;
@@ -1260,7 +1275,6 @@ int cz_compress_to_image(cz_ctx *c, const float *h_field, int nx, int ny, int nz
             CZ_CUDA(c, cz_launch_lz4_encode(stage, src_off, len, n, lzo, P<long long>(c->lz_off) + f0,
                                             P<int>(c->lz_len) + f0, p->shuffle ? 1 : 0, 16, lzgrid, ls,
                                             P<int4>(c->lz_hole) + f0, c->lz_effort));
-            CZ_CUDA(c, cz_launch_neg_reduce(P<int>(c->lz_len) + f0, n, P<int>(c->flag), ls));
             CZ_CUDA(c, cudaEventRecord(c->ev_lz[i], ls));
             src = lzo;
             src_off = P<long long>(c->lz_off) + f0;
@@ -1269,8 +1283,8 @@ int cz_compress_to_image(cz_ctx *c, const float *h_field, int nx, int ny, int nz
         }
         CZ_CUDA(c, cudaStreamWaitEvent(c->s_gather, ready, 0));
         CZ_CUDA(c, cz_launch_scan_from(len, n, P<long long>(c->out_off) + f0, c->s_gather));
-        CZ_CUDA(c, cz_launch_gather(src, src_off, len, n, dst, P<long long>(c->out_off) + f0, c->s_gather,
-                                    lz4 ? P<int4>(c->lz_hole) + f0 : nullptr, stage, P<long long>(c->in_off) + f0));
+        CZ_CUDA(c, cz_launch_gather(src, src_off, len, n, dst, P<long long>(c->out_off) + f0, false, &ctl->flag[0],
+                                    nullptr, c->s_gather, lz4 ? P<int4>(c->lz_hole) + f0 : nullptr, stage, P<long long>(c->in_off) + f0));
     }
     CZ_CUDA(c, cudaEventRecord(c->ev_join, c->s_gather));
     CZ_CUDA(c, cudaStreamWaitEvent(st, c->ev_join, 0));
@@ -1279,7 +1293,7 @@ int cz_compress_to_image(cz_ctx *c, const float *h_field, int nx, int ny, int nz
     int flag[2] = {0, 0};
     CZ_CUDA(c, cudaMemcpyAsync(off.data(), c->out_off.p, sizeof(long long) * (job.nchunks + 1), cudaMemcpyDeviceToHost,
                                st));
-    CZ_CUDA(c, cudaMemcpyAsync(flag, c->flag.p, 8, cudaMemcpyDeviceToHost, st));
+    CZ_CUDA(c, cudaMemcpyAsync(flag, ctl, 8, cudaMemcpyDeviceToHost, st));
     CZ_CUDA(c, cudaStreamSynchronize(st));
     if (flag[1] != 0) return fail(c, CZ_E_CUDA, "wavelet kernel: a tile copy did not complete");
     if (flag[0] != 0) return fail(c, CZ_E_CUDA, "LZ4 encoder output exceeded its bound");

@@ -322,12 +322,23 @@ struct Payload {
     bool shuffle;
 };
 
+// By one thread, once record g's size is known.
+__device__ __forceinline__ void record_done(const CzChunks &ch, long long g, int nb)
+{
+    if (ch.in_off) {
+        ch.in_off[g] = g * (long long)kSlotBytes;
+        ch.in_len[g] = 4 + nb;
+        ch.lz_off[g] = g * ch.lz_slot;
+    }
+    if (ch.raw_total) atomicAdd(ch.raw_total, (unsigned long long)(4 + nb));
+}
+
 // Record emission for block g once its coefficients sit in s.sb and its run
 // masks in s.seg*/s.mask32: [int32 nbytes][mask][survivors in the reference
 // order, zero-bits applied, byte planes when shuffling]
 // (WaveletCompressor.cpp:152-182, SerializerIO_WaveletCompression_MPI_Simple.h:236-240).
 __device__ __forceinline__ void emit_record(const Shared &s, long long g, uint32_t zmask, int shuffle, uint8_t *stage,
-                                            int *rec_bytes)
+                                            int *rec_bytes, const CzChunks &chunks)
 {
     // ---- offsets of every run, record header and mask
     const int S = scan_segments(s);
@@ -336,6 +347,7 @@ __device__ __forceinline__ void emit_record(const Shared &s, long long g, uint32
     if (threadIdx.x == 0) {
         *reinterpret_cast<int *>(slot) = nb;
         rec_bytes[g] = nb;
+        record_done(chunks, g, nb);
     }
     for (int i = threadIdx.x; i < kMaskBytes / 4; i += kNT)
         reinterpret_cast<uint32_t *>(slot + 4)[i] = s.mask32[i];

@@ -265,7 +265,7 @@ template <int KIND, bool AHEAD>
 __global__ void __launch_bounds__(kNT, 1)
 encode_kernel(const CzField *fields, int nfields, long long total_blocks, int zerobits, int shuffle, uint8_t *stage,
               int *rec_bytes, unsigned long long *queue, const __grid_constant__ CUtensorMap map0,
-              const CUtensorMap *maps, int *err)
+              const CUtensorMap *maps, int *err, CzChunks chunks)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -447,6 +447,7 @@ encode_kernel(const CzField *fields, int nfields, long long total_blocks, int ze
         if (threadIdx.x == 0) {
             *reinterpret_cast<int *>(rec) = nb;
             rec_bytes[g] = nb;
+            record_done(chunks, g, nb);
         }
         for (int i = threadIdx.x; i < kMaskBytes / 4; i += kNT) reinterpret_cast<uint32_t *>(rec + 4)[i] = mask32[i];
         {
@@ -610,9 +611,9 @@ __device__ __forceinline__ void unpack16(uint32_t p, unsigned bits, float (&v)[3
 
 template <int KIND, bool DIFF>
 __global__ void __launch_bounds__(kNT, 1)
-decode_kernel(const CzField *fields, int nfields, long long total_blocks, int shuffle, const uint8_t *base,
-              const long long *rec_off, int *status, unsigned long long *queue, const float *diff_ref,
-              double *diff_out, CzPlanes planes, const CUtensorMap *maps)
+decode_kernel(const CzField *fields, int nfields, long long total_blocks, int shuffle, CzRecords where, int *flag,
+              unsigned long long *queue, const float *diff_ref, double *diff_out, CzPlanes planes,
+              const CUtensorMap *maps)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -624,9 +625,9 @@ decode_kernel(const CzField *fields, int nfields, long long total_blocks, int sh
     // Record of block n of the CTA's sequence in two steps, so that none of
     // the dependent loads (offset, byte count, mask) waits on its own: where
     // it is ...
-    auto find = [&](uint32_t n, long long ro, int nb, const int4 &hole, long long src_off) {
-        const uint8_t *rec = base + (ro < 0 ? 0 : ro), *q12 = nullptr;
-        const bool ok = nb >= kMaskBytes && nb <= kMaxRecord + 4;
+    auto find = [&](uint32_t n, long long ro, long long len, int nb, const int4 &hole, long long src_off) {
+        const uint8_t *rec = where.base + (ro < 0 ? 0 : ro), *q12 = nullptr;
+        const bool ok = nb >= kMaskBytes && nb <= kMaxRecord + 4 && 4 + nb <= len;
         // byte planes 1 and 2 where the LZ4 stage left them in its input
         const int c4 = (nb - kMaskBytes) / 4;
         if (ok && hole.z > 0 && hole.z == 2 * c4 && hole.x == 4 + kMaskBytes + c4) q12 = planes.src + src_off + hole.y;
@@ -648,16 +649,28 @@ decode_kernel(const CzField *fields, int nfields, long long total_blocks, int sh
     // and used in a later one
     const bool scout = threadIdx.x == 32 * (kNW - 1);
     unsigned long long s_ticket = 0;
-    long long s_off = -1, s_src = 0;
+    long long s_off = -1, s_len = 0, s_src = 0;  // s_len: bytes from there on that can be the record's
     int s_nb = -1;
     int4 s_hole = make_int4(0, 0, 0, 0);
     auto scout_off = [&](uint32_t n) {
         const long long g = blk[n & 3].g;
-        s_off = g >= 0 ? rec_off[g] : -1;
+        s_off = -1;
+        s_len = 0x7fffffff;
+        if (g < 0) return;
+        if (where.rec_off) {
+            s_off = where.rec_off[g];
+        } else if (where.cap) {
+            s_off = g * where.cap;
+            s_len = where.dec_len[g];
+        } else {
+            s_off = where.off[g];
+            s_len = where.off[g + 1] - s_off;
+        }
+        if (s_len < 4 || s_len > 0x7fffffff) s_off = -1;
     };
     auto scout_rec = [&](uint32_t n) {
         const long long g = blk[n & 3].g;
-        s_nb = s_off >= 0 ? *reinterpret_cast<const int *>(base + s_off) : -1;
+        s_nb = s_off >= 0 ? *reinterpret_cast<const int *>(where.base + s_off) : -1;
         if (g >= 0 && holes) {
             s_hole = planes.hole[g];
             s_src = planes.src_off[g];
@@ -668,7 +681,7 @@ decode_kernel(const CzField *fields, int nfields, long long total_blocks, int sh
         take_ticket(blk, fields, nfields, total_blocks, queue);
         scout_off(0);
         scout_rec(0);
-        find(0, s_off, s_nb, s_hole, s_src);
+        find(0, s_off, s_len, s_nb, s_hole, s_src);
     }
     __syncthreads();
     if (blk[0].g < 0) return;
@@ -676,7 +689,7 @@ decode_kernel(const CzField *fields, int nfields, long long total_blocks, int sh
         take_second(blk + 1, fields, nfields, total_blocks, queue);
         scout_off(1);
         scout_rec(1);
-        find(1, s_off, s_nb, s_hole, s_src);
+        find(1, s_off, s_len, s_nb, s_hole, s_src);
     } else if (warp < kNW - 1) {
         fetch(0, threadIdx.x, kNT - 32);
     }
@@ -723,7 +736,7 @@ decode_kernel(const CzField *fields, int nfields, long long total_blocks, int sh
         if (nel - expected == 1) nel--;  // :247-250
         const bool ok = size_ok && nel == expected && !bad[it & 1];
         if (threadIdx.x == 0) {
-            status[g] = ok ? 0 : -1;
+            if (!ok) atomicMin(flag, -1);
             bad[(it + 1) & 1] = 0;
         }
         // ---- load (FullWaveletTransform.h:99-150): the survivors of every
@@ -878,7 +891,7 @@ decode_kernel(const CzField *fields, int nfields, long long total_blocks, int sh
             for (int j = 0; j < 32; ++j) at(sm, slab + j * 128 + lane * 4) = v[j];
         }
         __syncthreads();
-        if (scout) find(it + 2, s_off, s_nb, s_hole, s_src);
+        if (scout) find(it + 2, s_off, s_len, s_nb, s_hole, s_src);
         // ---- level 32, y then x: planes z = warp and warp + 16, then straight
         // to the field (copy_to, WaveletCompressor.h:73-82)
         DiffAcc acc;
@@ -1002,33 +1015,34 @@ template <int KIND>
 static cudaError_t launch_encode(const CzField *fields, int nfields, long long total_blocks, int zerobits,
                                  int shuffle, uint8_t *stage, int *rec_bytes, unsigned long long *queue, int grid,
                                  cudaStream_t st, const CUtensorMap *maps, const CUtensorMap &map0, int *err,
-                                 int variant)
+                                 int variant, const CzChunks &chunks)
 {
     auto k = variant == 1 ? encode_kernel<KIND, false> : encode_kernel<KIND, true>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCodecSmem);
     if (e != cudaSuccess) return e;
     k<<<grid, kNT, kCodecSmem, st>>>(fields, nfields, total_blocks, zerobits, shuffle, stage, rec_bytes, queue, map0,
-                                     maps, err);
+                                     maps, err, chunks);
     return cudaGetLastError();
 }
 
 template <int KIND>
 static cudaError_t launch_decode(const CzField *fields, int nfields, long long total_blocks, int shuffle,
-                                 const uint8_t *base, const long long *rec_off, int *status,
-                                 unsigned long long *queue, int grid, cudaStream_t st, const CUtensorMap *maps,
-                                 const float *diff_ref, double *diff_out, CzPlanes planes)
+                                 const CzRecords &recs, int *flag, unsigned long long *queue, int grid,
+                                 cudaStream_t st, const CUtensorMap *maps, const float *diff_ref, double *diff_out,
+                                 CzPlanes planes)
 {
     auto k = diff_ref ? decode_kernel<KIND, true> : decode_kernel<KIND, false>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCodecSmem);
     if (e != cudaSuccess) return e;
-    k<<<grid, kNT, kCodecSmem, st>>>(fields, nfields, total_blocks, shuffle, base, rec_off, status, queue, diff_ref,
-                                     diff_out, planes, maps);
+    k<<<grid, kNT, kCodecSmem, st>>>(fields, nfields, total_blocks, shuffle, recs, flag, queue, diff_ref, diff_out,
+                                     planes, maps);
     return cudaGetLastError();
 }
 
 cudaError_t cz_launch_encode(int wtype, const CzField *fields, int nfields, long long total_blocks, int zerobits,
                              int shuffle, uint8_t *stage, int *rec_bytes, unsigned long long *queue, int grid,
-                             cudaStream_t st, const CUtensorMap *maps, const CUtensorMap *map0, int *err, int variant)
+                             cudaStream_t st, const CUtensorMap *maps, const CUtensorMap *map0, int *err, int variant,
+                             CzChunks chunks)
 {
     if (!maps && !map0) return cudaErrorInvalidValue;
     CUtensorMap own = {};
@@ -1036,31 +1050,30 @@ cudaError_t cz_launch_encode(int wtype, const CzField *fields, int nfields, long
     switch (wkind(wtype)) {
     case 1:
         return launch_encode<1>(fields, nfields, total_blocks, zerobits, shuffle, stage, rec_bytes, queue, grid, st,
-                                maps, own, err, variant);
+                                maps, own, err, variant, chunks);
     case 2:
         return launch_encode<2>(fields, nfields, total_blocks, zerobits, shuffle, stage, rec_bytes, queue, grid, st,
-                                maps, own, err, variant);
+                                maps, own, err, variant, chunks);
     default:
         return launch_encode<3>(fields, nfields, total_blocks, zerobits, shuffle, stage, rec_bytes, queue, grid, st,
-                                maps, own, err, variant);
+                                maps, own, err, variant, chunks);
     }
 }
 
 cudaError_t cz_launch_decode(int wtype, const CzField *fields, int nfields, long long total_blocks, int shuffle,
-                             const uint8_t *base, const long long *rec_off, int *status, unsigned long long *queue,
-                             int grid, cudaStream_t st, const CUtensorMap *maps, const float *diff_ref,
-                             double *diff_out, CzPlanes planes)
+                             CzRecords recs, int *flag, unsigned long long *queue, int grid, cudaStream_t st,
+                             const CUtensorMap *maps, const float *diff_ref, double *diff_out, CzPlanes planes)
 {
     switch (wkind(wtype)) {
     case 1:
-        return launch_decode<1>(fields, nfields, total_blocks, shuffle, base, rec_off, status, queue, grid, st, maps,
-                                diff_ref, diff_out, planes);
+        return launch_decode<1>(fields, nfields, total_blocks, shuffle, recs, flag, queue, grid, st, maps, diff_ref,
+                                diff_out, planes);
     case 2:
-        return launch_decode<2>(fields, nfields, total_blocks, shuffle, base, rec_off, status, queue, grid, st, maps,
-                                diff_ref, diff_out, planes);
+        return launch_decode<2>(fields, nfields, total_blocks, shuffle, recs, flag, queue, grid, st, maps, diff_ref,
+                                diff_out, planes);
     default:
-        return launch_decode<3>(fields, nfields, total_blocks, shuffle, base, rec_off, status, queue, grid, st, maps,
-                                diff_ref, diff_out, planes);
+        return launch_decode<3>(fields, nfields, total_blocks, shuffle, recs, flag, queue, grid, st, maps, diff_ref,
+                                diff_out, planes);
     }
 }
 

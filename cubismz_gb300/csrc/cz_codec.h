@@ -20,6 +20,25 @@ struct CzField {
 // must be 16-byte aligned.
 bool cz_field_map(const CzField &f, CUtensorMap *map);
 
+// Where a record's kernel leaves what follows it in the pipeline (all
+// optional, indexed by block): the record as a one-record chunk (input offset
+// in the staging area, length, offset of the chunk's lossless output), and the
+// sum of the records' framed bytes.
+struct CzChunks {
+    long long *in_off = nullptr;
+    int *in_len = nullptr;
+    long long *lz_off = nullptr;
+    long long lz_slot = 0;
+    unsigned long long *raw_total = nullptr;
+    void at(long long *off, int *len, long long *lz, long long slot)
+    {
+        in_off = off;
+        in_len = len;
+        lz_off = lz;
+        lz_slot = slot;
+    }
+};
+
 // maps: the fields' tensor maps in device memory (64-byte aligned), or
 // nullptr with map0 (host) for a single field. err (optional, device): set
 // to 1 if a tile copy did not complete in time.
@@ -28,9 +47,20 @@ bool cz_field_map(const CzField &f, CUtensorMap *map);
 cudaError_t cz_launch_encode(int wtype, const CzField *fields, int nfields, long long total_blocks, int zerobits,
                              int shuffle, uint8_t *stage, int *rec_bytes, unsigned long long *queue, int grid,
                              cudaStream_t st, const CUtensorMap *maps, const CUtensorMap *map0, int *err,
-                             int variant = 0);
-// Record of block g at base + rec_off[g] ([int32 nbytes][record]); a
-// negative rec_off marks a block whose record is missing (status -1).
+                             int variant = 0, CzChunks chunks = CzChunks());
+// Where a launch's records are: block g's [int32 nbytes][record] at base +
+// rec_off[g] (negative: missing); or, without rec_off, one record per chunk:
+// chunk g at base + off[g], off[g + 1] - off[g] bytes (raw chunks, cap == 0), or
+// at base + g * cap with dec_len[g] bytes (decoded chunks).
+struct CzRecords {
+    const uint8_t *base = nullptr;
+    const long long *rec_off = nullptr;
+    const long long *off = nullptr;
+    const int *dec_len = nullptr;
+    long long cap = 0;
+};
+// A missing or malformed record leaves its block as decoded from an empty one
+// and sets *flag to -1.
 // diff_ref (optional, a field of the same geometry as fields[0]): per-block
 // error statistics into diff_out[8*g] (cz2diff's quantities). maps as for
 // cz_launch_encode (device memory).
@@ -43,8 +73,8 @@ struct CzPlanes {
     const long long *src_off = nullptr;
 };
 cudaError_t cz_launch_decode(int wtype, const CzField *fields, int nfields, long long total_blocks, int shuffle,
-                             const uint8_t *base, const long long *rec_off, int *status, unsigned long long *queue,
-                             int grid, cudaStream_t st, const CUtensorMap *maps, const float *diff_ref = nullptr,
+                             CzRecords recs, int *flag, unsigned long long *queue, int grid, cudaStream_t st,
+                             const CUtensorMap *maps, const float *diff_ref = nullptr,
                              double *diff_out = nullptr, CzPlanes planes = CzPlanes());
 cudaError_t cz_launch_diff_total(const double *per_block, long long nblocks, double *total, cudaStream_t st);
 
@@ -60,7 +90,7 @@ cudaError_t cz_launch_iwt_adjoint(int wtype, const float *in, float *coef, long 
 size_t cz_refit_scratch_floats(int grid);
 cudaError_t cz_launch_refit(int wtype, const CzField *fields, int nfields, long long total_blocks, int zerobits,
                             int shuffle, int iters, uint8_t *stage, int *rec_bytes, unsigned long long *queue,
-                            float *scratch, int grid, cudaStream_t st);
+                            float *scratch, int grid, cudaStream_t st, CzChunks chunks = CzChunks());
 
 // LZ4 stage (cz_lz4.cu). Chunk c's input is in[in_off[c] .. in_off[c]+in_len[c]);
 // the encoder reads it as aligned words, so in + in_off[c] must be a multiple
@@ -102,16 +132,22 @@ cudaError_t cz_launch_deflate(const uint8_t *in, const long long *in_off, const 
 // byte planes 1 and 2 when one literal run covers them whole -- the decoder
 // then leaves that span of its output unwritten and the record's reader
 // takes it from the input (CzPlanes); length 0 otherwise.
+// in_len == nullptr: chunk c is in[in_off[c] .. in_off[c + 1]); out_off ==
+// nullptr: its output goes to out + c * cap, cap bytes at most.
 cudaError_t cz_launch_lz4_decode(const uint8_t *in, const long long *in_off, const int *in_len, int nchunks,
                                  uint8_t *out, const long long *out_off, const int *out_cap, int *out_len,
-                                 cudaStream_t st, int4 *hole = nullptr);
+                                 cudaStream_t st, int4 *hole = nullptr, long long cap = 0);
 
 // Stream assembly helpers (cz_lz4.cu, cz_stream.cu)
-// With hole (from cz_launch_lz4_encode): the span of each chunk that the
-// encoder left unwritten comes from hsrc + hsrc_off[c] + hole[c].y.
+// Chunk payloads back to back at dst + dst_off[c]. With scan, dst_off[0..n] is
+// worked out here first (from 0), without it is given. A negative length sets
+// *flag to -1; *total gets the payload's size (both optional). With hole (from
+// cz_launch_lz4_encode): the span of each chunk that the encoder left
+// unwritten comes from hsrc + hsrc_off[c] + hole[c].y.
 cudaError_t cz_launch_gather(const uint8_t *src, const long long *src_off, const int *len, int nchunks,
-                             uint8_t *dst, const long long *dst_off, cudaStream_t st, const int4 *hole = nullptr,
-                             const uint8_t *hsrc = nullptr, const long long *hsrc_off = nullptr);
+                             uint8_t *dst, long long *dst_off, bool scan, int *flag, long long *total,
+                             cudaStream_t st, const int4 *hole = nullptr, const uint8_t *hsrc = nullptr,
+                             const long long *hsrc_off = nullptr);
 // Chunk layout of the encode side: chunk c holds blocks [c*bpc, (c+1)*bpc).
 // Fills in_off/in_len (chunk inputs in chunk_in, or in the slots when bpc=1),
 // blk_dst (where block g's [nbytes][record] goes inside chunk_in) and lz_off.
@@ -121,17 +157,14 @@ cudaError_t cz_launch_chunk_setup(int bpc, long long nblocks, int nchunks, const
 // Copies block g's [nbytes][record] from its slot to chunk_in + blk_dst[g].
 cudaError_t cz_launch_pack_records(const uint8_t *stage, const int *rec_bytes, long long nblocks,
                                    const long long *blk_dst, uint8_t *chunk_in, cudaStream_t st);
-// Exclusive scan of len[0..n) into off[0..n], off[n] = total (n <= 2^31).
-cudaError_t cz_launch_scan(const int *len, int n, long long *off, cudaStream_t st);
-// The same starting from the value already in off[0] (a running total).
+// Exclusive scan of len[0..n) into off[0..n], off[n] = total (n <= 2^31),
+// starting from the value already in off[0] (a running total).
 cudaError_t cz_launch_scan_from(const int *len, int n, long long *off, cudaStream_t st);
 // Decode side: walks the [nbytes] headers of each decoded chunk (chunk c at
 // base + c*chunk_cap, dec_len[c] bytes) and records where every block's
-// record starts (rec_off, relative to base); -1 and status -1 on a short or
-// malformed chunk. src_off/src_len, if not NULL, give raw (not LZ4) chunks.
+// record starts (rec_off, relative to base); -1 on a short or malformed chunk.
 cudaError_t cz_launch_locate_records(int bpc, long long nblocks, int nchunks, const long long *chunk_base,
-                                     const int *dec_len, long long *rec_off, int *status, const uint8_t *base,
-                                     cudaStream_t st);
+                                     const int *dec_len, long long *rec_off, const uint8_t *base, cudaStream_t st);
 cudaError_t cz_launch_decode_setup(int nchunks, const long long *off, int *in_len, long long *dec_off, int *dec_cap,
                                    long long cap, int raw, cudaStream_t st);
 cudaError_t cz_launch_chunk_records(int nchunks, int maxsub, const long long *chunk_base, const int *dec_len,
@@ -139,8 +172,6 @@ cudaError_t cz_launch_chunk_records(int nchunks, int maxsub, const long long *ch
 cudaError_t cz_launch_map_blocks(long long nblocks, int nchunks, int maxsub, const int *block_chunk,
                                  const int *block_subid, const long long *chunk_rec, long long *rec_off,
                                  cudaStream_t st);
-cudaError_t cz_launch_status_reduce(const int *status, long long n, int *flag, cudaStream_t st);
-cudaError_t cz_launch_neg_reduce(const int *v, int n, int *flag, cudaStream_t st);
 cudaError_t cz_launch_rebase(long long *off, int n, long long base, cudaStream_t st);
 
 // Layout of the reference's HDF5 tools (cz_ingest.cu): z-fastest arrays with
@@ -154,4 +185,5 @@ cudaError_t cz_launch_to_zfastest(const float *in, int nx, int ny, int nz, int n
 
 // zlib streams (cz_zlib.cu): one warp per chunk; out_len[c] = bytes or < 0.
 cudaError_t cz_launch_inflate(const uint8_t *in, const long long *in_off, const int *in_len, int nchunks, uint8_t *out,
-                              const long long *out_off, const int *out_cap, int *out_len, int grid, cudaStream_t st);
+                              const long long *out_off, const int *out_cap, int *out_len, int grid, cudaStream_t st,
+                              long long cap = 0);

@@ -648,6 +648,14 @@ __device__ __forceinline__ void cta_copy(uint8_t *__restrict__ d, const uint8_t 
     if ((int)threadIdx.x < t) d[h + 16 * nwd + threadIdx.x] = s2[16 * nwd + threadIdx.x];
 }
 
+// Input bytes of chunk c, -1 for a length that cannot be.
+__device__ __forceinline__ int chunk_len(const long long *in_off, const int *in_len, int c)
+{
+    if (in_len) return in_len[c];
+    const long long n = in_off[c + 1] - in_off[c];
+    return n < 0 || n > 0x7fffffffLL ? -1 : (int)n;
+}
+
 // One CTA per chunk, for few chunks. The chunk is one serial chain of sequences, each of a few
 // bytes; what bounds a decoder is that chain and, with many chunks, issue.
 // Both want many sequences per step, so a step takes kDecIn input bytes:
@@ -749,7 +757,7 @@ struct LzDecShared {
 __global__ void __launch_bounds__(kDecThreads, 3)
 lz4_decode_wide_kernel(const uint8_t *__restrict__ in, const long long *in_off, const int *in_len, int nchunks,
                   uint8_t *__restrict__ out, const long long *out_off, const int *out_cap, int *out_len,
-                  int4 *hole)
+                  int4 *hole, long long cap)
 {
     extern __shared__ __align__(16) unsigned char lz_dec_smem[];
     LzDecShared &s = *reinterpret_cast<LzDecShared *>(lz_dec_smem);
@@ -757,9 +765,9 @@ lz4_decode_wide_kernel(const uint8_t *__restrict__ in, const long long *in_off, 
     uint8_t *ring = s.ring;
     for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
         const uint8_t *src = in + in_off[c];
-        const int iend = in_len[c];
-        uint8_t *dst = out + out_off[c];
-        const int oend = out_cap[c];
+        const int iend = chunk_len(in_off, in_len, c);
+        uint8_t *dst = out + (out_off ? out_off[c] : c * cap);
+        const int oend = out_off ? out_cap[c] : (int)cap;
         int s0 = 0, op = 0, err = 0, ring_lo = 0;  // output before ring_lo is not in the ring
         bool done = false;
         LzHole hl;
@@ -1242,7 +1250,7 @@ __device__ __forceinline__ void copy_match_old(uint8_t *ring, int ms, int off, i
 __global__ void __launch_bounds__(128)
 lz4_decode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const int *in_len, int nchunks,
                   uint8_t *__restrict__ out, const long long *out_off, const int *out_cap, int *out_len,
-                  int4 *hole)
+                  int4 *hole, long long cap)
 {
     __shared__ int4 cand_all[4][kWin];           // (literal start, literal length, match length, flags)
     __shared__ int next_all[4][kWin];            // input position after the candidate's sequence
@@ -1260,9 +1268,9 @@ lz4_decode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
     for (int c = gw; c < nchunks; c += nw) {
         const uint8_t *src = in + in_off[c];
-        const int iend = in_len[c];
-        uint8_t *dst = out + out_off[c];
-        const int oend = out_cap[c];
+        const int iend = chunk_len(in_off, in_len, c);
+        uint8_t *dst = out + (out_off ? out_off[c] : c * cap);
+        const int oend = out_off ? out_cap[c] : (int)cap;
         int s0 = 0, op = 0, err = 0, ring_lo = 0;  // output before ring_lo is not in the ring
         bool done = false;
         LzHole hl;
@@ -1552,16 +1560,42 @@ lz4_decode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
 // One CTA per chunk: the chunk's bytes to dst + dst_off[c]. With `hole`
 // (LZ4 of block records), bytes [hole.x, hole.x + hole.z) of the chunk's
 // output are the input bytes at hsrc + hsrc_off[c] + hole.y, which the
-// encoder left unwritten.
-__global__ void gather_kernel(const uint8_t *__restrict__ src, const long long *src_off, const int *len,
-                              uint8_t *__restrict__ dst, const long long *dst_off, const int4 *hole,
-                              const uint8_t *__restrict__ hsrc, const long long *hsrc_off)
+// encoder left unwritten. SCAN: the chunk sums the lengths before its own and
+// writes its offset (for chunk counts where that is cheaper than a launch).
+template <bool SCAN>
+__global__ void __launch_bounds__(256)
+gather_kernel(const uint8_t *__restrict__ src, const long long *src_off, const int *len, int nchunks,
+              uint8_t *__restrict__ dst, long long *dst_off, int *flag, long long *total, const int4 *hole,
+              const uint8_t *__restrict__ hsrc, const long long *hsrc_off)
 {
     const int c = blockIdx.x;
     const int n = len[c];
+    long long at;
+    if (SCAN) {
+        __shared__ long long part[8];
+        long long sum = 0;
+        for (int i = threadIdx.x; i < c; i += 256) sum += len[i];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sum;
+        __syncthreads();
+        at = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) at += part[w];
+        if (threadIdx.x == 0) dst_off[c] = at;
+    } else {
+        at = dst_off[c];
+    }
+    if (threadIdx.x == 0) {
+        if (n < 0 && flag) atomicMin(flag, -1);
+        if (c == nchunks - 1) {
+            if (SCAN) dst_off[nchunks] = at + n;
+            if (total) *total = at + n;
+        }
+    }
     if (n <= 0) return;
     const uint8_t *s = src + src_off[c];
-    uint8_t *d = dst + dst_off[c];
+    uint8_t *d = dst + at;
     const int4 hl = hole ? hole[c] : make_int4(0, 0, 0, 0);
     if (hl.z > 0) {
         cta_copy(d, s, hl.x);
@@ -1675,7 +1709,7 @@ constexpr int kWideChunksPerSm = 8;
 
 cudaError_t cz_launch_lz4_decode(const uint8_t *in, const long long *in_off, const int *in_len, int nchunks,
                                  uint8_t *out, const long long *out_off, const int *out_cap, int *out_len,
-                                 cudaStream_t st, int4 *hole)
+                                 cudaStream_t st, int4 *hole, long long cap)
 {
     if (nchunks <= 0) return cudaSuccess;
     const int sms = sm_count();
@@ -1685,19 +1719,28 @@ cudaError_t cz_launch_lz4_decode(const uint8_t *in, const long long *in_off, con
             cudaFuncSetAttribute(lz4_decode_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
         if (e != cudaSuccess) return e;
         lz4_decode_wide_kernel<<<std::min(nchunks, 3 * sms), kDecThreads, sm, st>>>(in, in_off, in_len, nchunks, out,
-                                                                                   out_off, out_cap, out_len, hole);
+                                                                                   out_off, out_cap, out_len, hole, cap);
     } else {
         lz4_decode_kernel<<<std::min((nchunks + 3) / 4, 8 * sms), 128, 0, st>>>(in, in_off, in_len, nchunks, out, out_off,
-                                                                               out_cap, out_len, hole);
+                                                                               out_cap, out_len, hole, cap);
     }
     return cudaGetLastError();
 }
 
 cudaError_t cz_launch_gather(const uint8_t *src, const long long *src_off, const int *len, int nchunks,
-                             uint8_t *dst, const long long *dst_off, cudaStream_t st, const int4 *hole,
-                             const uint8_t *hsrc, const long long *hsrc_off)
+                             uint8_t *dst, long long *dst_off, bool scan, int *flag, long long *total,
+                             cudaStream_t st, const int4 *hole, const uint8_t *hsrc, const long long *hsrc_off)
 {
     if (nchunks <= 0) return cudaSuccess;
-    gather_kernel<<<nchunks, 256, 0, st>>>(src, src_off, len, dst, dst_off, hole, hsrc, hsrc_off);
+    // summed per chunk up to 1024 chunks: at most 4 KB of lengths per CTA
+    // (a scan launch of its own costs 4 us)
+    const bool own = scan && nchunks <= 1024;
+    if (scan && !own) {
+        cudaError_t e = cudaMemsetAsync(dst_off, 0, sizeof(long long), st);
+        if (e == cudaSuccess) e = cz_launch_scan_from(len, nchunks, dst_off, st);
+        if (e != cudaSuccess) return e;
+    }
+    auto k = own ? gather_kernel<true> : gather_kernel<false>;
+    k<<<nchunks, 256, 0, st>>>(src, src_off, len, nchunks, dst, dst_off, flag, total, hole, hsrc, hsrc_off);
     return cudaGetLastError();
 }

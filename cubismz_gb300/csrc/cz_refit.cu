@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(kNT, 1) iwt_adjoint_kernel(const float *in, fl
 template <int KIND>
 __global__ void __launch_bounds__(kNT, 1)
 refit_kernel(const CzField *fields, int nfields, long long total_blocks, int zerobits, int shuffle, int iters,
-             uint8_t *stage, int *rec_bytes, unsigned long long *queue, float *scratch)
+             uint8_t *stage, int *rec_bytes, unsigned long long *queue, float *scratch, CzChunks chunks)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const Shared s = carve(smem);
@@ -495,7 +495,7 @@ refit_kernel(const CzField *fields, int nfields, long long total_blocks, int zer
             sb[a + 3] = cv.w;
         }
         __syncthreads();
-        emit_record(s, g, zmask, shuffle, stage, rec_bytes);
+        emit_record(s, g, zmask, shuffle, stage, rec_bytes, chunks);
     }
 }
 
@@ -556,7 +556,7 @@ cudaError_t cz_launch_iwt_adjoint(int wtype, const float *in, float *coef, long 
 
 cudaError_t cz_launch_refit(int wtype, const CzField *fields, int nfields, long long total_blocks, int zerobits,
                             int shuffle, int iters, uint8_t *stage, int *rec_bytes, unsigned long long *queue,
-                            float *scratch, int grid, cudaStream_t st)
+                            float *scratch, int grid, cudaStream_t st, CzChunks chunks)
 {
     if (total_blocks <= 0) return cudaSuccess;
     const int smem = kSmBytes;
@@ -565,17 +565,17 @@ cudaError_t cz_launch_refit(int wtype, const CzField *fields, int nfields, long 
     case 1:
         if ((e = prep(refit_kernel<1>, smem)) != cudaSuccess) return e;
         refit_kernel<1><<<grid, kNT, smem, st>>>(fields, nfields, total_blocks, zerobits, shuffle, iters, stage,
-                                                 rec_bytes, queue, scratch);
+                                                 rec_bytes, queue, scratch, chunks);
         break;
     case 2:
         if ((e = prep(refit_kernel<2>, smem)) != cudaSuccess) return e;
         refit_kernel<2><<<grid, kNT, smem, st>>>(fields, nfields, total_blocks, zerobits, shuffle, iters, stage,
-                                                 rec_bytes, queue, scratch);
+                                                 rec_bytes, queue, scratch, chunks);
         break;
     default:
         if ((e = prep(refit_kernel<3>, smem)) != cudaSuccess) return e;
         refit_kernel<3><<<grid, kNT, smem, st>>>(fields, nfields, total_blocks, zerobits, shuffle, iters, stage,
-                                                 rec_bytes, queue, scratch);
+                                                 rec_bytes, queue, scratch, chunks);
     }
     return cudaGetLastError();
 }

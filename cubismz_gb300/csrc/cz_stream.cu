@@ -19,10 +19,10 @@ __global__ void chunk_setup_kernel(int bpc, long long nblocks, int nchunks, cons
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nchunks) return;
     const long long g0 = (long long)c * bpc;
-    const long long base = bpc == 1 ? g0 * kSlotBytes : (long long)c * bpc * kSlotBytes;
+    const long long base = g0 * kSlotBytes;
     long long acc = 0;
     for (long long g = g0; g < g0 + bpc && g < nblocks; ++g) {
-        if (blk_dst) blk_dst[g] = base + acc;
+        blk_dst[g] = base + acc;
         acc += 4 + rec_bytes[g];
     }
     in_off[c] = base;
@@ -51,13 +51,14 @@ __global__ void pack_records_kernel(const uint8_t *__restrict__ stage, const int
     }
 }
 
-// Single-CTA exclusive scan (chunk counts are at most a few hundred thousand).
-__global__ void __launch_bounds__(1024) scan_kernel(const int *len, int n, long long *off, int carry_in)
+// Single-CTA exclusive scan from off[0] on (chunk counts are at most a few
+// hundred thousand).
+__global__ void __launch_bounds__(1024) scan_kernel(const int *len, int n, long long *off)
 {
     __shared__ long long warp_sum[32];
     __shared__ long long carry;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) carry = carry_in ? off[0] : 0;
+    if (threadIdx.x == 0) carry = off[0];
     __syncthreads();
     for (int base = 0; base < n; base += 1024) {
         const int i = base + threadIdx.x;
@@ -91,7 +92,7 @@ __global__ void __launch_bounds__(1024) scan_kernel(const int *len, int n, long 
 
 // One thread per chunk walks its records (lz4.c output or raw chunk).
 __global__ void locate_records_kernel(int bpc, long long nblocks, int nchunks, const long long *chunk_base,
-                                      const int *dec_len, long long *rec_off, int *status, const uint8_t *base)
+                                      const int *dec_len, long long *rec_off, const uint8_t *base)
 {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nchunks) return;
@@ -106,11 +107,9 @@ __global__ void locate_records_kernel(int bpc, long long nblocks, int nchunks, c
         if (!ok || nb < kMaskBytes || nb > kMaxRecord + 4 || pos + 4 + nb > len) {
             ok = false;
             rec_off[g] = -1;
-            status[g] = -1;
             continue;
         }
         rec_off[g] = cb + pos;
-        status[g] = 0;
         pos += 4 + nb;
     }
 }
@@ -161,24 +160,6 @@ __global__ void map_blocks_kernel(long long nblocks, int nchunks, int maxsub, co
     rec_off[g] = (c < 0 || c >= nchunks || k < 0 || k >= maxsub) ? -1 : chunk_rec[(long long)c * maxsub + k];
 }
 
-// min over the per-block status words (0 ok, negative error) into *flag.
-__global__ void status_reduce_kernel(const int *status, long long n, int *flag)
-{
-    int worst = 0;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        worst = min(worst, status[i]);
-#pragma unroll
-    for (int o = 16; o; o >>= 1) worst = min(worst, __shfl_xor_sync(0xffffffffu, worst, o));
-    if ((threadIdx.x & 31) == 0 && worst < 0) atomicMin(flag, worst);
-}
-
-__global__ void neg_reduce_kernel(const int *v, int n, int *flag)
-{
-    int bad = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) bad |= v[i] < 0;
-    if (bad) atomicMin(flag, -1);
-}
-
 __global__ void rebase_kernel(long long *off, int n, long long base)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -222,22 +203,6 @@ cudaError_t cz_launch_map_blocks(long long nblocks, int nchunks, int maxsub, con
     return cudaGetLastError();
 }
 
-cudaError_t cz_launch_status_reduce(const int *status, long long n, int *flag, cudaStream_t st)
-{
-    if (n <= 0) return cudaSuccess;
-    const long long b = (n + 255) / 256;
-    status_reduce_kernel<<<(unsigned)(b < 1024 ? b : 1024), 256, 0, st>>>(status, n, flag);
-    return cudaGetLastError();
-}
-
-cudaError_t cz_launch_neg_reduce(const int *v, int n, int *flag, cudaStream_t st)
-{
-    if (n <= 0) return cudaSuccess;
-    const int b = (n + 255) / 256;
-    neg_reduce_kernel<<<b < 1024 ? b : 1024, 256, 0, st>>>(v, n, flag);
-    return cudaGetLastError();
-}
-
 cudaError_t cz_launch_chunk_setup(int bpc, long long nblocks, int nchunks, const int *rec_bytes, long long *in_off,
                                   int *in_len, long long *blk_dst, long long *lz_off, long long lz_slot,
                                   cudaStream_t st)
@@ -256,24 +221,17 @@ cudaError_t cz_launch_pack_records(const uint8_t *stage, const int *rec_bytes, l
     return cudaGetLastError();
 }
 
-cudaError_t cz_launch_scan(const int *len, int n, long long *off, cudaStream_t st)
-{
-    scan_kernel<<<1, 1024, 0, st>>>(len, n, off, 0);
-    return cudaGetLastError();
-}
-
 cudaError_t cz_launch_scan_from(const int *len, int n, long long *off, cudaStream_t st)
 {
-    scan_kernel<<<1, 1024, 0, st>>>(len, n, off, 1);
+    scan_kernel<<<1, 1024, 0, st>>>(len, n, off);
     return cudaGetLastError();
 }
 
 cudaError_t cz_launch_locate_records(int bpc, long long nblocks, int nchunks, const long long *chunk_base,
-                                     const int *dec_len, long long *rec_off, int *status, const uint8_t *base,
-                                     cudaStream_t st)
+                                     const int *dec_len, long long *rec_off, const uint8_t *base, cudaStream_t st)
 {
     if (nchunks <= 0) return cudaSuccess;
     locate_records_kernel<<<(nchunks + 127) / 128, 128, 0, st>>>(bpc, nblocks, nchunks, chunk_base, dec_len, rec_off,
-                                                                  status, base);
+                                                                  base);
     return cudaGetLastError();
 }

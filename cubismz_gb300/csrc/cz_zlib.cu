@@ -178,7 +178,7 @@ __device__ __forceinline__ void bar_sync64()
 
 __global__ void __launch_bounds__(64, 7)
 inflate_kernel(const uint8_t *__restrict__ in, const long long *in_off, const int *in_len, int nchunks,
-               uint8_t *__restrict__ out, const long long *out_off, const int *out_cap, int *out_len)
+               uint8_t *__restrict__ out, const long long *out_off, const int *out_cap, int *out_len, long long cap)
 {
     __shared__ Huff lit, dist;
     __shared__ unsigned char lens[320];
@@ -191,12 +191,14 @@ inflate_kernel(const uint8_t *__restrict__ in, const long long *in_off, const in
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
         const uint8_t *src = in + in_off[c];
-        uint8_t *dst = out + out_off[c];
-        const int oend = out_cap[c];
+        const long long span = in_len ? in_len[c] : in_off[c + 1] - in_off[c];
+        const int nin = span < 0 || span > 0x7fffffffLL ? -1 : (int)span;
+        uint8_t *dst = out + (out_off ? out_off[c] : c * cap);
+        const int oend = out_off ? out_cap[c] : (int)cap;
         // barriers 1, 2: batch k is full; 3, 4: batch k is free again
         if (warp == 0) {
             Inflater z;  // lane 0's decoder state, kept in registers
-            if (lane == 0) z.start(src, in_len[c]);
+            if (lane == 0) z.start(src, nin);
             uint32_t it = 0;
             for (int last = 0; !last; ++it) {
                 const int k = it & 1;
@@ -1262,9 +1264,10 @@ cudaError_t cz_launch_deflate(const uint8_t *in, const long long *in_off, const 
 }
 
 cudaError_t cz_launch_inflate(const uint8_t *in, const long long *in_off, const int *in_len, int nchunks, uint8_t *out,
-                              const long long *out_off, const int *out_cap, int *out_len, int grid, cudaStream_t st)
+                              const long long *out_off, const int *out_cap, int *out_len, int grid, cudaStream_t st,
+                              long long cap)
 {
     if (nchunks <= 0) return cudaSuccess;
-    inflate_kernel<<<grid, 64, 0, st>>>(in, in_off, in_len, nchunks, out, out_off, out_cap, out_len);
+    inflate_kernel<<<grid, 64, 0, st>>>(in, in_off, in_len, nchunks, out, out_off, out_cap, out_len, cap);
     return cudaGetLastError();
 }
