@@ -1,4 +1,4 @@
-// cz_lz4.cu -- LZ4 legacy block format on the GPU, one warp per chunk.
+// cz_lz4.cu -- LZ4 legacy block format on the GPU.
 //
 // Encoder: greedy parse, format-compatible with the reference decoder
 // LZ4_uncompress_unknownOutputSize (ThirdParty/lz4/lz4.c:802-905): minimum
@@ -16,7 +16,10 @@
 //     of the last kept match of lanes < k (one ballot when no match crosses
 //     a later lane's last start, the exact serial rule otherwise);
 //   * emit   -- a warp scan places every kept sequence, each lane writes its
-//     own; literal runs over 32 bytes are copied by the whole warp.
+//     own; literal runs over 32 bytes are copied by 8 lanes each, from 256 on
+//     by the whole warp.
+// With few chunks a second warp does the emission while the first parses on
+// (lz4_encode_pair_kernel).
 // Parse effort (a template level, cz_set_lz4_effort): 1 (default) extends
 // kept matches backwards over equal bytes (lz4.c's "catch up") and keeps
 // the tail of a match that a lower lane's match overlaps; 2 also takes
@@ -120,6 +123,20 @@ __device__ __forceinline__ void warp_copy(uint8_t *dst, const uint8_t *src, int 
     if (lane < t) dst[4 * nw + lane] = src[4 * nw + lane];
 }
 
+// n bytes by N lanes, as above.
+template <int N>
+__device__ __forceinline__ void lanes_copy(uint8_t *__restrict__ dst, const uint8_t *__restrict__ src, int n, int lane)
+{
+    const int h = min((int)((4 - (reinterpret_cast<uintptr_t>(dst) & 3)) & 3), n), nw = (n - h) >> 2;
+    const uint32_t first = rd32u(src), last = rd32u(src + max(n - 4, 0));
+    uint32_t *dw = reinterpret_cast<uint32_t *>(dst + h);
+#pragma unroll 4
+    for (int i = lane; i < nw; i += N) dw[i] = rd32u(src + h + 4 * i);
+    if (lane < h) dst[lane] = (uint8_t)(first >> 8 * lane);
+    const int t = n - h - 4 * nw;
+    if (lane < t) dst[n - t + lane] = (uint8_t)(last >> 8 * (4 - t + lane));
+}
+
 // n <= 32 bytes, 4 per step, so that the cost follows n (most literal runs
 // between matches are 0-4 bytes). Source and destination never overlap. May
 // read up to 7 bytes past s + n (inputs carry tail room).
@@ -178,7 +195,7 @@ __device__ __forceinline__ void next_skip(Skip &k, const uint8_t *src, int L)
 //             waiting for another;
 //   emit   -- every lane sizes its kept sequences, a warp scan places them,
 //             every lane writes its own; literal runs longer than 32 bytes
-//             are queued and copied by the whole warp.
+//             are queued and copied by several lanes.
 constexpr int kOvl = 8;
 // super-window sizes: 768 positions when every chunk of the launch is
 // resident at once (fewer windows per chunk), 512 otherwise (a smaller
@@ -262,59 +279,61 @@ __device__ __forceinline__ int match_len_back(const uint8_t *src, int p, int can
 // length, distance; zl::seq_pack) at out + out_off[c]; the last record holds
 // the tail literals. out_len[c] = record bytes, -1 past the capacity.
 // Shared memory of one encoder warp for super-windows of SW positions.
-template <int SW>
+// A lane's sequences, (start - base | back extension << 12 | offset << 16, match
+// length), take the place of its positions' candidates: the i-th sequence ends
+// at or after position 4 i + 4, where the walk's next read is. With OWN (effort
+// 2, whose walks read the end of the lower lane's segment) they have their
+// own.
+template <int SW, bool OWN>
 struct LzEncWarp {
     uint32_t table[1 << kHashLog];
     int4 longq[32];                   // (dst offset, src offset, n, -)
-    uint32_t seq[32][SW / 128];       // start - base | back extension << 12 | offset << 16
-    int lens[32][SW / 128];
     uint16_t info[SW];                // candidate offset per position, 0: none
+    uint2 own[OWN ? SW / 4 : 1];
     int nlong;
 };
 
-template <int kLzWarps, bool SEQ, int kEffort, int kSW>
-__global__ void __launch_bounds__(kLzWarps * 32)
-lz4_encode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const int *in_len, int nchunks,
-                  uint8_t *__restrict__ out, const long long *out_off, int *out_len, int records, int4 *hole)
+// With effort >= 1 a match [s, e) that starts before the literal position P is
+// kept from P on when that part is still a match (>= 4 bytes) that may follow a
+// literal run (P <= mflimit).
+template <int kEffort>
+__device__ __forceinline__ bool lz_survives(int s, int e, int P, int mflimit)
 {
-    constexpr int kSub = kSW / 32, kMaxSeqLane = kSub / 4;  // positions and sequences per lane
-    using LzEncWarp = cz::LzEncWarp<kSW>;
-    constexpr bool kThorough = kEffort >= 2;
-    constexpr int kMaxOff = SEQ ? zl::kMaxDist : 65535;
-    // up to 8 warps in static shared memory; 16 in dynamic
-    extern __shared__ __align__(16) unsigned char lz_enc_smem[];
-    __shared__ LzEncWarp lz_enc_static[kLzWarps <= 8 ? kLzWarps : 1];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    LzEncWarp &ws = (kLzWarps <= 8 ? lz_enc_static : reinterpret_cast<LzEncWarp *>(lz_enc_smem))[wib];
-    uint32_t *table = ws.table;
-    uint16_t *info = ws.info;
-    uint32_t *myseq = ws.seq[lane];
-    int *mylen = ws.lens[lane];
-    int4 *longq = ws.longq;
-    int &nlong = ws.nlong;
-    const int gw = blockIdx.x * kLzWarps + wib, nw = gridDim.x * kLzWarps;
+    return s >= P || (kEffort >= 1 && e - P >= kMinMatch && P <= mflimit);
+}
 
-    for (int c = gw; c < nchunks; c += nw) {
-        const uint8_t *src = in + in_off[c];
-        const int L = in_len[c];
-        uint8_t *dst = out + out_off[c];
-        const int cap = SEQ ? 8 * (L / 4 + 2) : L + L / 255 + 16;
-        for (int i = lane; i < (1 << kHashLog); i += 32) table[i] = kEmpty;
+// The parse of one chunk by one warp, window by window.
+template <bool SEQ, int kEffort, int kSW>
+struct LzParse {
+    static constexpr int kSub = kSW / 32;  // positions per lane; a quarter as many sequences
+    static constexpr bool kThorough = kEffort >= 2;
+    static constexpr int kMaxOff = SEQ ? zl::kMaxDist : 65535;
+    const uint8_t *src;
+    int L, pos, anchor, miss, mflimit, matchlimit;
+    int hlo, hhi;  // the literal-only planes last jumped over
+    Skip sk;
+
+    __device__ __forceinline__ void start(const uint8_t *s, int n, bool records, uint32_t *table)
+    {
+        for (int i = threadIdx.x & 31; i < (1 << kHashLog); i += 32) table[i] = kEmpty;
         __syncwarp();
-        int pos = 0, anchor = 0, op = 0, miss = 0;
-        bool overflow = false;
-        // the literal-only planes last jumped over, and whether the chunk's
-        // one deferred copy (left to the gather) is taken
-        int hlo = 0, hhi = 0;
-        bool deferred = hole == nullptr || !records;
-        if (hole && lane == 0) hole[c] = make_int4(0, 0, 0, 0);  // written for every chunk
-        Skip sk;
-        sk.on = records != 0;
+        src = s;
+        L = n;
+        pos = anchor = miss = hlo = hhi = 0;
+        sk.on = records;
         sk.next = 0;
         sk.lo = sk.hi = L + 1;
         if (sk.on) next_skip(sk, src, L);
-        const int mflimit = L - kMfLimit, matchlimit = L - kLastLiterals;
-        while (L >= kMfLimit + 1 && pos <= mflimit && !overflow) {
+        mflimit = L - kMfLimit;
+        matchlimit = L - kLastLiterals;
+    }
+
+    // Up to the next window with candidates: its start, and the lane's ns
+    // sequences (mine) from literal position myP on. False at the end.
+    __device__ __forceinline__ bool next(uint32_t *table, uint16_t *info, uint2 *mine, int &base, int &ns, int &myP)
+    {
+        const int lane = threadIdx.x & 31;
+        while (L >= kMfLimit + 1 && pos <= mflimit) {
             if (pos >= sk.lo) {  // literal-only planes: jump over them
                 if (pos < sk.hi) pos = sk.hi;
                 hlo = sk.lo;
@@ -323,7 +342,7 @@ lz4_encode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
                 miss = 0;
                 continue;
             }
-            const int base = pos;
+            base = pos;
             int end = base + kSW;
             if (end > mflimit + 1) end = mflimit + 1;
             if (end > sk.lo) end = sk.lo;
@@ -415,7 +434,8 @@ lz4_encode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
             // it equal the bytes before its source (at most 4), taken into
             // the match in the emission as far as the literal run allows
             // (effort >= 1: lz4.c's backward "catch up", lz4.c:586-587)
-            int ns = 0, last_start = -1, last_end = -1;
+            ns = 0;
+            int last_start = -1, last_end = -1;
             {
                 const int w0p = base + kSub * lane;
                 const int qe = min(w0p + kSub, end);
@@ -449,9 +469,8 @@ lz4_encode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
                                                    : match_len(src, q, q - off, 0, matchlimit);
                     if (len >= kMinMatch) {
                         if (q >= w0p) {
-                            myseq[ns] = (uint32_t)(q - base) | (uint32_t)ext << 12 | (uint32_t)off << 16;
-                            mylen[ns] = len;
-                            ++ns;
+                            mine[ns++] = make_uint2((uint32_t)(q - base) | (uint32_t)ext << 12 | (uint32_t)off << 16,
+                                                    (uint32_t)len);
                             last_start = q;
                             last_end = q + len;
                         }
@@ -465,18 +484,15 @@ lz4_encode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
             // effort >= 1 a match [s, e) that starts before the literal
             // position P is kept from P on when that part is still a match
             // (>= 4 bytes) that may follow a literal run (P <= mflimit).
-            auto survives = [&](int s, int e, int P) {
-                return s >= P || (kEffort >= 1 && e - P >= kMinMatch && P <= mflimit);
-            };
             // Usually every lane keeps its last sequence, so P_k is the end
             // of the nearest lower lane's last match; where a match reaches
             // past a later lane's last start, the exact serial rule runs.
             const unsigned has = __ballot_sync(0xffffffffu, ns > 0);
             const unsigned lower = has & lanemask_lt_();
-            int myP = __shfl_sync(0xffffffffu, last_end, lower ? 31 - __clz(lower) : 0);
+            myP = __shfl_sync(0xffffffffu, last_end, lower ? 31 - __clz(lower) : 0);
             if (!lower) myP = anchor;
             int P = has ? __shfl_sync(0xffffffffu, last_end, 31 - __clz(has)) : anchor;
-            const unsigned bad = __ballot_sync(0xffffffffu, ns > 0 && !survives(last_start, last_end, myP));
+            const unsigned bad = __ballot_sync(0xffffffffu, ns > 0 && !lz_survives<kEffort>(last_start, last_end, myP, mflimit));
             if (bad) {
                 // lanes below the first failing one are exact; from there the
                 // serial rule over the lanes that have sequences
@@ -487,110 +503,159 @@ lz4_encode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
                     const int ls = __shfl_sync(0xffffffffu, last_start, k);
                     const int le = __shfl_sync(0xffffffffu, last_end, k);
                     if (lane == k) myP = P;
-                    if (survives(ls, le, P)) P = le;
+                    if (lz_survives<kEffort>(ls, le, P, mflimit)) P = le;
                 }
             }
-            // ---- emit: kept sequences are those starting at or after myP
-            int lit_from = myP, bytes = 0, nkeep = 0;
-            for (int i = 0; i < ns; ++i) {
-                const int s0 = base + (int)(myseq[i] & 0xfff);
-                if (!survives(s0, s0 + mylen[i], lit_from)) continue;
-                const int st = max(s0 - (int)((myseq[i] >> 12) & 7), lit_from);
-                const int l = st - lit_from, ml = s0 + mylen[i] - st - kMinMatch;
-                bytes += SEQ ? 8 : 1 + (l >= 15 ? len_bytes(l - 15) : 0) + l + 2 + (ml >= 15 ? len_bytes(ml - 15) : 0);
-                lit_from = s0 + mylen[i];
-                ++nkeep;
-            }
-            int incl = bytes;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += t;
-            }
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            if ((long long)op + total + 1 + kLastLiterals > cap) {
-                overflow = true;
-                break;
-            }
-            if (lane == 0) nlong = 0;
-            __syncwarp();
-            if (SEQ) {
-                int at = op + incl - bytes;
-                lit_from = myP;
-                for (int i = 0; i < ns; ++i) {
-                    const int s0 = base + (int)(myseq[i] & 0xfff);
-                    if (!survives(s0, s0 + mylen[i], lit_from)) continue;
-                    const int st = max(s0 - (int)((myseq[i] >> 12) & 7), lit_from);
-                    *reinterpret_cast<unsigned long long *>(dst + at) =
-                        zl::seq_pack(st - lit_from, s0 + mylen[i] - st, (int)(myseq[i] >> 16));
-                    at += 8;
-                    lit_from = s0 + mylen[i];
-                }
-            } else {
-                int at = op + incl - bytes;
-                lit_from = myP;
-                for (int i = 0; i < ns; ++i) {
-                    const int s0 = base + (int)(myseq[i] & 0xfff);
-                    if (!survives(s0, s0 + mylen[i], lit_from)) continue;
-                    const int st = max(s0 - (int)((myseq[i] >> 12) & 7), lit_from);
-                    const int l = st - lit_from, ml = s0 + mylen[i] - st - kMinMatch, off = (int)(myseq[i] >> 16);
-                    uint8_t *d = dst + at;
-                    *d++ = (uint8_t)(((l >= 15 ? 15 : l) << 4) | (ml >= 15 ? 15 : ml));
-                    if (l >= 15) {
-                        put_len_serial(d, l - 15);
-                        d += len_bytes(l - 15);
-                    }
-                    if (l <= 32) {
-                        copy_short(d, src + lit_from, l);
-                    } else {
-                        const int slot = atomicAdd(&nlong, 1);
-                        if (slot < 32) longq[slot] = make_int4((int)(d - dst), lit_from, l, 0);
-                    }
-                    d += l;
-                    d[0] = (uint8_t)off;
-                    d[1] = (uint8_t)(off >> 8);
-                    if (ml >= 15) put_len_serial(d + 2, ml - 15);
-                    at += 1 + (l >= 15 ? len_bytes(l - 15) : 0) + l + 2 + (ml >= 15 ? len_bytes(ml - 15) : 0);
-                    lit_from = s0 + mylen[i];
-                }
-            }
-            __syncwarp();
-            const int nl = nlong;
-            if (nl > 32) {  // cannot happen: a long run (> 32 bytes) only before a lane's first sequence
-                overflow = true;
-                break;
-            }
-            for (int i = 0; i < nl; ++i) {
-                const int4 t = longq[i];
-                // the planes inside this run go to the gather (once per
-                // chunk): it copies them from the records into the stream
-                const int a = max(t.y, hlo), b = min(t.y + t.z, hhi);
-                if (!deferred && b - a >= kMinHole) {
-                    warp_copy(dst + t.x, src + t.y, a - t.y, lane);
-                    warp_copy(dst + t.x + (b - t.y), src + b, t.y + t.z - b, lane);
-                    if (lane == 0) hole[c] = make_int4(t.x + (a - t.y), a, b - a, 0);
-                    deferred = true;
-                } else {
-                    warp_copy(dst + t.x, src + t.y, t.z, lane);
-                }
-            }
-            __syncwarp();
-            op += total;
             anchor = P;
             pos = end > P ? end : P;
+            return true;
         }
-        if (!overflow && SEQ) {
+        return false;
+    }
+};
+
+// Its output.
+template <bool SEQ, int kEffort>
+struct LzEmit {
+    const uint8_t *src;
+    uint8_t *dst;
+    int L, cap, mflimit, op;
+    // whether the chunk's one deferred copy (left to the gather) is taken
+    bool deferred;
+    int4 *hole;  // the chunk's, or nullptr
+
+    __device__ __forceinline__ void start(const uint8_t *s, int n, uint8_t *d, int4 *h, bool records)
+    {
+        src = s;
+        dst = d;
+        L = n;
+        cap = SEQ ? 8 * (L / 4 + 2) : L + L / 255 + 16;
+        mflimit = L - kMfLimit;
+        op = 0;
+        hole = h;
+        deferred = h == nullptr || !records;
+        if (h && (threadIdx.x & 31) == 0) *h = make_int4(0, 0, 0, 0);  // written for every chunk
+    }
+
+    // A window's sequences; false past the capacity.
+    __device__ __forceinline__ bool window(int base, int ns, int myP, const uint2 *mine, int hlo, int hhi, int4 *longq,
+                                           int &nlong)
+    {
+        const int lane = threadIdx.x & 31;
+        auto survives = [&](int s, int e, int P) { return lz_survives<kEffort>(s, e, P, mflimit); };
+        // ---- emit: kept sequences are those starting at or after myP
+        int lit_from = myP, bytes = 0, nkeep = 0;
+        for (int i = 0; i < ns; ++i) {
+            const uint2 w = mine[i];
+            const int s0 = base + (int)(w.x & 0xfff), e0 = s0 + (int)w.y;
+            if (!survives(s0, e0, lit_from)) continue;
+            const int st = max(s0 - (int)((w.x >> 12) & 7), lit_from);
+            const int l = st - lit_from, ml = e0 - st - kMinMatch;
+            bytes += SEQ ? 8 : 1 + (l >= 15 ? len_bytes(l - 15) : 0) + l + 2 + (ml >= 15 ? len_bytes(ml - 15) : 0);
+            lit_from = e0;
+            ++nkeep;
+        }
+        int incl = bytes;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        if ((long long)op + total + 1 + kLastLiterals > cap) {
+            return false;
+        }
+        if (lane == 0) nlong = 0;
+        __syncwarp();
+        if (SEQ) {
+            int at = op + incl - bytes;
+            lit_from = myP;
+            for (int i = 0; i < ns; ++i) {
+                const uint2 w = mine[i];
+                const int s0 = base + (int)(w.x & 0xfff), e0 = s0 + (int)w.y;
+                if (!survives(s0, e0, lit_from)) continue;
+                const int st = max(s0 - (int)((w.x >> 12) & 7), lit_from);
+                *reinterpret_cast<unsigned long long *>(dst + at) =
+                    zl::seq_pack(st - lit_from, e0 - st, (int)(w.x >> 16));
+                at += 8;
+                lit_from = e0;
+            }
+        } else {
+            int at = op + incl - bytes;
+            lit_from = myP;
+            for (int i = 0; i < ns; ++i) {
+                const uint2 w = mine[i];
+                const int s0 = base + (int)(w.x & 0xfff), e0 = s0 + (int)w.y;
+                if (!survives(s0, e0, lit_from)) continue;
+                const int st = max(s0 - (int)((w.x >> 12) & 7), lit_from);
+                const int l = st - lit_from, ml = e0 - st - kMinMatch, off = (int)(w.x >> 16);
+                uint8_t *d = dst + at;
+                *d++ = (uint8_t)(((l >= 15 ? 15 : l) << 4) | (ml >= 15 ? 15 : ml));
+                if (l >= 15) {
+                    put_len_serial(d, l - 15);
+                    d += len_bytes(l - 15);
+                }
+                if (l <= 32) {
+                    copy_short(d, src + lit_from, l);
+                } else {
+                    const int slot = atomicAdd(&nlong, 1);
+                    if (slot < 32) longq[slot] = make_int4((int)(d - dst), lit_from, l, 0);
+                }
+                d += l;
+                d[0] = (uint8_t)off;
+                d[1] = (uint8_t)(off >> 8);
+                if (ml >= 15) put_len_serial(d + 2, ml - 15);
+                at += 1 + (l >= 15 ? len_bytes(l - 15) : 0) + l + 2 + (ml >= 15 ? len_bytes(ml - 15) : 0);
+                lit_from = e0;
+            }
+        }
+        __syncwarp();
+        const int nl = nlong;
+        if (nl > 32) {  // cannot happen: a long run (> 32 bytes) only before a lane's first sequence
+            return false;
+        }
+        // runs shorter than a hole: four at a time, 8 lanes each, so that
+        // their loads overlap (a window has 3 to 4, of 33 to 100 bytes)
+        for (int i = 0; i < nl; i += 4) {
+            const int4 t = longq[min(i + (lane >> 3), 31)];
+            if (i + (lane >> 3) < nl && t.z < kMinHole) lanes_copy<8>(dst + t.x, src + t.y, t.z, lane & 7);
+        }
+        for (int i = 0; i < nl; ++i) {
+            const int4 t = longq[i];
+            if (t.z < kMinHole) continue;
+            // the planes inside this run go to the gather (once per
+            // chunk): it copies them from the records into the stream
+            const int a = max(t.y, hlo), b = min(t.y + t.z, hhi);
+            if (!deferred && b - a >= kMinHole) {
+                warp_copy(dst + t.x, src + t.y, a - t.y, lane);
+                warp_copy(dst + t.x + (b - t.y), src + b, t.y + t.z - b, lane);
+                if (lane == 0) *hole = make_int4(t.x + (a - t.y), a, b - a, 0);
+                deferred = true;
+            } else {
+                warp_copy(dst + t.x, src + t.y, t.z, lane);
+            }
+        }
+        __syncwarp();
+        op += total;
+        return true;
+    }
+
+    // The literals from anchor on; false past the capacity.
+    __device__ __forceinline__ bool tail(int anchor, int hlo, int hhi)
+    {
+        const int lane = threadIdx.x & 31;
+        if (SEQ) {
             if (op + 8 > cap) {
-                overflow = true;
+                return false;
             } else {
                 if (lane == 0) *reinterpret_cast<unsigned long long *>(dst + op) = zl::seq_pack(L - anchor, 0, 0);
                 op += 8;
             }
-        } else if (!overflow) {
+        } else {
             const int lit = L - anchor;
             const int need = 1 + (lit >= 15 ? len_bytes(lit - 15) : 0) + lit;
             if (op + need > cap) {
-                overflow = true;
+                return false;
             } else {
                 if (lane == 0) {
                     dst[op] = (uint8_t)((lit >= 15 ? 15 : lit) << 4);
@@ -601,7 +666,7 @@ lz4_encode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
                 if (!deferred && b - a >= kMinHole) {  // the planes to the gather, as above
                     warp_copy(dst + op, src + anchor, a - anchor, lane);
                     warp_copy(dst + op + (b - anchor), src + b, L - b, lane);
-                    if (lane == 0) hole[c] = make_int4(op + (a - anchor), a, b - a, 0);
+                    if (lane == 0) *hole = make_int4(op + (a - anchor), a, b - a, 0);
                     deferred = true;
                 } else {
                     warp_copy(dst + op, src + anchor, lit, lane);
@@ -609,8 +674,124 @@ lz4_encode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
                 op += lit;
             }
         }
-        if (lane == 0) out_len[c] = overflow ? -1 : op;
+        return true;
+    }
+};
+
+template <int kLzWarps, bool SEQ, int kEffort, int kSW>
+__global__ void __launch_bounds__(kLzWarps * 32, 32 / kLzWarps)
+lz4_encode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const int *in_len, int nchunks,
+                  uint8_t *__restrict__ out, const long long *out_off, int *out_len, int records, int4 *hole)
+{
+    using Parse = LzParse<SEQ, kEffort, kSW>;
+    using LzEncWarp = cz::LzEncWarp<kSW, Parse::kThorough>;
+    // up to 8 warps in static shared memory; 16 in dynamic
+    extern __shared__ __align__(16) unsigned char lz_enc_smem[];
+    __shared__ LzEncWarp lz_enc_static[kLzWarps <= 8 ? kLzWarps : 1];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    LzEncWarp &ws = (kLzWarps <= 8 ? lz_enc_static : reinterpret_cast<LzEncWarp *>(lz_enc_smem))[wib];
+    uint2 *mine = (Parse::kThorough ? ws.own : reinterpret_cast<uint2 *>(ws.info)) + Parse::kSub / 4 * lane;
+    const int gw = blockIdx.x * kLzWarps + wib, nw = gridDim.x * kLzWarps;
+
+    for (int c = gw; c < nchunks; c += nw) {
+        const uint8_t *src = in + in_off[c];
+        const int L = in_len[c];
+        Parse p;
+        LzEmit<SEQ, kEffort> e;
+        p.start(src, L, records != 0, ws.table);
+        e.start(src, L, out + out_off[c], hole ? hole + c : nullptr, records != 0);
+        bool ok = true;
+        int base, ns, myP;
+        while (ok && p.next(ws.table, ws.info, mine, base, ns, myP))
+            ok = e.window(base, ns, myP, mine, p.hlo, p.hhi, ws.longq, ws.nlong);
+        ok = ok && e.tail(p.anchor, p.hlo, p.hhi);
+        if (lane == 0) out_len[c] = ok ? e.op : -1;
         __syncwarp();
+    }
+}
+
+// Two warps per chunk, for few chunks: one parses, the other writes what the
+// window before gave. A chunk is one serial chain of windows (a window's start
+// and its table depend on the window before; about 6 k cycles of parse and
+// 5 k of output each, nearly all latency), so this takes it through nearly
+// twice as fast while there are SMs for the second warps. Same bytes.
+template <int SW>
+struct LzPairShared {
+    uint32_t table[1 << kHashLog];
+    int4 longq[32];
+    uint16_t info[SW];
+    uint2 seq[2][SW / 4];  // two windows in flight
+    int2 lane[2][32];      // ns, myP
+    int4 win[2];           // base (-1: the end, with the anchor), anchor, hlo, hhi
+    int nlong, stop;       // stop: 1 + the chunk whose output is past its capacity
+};
+// Named barriers, one per buffer b: 1 + b full, 3 + b empty. Immediate ids, so
+// that a CTA holds 5 of the SM's barriers and not 16.
+template <int ID>
+__device__ __forceinline__ void pair_wait(int b)
+{
+    if (b) asm volatile("bar.sync %0, 64;" ::"n"(ID + 1) : "memory");
+    else asm volatile("bar.sync %0, 64;" ::"n"(ID) : "memory");
+}
+template <int ID>
+__device__ __forceinline__ void pair_signal(int b)
+{
+    if (b) asm volatile("bar.arrive %0, 64;" ::"n"(ID + 1) : "memory");
+    else asm volatile("bar.arrive %0, 64;" ::"n"(ID) : "memory");
+}
+constexpr int kPairFull = 1, kPairEmpty = 3;
+
+template <bool SEQ, int kEffort, int kSW>
+__global__ void __launch_bounds__(64)
+lz4_encode_pair_kernel(const uint8_t *__restrict__ in, const long long *in_off, const int *in_len, int nchunks,
+                       uint8_t *__restrict__ out, const long long *out_off, int *out_len, int records, int4 *hole)
+{
+    using Parse = LzParse<SEQ, kEffort, kSW>;
+    __shared__ LzPairShared<kSW> ps;
+    const int lane = threadIdx.x & 31;
+    int buf = 0;
+    if (threadIdx.x == 0) ps.stop = 0;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
+            Parse p;
+            p.start(in + in_off[c], in_len[c], records != 0, ps.table);
+            for (bool more = true; more; buf ^= 1) {
+                pair_wait<kPairEmpty>(buf);
+                int base, ns, myP;
+                more = *(volatile int *)&ps.stop != c + 1 &&
+                       p.next(ps.table, ps.info, ps.seq[buf] + Parse::kSub / 4 * lane, base, ns, myP);
+                if (more) ps.lane[buf][lane] = make_int2(ns, myP);
+                if (lane == 0) ps.win[buf] = make_int4(more ? base : -1, p.anchor, p.hlo, p.hhi);
+                pair_signal<kPairFull>(buf);
+            }
+        }
+        // the buffers' last signals
+        pair_wait<kPairEmpty>(buf);
+        pair_wait<kPairEmpty>(buf ^ 1);
+    } else {
+        pair_signal<kPairEmpty>(0);
+        pair_signal<kPairEmpty>(1);
+        for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
+            LzEmit<SEQ, kEffort> e;
+            e.start(in + in_off[c], in_len[c], out + out_off[c], hole ? hole + c : nullptr, records != 0);
+            bool ok = true;
+            for (bool more = true; more; buf ^= 1) {
+                pair_wait<kPairFull>(buf);
+                const int4 w = ps.win[buf];
+                more = w.x >= 0;
+                if (more && ok) {
+                    const int2 l = ps.lane[buf][lane];
+                    ok = e.window(w.x, l.x, l.y, ps.seq[buf] + Parse::kSub / 4 * lane, w.z, w.w, ps.longq, ps.nlong);
+                } else if (ok) {
+                    ok = e.tail(w.y, w.z, w.w);
+                }
+                if (!ok && lane == 0) *(volatile int *)&ps.stop = c + 1;  // no more of this chunk
+                __syncwarp();
+                pair_signal<kPairEmpty>(buf);
+            }
+            if (lane == 0) out_len[c] = ok ? e.op : -1;
+        }
     }
 }
 
@@ -1622,12 +1803,24 @@ static int sm_count()
 // kLzWarps chunks per CTA; 16 (512 threads, ~123 KB of shared memory)
 // takes an SM, so that CTAs of this kernel and the wavelet kernel, which
 // also takes a whole SM, share the machine SM by SM.
+// Up to 9 chunks per SM: two warps per chunk. One-record chunks, ms with two
+// warps / with one: 64 chunks 0.17 / 0.29, 512 0.23 / 0.33, 1 024 0.22 / 0.30,
+// 2 048 0.30 / 0.27, 4 096 0.90 / 0.67 (there the warps fill the SMs either way
+// and two need more registers); 128 chunks of 4 records 1.03 / 1.56, 69 of 15
+// 2.99 / 4.30. The CTA width asked for only shapes the other kernel.
+constexpr int kPairChunksPerSm = 9;
+
 template <int W, bool SEQ, int E, int SW>
 static cudaError_t launch_enc_t(const uint8_t *in, const long long *in_off, const int *in_len, int nchunks,
                                 uint8_t *out, const long long *out_off, int *out_len, int records, int grid,
                                 cudaStream_t st, int4 *hole)
 {
-    const int sm = W <= 8 ? 0 : (int)sizeof(LzEncWarp<SW>) * W;
+    if (nchunks <= kPairChunksPerSm * sm_count()) {
+        lz4_encode_pair_kernel<SEQ, E, SW>
+            <<<nchunks, 64, 0, st>>>(in, in_off, in_len, nchunks, out, out_off, out_len, records, hole);
+        return cudaGetLastError();
+    }
+    const int sm = W <= 8 ? 0 : (int)sizeof(LzEncWarp<SW, (E >= 2)>) * W;
     auto k = lz4_encode_kernel<W, SEQ, E, SW>;
     if (sm > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
