@@ -196,19 +196,21 @@ void collect(cz_ctx *c)
     }
 }
 
-// The field descriptors and, behind them, the fields' tensor maps to the
-// device in one copy; `extra` bytes of pinned scratch stay free after them.
+// A single field by value; several (or `list`) as descriptors and, behind
+// them, tensor maps in device memory, in one copy. `extra` bytes of pinned
+// scratch stay free from pin_extra(n) on.
 size_t maps_at(size_t nfields) { return (sizeof(CzField) * nfields + 127) / 128 * 128; }
-size_t fields_bytes(size_t nfields) { return maps_at(nfields) + sizeof(CUtensorMap) * nfields; }
-const CUtensorMap *maps_of(cz_ctx *c, size_t nfields)
+size_t pin_extra(size_t nfields) { return maps_at(nfields) + sizeof(CUtensorMap) * nfields; }
+int put_fields(cz_ctx *c, const std::vector<CzField> &fields, bool list, size_t extra, cudaStream_t st, CzFields *out)
 {
-    return reinterpret_cast<const CUtensorMap *>(P<uint8_t>(c->fields) + maps_at(nfields));
-}
-int put_fields(cz_ctx *c, const std::vector<CzField> &fields, size_t extra, cudaStream_t st)
-{
-    const size_t n = fields.size(), bytes = fields_bytes(n);
-    CZ_TRY(grow(c, c->fields, bytes));
+    const size_t n = fields.size(), bytes = pin_extra(n);
     CZ_TRY(grow_pin(c, std::max<size_t>(4096, bytes + extra)));
+    *out = CzFields();
+    out->n = (int)n;
+    out->one = fields[0];
+    if (!cz_field_map(fields[0], &out->map)) return fail(c, CZ_E_CUDA, "no tensor map for a field");
+    if (n == 1 && !list) return CZ_OK;
+    CZ_TRY(grow(c, c->fields, bytes));
     memcpy(c->pin, fields.data(), sizeof(CzField) * n);
     for (size_t i = 0; i < n; ++i) {
         CUtensorMap m;
@@ -216,6 +218,8 @@ int put_fields(cz_ctx *c, const std::vector<CzField> &fields, size_t extra, cuda
         memcpy(static_cast<char *>(c->pin) + maps_at(n) + sizeof(m) * i, &m, sizeof(m));
     }
     CZ_CUDA(c, cudaMemcpyAsync(c->fields.p, c->pin, bytes, cudaMemcpyHostToDevice, st));
+    out->list = P<CzField>(c->fields);
+    out->maps = reinterpret_cast<const CUtensorMap *>(P<uint8_t>(c->fields) + maps_at(n));
     return CZ_OK;
 }
 
@@ -227,7 +231,8 @@ int put_fields(cz_ctx *c, const std::vector<CzField> &fields, size_t extra, cuda
 //   finish   waits for the stream, reads the totals, fills *out.
 struct Job {
     long long nblocks = 0;
-    int nfields = 0, nchunks = 0, bpc = 1, lz_warps = 4, refit_iters = 0, enc_variant = 0;
+    CzFields fields;
+    int nchunks = 0, bpc = 1, lz_warps = 4, refit_iters = 0, enc_variant = 0;
     long long lz_slot = 0, z_slot = 0;  // per chunk: LZ4 output or DEFLATE parse; zlib output
     cz_params p{};
 };
@@ -239,7 +244,6 @@ int prepare(cz_ctx *c, const std::vector<CzField> &fields, long long nblocks, co
     const long long nch_ll = (nblocks + bpc - 1) / bpc;
     if (nch_ll > 0x7fffffffLL) return fail(c, CZ_E_ARG, "too many chunks");
     job.nblocks = nblocks;
-    job.nfields = (int)fields.size();
     job.nchunks = (int)nch_ll;
     job.bpc = bpc;
     job.p = *p;
@@ -275,7 +279,7 @@ int prepare(cz_ctx *c, const std::vector<CzField> &fields, long long nblocks, co
     const int grid = (int)std::min<long long>(nblocks, c->sms);
     if (refit_iters > 0) CZ_TRY(grow(c, c->refit, sizeof(float) * cz_refit_scratch_floats(grid)));
     // finish() reuses the pinned staging only after this copy (stream order)
-    return put_fields(c, fields, 0, st);
+    return put_fields(c, fields, refit_iters > 0, 0, st, &job.fields);
 }
 
 int enqueue(cz_ctx *c, const Job &job, cudaStream_t st, bool marks)
@@ -291,13 +295,13 @@ int enqueue(cz_ctx *c, const Job &job, cudaStream_t st, bool marks)
     if (bpc == 1) chunks.at(P<long long>(c->in_off), P<int>(c->in_len), P<long long>(c->lz_off), job.lz_slot);
     if (marks) CZ_TRY(mark(c, 0, st));
     if (job.refit_iters > 0)
-        CZ_CUDA(c, cz_launch_refit(p->wtype, P<CzField>(c->fields), job.nfields, nblocks, p->zerobits,
+        CZ_CUDA(c, cz_launch_refit(p->wtype, job.fields.list, job.fields.n, nblocks, p->zerobits,
                                    p->shuffle ? 1 : 0, job.refit_iters, P<uint8_t>(c->stage), P<int>(c->rec_bytes),
                                    ctl->queue, P<float>(c->refit), grid, st, chunks));
     else
-        CZ_CUDA(c, cz_launch_encode(p->wtype, P<CzField>(c->fields), job.nfields, nblocks, p->zerobits,
-                                    p->shuffle ? 1 : 0, P<uint8_t>(c->stage), P<int>(c->rec_bytes), ctl->queue, grid,
-                                    st, maps_of(c, job.nfields), nullptr, &ctl->flag[1], job.enc_variant, chunks));
+        CZ_CUDA(c, cz_launch_encode(p->wtype, job.fields, nblocks, p->zerobits, p->shuffle ? 1 : 0,
+                                    P<uint8_t>(c->stage), P<int>(c->rec_bytes), ctl->queue, grid, st, &ctl->flag[1],
+                                    job.enc_variant, chunks));
     if (marks) CZ_TRY(mark(c, 1, st));
     const uint8_t *chunk_src = P<uint8_t>(c->stage);
     if (bpc > 1) {
@@ -402,9 +406,10 @@ int decompress_fields(cz_ctx *c, const std::vector<CzField> &fields, long long n
     CZ_TRY(grow(c, c->ctl, sizeof(Ctl)));
     if (encoder != CZ_ENCODER_NONE) CZ_TRY(grow(c, c->dec, (size_t)nchunks * dcap));
     // pinned scratch: [fields and tensor maps | flag (64 B) | block map]
-    const size_t pin_fields = fields_bytes(fields.size());
+    const size_t pin_fields = pin_extra(fields.size());
     const size_t map_bytes = h_block_chunk ? sizeof(int) * 2 * nblocks : 0;
-    CZ_TRY(put_fields(c, fields, 64 + map_bytes, st));
+    CzFields fs;
+    CZ_TRY(put_fields(c, fields, false, 64 + map_bytes, st, &fs));
     Ctl *ctl = P<Ctl>(c->ctl);
     CZ_CUDA(c, cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
     const int raw = encoder == CZ_ENCODER_NONE;
@@ -466,9 +471,8 @@ int decompress_fields(cz_ctx *c, const std::vector<CzField> &fields, long long n
     const int grid = (int)std::min<long long>(nblocks, c->sms);
     CZ_TRY(mark(c, 2, st));
     double *per_block = diff_ref ? P<double>(c->diff) : nullptr;
-    CZ_CUDA(c, cz_launch_decode(wtype, P<CzField>(c->fields), (int)fields.size(), nblocks, shuffle ? 1 : 0, recs,
-                                &ctl->flag[0], ctl->queue, grid, st, maps_of(c, fields.size()), diff_ref, per_block,
-                                planes));
+    CZ_CUDA(c, cz_launch_decode(wtype, fs, nblocks, shuffle ? 1 : 0, recs, &ctl->flag[0], ctl->queue, grid, st,
+                                diff_ref, per_block, planes));
     if (diff_ref) CZ_CUDA(c, cz_launch_diff_total(per_block, nblocks, per_block + 8 * nblocks, st));
     CZ_TRY(mark(c, 3, st));
     int *hflag = reinterpret_cast<int *>(reinterpret_cast<char *>(c->pin) + pin_fields);
@@ -1224,7 +1228,7 @@ int cz_compress_to_image(cz_ctx *c, const float *h_field, int nx, int ny, int nz
         slabs[i] = CzField{P<float>(c->tmp_field) + z0 * ny * nx, nx, ny, (int)depth, p->eps, 0};
     }
     Job job;
-    CZ_TRY(prepare(c, slabs, nblocks, p, 0, st, job));
+    CZ_TRY(prepare(c, {CzField{P<float>(c->tmp_field), nx, ny, nz, p->eps, 0}}, nblocks, p, 0, st, job));
     // the payload goes straight to the image when the device can write it
     const std::string hdr = czf::header_text(bx, by, bz, p->eps, p->wtype, p->encoder);
     const long long mini = czf::mini_header_bytes();
@@ -1257,9 +1261,12 @@ int cz_compress_to_image(cz_ctx *c, const float *h_field, int nx, int ny, int nz
         CZ_CUDA(c, cudaStreamWaitEvent(cs, c->ev_h2d[i], 0));
         CzChunks chunks;
         chunks.at(P<long long>(c->in_off) + f0, P<int>(c->in_len) + f0, P<long long>(c->lz_off) + f0, job.lz_slot);
-        CZ_CUDA(c, cz_launch_encode(p->wtype, P<CzField>(c->fields) + i, 1, n, p->zerobits, p->shuffle ? 1 : 0, stage,
-                                    P<int>(c->rec_bytes) + f0, &ctl->queue[i], std::min(n, c->sms), cs,
-                                    maps_of(c, nslab) + i, nullptr, &ctl->flag[1], 0, chunks));
+        CzFields slab;
+        slab.one = slabs[i];
+        if (!cz_field_map(slab.one, &slab.map)) return fail(c, CZ_E_CUDA, "no tensor map for a field");
+        CZ_CUDA(c, cz_launch_encode(p->wtype, slab, n, p->zerobits, p->shuffle ? 1 : 0, stage,
+                                    P<int>(c->rec_bytes) + f0, &ctl->queue[i], std::min(n, c->sms), cs, &ctl->flag[1],
+                                    0, chunks));
         CZ_CUDA(c, cudaEventRecord(c->ev_enc[i], cs));
         const uint8_t *src = stage;
         const long long *src_off = P<long long>(c->in_off) + f0;

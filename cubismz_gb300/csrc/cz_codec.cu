@@ -84,17 +84,18 @@ __device__ __forceinline__ void set_block(Blk *b, long long g, const CzField *fi
     }
 }
 
-__device__ __forceinline__ void take_ticket(Blk *b, const CzField *fields, int nfields, long long total,
-                                            unsigned long long *queue)
+// The CTA's blocks come from the queue, the second one with the first; where
+// every block can have a CTA of its own, without it.
+__device__ __forceinline__ void take_first(Blk *b, const CzField *fields, int nfields, long long total,
+                                           unsigned long long *queue)
 {
-    set_block(b, (long long)atomicAdd(queue, 1ull), fields, nfields, total);
+    const long long g = total <= gridDim.x ? (long long)blockIdx.x : (long long)atomicAdd(queue, 1ull);
+    set_block(b, g, fields, nfields, total);
 }
-// The CTA's second block is taken with the first one: not when every block
-// can have a CTA of its own.
-__device__ __forceinline__ void take_second(Blk *b, const CzField *fields, int nfields, long long total,
-                                            unsigned long long *queue)
+__device__ __forceinline__ void take_later(Blk *b, const CzField *fields, int nfields, long long total,
+                                           unsigned long long *queue)
 {
-    if (total > gridDim.x) take_ticket(b, fields, nfields, total, queue);
+    if (total > gridDim.x) set_block(b, (long long)atomicAdd(queue, 1ull), fields, nfields, total);
     else b->g = -1;
 }
 
@@ -263,10 +264,11 @@ __device__ __forceinline__ void emit_quarter(unsigned char *sm, uint32_t p, int 
 // into L2 while this block is finished (the autotuner times both).
 template <int KIND, bool AHEAD>
 __global__ void __launch_bounds__(kNT, 1)
-encode_kernel(const CzField *fields, int nfields, long long total_blocks, int zerobits, int shuffle, uint8_t *stage,
-              int *rec_bytes, unsigned long long *queue, const __grid_constant__ CUtensorMap map0,
-              const CUtensorMap *maps, int *err, CzChunks chunks)
+encode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int zerobits, int shuffle, uint8_t *stage,
+              int *rec_bytes, unsigned long long *queue, int *err, CzChunks chunks)
 {
+    const CzField *fields = fs.list ? fs.list : &fs.one;
+    const int nfields = fs.n;
     extern __shared__ __align__(1024) unsigned char sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t zmask = zerobits > 0 ? ~((1u << zerobits) - 1u) : 0xffffffffu;
@@ -280,7 +282,7 @@ encode_kernel(const CzField *fields, int nfields, long long total_blocks, int ze
         for (int s = 0; s < kSlots; ++s) mbar_init(bars + 8 * s, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         *fail = 0;
-        take_ticket(blk, fields, nfields, total_blocks, queue);
+        take_first(blk, fields, nfields, total_blocks, queue);
     }
     __syncthreads();
     // plane n of the CTA's sequence (plane n & 31 of its block n >> 5) into
@@ -289,14 +291,14 @@ encode_kernel(const CzField *fields, int nfields, long long total_blocks, int ze
         const Blk &b = blk[(n >> 5) & 3];
         if (b.g < 0) return;
         const uint32_t s = n % kSlots;
-        tma_load_3d(ring + s * kPlane, maps ? maps + b.field : &map0, b.x, b.y, b.z + (int)(n & 31), bars + 8 * s,
+        tma_load_3d(ring + s * kPlane, fs.list ? fs.maps + b.field : &fs.map, b.x, b.y, b.z + (int)(n & 31), bars + 8 * s,
                     kPlane);
     };
     if (lane == 0) {
         bring(warp);
         if (warp + 16 < kSlots) bring(warp + 16);
     }
-    if (threadIdx.x == 0) take_second(blk + 1, fields, nfields, total_blocks, queue);
+    if (threadIdx.x == 0) take_later(blk + 1, fields, nfields, total_blocks, queue);
     __syncthreads();
 
     uint32_t it = 0;
@@ -369,10 +371,10 @@ encode_kernel(const CzField *fields, int nfields, long long total_blocks, int ze
             }
         }
         __syncthreads();
-        if (warp == kNW - 1 && lane == 0) take_ticket(blk + ((it + 2) & 3), fields, nfields, total_blocks, queue);
+        if (warp == kNW - 1 && lane == 0) take_later(blk + ((it + 2) & 3), fields, nfields, total_blocks, queue);
         if (AHEAD && warp == kNW - 2 && lane >= kSlots) {
             const Blk &b = blk[(it + 1) & 3];
-            if (b.g >= 0) tma_prefetch_3d(maps ? maps + b.field : &map0, b.x, b.y, b.z + lane);
+            if (b.g >= 0) tma_prefetch_3d(fs.list ? fs.maps + b.field : &fs.map, b.x, b.y, b.z + lane);
         }
         if (warp < 8) {
             // ---- level 16, x (lines (y, z)) and y (lines (x, z)), level 8, y
@@ -611,10 +613,11 @@ __device__ __forceinline__ void unpack16(uint32_t p, unsigned bits, float (&v)[3
 
 template <int KIND, bool DIFF>
 __global__ void __launch_bounds__(kNT, 1)
-decode_kernel(const CzField *fields, int nfields, long long total_blocks, int shuffle, CzRecords where, int *flag,
-              unsigned long long *queue, const float *diff_ref, double *diff_out, CzPlanes planes,
-              const CUtensorMap *maps)
+decode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int shuffle, CzRecords where, int *flag,
+              unsigned long long *queue, const float *diff_ref, double *diff_out, CzPlanes planes)
 {
+    const CzField *fields = fs.list ? fs.list : &fs.one;
+    const int nfields = fs.n;
     extern __shared__ __align__(1024) unsigned char sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int *seg_cnt = reinterpret_cast<int *>(sm + kSegCnt), *warp_cnt = reinterpret_cast<int *>(sm + kWarpCnt);
@@ -678,7 +681,7 @@ decode_kernel(const CzField *fields, int nfields, long long total_blocks, int sh
     };
     if (scout) {
         bad[0] = bad[1] = 0;
-        take_ticket(blk, fields, nfields, total_blocks, queue);
+        take_first(blk, fields, nfields, total_blocks, queue);
         scout_off(0);
         scout_rec(0);
         find(0, s_off, s_len, s_nb, s_hole, s_src);
@@ -686,7 +689,7 @@ decode_kernel(const CzField *fields, int nfields, long long total_blocks, int sh
     __syncthreads();
     if (blk[0].g < 0) return;
     if (scout) {
-        take_second(blk + 1, fields, nfields, total_blocks, queue);
+        take_later(blk + 1, fields, nfields, total_blocks, queue);
         scout_off(1);
         scout_rec(1);
         find(1, s_off, s_len, s_nb, s_hole, s_src);
@@ -912,7 +915,7 @@ decode_kernel(const CzField *fields, int nfields, long long total_blocks, int sh
             st_row(slot, lane, v);
             fence_async_smem();
             __syncwarp();
-            if (lane == 0) tma_store_3d(maps + cur.field, cur.x, cur.y, cur.z + z, smem_u32(slot));
+            if (lane == 0) tma_store_3d(fs.list ? fs.maps + cur.field : &fs.map, cur.x, cur.y, cur.z + z, smem_u32(slot));
             if (DIFF) {
                 const CzField &f = fields[cur.field];
                 const float4 *rr = reinterpret_cast<const float4 *>(
@@ -1011,69 +1014,43 @@ bool cz_field_map(const CzField &f, CUtensorMap *map)
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int KIND>
-static cudaError_t launch_encode(const CzField *fields, int nfields, long long total_blocks, int zerobits,
-                                 int shuffle, uint8_t *stage, int *rec_bytes, unsigned long long *queue, int grid,
-                                 cudaStream_t st, const CUtensorMap *maps, const CUtensorMap &map0, int *err,
-                                 int variant, const CzChunks &chunks)
+cudaError_t cz_launch_encode(int wtype, const CzFields &fields, long long total_blocks, int zerobits, int shuffle,
+                             uint8_t *stage, int *rec_bytes, unsigned long long *queue, int grid, cudaStream_t st,
+                             int *err, int variant, CzChunks chunks)
 {
-    auto k = variant == 1 ? encode_kernel<KIND, false> : encode_kernel<KIND, true>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCodecSmem);
-    if (e != cudaSuccess) return e;
-    k<<<grid, kNT, kCodecSmem, st>>>(fields, nfields, total_blocks, zerobits, shuffle, stage, rec_bytes, queue, map0,
-                                     maps, err, chunks);
-    return cudaGetLastError();
-}
-
-template <int KIND>
-static cudaError_t launch_decode(const CzField *fields, int nfields, long long total_blocks, int shuffle,
-                                 const CzRecords &recs, int *flag, unsigned long long *queue, int grid,
-                                 cudaStream_t st, const CUtensorMap *maps, const float *diff_ref, double *diff_out,
-                                 CzPlanes planes)
-{
-    auto k = diff_ref ? decode_kernel<KIND, true> : decode_kernel<KIND, false>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCodecSmem);
-    if (e != cudaSuccess) return e;
-    k<<<grid, kNT, kCodecSmem, st>>>(fields, nfields, total_blocks, shuffle, recs, flag, queue, diff_ref, diff_out,
-                                     planes, maps);
-    return cudaGetLastError();
-}
-
-cudaError_t cz_launch_encode(int wtype, const CzField *fields, int nfields, long long total_blocks, int zerobits,
-                             int shuffle, uint8_t *stage, int *rec_bytes, unsigned long long *queue, int grid,
-                             cudaStream_t st, const CUtensorMap *maps, const CUtensorMap *map0, int *err, int variant,
-                             CzChunks chunks)
-{
-    if (!maps && !map0) return cudaErrorInvalidValue;
-    CUtensorMap own = {};
-    if (map0) own = *map0;
+    auto launch = [&](auto k) {
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCodecSmem);
+        if (e != cudaSuccess) return e;
+        k<<<grid, kNT, kCodecSmem, st>>>(fields, total_blocks, zerobits, shuffle, stage, rec_bytes, queue, err, chunks);
+        return cudaGetLastError();
+    };
     switch (wkind(wtype)) {
     case 1:
-        return launch_encode<1>(fields, nfields, total_blocks, zerobits, shuffle, stage, rec_bytes, queue, grid, st,
-                                maps, own, err, variant, chunks);
+        return launch(variant == 1 ? encode_kernel<1, false> : encode_kernel<1, true>);
     case 2:
-        return launch_encode<2>(fields, nfields, total_blocks, zerobits, shuffle, stage, rec_bytes, queue, grid, st,
-                                maps, own, err, variant, chunks);
+        return launch(variant == 1 ? encode_kernel<2, false> : encode_kernel<2, true>);
     default:
-        return launch_encode<3>(fields, nfields, total_blocks, zerobits, shuffle, stage, rec_bytes, queue, grid, st,
-                                maps, own, err, variant, chunks);
+        return launch(variant == 1 ? encode_kernel<3, false> : encode_kernel<3, true>);
     }
 }
 
-cudaError_t cz_launch_decode(int wtype, const CzField *fields, int nfields, long long total_blocks, int shuffle,
-                             CzRecords recs, int *flag, unsigned long long *queue, int grid, cudaStream_t st,
-                             const CUtensorMap *maps, const float *diff_ref, double *diff_out, CzPlanes planes)
+cudaError_t cz_launch_decode(int wtype, const CzFields &fields, long long total_blocks, int shuffle, CzRecords recs,
+                             int *flag, unsigned long long *queue, int grid, cudaStream_t st, const float *diff_ref,
+                             double *diff_out, CzPlanes planes)
 {
+    auto launch = [&](auto k) {
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCodecSmem);
+        if (e != cudaSuccess) return e;
+        k<<<grid, kNT, kCodecSmem, st>>>(fields, total_blocks, shuffle, recs, flag, queue, diff_ref, diff_out, planes);
+        return cudaGetLastError();
+    };
     switch (wkind(wtype)) {
     case 1:
-        return launch_decode<1>(fields, nfields, total_blocks, shuffle, recs, flag, queue, grid, st, maps, diff_ref,
-                                diff_out, planes);
+        return launch(diff_ref ? decode_kernel<1, true> : decode_kernel<1, false>);
     case 2:
-        return launch_decode<2>(fields, nfields, total_blocks, shuffle, recs, flag, queue, grid, st, maps, diff_ref,
-                                diff_out, planes);
+        return launch(diff_ref ? decode_kernel<2, true> : decode_kernel<2, false>);
     default:
-        return launch_decode<3>(fields, nfields, total_blocks, shuffle, recs, flag, queue, grid, st, maps, diff_ref,
-                                diff_out, planes);
+        return launch(diff_ref ? decode_kernel<3, true> : decode_kernel<3, false>);
     }
 }
 

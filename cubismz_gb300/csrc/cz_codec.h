@@ -19,6 +19,16 @@ struct CzField {
 // codec kernels' tile copies; false if the driver cannot make it. The field
 // must be 16-byte aligned.
 bool cz_field_map(const CzField &f, CUtensorMap *map);
+// The fields of a launch: n descriptors and their tensor maps (64-byte aligned)
+// in device memory, or (list == nullptr) a single field by value, which costs
+// no copy to the device and no read of it at the start of every CTA.
+struct CzFields {
+    CUtensorMap map = {};
+    CzField one = {};
+    const CzField *list = nullptr;
+    const CUtensorMap *maps = nullptr;
+    int n = 1;
+};
 
 // Where a record's kernel leaves what follows it in the pipeline (all
 // optional, indexed by block): the record as a one-record chunk (input offset
@@ -39,15 +49,12 @@ struct CzChunks {
     }
 };
 
-// maps: the fields' tensor maps in device memory (64-byte aligned), or
-// nullptr with map0 (host) for a single field. err (optional, device): set
-// to 1 if a tile copy did not complete in time.
+// err (optional, device): set to 1 if a tile copy did not complete in time.
 // variant 0: the part of the next block that shared memory does not hold yet
 // is brought into L2 ahead; 1: it is not (same records)
-cudaError_t cz_launch_encode(int wtype, const CzField *fields, int nfields, long long total_blocks, int zerobits,
-                             int shuffle, uint8_t *stage, int *rec_bytes, unsigned long long *queue, int grid,
-                             cudaStream_t st, const CUtensorMap *maps, const CUtensorMap *map0, int *err,
-                             int variant = 0, CzChunks chunks = CzChunks());
+cudaError_t cz_launch_encode(int wtype, const CzFields &fields, long long total_blocks, int zerobits, int shuffle,
+                             uint8_t *stage, int *rec_bytes, unsigned long long *queue, int grid, cudaStream_t st,
+                             int *err, int variant = 0, CzChunks chunks = CzChunks());
 // Where a launch's records are: block g's [int32 nbytes][record] at base +
 // rec_off[g] (negative: missing); or, without rec_off, one record per chunk:
 // chunk g at base + off[g], off[g + 1] - off[g] bytes (raw chunks, cap == 0), or
@@ -61,9 +68,8 @@ struct CzRecords {
 };
 // A missing or malformed record leaves its block as decoded from an empty one
 // and sets *flag to -1.
-// diff_ref (optional, a field of the same geometry as fields[0]): per-block
-// error statistics into diff_out[8*g] (cz2diff's quantities). maps as for
-// cz_launch_encode (device memory).
+// diff_ref (optional, a field of the same geometry as the first): per-block
+// error statistics into diff_out[8*g] (cz2diff's quantities).
 // Byte planes 1 and 2 of one-record chunks left in the LZ4 input by
 // cz_launch_lz4_decode (hole per chunk = per block, chunk c at src +
 // src_off[c]); hole == nullptr: every record is whole.
@@ -72,10 +78,10 @@ struct CzPlanes {
     const uint8_t *src = nullptr;
     const long long *src_off = nullptr;
 };
-cudaError_t cz_launch_decode(int wtype, const CzField *fields, int nfields, long long total_blocks, int shuffle,
-                             CzRecords recs, int *flag, unsigned long long *queue, int grid, cudaStream_t st,
-                             const CUtensorMap *maps, const float *diff_ref = nullptr,
-                             double *diff_out = nullptr, CzPlanes planes = CzPlanes());
+cudaError_t cz_launch_decode(int wtype, const CzFields &fields, long long total_blocks, int shuffle, CzRecords recs,
+                             int *flag, unsigned long long *queue, int grid, cudaStream_t st,
+                             const float *diff_ref = nullptr, double *diff_out = nullptr,
+                             CzPlanes planes = CzPlanes());
 cudaError_t cz_launch_diff_total(const double *per_block, long long nblocks, double *total, cudaStream_t st);
 
 // Linear inverse transform and its adjoint on stacked 32^3 blocks; block

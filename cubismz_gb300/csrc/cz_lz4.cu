@@ -1738,7 +1738,7 @@ lz4_decode_kernel(const uint8_t *__restrict__ in, const long long *in_off, const
     }
 }
 
-// One CTA per chunk: the chunk's bytes to dst + dst_off[c]. With `hole`
+// gridDim.y CTAs per chunk: the chunk's bytes to dst + dst_off[c]. With `hole`
 // (LZ4 of block records), bytes [hole.x, hole.x + hole.z) of the chunk's
 // output are the input bytes at hsrc + hsrc_off[c] + hole.y, which the
 // encoder left unwritten. SCAN: the chunk sums the lengths before its own and
@@ -1763,11 +1763,11 @@ gather_kernel(const uint8_t *__restrict__ src, const long long *src_off, const i
         at = 0;
 #pragma unroll
         for (int w = 0; w < 8; ++w) at += part[w];
-        if (threadIdx.x == 0) dst_off[c] = at;
+        if (threadIdx.x == 0 && blockIdx.y == 0) dst_off[c] = at;
     } else {
         at = dst_off[c];
     }
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && blockIdx.y == 0) {
         if (n < 0 && flag) atomicMin(flag, -1);
         if (c == nchunks - 1) {
             if (SCAN) dst_off[nchunks] = at + n;
@@ -1775,15 +1775,23 @@ gather_kernel(const uint8_t *__restrict__ src, const long long *src_off, const i
         }
     }
     if (n <= 0) return;
+    // this CTA's part of the chunk
+    const int share = ((n + (int)gridDim.y - 1) / (int)gridDim.y + 15) & ~15;
+    const int lo = min(share * (int)blockIdx.y, n), hi = min(lo + share, n);
     const uint8_t *s = src + src_off[c];
     uint8_t *d = dst + at;
     const int4 hl = hole ? hole[c] : make_int4(0, 0, 0, 0);
+    auto copy = [&](const uint8_t *from, int a, int b) {  // output bytes [a, b) from `from` + a
+        a = max(a, lo);
+        b = min(b, hi);
+        if (b > a) cta_copy(d + a, from + a, b - a);
+    };
     if (hl.z > 0) {
-        cta_copy(d, s, hl.x);
-        cta_copy(d + hl.x, hsrc + hsrc_off[c] + hl.y, hl.z);
-        cta_copy(d + hl.x + hl.z, s + hl.x + hl.z, n - hl.x - hl.z);
+        copy(s, 0, hl.x);
+        copy(hsrc + hsrc_off[c] + hl.y - hl.x, hl.x, hl.x + hl.z);
+        copy(s, hl.x + hl.z, n);
     } else {
-        cta_copy(d, s, n);
+        copy(s, 0, n);
     }
 }
 
@@ -1799,6 +1807,7 @@ static int sm_count()
         sms = 1;
     return sms;
 }
+
 
 // kLzWarps chunks per CTA; 16 (512 threads, ~123 KB of shared memory)
 // takes an SM, so that CTAs of this kernel and the wavelet kernel, which
@@ -1933,7 +1942,10 @@ cudaError_t cz_launch_gather(const uint8_t *src, const long long *src_off, const
         if (e == cudaSuccess) e = cz_launch_scan_from(len, nchunks, dst_off, st);
         if (e != cudaSuccess) return e;
     }
+    // a CTA moves 4 KB per round trip to memory: few chunks go to several CTAs
+    // (64 raw records 12 -> 6 us), unless the other streams' kernels share the GPU
+    const int parts = scan ? std::max(1, std::min(8, 8 * sm_count() / nchunks)) : 1;
     auto k = own ? gather_kernel<true> : gather_kernel<false>;
-    k<<<nchunks, 256, 0, st>>>(src, src_off, len, nchunks, dst, dst_off, flag, total, hole, hsrc, hsrc_off);
+    k<<<dim3(nchunks, parts), 256, 0, st>>>(src, src_off, len, nchunks, dst, dst_off, flag, total, hole, hsrc, hsrc_off);
     return cudaGetLastError();
 }

@@ -5,8 +5,8 @@
 // allocation would implicitly synchronise the device and stall work running
 // beside the compressor. For them cz_blocks_compress_noalloc runs the same
 // encode kernel as every other entry point, but its scratch memory (the
-// block descriptor, the work-queue counter, the per-block record sizes and
-// one staging slot per block) lives in the file-scope device array below,
+// work-queue counter, the per-block record sizes and one staging slot per
+// block) lives in the file-scope device array below,
 // sized for CZ_NOALLOC_MAX_BLOCKS blocks (about 2.2 MB). Every GPU that
 // loads the library holds that array until the process exits.
 //
@@ -33,9 +33,9 @@ namespace {
 using cz::kSlotBytes;
 
 constexpr int kMaxBlocks = CZ_NOALLOC_MAX_BLOCKS;
-constexpr size_t kHdrBytes = 1024;  // descriptor, queue counter, record sizes
+constexpr size_t kHdrBytes = 1024;  // queue counter, record sizes
 constexpr size_t kScratchBytes = kHdrBytes + (size_t)kMaxBlocks * kSlotBytes;
-static_assert(sizeof(CzField) <= 256 && 512 + 4 * kMaxBlocks <= 768, "scratch header too small");
+static_assert(512 + 4 * kMaxBlocks <= 768, "scratch header too small");
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -44,7 +44,6 @@ std::mutex g_mu;
 unsigned char *g_addr[kMaxDevices] = {};
 
 struct Layout {
-    CzField *field;
     unsigned long long *queue;
     int *rec_bytes;
     int *err;
@@ -54,7 +53,6 @@ struct Layout {
 __host__ __device__ inline Layout layout(unsigned char *base)
 {
     Layout l;
-    l.field = reinterpret_cast<CzField *>(base);
     l.queue = reinterpret_cast<unsigned long long *>(base + 256);
     l.rec_bytes = reinterpret_cast<int *>(base + 512);
     l.err = reinterpret_cast<int *>(base + 768);
@@ -62,21 +60,12 @@ __host__ __device__ inline Layout layout(unsigned char *base)
     return l;
 }
 
-// Resets the queue counter and writes the descriptor: the blocks are a
-// stack of 32^3 blocks along z (block g at d_blocks + g*32768).
-__global__ void noalloc_init(unsigned char *base, const float *d_blocks, int nblocks, float eps)
+// Resets the queue counter and the error flag.
+__global__ void noalloc_init(unsigned char *base)
 {
     const Layout l = layout(base);
     *l.queue = 0ull;
     *l.err = 0;
-    CzField f;
-    f.data = d_blocks;
-    f.nx = 32;
-    f.ny = 32;
-    f.nz = 32 * nblocks;
-    f.eps = eps;
-    f.block0 = 0;
-    *l.field = f;
 }
 
 // Staging slot [int32 nbytes][record] -> caller's record buffer and size
@@ -134,17 +123,20 @@ extern "C" int cz_blocks_compress_noalloc(const float *d_blocks, int nblocks, fl
     if (rc != CZ_OK) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const Layout l = layout(base);
-    noalloc_init<<<1, 1, 0, st>>>(base, d_blocks, nblocks, eps);
+    noalloc_init<<<1, 1, 0, st>>>(base);
     if (cudaGetLastError() != cudaSuccess) return CZ_E_CUDA;
     int sms = 1;
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int grid = nblocks < sms ? nblocks : sms;
-    CUtensorMap map;
-    if (!cz_field_map(CzField{d_blocks, 32, 32, 32 * nblocks, eps, 0}, &map)) return CZ_E_CUDA;
-    if (cz_launch_encode(wtype, l.field, 1, nblocks, zerobits, shuffle ? 1 : 0, l.stage, l.rec_bytes, l.queue, grid,
-                         st, nullptr, &map, l.err) != cudaSuccess) {
+    // the blocks are a stack of 32^3 blocks along z (block g at d_blocks +
+    // g*32768)
+    CzFields f;
+    f.one = CzField{d_blocks, 32, 32, 32 * nblocks, eps, 0};
+    if (!cz_field_map(f.one, &f.map)) return CZ_E_CUDA;
+    if (cz_launch_encode(wtype, f, nblocks, zerobits, shuffle ? 1 : 0, l.stage, l.rec_bytes, l.queue, grid, st,
+                         l.err) != cudaSuccess) {
         cudaGetLastError();
         return CZ_E_CUDA;
     }
