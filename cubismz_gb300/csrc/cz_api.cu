@@ -64,7 +64,7 @@ struct cz_ctx {
     std::string err;
     DevBuf fields, stage, rec_bytes, chunk_in, in_off, in_len, blk_dst, lz_off, lz_out, lz_len, out_off, out_data,
         ctl, rec_off, dec, dec_off, dec_cap, dec_len, chunk_rec, block_chunk, block_subid,
-        tmp_field, tmp_in, refit, diff, zout, zoff, zlen, ierr, lz_hole;
+        tmp_field, tmp_in, refit, diff, zout, zoff, zlen, lz_hole;
     void *pin = nullptr;  // small pinned host scratch
     size_t pin_cap = 0;
     // geometry of the last compressed stream
@@ -513,7 +513,7 @@ int cz_destroy(cz_ctx *c)
 {
     if (!c) return CZ_OK;
     cudaSetDevice(c->device);
-    DevBuf *all[] = {&c->ierr, &c->zout, &c->zoff, &c->zlen, &c->diff, &c->refit, &c->fields,  &c->stage,   &c->rec_bytes, &c->chunk_in,  &c->in_off,      &c->in_len,
+    DevBuf *all[] = {&c->zout, &c->zoff, &c->zlen, &c->diff, &c->refit, &c->fields,  &c->stage,   &c->rec_bytes, &c->chunk_in,  &c->in_off,      &c->in_len,
                      &c->blk_dst, &c->lz_off,  &c->lz_out,    &c->lz_len,    &c->out_off,     &c->out_data,
                      &c->ctl,     &c->rec_off,   &c->dec,         &c->dec_off,
                      &c->dec_cap, &c->dec_len, &c->chunk_rec, &c->block_chunk, &c->block_subid,
@@ -688,15 +688,20 @@ int cz_res_line(const double *st, long long compressed_bytes, char *buf, int len
     return w < len ? CZ_OK : CZ_E_SPACE;
 }
 
-// After a TMA transpose: the kernel's error flag (a bounded mbarrier wait
-// that ran out); waits for the stream.
-static int ingest_check(cz_ctx *c, cudaStream_t st)
+// A TMA transpose reports a bounded mbarrier wait that ran out in pinned host
+// memory, which costs no clearing launch and no copy back: cleared here, read
+// after waiting for the stream.
+static int ingest_flag(cz_ctx *c, int **flag)
 {
     CZ_TRY(grow_pin(c, 4096));
-    int *h = reinterpret_cast<int *>(c->pin);
-    CZ_CUDA(c, cudaMemcpyAsync(h, c->ierr.p, 4, cudaMemcpyDeviceToHost, st));
+    *flag = reinterpret_cast<int *>(c->pin);
+    **flag = 0;
+    return CZ_OK;
+}
+static int ingest_check(cz_ctx *c, const int *flag, cudaStream_t st)
+{
     CZ_CUDA(c, cudaStreamSynchronize(st));
-    if (*h != 0) return fail(c, CZ_E_CUDA, "layout transform: a tile copy did not complete");
+    if (*(const volatile int *)flag != 0) return fail(c, CZ_E_CUDA, "layout transform: a tile copy did not complete");
     return CZ_OK;
 }
 
@@ -708,11 +713,11 @@ int cz_field_from_zfastest(cz_ctx *c, const void *d_in, int bytes, int nch, int 
         return fail(c, CZ_E_ARG, "bad layout arguments");
     CZ_TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
-    CZ_TRY(grow(c, c->ierr, 64));
-    CZ_CUDA(c, cudaMemsetAsync(c->ierr.p, 0, 4, st));
+    int *flag = nullptr;
+    CZ_TRY(ingest_flag(c, &flag));
     bool tma = false;
-    CZ_CUDA(c, cz_launch_from_zfastest(d_in, bytes, nch, ch, nx, ny, nz, d_field, st, P<int>(c->ierr), &tma));
-    return tma ? ingest_check(c, st) : CZ_OK;
+    CZ_CUDA(c, cz_launch_from_zfastest(d_in, bytes, nch, ch, nx, ny, nz, d_field, st, flag, &tma));
+    return tma ? ingest_check(c, flag, st) : CZ_OK;
 }
 
 int cz_field_to_zfastest(cz_ctx *c, const float *d_field, int nx, int ny, int nz, int nch, int ch, float *d_out,
@@ -722,11 +727,11 @@ int cz_field_to_zfastest(cz_ctx *c, const float *d_field, int nx, int ny, int nz
         return fail(c, CZ_E_ARG, "bad layout arguments");
     CZ_TRY(set_device(c));
     cudaStream_t st = (cudaStream_t)stream;
-    CZ_TRY(grow(c, c->ierr, 64));
-    CZ_CUDA(c, cudaMemsetAsync(c->ierr.p, 0, 4, st));
+    int *flag = nullptr;
+    CZ_TRY(ingest_flag(c, &flag));
     bool tma = false;
-    CZ_CUDA(c, cz_launch_to_zfastest(d_field, nx, ny, nz, nch, ch, d_out, st, P<int>(c->ierr), &tma));
-    return tma ? ingest_check(c, st) : CZ_OK;
+    CZ_CUDA(c, cz_launch_to_zfastest(d_field, nx, ny, nz, nch, ch, d_out, st, flag, &tma));
+    return tma ? ingest_check(c, flag, st) : CZ_OK;
 }
 
 int cz_batch_compress(cz_ctx *c, int nfields, const float *const *d_fields, const int *dims, const float *eps,

@@ -182,6 +182,7 @@ cudaError_t cz_launch_rebase(long long *off, int n, long long base, cudaStream_t
 
 // Layout of the reference's HDF5 tools (cz_ingest.cu): z-fastest arrays with
 // interleaved channels <-> the x-fastest field. bytes: 4 (float) or 8 (double).
+// err: pinned host memory, set to 1 if a tile copy did not complete in time.
 cudaError_t cz_launch_from_zfastest(const void *in, int bytes, int nch, int ch, int nx, int ny, int nz, float *out,
                                     cudaStream_t st, int *err = nullptr,
                                     bool *used_tma = nullptr);

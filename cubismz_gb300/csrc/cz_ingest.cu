@@ -12,12 +12,16 @@
 // nearest binary32.
 //
 // Single-channel arrays whose two transposed extents are multiples of the
-// tile take the TMA path: tiles of 4 planes x 32 rows x 128 bytes move from
+// tile take the TMA path: tiles of 128 rows x 128 bytes in one y plane (64 or
+// 32 rows in 2 or 4 planes where the extent is a multiple of no more) move from
 // HBM into shared memory by cp.async.bulk.tensor (128-byte swizzle, so that
 // the column reads of the transpose hit at most 4 ways per bank; planes past
 // the array come in zero-filled and are not stored), four tiles in flight
-// per CTA on mbarriers, and every warp writes whole 128-byte rows of the
-// destination. Each wait on an mbarrier is bounded; past the bound the
+// per CTA on mbarriers, and every warp writes whole rows of the destination,
+// 512 bytes for 128 rows: memory is what bounds this, and it takes runs of 512
+// bytes better than runs of 128 that lie a plane apart (384^3: from binary64 130
+// -> 119 us, to z-fastest 86 -> 76; 256^3: 42 -> 41, 27 -> 19; at the memory's
+// rate 100 and 67). Rows past the extent would waste more than that gives. Each wait on an mbarrier is bounded; past the bound the
 // CTA records an error, drains its copies in flight (bounded too) and
 // returns, and the call reports the error.
 #include <algorithm>
@@ -72,21 +76,22 @@ to_zfastest_kernel(const float *__restrict__ in, int nx, int ny, int nz, int nch
 
 // ------------------------------------------------------------------ TMA path
 constexpr int kStages = 4;
-constexpr int kPlanes = 4;                                   // y planes per tile
-constexpr int kTileBytes = kPlanes * 32 * 128;               // 16 KB
+constexpr int kTileRows = 128;                               // rows x planes of a tile
+constexpr int kTileBytes = kTileRows * 128;                  // 16 KB
 constexpr int kTmaSmem = kStages * kTileBytes + 1024;        // + alignment slack
 
-// Tile t of the source: planes y0..y0+3, 32 rows each (along the
+// Tile t of the source: planes y0 .. y0 + 128 / R - 1, R rows each (along the
 // destination's fastest axis, r) of BC elements (along the source's fastest
 // axis, c). Element (p, r, c) of the tile is written to
 // out[(c0 + c)*sc + (y0 + p)*sy + r0 + r].
-template <class T>
+template <class T, int R>
 __global__ void __launch_bounds__(256)
 tma_transpose_kernel(const __grid_constant__ CUtensorMap map, int ncb, int ny, int nrb, float *__restrict__ out,
                      long long sc, long long sy, int *err)
 {
     constexpr int BC = 128 / (int)sizeof(T);  // elements per 128-byte row
     constexpr uint32_t kTile = kTileBytes;
+    constexpr int kPlanes = kTileRows / R;
     extern __shared__ unsigned char tma_smem[];
     unsigned char *base = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tma_smem) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) unsigned long long bar[kStages];
@@ -110,7 +115,7 @@ tma_transpose_kernel(const __grid_constant__ CUtensorMap map, int ncb, int ny, i
             if (t >= ntiles) break;
             int cb, y, rb;
             coords(t, cb, y, rb);
-            tma_load_3d(smem_u32(base + s * kTile), &map, cb * BC, rb * 32, y, smem_u32(&bar[s]), kTile);
+            tma_load_3d(smem_u32(base + s * kTile), &map, cb * BC, rb * R, y, smem_u32(&bar[s]), kTile);
         }
     bool ok = true;
     long long i = 0;
@@ -129,9 +134,13 @@ tma_transpose_kernel(const __grid_constant__ CUtensorMap map, int ncb, int ny, i
         for (int pc = warp; pc < np * BC; pc += 8) {
             const int p = pc / BC, c = pc - p * BC;
             const int cbyte = c * (int)sizeof(T);
-            const int off = p * 4096 + lane * 128 + ((((cbyte >> 4) ^ (lane & 7))) << 4) + (cbyte & 15);
-            const T v = *reinterpret_cast<const T *>(tile + off);
-            out[(long long)(cb * BC + c) * sc + (long long)(y + p) * sy + rb * 32 + lane] = (float)v;
+            const int off = p * R * 128 + lane * 128 + ((((cbyte >> 4) ^ (lane & 7))) << 4) + (cbyte & 15);
+            float *o = out + (long long)(cb * BC + c) * sc + (long long)(y + p) * sy + rb * R + lane;
+            T v[R / 32];
+#pragma unroll
+            for (int k = 0; k < R / 32; ++k) v[k] = *reinterpret_cast<const T *>(tile + off + 4096 * k);
+#pragma unroll
+            for (int k = 0; k < R / 32; ++k) o[32 * k] = (float)v[k];
         }
         __syncthreads();  // every thread is done with buf[s]
         if (threadIdx.x == 0) {
@@ -139,14 +148,15 @@ tma_transpose_kernel(const __grid_constant__ CUtensorMap map, int ncb, int ny, i
             if (tn < ntiles) {
                 int cb2, y2, rb2;
                 coords(tn, cb2, y2, rb2);
-                tma_load_3d(smem_u32(base + s * kTile), &map, cb2 * BC, rb2 * 32, y2, smem_u32(&bar[s]), kTile);
+                tma_load_3d(smem_u32(base + s * kTile), &map, cb2 * BC, rb2 * R, y2, smem_u32(&bar[s]), kTile);
             }
         }
     }
     if (!ok) {  // uniform across the CTA
         // record the error, then wait (bounded) for the copies still in flight
         if (threadIdx.x == 0) {
-            atomicExch(err, 1);
+            *(volatile int *)err = 1;  // host memory
+            __threadfence_system();
             for (int k = 0; k < kStages; ++k) {
                 const long long j = i + k;
                 if (first + j * step >= ntiles) break;
@@ -164,21 +174,22 @@ using namespace cz;
 namespace {
 
 // The TMA transpose of a 3-D array (d0 fastest, then d1, d2) whose tiles are
-// 128 bytes along d0 and 32 rows along d2; false if the map cannot be made
+// 128 bytes along d0 and R rows along d2; false if the map cannot be made
 // (the caller then takes the plain kernel).
-bool launch_tma(const void *in, int bytes, long long d0, long long d1, long long d2, float *out, long long sc,
-                long long sy, int *err, cudaStream_t st)
+template <int R>
+bool launch_tma_rows(const void *in, int bytes, long long d0, long long d1, long long d2, float *out, long long sc,
+                     long long sy, int *err, cudaStream_t st)
 {
+    constexpr int kPlanes = kTileRows / R;
     CzEncodeTiled enc = cz_encode_tiled();
     if (!enc) return false;
     const int bc = 128 / bytes;
-    if (d0 % bc || d2 % 32 || reinterpret_cast<uintptr_t>(in) % 16) return false;
     // the map lists the rows' axis (d2) before the planes' (d1), so that a
-    // box lands in shared memory as kPlanes whole 32-row tiles
+    // box lands in shared memory as kPlanes whole tiles of R rows
     CUtensorMap map;
     const cuuint64_t dim[3] = {(cuuint64_t)d0, (cuuint64_t)d2, (cuuint64_t)d1};
     const cuuint64_t stride[2] = {(cuuint64_t)(d0 * d1 * bytes), (cuuint64_t)(d0 * bytes)};
-    const cuuint32_t box[3] = {(cuuint32_t)bc, 32, (cuuint32_t)kPlanes}, es[3] = {1, 1, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)bc, (cuuint32_t)R, (cuuint32_t)kPlanes}, es[3] = {1, 1, 1};
     if (stride[0] % 16 || stride[1] % 16) return false;
     if (enc(&map, bytes == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
             const_cast<void *>(in), dim, stride, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -187,16 +198,24 @@ bool launch_tma(const void *in, int bytes, long long d0, long long d1, long long
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int ncb = (int)(d0 / bc), nrb = (int)(d2 / 32);
+    const int ncb = (int)(d0 / bc), nrb = (int)(d2 / R);
     const long long ntiles = (long long)ncb * ((d1 + kPlanes - 1) / kPlanes) * nrb;
     const int grid = (int)std::min<long long>(ntiles, (long long)sms * 3);
-    auto k = bytes == 8 ? tma_transpose_kernel<double> : tma_transpose_kernel<float>;
+    auto k = bytes == 8 ? tma_transpose_kernel<double, R> : tma_transpose_kernel<float, R>;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kTmaSmem) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
     k<<<grid, 256, kTmaSmem, st>>>(map, ncb, (int)d1, nrb, out, sc, sy, err);
     return true;
+}
+bool launch_tma(const void *in, int bytes, long long d0, long long d1, long long d2, float *out, long long sc,
+                long long sy, int *err, cudaStream_t st)
+{
+    if (d0 % (128 / bytes) || d2 % 32 || reinterpret_cast<uintptr_t>(in) % 16) return false;
+    if (d2 % 128 == 0) return launch_tma_rows<128>(in, bytes, d0, d1, d2, out, sc, sy, err, st);
+    if (d2 % 64 == 0) return launch_tma_rows<64>(in, bytes, d0, d1, d2, out, sc, sy, err, st);
+    return launch_tma_rows<32>(in, bytes, d0, d1, d2, out, sc, sy, err, st);
 }
 
 }  // namespace
