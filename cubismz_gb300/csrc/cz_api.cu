@@ -777,7 +777,8 @@ struct cz_plan {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     // autotuner timings (-1: not tuned): the LZ4 stage at 2, 4, 8, 16 chunks
-    // per CTA, the wavelet kernel in its two row-prefetch variants
+    // per CTA, the wavelet kernel with and without bringing the next block
+    // into L2 ahead
     float lz_ms[4] = {-1.f, -1.f, -1.f, -1.f};
     float enc_ms[2] = {-1.f, -1.f};
 };
@@ -834,8 +835,8 @@ int cz_plan_create(cz_ctx *c, int nfields, const float *const *d_fields, const i
     // autotuner, timed on this batch with CUDA events (best of the second
     // and third run of each shape): first the LZ4 stage's CTA width (2, 4,
     // 8 or 16 chunks per CTA) with the wavelet kernel's default variant,
-    // then the wavelet kernel's row-prefetch variant with that width. Every
-    // shape writes the same bytes.
+    // then the wavelet kernel with the next block brought into L2 ahead or
+    // not, with that width. Every shape writes the same bytes.
     cz_stream tmp;
     if (tune) {
         pl->c->timing = true;

@@ -98,15 +98,14 @@ __device__ __forceinline__ void st_line(float *sb, int base, const float (&v)[N]
     for (int j = 0; j < N; ++j) sb[base + j * stride<AXIS>()] = v[j];
 }
 
-template <int N, int AXIS, bool FWD, int KIND>
-__device__ __forceinline__ void sweep(float *sb)
+template <int N, int AXIS, int KIND>
+__device__ __forceinline__ void sweep_fwd(float *sb)
 {
     for (int l = threadIdx.x; l < N * N; l += kNT) {
         const int base = line_base<N, AXIS>(l);
         float v[N];
         ld_line<N, AXIS>(sb, base, v);
-        if (FWD) line_fwd<N, KIND>(v);
-        else line_inv<N, KIND>(v);
+        line_fwd<N, KIND>(v);
         st_line<N, AXIS>(sb, base, v);
     }
 }

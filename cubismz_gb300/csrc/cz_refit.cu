@@ -536,7 +536,7 @@ refit_kernel(const CzField *fields, int nfields, long long total_blocks, int zer
             st_line<32, 0>(sb, pidx(0, y, z), v);
         }
         __syncthreads();
-        sweep<32, 1, true, KIND>(sb);
+        sweep_fwd<32, 1, KIND>(sb);
         __syncthreads();
         for (int l = threadIdx.x; l < 1024; l += kNT) {
             const int x = l & 31, y = l >> 5;
@@ -548,9 +548,9 @@ refit_kernel(const CzField *fields, int nfields, long long total_blocks, int zer
             emit32(s, x, y, keep_bits<32>(v, eps));
         }
         __syncthreads();
-        sweep<16, 2, true, KIND>(sb);
+        sweep_fwd<16, 2, KIND>(sb);
         __syncthreads();
-        sweep<16, 0, true, KIND>(sb);
+        sweep_fwd<16, 0, KIND>(sb);
         __syncthreads();
         if (threadIdx.x < 256) {
             const int x = threadIdx.x & 15, z = threadIdx.x >> 4;
@@ -562,9 +562,9 @@ refit_kernel(const CzField *fields, int nfields, long long total_blocks, int zer
             emit16(s, x, z, keep_bits<16>(v, eps));
         }
         __syncthreads();
-        sweep<8, 1, true, KIND>(sb);
+        sweep_fwd<8, 1, KIND>(sb);
         __syncthreads();
-        sweep<8, 2, true, KIND>(sb);
+        sweep_fwd<8, 2, KIND>(sb);
         __syncthreads();
         if (threadIdx.x < 64) {
             const int y = threadIdx.x & 7, z = threadIdx.x >> 3;

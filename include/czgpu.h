@@ -236,10 +236,10 @@ int cz_refit(cz_ctx *ctx, const float *d_field, int nx, int ny, int nz, const cz
  * compressed many times: cz_plan_create sizes a private set of buffers,
  * optionally tunes the launch shape on the batch itself (tune != 0, timed
  * with CUDA events: the LZ4 stage's CTA width, 2, 4, 8 or 16 chunks per
- * CTA, then the wavelet kernel's row-prefetch variant; every shape writes
- * the same bytes), and captures the whole pipeline (one persistent wavelet
- * launch over every field's blocks through the device work queue, chunk
- * setup, scans, LZ4, gather) in a CUDA graph. cz_plan_launch is one graph
+ * CTA, then the wavelet kernel with and without bringing the next block
+ * into L2 ahead; every shape writes the same bytes), and captures the whole
+ * pipeline (one persistent wavelet launch over every field's blocks through
+ * the device work queue, LZ4, scan, gather) in a CUDA graph. cz_plan_launch is one graph
  * launch with no host work; the fields' contents may change between
  * launches. cz_plan_result waits for `stream` and describes the shared
  * stream (all) and, if per_field is not NULL, each field's chunks as in
@@ -252,8 +252,8 @@ int cz_plan_launch(cz_plan *plan, void *stream);
 int cz_plan_result(cz_plan *plan, void *stream, cz_stream *all, cz_stream *per_field);
 int cz_plan_info(const cz_plan *plan, int *lz_warps, float *tune_ms /* 3: LZ4 ms at 2, 4, 8 */);
 /* The tuned shape: shape[0] = LZ4 chunks per CTA, shape[1] = wavelet kernel
- * variant (0: the next block's rows load in two halves by the warps each
- * level leaves idle, 1: all at once after level 32); ms[0..3] = LZ4 stage at
+ * variant (0: the part of the next block that shared memory does not hold
+ * yet is brought into L2 ahead, 1: it is not); ms[0..3] = LZ4 stage at
  * 2, 4, 8, 16 chunks per CTA, ms[4..5] = wavelet kernel in variant 0, 1
  * (-1 where not timed). No counterpart in the reference. */
 int cz_plan_shape(const cz_plan *plan, int *shape /* 2 */, float *ms /* 6 */);
