@@ -1283,10 +1283,15 @@ int cz_compress_to_image(cz_ctx *c, const float *h_field, int nx, int ny, int nz
             CZ_CUDA(c, cudaStreamWaitEvent(ls, c->ev_enc[i], 0));
             uint8_t *lzo = P<uint8_t>(c->lz_out) + f0 * job.lz_slot;
             // whole-SM CTAs (16 chunks each): LZ4 and the wavelet kernel of
-            // the next slabs then share the GPU SM by SM
-            const int lzgrid = std::max(1, std::min((n + 15) / 16, c->sms));
+            // the next slabs then share the GPU SM by SM. Two warps per chunk
+            // where that leaves the wavelet kernel SMs (small slabs) or little
+            // is left of it (the last two): 256^3 0.79 -> 0.71 ms, 256x512x512
+            // 1.73 -> 1.66, 512^3 3.33 -> 3.30, but 3.42 with all slabs so.
+            const bool pairs = (n <= c->sms || i >= nslab - 2) && n <= kLzPairChunksPerSm * c->sms;
+            const int per = pairs ? 4 : 16;
+            const int lzgrid = std::max(1, std::min((n + per - 1) / per, c->sms));
             CZ_CUDA(c, cz_launch_lz4_encode(stage, src_off, len, n, lzo, P<long long>(c->lz_off) + f0,
-                                            P<int>(c->lz_len) + f0, p->shuffle ? 1 : 0, 16, lzgrid, ls,
+                                            P<int>(c->lz_len) + f0, p->shuffle ? 1 : 0, per, lzgrid, ls,
                                             P<int4>(c->lz_hole) + f0, c->lz_effort));
             CZ_CUDA(c, cudaEventRecord(c->ev_lz[i], ls));
             src = lzo;

@@ -98,6 +98,7 @@ cudaError_t cz_launch_refit(int wtype, const CzField *fields, int nfields, long 
                             int shuffle, int iters, uint8_t *stage, int *rec_bytes, unsigned long long *queue,
                             float *scratch, int grid, cudaStream_t st, CzChunks chunks = CzChunks());
 
+constexpr int kLzPairChunksPerSm = 9;  // up to here the LZ4 encoder takes two warps per chunk (warps < 16)
 // LZ4 stage (cz_lz4.cu). Chunk c's input is in[in_off[c] .. in_off[c]+in_len[c]);
 // the encoder reads it as aligned words, so in + in_off[c] must be a multiple
 // of 4 bytes (records and the staged host inputs are), and reads up to 64

@@ -1776,7 +1776,7 @@ gather_kernel(const uint8_t *__restrict__ src, const long long *src_off, const i
     }
     if (n <= 0) return;
     // this CTA's part of the chunk
-    const int share = ((n + (int)gridDim.y - 1) / (int)gridDim.y + 15) & ~15;
+    const int share = gridDim.y == 1 ? n : ((n + (int)gridDim.y - 1) / (int)gridDim.y + 15) & ~15;
     const int lo = min(share * (int)blockIdx.y, n), hi = min(lo + share, n);
     const uint8_t *s = src + src_off[c];
     uint8_t *d = dst + at;
@@ -1816,15 +1816,15 @@ static int sm_count()
 // warps / with one: 64 chunks 0.17 / 0.29, 512 0.23 / 0.33, 1 024 0.22 / 0.30,
 // 2 048 0.30 / 0.27, 4 096 0.90 / 0.67 (there the warps fill the SMs either way
 // and two need more registers); 128 chunks of 4 records 1.03 / 1.56, 69 of 15
-// 2.99 / 4.30. The CTA width asked for only shapes the other kernel.
-constexpr int kPairChunksPerSm = 9;
+// 2.99 / 4.30. The CTA width asked for only shapes the other kernel; 16, whole-SM
+// CTAs that leave the other SMs free, is never taken over.
 
 template <int W, bool SEQ, int E, int SW>
 static cudaError_t launch_enc_t(const uint8_t *in, const long long *in_off, const int *in_len, int nchunks,
                                 uint8_t *out, const long long *out_off, int *out_len, int records, int grid,
                                 cudaStream_t st, int4 *hole)
 {
-    if (nchunks <= kPairChunksPerSm * sm_count()) {
+    if (W < 16 && nchunks <= kLzPairChunksPerSm * sm_count()) {
         lz4_encode_pair_kernel<SEQ, E, SW>
             <<<nchunks, 64, 0, st>>>(in, in_off, in_len, nchunks, out, out_off, out_len, records, hole);
         return cudaGetLastError();
