@@ -534,19 +534,6 @@ struct DiffAcc {
     }
 };
 
-__device__ __forceinline__ double warp_max(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-__device__ __forceinline__ double warp_sum(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 // ------------------------------------------------------------------ decode
 // Where a block's record is.
 struct Rec {
@@ -609,6 +596,26 @@ __device__ __forceinline__ void unpack16(uint32_t p, unsigned bits, float (&v)[3
                      : "memory");
         v[J0 + j] = x;
     }
+}
+
+__device__ __forceinline__ double diff_fold(int k, double r, double x)
+{
+    return (k == 0 || k == 1 || k == 7) ? fmax(r, x) : (k == 6 ? fmin(r, x) : r + x);
+}
+// Four quantities over the warp by f, quantity k in lane 8 k. Halves of the warp
+// take two each, quarters one (6 operations instead of 20; binary64 runs at 2
+// lanes a cycle and SM), in the order of a butterfly over all lanes.
+template <class F>
+__device__ __forceinline__ double warp_fold4(double a0, double a1, double a2, double a3, F &&f)
+{
+    const int lane = threadIdx.x & 31;
+    const bool h = lane & 16, q = lane & 8;
+    const double b0 = f(h ? a2 : a0, __shfl_xor_sync(0xffffffffu, h ? a0 : a2, 16));
+    const double b1 = f(h ? a3 : a1, __shfl_xor_sync(0xffffffffu, h ? a1 : a3, 16));
+    double c = f(q ? b1 : b0, __shfl_xor_sync(0xffffffffu, q ? b0 : b1, 8));
+#pragma unroll
+    for (int o = 4; o; o >>= 1) c = f(c, __shfl_xor_sync(0xffffffffu, c, o));
+    return c;
 }
 
 template <int KIND, bool DIFF>
@@ -931,27 +938,26 @@ decode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int s
             }
         }
         if (DIFF) {
-            // block totals in binary64: maxima exact, sums of the compensated partials
+            // block totals in binary64: maxima exact, sums of the compensated
+            // partials; order of the record: {e_inf, n_inf, e_1, e_2, n_1, n_2,
+            // min, max}, the first two and the last two as maxima
             double(*red)[8] = reinterpret_cast<double(*)[8]>(sm + kRing + kStores * kPlane);
-            double t[8];
-            t[0] = warp_max(fabs((double)acc.es + acc.ee));
-            t[1] = warp_max(acc.ninf);
-            t[6] = -warp_max(-(double)acc.mn);
-            t[7] = warp_max(acc.mx);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) t[2 + k] = warp_sum((double)acc.s[k] + (double)acc.c[k]);
-            if (lane == 0)
-                for (int k = 0; k < 8; ++k) red[warp][k] = t[k];
+            const double m = warp_fold4(fabs((double)acc.es + acc.ee), (double)acc.ninf, -(double)acc.mn, (double)acc.mx,
+                                        [](double a, double b) { return fmax(a, b); });
+            const double u = warp_fold4((double)acc.s[0] + (double)acc.c[0], (double)acc.s[1] + (double)acc.c[1],
+                                        (double)acc.s[2] + (double)acc.c[2], (double)acc.s[3] + (double)acc.c[3],
+                                        [](double a, double b) { return a + b; });
+            if ((lane & 7) == 0) {
+                const int k = lane >> 3;
+                red[warp][k < 2 ? k : k + 4] = k == 2 ? -m : m;
+                red[warp][2 + k] = u;
+            }
             __syncthreads();
-            if (threadIdx.x < 8) {
-                const int k = threadIdx.x;
-                double r = red[0][k];
-                for (int w = 1; w < kNW; ++w) {
-                    const double x = red[w][k];
-                    r = (k == 0 || k == 1 || k == 7) ? fmax(r, x) : (k == 6 ? fmin(r, x) : r + x);
-                }
-                // e_1 n_1 e_2 n_2 order of the record: {e_inf, n_inf, e_1, e_2, n_1, n_2, min, max}
-                diff_out[g * 8 + k] = r;
+            if (lane == 0 && warp < 8) {  // a warp per quantity: one chain of binary64 operations each
+                double r = red[0][warp];
+#pragma unroll
+                for (int w = 1; w < kNW; ++w) r = diff_fold(warp, r, red[w][warp]);
+                diff_out[g * 8 + warp] = r;
             }
         }
     }
@@ -964,10 +970,6 @@ decode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int s
 // in flight, folded in block order), then the groups fold in order j = 0, 1,
 // ... Deterministic for a given block count.
 constexpr int kDiffGroups = 128;
-__device__ __forceinline__ double diff_fold(int k, double r, double x)
-{
-    return (k == 0 || k == 1 || k == 7) ? fmax(r, x) : (k == 6 ? fmin(r, x) : r + x);
-}
 __global__ void __launch_bounds__(8 * kDiffGroups)
 diff_total_kernel(const double *per_block, long long nblocks, double *total)
 {
