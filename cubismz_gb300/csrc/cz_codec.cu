@@ -70,12 +70,16 @@ struct Blk {
 };
 static_assert(sizeof(Blk) == 32, "Blk");
 
-__device__ __forceinline__ void set_block(Blk *b, long long g, const CzField *fields, int nfields, long long total)
+// Block g of the launch, and its field's tensor map made ready for the CTA: every
+// use of it lies behind a CTA-wide barrier after this.
+__device__ __forceinline__ void set_block(Blk *b, long long g, const CzFields &fs, long long total)
 {
     b->g = -1;
     if (g < total) {
-        const BlockRef r = locate(fields, nfields, g);
+        const CzField *fields = fs.list ? fs.list : &fs.one;
+        const BlockRef r = locate(fields, fs.n, g);
         b->field = (int)(r.f - fields);
+        if (fs.list) tma_map_acquire(fs.maps + b->field);
         b->x = 32 * r.bx;
         b->y = 32 * r.by;
         b->z = 32 * r.bz;
@@ -86,16 +90,14 @@ __device__ __forceinline__ void set_block(Blk *b, long long g, const CzField *fi
 
 // The CTA's blocks come from the queue, the second one with the first; where
 // every block can have a CTA of its own, without it.
-__device__ __forceinline__ void take_first(Blk *b, const CzField *fields, int nfields, long long total,
-                                           unsigned long long *queue)
+__device__ __forceinline__ void take_first(Blk *b, const CzFields &fs, long long total, unsigned long long *queue)
 {
     const long long g = total <= gridDim.x ? (long long)blockIdx.x : (long long)atomicAdd(queue, 1ull);
-    set_block(b, g, fields, nfields, total);
+    set_block(b, g, fs, total);
 }
-__device__ __forceinline__ void take_later(Blk *b, const CzField *fields, int nfields, long long total,
-                                           unsigned long long *queue)
+__device__ __forceinline__ void take_later(Blk *b, const CzFields &fs, long long total, unsigned long long *queue)
 {
-    if (total > gridDim.x) set_block(b, (long long)atomicAdd(queue, 1ull), fields, nfields, total);
+    if (total > gridDim.x) set_block(b, (long long)atomicAdd(queue, 1ull), fs, total);
     else b->g = -1;
 }
 
@@ -267,8 +269,6 @@ __global__ void __launch_bounds__(kNT, 1)
 encode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int zerobits, int shuffle, uint8_t *stage,
               int *rec_bytes, unsigned long long *queue, int *err, CzChunks chunks)
 {
-    const CzField *fields = fs.list ? fs.list : &fs.one;
-    const int nfields = fs.n;
     extern __shared__ __align__(1024) unsigned char sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t zmask = zerobits > 0 ? ~((1u << zerobits) - 1u) : 0xffffffffu;
@@ -282,7 +282,7 @@ encode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int z
         for (int s = 0; s < kSlots; ++s) mbar_init(bars + 8 * s, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         *fail = 0;
-        take_first(blk, fields, nfields, total_blocks, queue);
+        take_first(blk, fs, total_blocks, queue);
     }
     __syncthreads();
     // plane n of the CTA's sequence (plane n & 31 of its block n >> 5) into
@@ -298,7 +298,7 @@ encode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int z
         bring(warp);
         if (warp + 16 < kSlots) bring(warp + 16);
     }
-    if (threadIdx.x == 0) take_later(blk + 1, fields, nfields, total_blocks, queue);
+    if (threadIdx.x == 0) take_later(blk + 1, fs, total_blocks, queue);
     __syncthreads();
 
     uint32_t it = 0;
@@ -371,7 +371,7 @@ encode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int z
             }
         }
         __syncthreads();
-        if (warp == kNW - 1 && lane == 0) take_later(blk + ((it + 2) & 3), fields, nfields, total_blocks, queue);
+        if (warp == kNW - 1 && lane == 0) take_later(blk + ((it + 2) & 3), fs, total_blocks, queue);
         if (AHEAD && warp == kNW - 2 && lane >= kSlots) {
             const Blk &b = blk[(it + 1) & 3];
             if (b.g >= 0) tma_prefetch_3d(fs.list ? fs.maps + b.field : &fs.map, b.x, b.y, b.z + lane);
@@ -623,8 +623,6 @@ __global__ void __launch_bounds__(kNT, 1)
 decode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int shuffle, CzRecords where, int *flag,
               unsigned long long *queue, const float *diff_ref, double *diff_out, CzPlanes planes)
 {
-    const CzField *fields = fs.list ? fs.list : &fs.one;
-    const int nfields = fs.n;
     extern __shared__ __align__(1024) unsigned char sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int *seg_cnt = reinterpret_cast<int *>(sm + kSegCnt), *warp_cnt = reinterpret_cast<int *>(sm + kWarpCnt);
@@ -688,7 +686,7 @@ decode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int s
     };
     if (scout) {
         bad[0] = bad[1] = 0;
-        take_first(blk, fields, nfields, total_blocks, queue);
+        take_first(blk, fs, total_blocks, queue);
         scout_off(0);
         scout_rec(0);
         find(0, s_off, s_len, s_nb, s_hole, s_src);
@@ -696,7 +694,7 @@ decode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int s
     __syncthreads();
     if (blk[0].g < 0) return;
     if (scout) {
-        take_later(blk + 1, fields, nfields, total_blocks, queue);
+        take_later(blk + 1, fs, total_blocks, queue);
         scout_off(1);
         scout_rec(1);
         find(1, s_off, s_len, s_nb, s_hole, s_src);
@@ -868,7 +866,7 @@ decode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int s
             for (int j = 0; j < 16; ++j) at(sm, corner(j, y, z)) = u[j];
         } else if (scout) {  // idle meanwhile
             blk[(it + 2) & 3].g = -1;
-            if (more) set_block(blk + ((it + 2) & 3), (long long)s_ticket, fields, nfields, total_blocks);
+            if (more) set_block(blk + ((it + 2) & 3), (long long)s_ticket, fs, total_blocks);
             scout_off(it + 2);
         } else if (more && warp < kNW - 1) {
             fetch(it + 1, threadIdx.x - 256, kNT - 256 - 32);
@@ -926,7 +924,7 @@ decode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int s
             if (DIFF) {
                 // a lane reads its row 16 bytes at a time: the line must stay in L1
                 // between the reads (as streaming loads: 1.42 instead of 1.17 ms at 512^3)
-                const CzField &f = fields[cur.field];
+                const CzField &f = fs.list ? fs.list[cur.field] : fs.one;
                 const float4 *rr = reinterpret_cast<const float4 *>(
                     diff_ref + ((size_t)(cur.z + z) * f.ny + (size_t)(cur.y + lane)) * f.nx + (size_t)cur.x);
 #pragma unroll

@@ -20,8 +20,10 @@ struct CzField {
 // must be 16-byte aligned.
 bool cz_field_map(const CzField &f, CUtensorMap *map);
 // The fields of a launch: n descriptors and their tensor maps (64-byte aligned)
-// in device memory, or (list == nullptr) a single field by value, which costs
-// no copy to the device and no read of it at the start of every CTA.
+// in device memory (the kernels acquire each map before they use it: it may have
+// been copied to where an earlier launch had another), or (list == nullptr) a
+// single field by value, which costs no copy to the device and no read of it at
+// the start of every CTA.
 struct CzFields {
     CUtensorMap map = {};
     CzField one = {};

@@ -29,6 +29,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long lo
     }
     return false;
 }
+// Before a CTA uses a tensor map that a copy from the host has written to global
+// memory: maps are read through a cache of their own, which may still hold what
+// an earlier copy left at that address. By one thread, with a CTA-wide barrier
+// before the others use the map.
+__device__ __forceinline__ void tma_map_acquire(const CUtensorMap *map)
+{
+    asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
 // Box at (c0, c1, c2) of `map` into shared memory; `bar` completes after
 // `bytes` bytes.
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, uint32_t bar,
