@@ -890,6 +890,11 @@ int cz_plan_create(cz_ctx *c, int nfields, const float *const *d_fields, const i
         cudaGetLastError();
         return bail(CZ_E_CUDA, "graph instantiation");
     }
+    // the fields' list is on the device before a launch on another stream reads it
+    if (cudaStreamSynchronize(pl->st) != cudaSuccess) {
+        cudaGetLastError();
+        return bail(CZ_E_CUDA, "plan stream");
+    }
     *out = pl;
     return CZ_OK;
 }

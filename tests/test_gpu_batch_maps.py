@@ -46,3 +46,30 @@ def test_plans_one_after_the_other(gpu_lib):
             sd, so = cz.compress_field(f, e, 1, 4, True, encoder="none").to_device()
             assert torch.equal(o, so) and torch.equal(d, sd)
         plan.close()
+
+
+def test_plan_list_is_there_before_its_first_launch(gpu_lib):
+    """cz_plan_create copies the fields' list on a stream of its own; a launch
+    on another stream right after it, with the copy engine still busy with
+    something else, reads the whole list."""
+    import torch
+    import cubismz_gb300 as cz
+    shapes = SHAPES * 3
+    fields = [torch.from_numpy(np.random.default_rng(50 + i).standard_normal(s).astype(np.float32)).cuda()
+              for i, s in enumerate(shapes)]
+    eps = [1e-3 * (i + 1) for i in range(len(fields))]
+    host = torch.empty(1 << 28, pin_memory=True).fill_(1.0)
+    dev = torch.empty(1 << 28, device="cuda")
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        dev.copy_(host, non_blocking=True)
+    plan = cz.Plan(fields, eps, 1, 4, True, "none", tune=False)
+    plan.launch()
+    data, off = plan.result().to_device()
+    torch.cuda.synchronize()
+    for i, (f, e) in enumerate(zip(fields, eps)):
+        d, o = plan.field_chunks(data, off, i)
+        sd, so = cz.compress_field(f, e, 1, 4, True, encoder="none").to_device()
+        assert torch.equal(o, so) and torch.equal(d, sd)
+    plan.close()
