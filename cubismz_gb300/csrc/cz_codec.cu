@@ -55,7 +55,8 @@ constexpr int kWarpCnt = kSegCnt + 112 * 4;        // int x 16: survivors per wa
 constexpr int kBlkAt = kWarpCnt + 64;              // Blk x 4
 constexpr int kBarAt = kBlkAt + 4 * 32;            // mbarrier per slot
 constexpr int kFailAt = kBarAt + 8 * kSlots;
-constexpr int kCodecSmem = kFailAt + 16;
+constexpr int kBroughtAt = kFailAt + 16;           // encode: u32 per slot, 1 + the last plane brought into it
+constexpr int kCodecSmem = kBroughtAt + 4 * kSlots;
 constexpr int kMaskOdd = kRing + (kStores + 1) * kPlane;  // decode: the mask of every second block
 constexpr int kRecAt = kRing + (kStores + 2) * kPlane;    // decode: Rec x 4
 static_assert(kCodecSmem <= 232448, "shared memory of one CTA");
@@ -276,10 +277,14 @@ encode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int z
     int *seg_cnt = reinterpret_cast<int *>(sm + kSegCnt), *warp_cnt = reinterpret_cast<int *>(sm + kWarpCnt);
     Blk *blk = reinterpret_cast<Blk *>(sm + kBlkAt);
     volatile int *fail = reinterpret_cast<volatile int *>(sm + kFailAt);
+    uint32_t *brought = reinterpret_cast<uint32_t *>(sm + kBroughtAt);
     const uint32_t bars = smem_u32(sm + kBarAt), ring = smem_u32(sm + kRing);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kSlots; ++s) mbar_init(bars + 8 * s, 1);
+        for (int s = 0; s < kSlots; ++s) {
+            mbar_init(bars + 8 * s, 1);
+            brought[s] = 0;
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         *fail = 0;
         take_first(blk, fs, total_blocks, queue);
@@ -291,6 +296,7 @@ encode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int z
         const Blk &b = blk[(n >> 5) & 3];
         if (b.g < 0) return;
         const uint32_t s = n % kSlots;
+        brought[s] = n + 1;
         tma_load_3d(ring + s * kPlane, fs.list ? fs.maps + b.field : &fs.map, b.x, b.y, b.z + (int)(n & 31), bars + 8 * s,
                     kPlane);
     };
@@ -313,9 +319,10 @@ encode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int z
             const int z = warp + 16 * r;
             const uint32_t n = 32 * it + z, s = n % kSlots;
             unsigned char *slot = sm + kRing + s * kPlane;
-            // after one wait ran out the others poll only briefly: the
-            // launch ends, and its error is reported
-            if (!mbar_wait(bars + 8 * s, (n / kSlots) & 1, *fail ? 64 : kWaitLimit)) *fail = 1;
+            // after one wait ran out the others poll only briefly: the CTA
+            // ends, and its error is reported
+            const bool here = mbar_wait(bars + 8 * s, (n / kSlots) & 1, *fail ? 64 : kTilePolls);
+            if (!here) *fail = 1;
             float v[32];
             ld_row(slot, lane, v);
             line_fwd<32, KIND>(v);
@@ -324,7 +331,9 @@ encode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int z
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = at(slot, col_at(lane, j));
             __syncwarp();
-            if (lane == 0) {
+            // a slot whose copy is still to come gets no second one: planes 22 to 31
+            // follow planes 0 to 9 of the same block, whose waits are over at r == 1
+            if (lane == 0 && here && !*fail) {
                 fence_async_smem();
                 bring(n + kSlots);
             }
@@ -334,6 +343,7 @@ encode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int z
             for (int j = 0; j < 32; ++j) at(sm, kMain + j * kPlane + z * 128 + lane * 4) = v[j];
         }
         __syncthreads();
+        if (*fail) break;  // the same for all: the waits are over until the next block
         // ---- level 32, z: slabs y = warp and warp + 16
 #pragma unroll 1
         for (int r = 0; r < 2; ++r) {
@@ -473,17 +483,23 @@ encode_kernel(const __grid_constant__ CzFields fs, long long total_blocks, int z
                          lane);
         }
     }
-    // every plane brought in was waited for; a launch that gave up waiting
-    // lets its copies land (bounded) before it leaves
-    __syncthreads();
+    // every plane brought in was waited for; a CTA that gave up waiting lets its
+    // copies land (bounded) before it leaves, and gives the blocks that it has
+    // taken, and those that nobody has yet, the sizes that what follows reads
     if (*fail && threadIdx.x == 0) {
         if (err) atomicExch(err, 1);
-        for (uint32_t s = 0; s < kSlots && s < 32 * it; ++s) {
-            const uint32_t last = (32 * it - 1 - s) / kSlots;  // the slot's last use
-            mbar_wait(bars + 8 * s, last & 1);
-        }
+        for (uint32_t s = 0; s < kSlots; ++s)
+            if (brought[s]) mbar_wait(bars + 8 * s, ((brought[s] - 1) / kSlots) & 1);
+        auto skip = [&](long long g) {
+            *reinterpret_cast<int *>(stage + (size_t)g * kSlotBytes) = kMaskBytes;
+            rec_bytes[g] = kMaskBytes;
+            record_done(chunks, g, kMaskBytes);
+        };
+        for (uint32_t k = it; k < it + 2; ++k)
+            if (blk[k & 3].g >= 0) skip(blk[k & 3].g);
+        if (total_blocks > gridDim.x)
+            for (long long g; (g = (long long)atomicAdd(queue, 1ull)) < total_blocks;) skip(g);
     }
-    __syncthreads();
 }
 
 // Error statistics of a decoded block against a reference field (the

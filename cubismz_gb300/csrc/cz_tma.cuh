@@ -8,6 +8,11 @@
 namespace cz {
 
 constexpr long long kWaitLimit = 1ll << 22;  // try_wait polls before giving up
+#if defined(CZ_TILE_POLLS)  // the polls for a tile of the wavelet kernel; a test build's waits run out with it
+constexpr long long kTilePolls = CZ_TILE_POLLS;
+#else
+constexpr long long kTilePolls = kWaitLimit;
+#endif
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
 {
