@@ -25,19 +25,21 @@
 //     stencil's own maximum, and binary64 only when even that is too wide.
 //
 // Signed zeros follow the binary64 chain: when the hi sum is zero the result
-// is the lo chain itself, evaluated left to right like the reference. A line
-// without a -0 among its sources needs no such case: every zero hi and lo is
-// then +0, every stencil has a positive coefficient, so both chains end in +0
-// where they vanish, and the plain sum is right.
+// is the lo chain itself, whose zeros have the chain's signs. That costs no
+// instruction: hi is carried negated, with -0 for a hi that vanishes, so that
+// its chain (every stencil has coefficients of both signs) vanishes to +0 and
+// lo - (+0) is lo. A line with a -0 thus needs no path of its own: a field with
+// a -0 background takes the encode kernel 62 us at 256^3; with such lines on the
+// out-of-line path below it took 172.
 //
 // What bounds a line on the GPU is instruction issue, so the main path keeps
-// (hi, lo) as a register pair and evaluates both chains with packed binary32
+// (-hi, lo) as a register pair and evaluates both chains with packed binary32
 // arithmetic (two roundings per instruction, each as the scalar one's):
 // 5 instructions per 4-point stencil instead of 10; and it finds the line's
 // largest and smallest non-zero magnitude with three-input minima and maxima,
-// 2.5 instructions per source instead of 4. Encode
-// kernel at 512^3: 0.516 -> 0.429 ms, decode 0.706 -> 0.646 ms. The other
-// paths are rare and stay out of line, which keeps the kernels' code small.
+// 2 instructions per source instead of 4. Encode kernel at 512^3: 0.516 -> 0.412
+// ms (wtype 1). The other paths are rare and stay out of line, which keeps the
+// kernels' code small.
 //
 // All binary32 arithmetic goes through explicit round-to-nearest intrinsics so
 // the compiler cannot contract or reassociate it; host builds use
@@ -60,8 +62,8 @@
 #define CZ_ADD(a, b) __fadd_rn((a), (b))
 #define CZ_SUB(a, b) __fsub_rn((a), (b))
 #define CZ_MUL(a, b) __fmul_rn((a), (b))
-#define CZ_DADD(a, b) __dadd_rn((a), (b))
 #define CZ_DMUL(a, b) __dmul_rn((a), (b))
+#define CZ_DFMA(a, b, c) __fma_rn((a), (b), (c))
 #define CZ_D2F(a) __double2float_rn(a)
 #define CZ_BITS(x) __float_as_uint(x)
 #define CZ_FLT(u) __uint_as_float(u)
@@ -72,8 +74,8 @@
 #define CZ_ADD(a, b) ((float)((a) + (b)))
 #define CZ_SUB(a, b) ((float)((a) - (b)))
 #define CZ_MUL(a, b) ((float)((a) * (b)))
-#define CZ_DADD(a, b) ((double)(a) + (double)(b))
 #define CZ_DMUL(a, b) ((double)(a) * (double)(b))
+#define CZ_DFMA(a, b, c) fma((a), (b), (c))
 #define CZ_D2F(a) ((float)(a))
 CZ_HD uint32_t cz_bits_h(float x)
 {
@@ -164,19 +166,11 @@ CZ_HD void split(const float (&v)[H], float C, float (&hi)[H], float (&lo)[H])
     }
 }
 
-// Minima and maxima of three.
+// Minimum of three.
 CZ_HD uint32_t umin3(uint32_t a, uint32_t b, uint32_t c)
 {
 #if defined(__CUDA_ARCH__)
     return __vimin3_u32(a, b, c);
-#else
-    return CZ_UMIN(CZ_UMIN(a, b), c);
-#endif
-}
-CZ_HD int32_t smin3(int32_t a, int32_t b, int32_t c)
-{
-#if defined(__CUDA_ARCH__)
-    return __vimin3_s32(a, b, c);
 #else
     return CZ_UMIN(CZ_UMIN(a, b), c);
 #endif
@@ -194,29 +188,37 @@ CZ_HD float amax3(float a, float b, float c)
 #endif
 }
 
+// Whether the split grids are exact for sources of largest magnitude amax and
+// smallest non-zero magnitude lo2 (as 2 bits - 1, which orders the non-zero
+// magnitudes and puts zeros past them all): all non-zero ones within `spread`
+// binades of the largest, and that one within the grids' range (or everything
+// zero).
+CZ_HD bool in_range(uint32_t amax, uint32_t lo2, int spread)
+{
+    const uint32_t eb = CZ_UMIN(CZ_UMAX(amax >> 23, 27u), 247u);
+    return (amax == 0u || (amax >> 23) == eb) && lo2 >= ((eb - (uint32_t)spread) << 24) - 1u;
+}
+
 // Exponent analysis of a line's sources (H even). Returns whether the main
-// path is exact for every stencil with K <= 32 on this line: no -0, all
-// non-zero magnitudes within kSpread binades of the largest, and that one
-// within the grids' range (or everything zero). `narrow`: within kLastSpread.
-// 2 bits - 1 orders the non-zero magnitudes and puts zeros past them all; as
-// signed integers the bits of -0 are the least.
+// path is exact for every stencil with K <= 32 on this line. `narrow`: the last
+// four, which interp_last takes, lie within kLastSpread binades of the largest
+// (noise-like sources: all but one line in 170; for all 16 of them it would be
+// one in 40).
 template <int H>
 CZ_HD bool line_grid(const float (&v)[H], uint32_t &amax, bool &narrow)
 {
+    auto x = [&](int i) { return 2u * CZ_BITS(v[i]) - 1u; };
     float m = amax3(v[0], v[1], v[1]);
-    uint32_t lo = CZ_UMIN(2u * CZ_BITS(v[0]) - 1u, 2u * CZ_BITS(v[1]) - 1u);
-    int32_t neg = CZ_UMIN((int32_t)CZ_BITS(v[0]), (int32_t)CZ_BITS(v[1]));
+    const uint32_t last = umin3(CZ_UMIN(x(H - 4), x(H - 3)), x(H - 2), x(H - 1));
+    uint32_t lo = last;
 #pragma unroll
-    for (int i = 2; i < H; i += 2) {
-        m = amax3(m, v[i], v[i + 1]);
-        lo = umin3(lo, 2u * CZ_BITS(v[i]) - 1u, 2u * CZ_BITS(v[i + 1]) - 1u);
-        neg = smin3(neg, (int32_t)CZ_BITS(v[i]), (int32_t)CZ_BITS(v[i + 1]));
-    }
+    for (int i = 2; i < H; i += 2) m = amax3(m, v[i], v[i + 1]);
+#pragma unroll
+    for (int i = 0; i < H - 4; i += 2) lo = umin3(lo, x(i), x(i + 1));
     amax = CZ_BITS(m);
     const uint32_t eb = CZ_UMIN(CZ_UMAX(amax >> 23, 27u), 247u);
-    narrow = lo >= ((eb - (uint32_t)kLastSpread) << 24) - 1u;
-    return (amax == 0u || (amax >> 23) == eb) && neg != INT32_MIN &&
-           lo >= ((eb - (uint32_t)kSpread) << 24) - 1u;
+    narrow = last >= ((eb - (uint32_t)kLastSpread) << 24) - 1u;
+    return (amax == 0u || (amax >> 23) == eb) && lo >= ((eb - (uint32_t)kSpread) << 24) - 1u;
 }
 
 // Line-level analysis and split on the main grid.
@@ -229,7 +231,7 @@ CZ_HD bool line_split(const float (&v)[H], float (&hi)[H], float (&lo)[H], uint3
     return ok;
 }
 
-// A (hi, lo) pair and packed binary32 arithmetic on it.
+// A (-hi, lo) pair and packed binary32 arithmetic on it.
 struct Pair {
 #if defined(__CUDA_ARCH__)
     unsigned long long v;
@@ -281,27 +283,30 @@ CZ_HD Pair padd(Pair x, Pair y)
 #endif
     return p;
 }
-CZ_HD float psum(Pair x)
+// The sum rounded down: exact operands, so only its zeros differ (-0 unless
+// both are +0).
+CZ_HD Pair padd_rd(Pair x, Pair y)
 {
+    Pair p;
 #if defined(__CUDA_ARCH__)
-    float a, b;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
-    return CZ_ADD(a, b);
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(p.v) : "l"(x.v), "l"(y.v));
 #else
-    return CZ_ADD(x.a, x.b);
+    p.a = CZ_ADD(x.a, y.a);
+    p.b = CZ_ADD(x.b, y.b);
+    if (p.a == 0.f) p.a = CZ_BITS(x.a) | CZ_BITS(y.a) ? -0.f : 0.f;
+    if (p.b == 0.f) p.b = CZ_BITS(x.b) | CZ_BITS(y.b) ? -0.f : 0.f;
 #endif
+    return p;
 }
-CZ_HD Pair split_pair(float v, float C)
+CZ_HD Pair pfma_rd(Pair x, Pair y, Pair z)
 {
-    const float hi = CZ_SUB(CZ_ADD(v, C), C);
-    return pair(hi, CZ_SUB(v, hi));
-}
-// RN32 of sum c_i*(hi_i+lo_i) for lines without -0.
-template <class S>
-CZ_HD float st4_pair(Pair p0, Pair p1, Pair p2, Pair p3)
-{
-    constexpr float k0 = S::c[0], k1 = S::c[1], k2 = S::c[2], k3 = S::c[3];
-    return psum(pfma(pair(k3, k3), p3, pfma(pair(k2, k2), p2, pfma(pair(k1, k1), p1, pmul(pair(k0, k0), p0)))));
+    Pair p;
+#if defined(__CUDA_ARCH__)
+    asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(p.v) : "l"(x.v), "l"(y.v), "l"(z.v));
+#else
+    p = padd_rd(pmul(x, y), z);
+#endif
+    return p;
 }
 CZ_HD void unpair(Pair x, float &a, float &b)
 {
@@ -312,19 +317,31 @@ CZ_HD void unpair(Pair x, float &a, float &b)
     b = x.b;
 #endif
 }
-// 16 times the W1M stencil, RN32 of 9 (p1 + p2) - (p0 + p3), from the pair
-// sums u_i = p_i + p_{i+1} as 10 u_1 - (u_0 + u_2). Scaling by a power of two
-// commutes with the rounding (line_grid keeps a line's sums clear of the
-// subnormals), so the caller's fma with 1/16 gives the bits of the stencil's
-// own rounding followed by the add. Every step is exact (sums below
-// 22 * 2^19), zeros come out +0 as from the chain, and a stencil takes 8
-// cycles of the fma pipe instead of 10.
-CZ_HD float w1m_16(Pair u0, Pair u1, Pair u2)
+// hi + lo of a chain's (-hi, lo).
+CZ_HD float psum(Pair x)
 {
-    float uh, ul, wh, wl;
-    unpair(u1, uh, ul);
-    unpair(padd(u0, u2), wh, wl);
-    return CZ_ADD(CZ_FMA(10.f, uh, -wh), CZ_FMA(10.f, ul, -wl));
+    float a, b;
+    unpair(x, a, b);
+    return CZ_SUB(b, a);
+}
+// -hi rounded down: exact, and -0 where it vanishes; lo then keeps the sign of a
+// zero v.
+CZ_HD Pair split_pair(float v, float C)
+{
+#if defined(__CUDA_ARCH__)
+    const float n = __fsub_rd(C, CZ_ADD(v, C));
+#else
+    float n = CZ_SUB(C, CZ_ADD(v, C));
+    if (n == 0.f) n = -0.f;
+#endif
+    return pair(n, CZ_ADD(v, n));
+}
+// RN32 of sum c_i*(hi_i+lo_i) given an exact split (see header).
+template <class S>
+CZ_HD float st4_pair(Pair p0, Pair p1, Pair p2, Pair p3)
+{
+    constexpr float k0 = S::c[0], k1 = S::c[1], k2 = S::c[2], k3 = S::c[3];
+    return psum(pfma(pair(k3, k3), p3, pfma(pair(k2, k2), p2, pfma(pair(k1, k1), p1, pmul(pair(k0, k0), p0)))));
 }
 template <class S>
 CZ_HD float st3_pair(Pair p0, Pair p1, Pair p2)
@@ -332,65 +349,58 @@ CZ_HD float st3_pair(Pair p0, Pair p1, Pair p2)
     constexpr float k0 = S::c[0], k1 = S::c[1], k2 = S::c[2];
     return psum(pfma(pair(k2, k2), p2, pfma(pair(k1, k1), p1, pmul(pair(k0, k0), p0))));
 }
-
-// RN32 of sum c_i*(hi_i+lo_i) given an exact split (see header).
+// The stencil on the grid of split constant C.
 template <class S>
-CZ_HD float st4_fast(float h0, float h1, float h2, float h3, float l0, float l1, float l2, float l3)
+CZ_HD float st4_on(float v0, float v1, float v2, float v3, float C)
 {
-    float sh = CZ_MUL(S::c[0], h0);
-    sh = CZ_FMA(S::c[1], h1, sh);
-    sh = CZ_FMA(S::c[2], h2, sh);
-    sh = CZ_FMA(S::c[3], h3, sh);
-    float sl = CZ_MUL(S::c[0], l0);
-    sl = CZ_FMA(S::c[1], l1, sl);
-    sl = CZ_FMA(S::c[2], l2, sl);
-    sl = CZ_FMA(S::c[3], l3, sl);
-    return sh == 0.f ? sl : CZ_ADD(sh, sl);
+    return st4_pair<S>(split_pair(v0, C), split_pair(v1, C), split_pair(v2, C), split_pair(v3, C));
 }
-template <class S>
-CZ_HD float st3_fast(float h0, float h1, float h2, float l0, float l1, float l2)
+// 16 times the W1M stencil, RN32 of 9 (p1 + p2) - (p0 + p3). Scaling by a power
+// of two commutes with the rounding (line_grid keeps a line's sums clear of the
+// subnormals), so the caller's fma with 1/16 gives the bits of the stencil's
+// own rounding followed by the add. Every step is exact (sums below 20 * 2^19);
+// the zeros of lo are the chain's: 9 (p1 + p2) is -0 where both are -0, and
+// -(p0 + p3), rounded so, where both are +0. 8 cycles of the fma pipe instead of
+// the chain's 10.
+CZ_HD float w1m_16(Pair p0, Pair p1, Pair p2, Pair p3)
 {
-    float sh = CZ_MUL(S::c[0], h0);
-    sh = CZ_FMA(S::c[1], h1, sh);
-    sh = CZ_FMA(S::c[2], h2, sh);
-    float sl = CZ_MUL(S::c[0], l0);
-    sl = CZ_FMA(S::c[1], l1, sl);
-    sl = CZ_FMA(S::c[2], l2, sl);
-    return sh == 0.f ? sl : CZ_ADD(sh, sl);
+    float un, ul, wn, wl;
+    unpair(padd(p1, p2), un, ul);
+    unpair(padd_rd(p0, p3), wn, wl);
+    return CZ_SUB(CZ_FMA(9.f, ul, -wl), CZ_FMA(9.f, un, -wn));
+}
+// The P0M and P1M stencils: p1 +- (p0 - p2) / 8. The difference is -0 where p0
+// is -0 and p2 is +0, as P0M's products are; rounded down, +0 where P1M's are.
+CZ_HD void avg_mid(Pair p0, Pair p1, Pair p2, float &even, float &odd)
+{
+    const Pair m = pair(-1.f, -1.f), t = pfma(m, p2, p0), u = pfma_rd(m, p2, p0);
+    even = psum(pfma(pair(0.125f, 0.125f), t, p1));
+    odd = psum(pfma(pair(-0.125f, -0.125f), u, p1));
 }
 
 // The reference arithmetic itself: binary64 products summed left to right,
-// rounded to binary32 once (used when no exact binary32 split exists).
+// rounded to binary32 once (used when no exact binary32 split exists). The
+// products are exact, so an fma rounds like the sum alone.
 template <class S>
 CZ_HD float st4_f64(float v0, float v1, float v2, float v3)
 {
-    double s = CZ_DMUL((double)S::c[0], (double)v0);
-    s = CZ_DADD(s, CZ_DMUL((double)S::c[1], (double)v1));
-    s = CZ_DADD(s, CZ_DMUL((double)S::c[2], (double)v2));
-    s = CZ_DADD(s, CZ_DMUL((double)S::c[3], (double)v3));
-    return CZ_D2F(s);
+    constexpr double k0 = S::c[0], k1 = S::c[1], k2 = S::c[2], k3 = S::c[3];
+    return CZ_D2F(CZ_DFMA(k3, (double)v3, CZ_DFMA(k2, (double)v2, CZ_DFMA(k1, (double)v1, CZ_DMUL(k0, (double)v0)))));
 }
 template <class S>
 CZ_HD float st3_f64(float v0, float v1, float v2)
 {
-    double s = CZ_DMUL((double)S::c[0], (double)v0);
-    s = CZ_DADD(s, CZ_DMUL((double)S::c[1], (double)v1));
-    s = CZ_DADD(s, CZ_DMUL((double)S::c[2], (double)v2));
-    return CZ_D2F(s);
+    constexpr double k0 = S::c[0], k1 = S::c[1], k2 = S::c[2];
+    return CZ_D2F(CZ_DFMA(k2, (double)v2, CZ_DFMA(k1, (double)v1, CZ_DMUL(k0, (double)v0))));
 }
 
-// Per-stencil path: split against the stencil's own maximum (grid chosen by
-// the stencil's coefficient sum); binary64 when even that is too wide.
-template <class S, int B, int SPREAD>
+// Per-stencil path: the stencil's own grid, or binary64.
+template <class S>
 CZ_HD float st4_any(float v0, float v1, float v2, float v3)
 {
     const float v[4] = {v0, v1, v2, v3};
     const uint32_t amax = max_bits<4>(v);
-    if (within<4>(v, amax, SPREAD)) {
-        float h[4], l[4];
-        split<4>(v, split_const<B>(amax), h, l);
-        return st4_fast<S>(h[0], h[1], h[2], h[3], l[0], l[1], l[2], l[3]);
-    }
+    if (within<4>(v, amax, kSpread)) return st4_on<S>(v0, v1, v2, v3, split_const<kGridBits>(amax));
     return st4_f64<S>(v0, v1, v2, v3);
 }
 template <class S>
@@ -399,40 +409,26 @@ CZ_HD float st3_any(float v0, float v1, float v2)
     const float v[3] = {v0, v1, v2};
     const uint32_t amax = max_bits<3>(v);
     if (within<3>(v, amax, kSpread)) {
-        float h[3], l[3];
-        split<3>(v, split_const<kGridBits>(amax), h, l);
-        return st3_fast<S>(h[0], h[1], h[2], l[0], l[1], l[2]);
+        const float C = split_const<kGridBits>(amax);
+        return st3_pair<S>(split_pair(v0, C), split_pair(v1, C), split_pair(v2, C));
     }
     return st3_f64<S>(v0, v1, v2);
 }
 
-template <class S>
-CZ_HD float st4_main(float v0, float v1, float v2, float v3)
-{
-    return st4_any<S, kGridBits, kSpread>(v0, v1, v2, v3);
-}
-CZ_HD float st4_lastany(float v0, float v1, float v2, float v3)
-{
-    return st4_any<W1L, kLastGridBits, kLastSpread>(v0, v1, v2, v3);
-}
-
 // interp_last on a line's last four sources (K = 96, its own coarser grid),
-// given the line maximum and a line without -0; `narrow` as line_grid says.
-CZ_RARE float interp_last_wide(float v0, float v1, float v2, float v3, uint32_t line_amax)
+// given the line maximum; `narrow` as line_grid says. Otherwise their own
+// maximum's grid, or binary64.
+CZ_RARE float interp_last_wide(float v0, float v1, float v2, float v3)
 {
     const float v[4] = {v0, v1, v2, v3};
-    if (within<4>(v, line_amax, kLastSpread)) {
-        float h[4], l[4];
-        split<4>(v, split_const<kLastGridBits>(line_amax), h, l);
-        return st4_fast<W1L>(h[0], h[1], h[2], h[3], l[0], l[1], l[2], l[3]);
-    }
-    return st4_lastany(v0, v1, v2, v3);
+    const uint32_t amax = max_bits<4>(v);
+    if (within<4>(v, amax, kLastSpread)) return st4_on<W1L>(v0, v1, v2, v3, split_const<kLastGridBits>(amax));
+    return st4_f64<W1L>(v0, v1, v2, v3);
 }
 CZ_HD float interp_last(float v0, float v1, float v2, float v3, uint32_t line_amax, bool narrow)
 {
-    if (!narrow) return interp_last_wide(v0, v1, v2, v3, line_amax);
-    const float C = split_const<kLastGridBits>(line_amax);
-    return st4_pair<W1L>(split_pair(v0, C), split_pair(v1, C), split_pair(v2, C), split_pair(v3, C));
+    if (!narrow) return interp_last_wide(v0, v1, v2, v3);
+    return st4_on<W1L>(v0, v1, v2, v3, split_const<kLastGridBits>(line_amax));
 }
 
 }  // namespace cz

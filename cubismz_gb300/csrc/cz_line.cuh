@@ -12,14 +12,31 @@ namespace cz {
 
 // ---------------------------------------------------------------- wtype 1/2
 // Predictions of a line's odd samples from its H scalings e
-// (WaveletsOnInterval.h:33-51), stencil by stencil.
-CZ_RARE void interp_rare(const float *e, float *o, int H)
+// (WaveletsOnInterval.h:33-51) where one grid does not do for the line: every
+// four neighbours on a grid of their own, binary64 where even that is not exact.
+// Out of line and rolled, one prediction after the other: noise has a few such
+// lines, and unrolled whole it took more from the kernels' other code (encode at
+// 512^3 0.429 ms instead of 0.417) than it gave where most lines come here.
+CZ_RARE void interp_wide(const float *__restrict__ e, float *__restrict__ o, int H)
 {
-    o[0] = st4_main<W1F>(e[0], e[1], e[2], e[3]);
+    float v0 = e[0], v1 = e[1], v2 = e[2], v3 = e[3];
+    o[0] = st4_any<W1F>(v0, v1, v2, v3);
 #pragma unroll 1
-    for (int i = 1; i < H - 2; ++i) o[i] = st4_main<W1M>(e[i - 1], e[i], e[i + 1], e[i + 2]);
-    o[H - 2] = st4_main<W1O>(e[H - 4], e[H - 3], e[H - 2], e[H - 1]);
-    o[H - 1] = st4_lastany(e[H - 4], e[H - 3], e[H - 2], e[H - 1]);
+    for (int i = 1;; ++i) {
+        const uint32_t amax = CZ_BITS(amax3(v0, v1, amax3(v2, v3, v3)));
+        const uint32_t lo = umin3(2u * CZ_BITS(v0) - 1u, 2u * CZ_BITS(v1) - 1u,
+                                  CZ_UMIN(2u * CZ_BITS(v2) - 1u, 2u * CZ_BITS(v3) - 1u));
+        float r = st4_on<W1M>(v0, v1, v2, v3, split_const<kGridBits>(amax));
+        if (!in_range(amax, lo, kSpread)) r = st4_f64<W1M>(v0, v1, v2, v3);
+        o[i] = r;
+        if (i == H - 3) break;
+        v0 = v1;
+        v1 = v2;
+        v2 = v3;
+        v3 = e[i + 3];
+    }
+    o[H - 2] = st4_any<W1O>(v0, v1, v2, v3);
+    o[H - 1] = interp_last_wide(v0, v1, v2, v3);
 }
 // o[i] = base[i] + sign * prediction i, each rounded as the reference rounds
 // (the prediction, then the sum).
@@ -34,18 +51,16 @@ CZ_HD void interp_predict(const float (&e)[H], float sign, const float (&base)[H
 #pragma unroll
         for (int i = 0; i < H; ++i) p[i] = split_pair(e[i], C);
         o[0] = CZ_FMA(sign, st4_pair<W1F>(p[0], p[1], p[2], p[3]), base[0]);
-        Pair u[H - 1];
 #pragma unroll
-        for (int i = 0; i < H - 1; ++i) u[i] = padd(p[i], p[i + 1]);
-#pragma unroll
-        for (int i = 1; i < H - 2; ++i) o[i] = CZ_FMA(0.0625f * sign, w1m_16(u[i - 1], u[i], u[i + 1]), base[i]);
+        for (int i = 1; i < H - 2; ++i)
+            o[i] = CZ_FMA(0.0625f * sign, w1m_16(p[i - 1], p[i], p[i + 1], p[i + 2]), base[i]);
         o[H - 2] = CZ_FMA(sign, st4_pair<W1O>(p[H - 4], p[H - 3], p[H - 2], p[H - 1]), base[H - 2]);
         o[H - 1] = CZ_FMA(sign, interp_last(e[H - 4], e[H - 3], e[H - 2], e[H - 1], amax, narrow), base[H - 1]);
     } else {
         float te[H], to[H];  // the call's arrays live in memory, e and o in registers
 #pragma unroll
         for (int i = 0; i < H; ++i) te[i] = e[i];
-        interp_rare(te, to, H);
+        interp_wide(te, to, H);
 #pragma unroll
         for (int i = 0; i < H; ++i) o[i] = CZ_FMA(sign, to[i], base[i]);
     }
@@ -91,18 +106,33 @@ CZ_HD void inv_interp(float (&x)[N], bool lifting)
 
 // ---------------------------------------------------------------- wtype 3
 // Predictions of a line's even and odd samples from its H scalings s
-// (WaveletsOnInterval.h:55-83).
-CZ_RARE void avg_rare(const float *s, float *p0, float *p1, int H)
+// (WaveletsOnInterval.h:55-83), as interp_wide: every three neighbours on a grid
+// of their own.
+CZ_RARE void avg_wide(const float *__restrict__ s, float *__restrict__ o0, float *__restrict__ o1, int H)
 {
-    p0[0] = st3_any<P0F>(s[0], s[1], s[2]);
-    p1[0] = st3_any<P1F>(s[0], s[1], s[2]);
+    float v0 = s[0], v1 = s[1], v2 = s[2];
+    o0[0] = st3_any<P0F>(v0, v1, v2);
+    o1[0] = st3_any<P1F>(v0, v1, v2);
 #pragma unroll 1
-    for (int i = 1; i < H - 1; ++i) {
-        p0[i] = st3_any<P0M>(s[i - 1], s[i], s[i + 1]);
-        p1[i] = st3_any<P1M>(s[i - 1], s[i], s[i + 1]);
+    for (int i = 1;; ++i) {
+        const uint32_t amax = CZ_BITS(amax3(v0, v1, v2));
+        const uint32_t lo = umin3(2u * CZ_BITS(v0) - 1u, 2u * CZ_BITS(v1) - 1u, 2u * CZ_BITS(v2) - 1u);
+        const float C = split_const<kGridBits>(amax);
+        float even, odd;
+        avg_mid(split_pair(v0, C), split_pair(v1, C), split_pair(v2, C), even, odd);
+        if (!in_range(amax, lo, kSpread)) {
+            even = st3_f64<P0M>(v0, v1, v2);
+            odd = st3_f64<P1M>(v0, v1, v2);
+        }
+        o0[i] = even;
+        o1[i] = odd;
+        if (i == H - 2) break;
+        v0 = v1;
+        v1 = v2;
+        v2 = s[i + 2];
     }
-    p0[H - 1] = st3_any<P0L>(s[H - 3], s[H - 2], s[H - 1]);
-    p1[H - 1] = st3_any<P1L>(s[H - 3], s[H - 2], s[H - 1]);
+    o0[H - 1] = st3_any<P0L>(v0, v1, v2);
+    o1[H - 1] = st3_any<P1L>(v0, v1, v2);
 }
 template <int H>
 CZ_HD void avg_predict(const float (&s)[H], float (&p0)[H], float (&p1)[H])
@@ -110,27 +140,21 @@ CZ_HD void avg_predict(const float (&s)[H], float (&p0)[H], float (&p1)[H])
     uint32_t amax;
     bool narrow;
     if (line_grid<H>(s, amax, narrow)) {
-        const float C = split_const<kGridBits>(amax);
-        Pair p[H];
+    const float C = split_const<kGridBits>(amax);
+    Pair p[H];
 #pragma unroll
-        for (int i = 0; i < H; ++i) p[i] = split_pair(s[i], C);
-        p0[0] = st3_pair<P0F>(p[0], p[1], p[2]);
-        p1[0] = st3_pair<P1F>(p[0], p[1], p[2]);
+    for (int i = 0; i < H; ++i) p[i] = split_pair(s[i], C);
+    p0[0] = st3_pair<P0F>(p[0], p[1], p[2]);
+    p1[0] = st3_pair<P1F>(p[0], p[1], p[2]);
 #pragma unroll
-        for (int i = 1; i < H - 1; ++i) {
-            // p[i] +- (p[i-1] - p[i+1]) / 8: the difference is shared (exact,
-            // and +0 where it vanishes)
-            const Pair t = pfma(pair(-1.f, -1.f), p[i + 1], p[i - 1]);
-            p0[i] = psum(pfma(pair(0.125f, 0.125f), t, p[i]));
-            p1[i] = psum(pfma(pair(-0.125f, -0.125f), t, p[i]));
-        }
-        p0[H - 1] = st3_pair<P0L>(p[H - 3], p[H - 2], p[H - 1]);
-        p1[H - 1] = st3_pair<P1L>(p[H - 3], p[H - 2], p[H - 1]);
+    for (int i = 1; i < H - 1; ++i) avg_mid(p[i - 1], p[i], p[i + 1], p0[i], p1[i]);
+    p0[H - 1] = st3_pair<P0L>(p[H - 3], p[H - 2], p[H - 1]);
+    p1[H - 1] = st3_pair<P1L>(p[H - 3], p[H - 2], p[H - 1]);
     } else {
-        float t[H], t0[H], t1[H];
+        float t[H], t0[H], t1[H];  // the call's arrays live in memory
 #pragma unroll
         for (int i = 0; i < H; ++i) t[i] = s[i];
-        avg_rare(t, t0, t1, H);
+        avg_wide(t, t0, t1, H);
 #pragma unroll
         for (int i = 0; i < H; ++i) {
             p0[i] = t0[i];
