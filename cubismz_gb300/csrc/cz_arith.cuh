@@ -24,22 +24,25 @@
 //     binary32 range, take the per-stencil path: the same split against the
 //     stencil's own maximum, and binary64 only when even that is too wide.
 //
-// Signed zeros follow the binary64 chain: when the hi sum is zero the result
-// is the lo chain itself, whose zeros have the chain's signs. That costs no
-// instruction: hi is carried negated, with -0 for a hi that vanishes, so that
-// its chain (every stencil has coefficients of both signs) vanishes to +0 and
-// lo - (+0) is lo. A line with a -0 thus needs no path of its own: a field with
+// Signed zeros follow the binary64 chain, whose zero is -0 only where all its
+// products are: -0 under every positive coefficient, +0 under every negative
+// one. That costs no instruction. The result is lo - (-hi): a hi sum that
+// vanishes comes out as -hi = +0 (every stencil has coefficients of both signs),
+// so the result is the lo sum, whose zeros have the signs of its sources'. Only
+// where sources that are not zero cancel would their lo (+0) pass for a zero
+// source's; that takes two sources of one coefficient sign, so it concerns W1M
+// and W1L (see there). A line with a -0 thus needs no path of its own: a field with
 // a -0 background takes the encode kernel 62 us at 256^3; with such lines on the
 // out-of-line path below it took 172.
 //
 // What bounds a line on the GPU is instruction issue, so the main path keeps
-// (-hi, lo) as a register pair and evaluates both chains with packed binary32
+// (hi, lo) as a register pair and evaluates both chains with packed binary32
 // arithmetic (two roundings per instruction, each as the scalar one's):
 // 5 instructions per 4-point stencil instead of 10; and it finds the line's
 // largest and smallest non-zero magnitude with three-input minima and maxima,
 // 2 instructions per source instead of 4. Encode kernel at 512^3: 0.516 -> 0.412
-// ms (wtype 1). The other paths are rare and stay out of line, which keeps the
-// kernels' code small.
+// ms (wtype 1), 0.420 with the signs of cancelling zeros. The other paths are
+// rare and stay out of line, which keeps the kernels' code small.
 //
 // All binary32 arithmetic goes through explicit round-to-nearest intrinsics so
 // the compiler cannot contract or reassociate it; host builds use
@@ -231,7 +234,7 @@ CZ_HD bool line_split(const float (&v)[H], float (&hi)[H], float (&lo)[H], uint3
     return ok;
 }
 
-// A (-hi, lo) pair and packed binary32 arithmetic on it.
+// A pair of hi (or -hi) and lo, and packed binary32 arithmetic on it.
 struct Pair {
 #if defined(__CUDA_ARCH__)
     unsigned long long v;
@@ -324,9 +327,13 @@ CZ_HD float psum(Pair x)
     unpair(x, a, b);
     return CZ_SUB(b, a);
 }
-// -hi rounded down: exact, and -0 where it vanishes; lo then keeps the sign of a
-// zero v.
 CZ_HD Pair split_pair(float v, float C)
+{
+    const float hi = CZ_SUB(CZ_ADD(v, C), C);
+    return pair(hi, CZ_SUB(v, hi));
+}
+// (-hi, lo): -hi rounded down, which is exact, and -0 where it vanishes.
+CZ_HD Pair split_neg(float v, float C)
 {
 #if defined(__CUDA_ARCH__)
     const float n = __fsub_rd(C, CZ_ADD(v, C));
@@ -336,12 +343,14 @@ CZ_HD Pair split_pair(float v, float C)
 #endif
     return pair(n, CZ_ADD(v, n));
 }
-// RN32 of sum c_i*(hi_i+lo_i) given an exact split (see header).
+// RN32 of sum c_i*(hi_i+lo_i) given an exact split (see header): the
+// interpolating stencils from (hi, lo), the averaging ones from (-hi, lo), whose
+// middle has no product to negate hi with.
 template <class S>
 CZ_HD float st4_pair(Pair p0, Pair p1, Pair p2, Pair p3)
 {
     constexpr float k0 = S::c[0], k1 = S::c[1], k2 = S::c[2], k3 = S::c[3];
-    return psum(pfma(pair(k3, k3), p3, pfma(pair(k2, k2), p2, pfma(pair(k1, k1), p1, pmul(pair(k0, k0), p0)))));
+    return psum(pfma(pair(-k3, k3), p3, pfma(pair(-k2, k2), p2, pfma(pair(-k1, k1), p1, pmul(pair(-k0, k0), p0)))));
 }
 template <class S>
 CZ_HD float st3_pair(Pair p0, Pair p1, Pair p2)
@@ -349,25 +358,43 @@ CZ_HD float st3_pair(Pair p0, Pair p1, Pair p2)
     constexpr float k0 = S::c[0], k1 = S::c[1], k2 = S::c[2];
     return psum(pfma(pair(k2, k2), p2, pfma(pair(k1, k1), p1, pmul(pair(k0, k0), p0))));
 }
-// The stencil on the grid of split constant C.
+// The two interpolating stencils with two negative coefficients: from u and w,
+// the exact sums of what is added and of what is taken away, u - w. w is rounded
+// down: its lo is +0 only where both its sources are, its hi -0 only where two
+// that are not zero cancel, which makes the zero +0 again. Here:
+// 16 times W1M, RN32 of 9 (p1 + p2) - (p0 + p3). Scaling by a power of two
+// commutes with the rounding (line_grid keeps a line's sums clear of the
+// subnormals), so the caller's fma with 1/16 gives the bits of the stencil's
+// own rounding followed by the add. 8 cycles of the fma pipe instead of the
+// chain's 10.
+CZ_HD float w1m_16(Pair p0, Pair p1, Pair p2, Pair p3)
+{
+    float uh, ul, wh, wl;
+    unpair(padd(p1, p2), uh, ul);
+    unpair(padd_rd(p0, p3), wh, wl);
+    return CZ_SUB(CZ_FMA(9.f, ul, -wl), CZ_FMA(-9.f, uh, wh));
+}
+CZ_HD float w1l(Pair p0, Pair p1, Pair p2, Pair p3)
+{
+    constexpr float k0 = -W1L::c[0], k1 = W1L::c[1], k2 = -W1L::c[2], k3 = W1L::c[3];
+    float uh, ul, wh, wl;
+    unpair(pfma(pair(k3, k3), p3, pmul(pair(k1, k1), p1)), uh, ul);
+    unpair(pfma_rd(pair(k2, k2), p2, pmul(pair(k0, k0), p0)), wh, wl);
+    return CZ_SUB(CZ_SUB(ul, wl), CZ_SUB(wh, uh));
+}
+// Stencils on the grid of split constant C.
 template <class S>
 CZ_HD float st4_on(float v0, float v1, float v2, float v3, float C)
 {
     return st4_pair<S>(split_pair(v0, C), split_pair(v1, C), split_pair(v2, C), split_pair(v3, C));
 }
-// 16 times the W1M stencil, RN32 of 9 (p1 + p2) - (p0 + p3). Scaling by a power
-// of two commutes with the rounding (line_grid keeps a line's sums clear of the
-// subnormals), so the caller's fma with 1/16 gives the bits of the stencil's
-// own rounding followed by the add. Every step is exact (sums below 20 * 2^19);
-// the zeros of lo are the chain's: 9 (p1 + p2) is -0 where both are -0, and
-// -(p0 + p3), rounded so, where both are +0. 8 cycles of the fma pipe instead of
-// the chain's 10.
-CZ_HD float w1m_16(Pair p0, Pair p1, Pair p2, Pair p3)
+CZ_HD float w1m_on(float v0, float v1, float v2, float v3, float C)
 {
-    float un, ul, wn, wl;
-    unpair(padd(p1, p2), un, ul);
-    unpair(padd_rd(p0, p3), wn, wl);
-    return CZ_SUB(CZ_FMA(9.f, ul, -wl), CZ_FMA(9.f, un, -wn));
+    return 0.0625f * w1m_16(split_pair(v0, C), split_pair(v1, C), split_pair(v2, C), split_pair(v3, C));
+}
+CZ_HD float w1l_on(float v0, float v1, float v2, float v3, float C)
+{
+    return w1l(split_pair(v0, C), split_pair(v1, C), split_pair(v2, C), split_pair(v3, C));
 }
 // The P0M and P1M stencils: p1 +- (p0 - p2) / 8. The difference is -0 where p0
 // is -0 and p2 is +0, as P0M's products are; rounded down, +0 where P1M's are.
@@ -410,7 +437,7 @@ CZ_HD float st3_any(float v0, float v1, float v2)
     const uint32_t amax = max_bits<3>(v);
     if (within<3>(v, amax, kSpread)) {
         const float C = split_const<kGridBits>(amax);
-        return st3_pair<S>(split_pair(v0, C), split_pair(v1, C), split_pair(v2, C));
+        return st3_pair<S>(split_neg(v0, C), split_neg(v1, C), split_neg(v2, C));
     }
     return st3_f64<S>(v0, v1, v2);
 }
@@ -422,13 +449,13 @@ CZ_RARE float interp_last_wide(float v0, float v1, float v2, float v3)
 {
     const float v[4] = {v0, v1, v2, v3};
     const uint32_t amax = max_bits<4>(v);
-    if (within<4>(v, amax, kLastSpread)) return st4_on<W1L>(v0, v1, v2, v3, split_const<kLastGridBits>(amax));
+    if (within<4>(v, amax, kLastSpread)) return w1l_on(v0, v1, v2, v3, split_const<kLastGridBits>(amax));
     return st4_f64<W1L>(v0, v1, v2, v3);
 }
 CZ_HD float interp_last(float v0, float v1, float v2, float v3, uint32_t line_amax, bool narrow)
 {
     if (!narrow) return interp_last_wide(v0, v1, v2, v3);
-    return st4_on<W1L>(v0, v1, v2, v3, split_const<kLastGridBits>(line_amax));
+    return w1l_on(v0, v1, v2, v3, split_const<kLastGridBits>(line_amax));
 }
 
 }  // namespace cz

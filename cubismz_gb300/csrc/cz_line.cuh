@@ -26,7 +26,7 @@ CZ_RARE void interp_wide(const float *__restrict__ e, float *__restrict__ o, int
         const uint32_t amax = CZ_BITS(amax3(v0, v1, amax3(v2, v3, v3)));
         const uint32_t lo = umin3(2u * CZ_BITS(v0) - 1u, 2u * CZ_BITS(v1) - 1u,
                                   CZ_UMIN(2u * CZ_BITS(v2) - 1u, 2u * CZ_BITS(v3) - 1u));
-        float r = st4_on<W1M>(v0, v1, v2, v3, split_const<kGridBits>(amax));
+        float r = w1m_on(v0, v1, v2, v3, split_const<kGridBits>(amax));
         if (!in_range(amax, lo, kSpread)) r = st4_f64<W1M>(v0, v1, v2, v3);
         o[i] = r;
         if (i == H - 3) break;
@@ -119,7 +119,7 @@ CZ_RARE void avg_wide(const float *__restrict__ s, float *__restrict__ o0, float
         const uint32_t lo = umin3(2u * CZ_BITS(v0) - 1u, 2u * CZ_BITS(v1) - 1u, 2u * CZ_BITS(v2) - 1u);
         const float C = split_const<kGridBits>(amax);
         float even, odd;
-        avg_mid(split_pair(v0, C), split_pair(v1, C), split_pair(v2, C), even, odd);
+        avg_mid(split_neg(v0, C), split_neg(v1, C), split_neg(v2, C), even, odd);
         if (!in_range(amax, lo, kSpread)) {
             even = st3_f64<P0M>(v0, v1, v2);
             odd = st3_f64<P1M>(v0, v1, v2);
@@ -143,7 +143,7 @@ CZ_HD void avg_predict(const float (&s)[H], float (&p0)[H], float (&p1)[H])
     const float C = split_const<kGridBits>(amax);
     Pair p[H];
 #pragma unroll
-    for (int i = 0; i < H; ++i) p[i] = split_pair(s[i], C);
+    for (int i = 0; i < H; ++i) p[i] = split_neg(s[i], C);
     p0[0] = st3_pair<P0F>(p[0], p[1], p[2]);
     p1[0] = st3_pair<P1F>(p[0], p[1], p[2]);
 #pragma unroll

@@ -63,3 +63,36 @@ def test_wide_lines_bit_exact(emu, wtype):  # noqa: F811
 def _same(a, b):
     both = np.isnan(a) & np.isnan(b)
     return np.array_equal(np.where(both, 0, a.view(np.uint32)), np.where(both, 0, b.view(np.uint32)))
+
+
+def signed_zero_fields():
+    """Zeros of both signs beside values that cancel exactly in a stencil."""
+    rng = np.random.default_rng(12)
+    yield rng.choice(np.array([0.0, -0.0, -0.0, 1.0, -1.0, 0.5, -0.5], np.float32), size=N)
+    yield rng.choice(np.array([0.0, -0.0, -0.0, 7.0, -1.0, 1.0, -7.0], np.float32), size=N)  # -5 v0 = 35 v2
+    yield np.where(rng.random(N) < 0.7, rng.choice(np.array([0.0, -0.0], np.float32), size=N),
+                   rng.integers(-2, 3, N)).astype(np.float32)
+
+
+@pytest.mark.parametrize("wtype", [1, 2, 3])
+def test_signs_of_zeros(emu, wtype):  # noqa: F811
+    for b in signed_zero_fields():
+        phys, pos = b.copy(), np.zeros(N, np.float32)
+        emu.emu_fwt(phys.ctypes.data_as(fp), wtype, None)
+        emu.emu_to_positional(phys.ctypes.data_as(fp), pos.ctypes.data_as(fp))
+        assert np.array_equal(pos.view(np.uint32), O.fwt(b, wtype).view(np.uint32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("wtype", [1, 2, 3])
+def test_signs_of_zeros_on_the_gpu(gpu_lib, wtype):
+    """The same fields through the kernels, everything kept, bit for bit."""
+    import torch
+    import cubismz_gb300 as cz
+    f = np.concatenate(list(signed_zero_fields()) * 60)  # several blocks per CTA
+    cf = cz.compress_field(torch.from_numpy(f).cuda(), -1.0, wtype, 0, False, encoder="none")
+    data, off = cf.to_device()
+    raw, ooff = O.field_compress(f, -1.0, wtype, 0, 0, 0, 1)
+    assert np.array_equal(off.cpu().numpy(), ooff) and np.array_equal(data.cpu().numpy(), raw)
+    dec = cz.decompress_field(data, off, f.shape, wtype, False, encoder="none").cpu().numpy()
+    assert np.array_equal(dec.view(np.uint32), O.field_decompress(raw, ooff, f.shape, wtype, 0).view(np.uint32))
