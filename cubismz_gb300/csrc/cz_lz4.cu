@@ -723,7 +723,7 @@ struct LzPairShared {
     uint2 seq[2][SW / 4];  // two windows in flight
     int2 lane[2][32];      // ns, myP
     int4 win[2];           // base (-1: the end, with the anchor), anchor, hlo, hhi
-    int nlong, stop;       // stop: 1 + the chunk whose output is past its capacity
+    int nlong;
 };
 // Named barriers, one per buffer b: 1 + b full, 3 + b empty. Immediate ids, so
 // that a CTA holds 5 of the SM's barriers and not 16.
@@ -750,8 +750,6 @@ lz4_encode_pair_kernel(const uint8_t *__restrict__ in, const long long *in_off, 
     __shared__ LzPairShared<kSW> ps;
     const int lane = threadIdx.x & 31;
     int buf = 0;
-    if (threadIdx.x == 0) ps.stop = 0;
-    __syncthreads();
     if (threadIdx.x < 32) {
         for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
             Parse p;
@@ -759,8 +757,7 @@ lz4_encode_pair_kernel(const uint8_t *__restrict__ in, const long long *in_off, 
             for (bool more = true; more; buf ^= 1) {
                 pair_wait<kPairEmpty>(buf);
                 int base, ns, myP;
-                more = *(volatile int *)&ps.stop != c + 1 &&
-                       p.next(ps.table, ps.info, ps.seq[buf] + Parse::kSub / 4 * lane, base, ns, myP);
+                more = p.next(ps.table, ps.info, ps.seq[buf] + Parse::kSub / 4 * lane, base, ns, myP);
                 if (more) ps.lane[buf][lane] = make_int2(ns, myP);
                 if (lane == 0) ps.win[buf] = make_int4(more ? base : -1, p.anchor, p.hlo, p.hhi);
                 pair_signal<kPairFull>(buf);
@@ -775,7 +772,7 @@ lz4_encode_pair_kernel(const uint8_t *__restrict__ in, const long long *in_off, 
         for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
             LzEmit<SEQ, kEffort> e;
             e.start(in + in_off[c], in_len[c], out + out_off[c], hole ? hole + c : nullptr, records != 0);
-            bool ok = true;
+            bool ok = true;  // past the capacity the rest of the chunk's windows are passed over
             for (bool more = true; more; buf ^= 1) {
                 pair_wait<kPairFull>(buf);
                 const int4 w = ps.win[buf];
@@ -786,7 +783,6 @@ lz4_encode_pair_kernel(const uint8_t *__restrict__ in, const long long *in_off, 
                 } else if (ok) {
                     ok = e.tail(w.y, w.z, w.w);
                 }
-                if (!ok && lane == 0) *(volatile int *)&ps.stop = c + 1;  // no more of this chunk
                 __syncwarp();
                 pair_signal<kPairEmpty>(buf);
             }
