@@ -279,7 +279,10 @@ inflate_kernel(const uint8_t *__restrict__ in, const long long *in_off, const in
                     }
                     const int total = __shfl_sync(0xffffffffu, incl, 31);
                     const int at = op + incl - nl - len, p = at + nl;  // the record's literals, its match
-                    const int bad = p > oend ? 15 : len && d > p ? 19 : p + len > oend ? 20 : 0;
+                    // against the room left: with a capacity near 2^31 the ends
+                    // themselves may not be ints
+                    const int room = oend - op;
+                    const int bad = incl - len > room ? 15 : len && d > p ? 19 : incl > room ? 20 : 0;
                     const unsigned bb = __ballot_sync(0xffffffffu, bad != 0);
                     if (bb) {
                         err = __shfl_sync(0xffffffffu, bad, __ffs(bb) - 1);
