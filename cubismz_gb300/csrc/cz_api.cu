@@ -652,6 +652,13 @@ int cz_field_diff(cz_ctx *c, const uint8_t *d_data, const long long *d_off, int 
     const long long nblocks = (long long)(nx / 32) * (ny / 32) * (nz / 32);
     const int bpc = p->blocks_per_chunk;
     if ((long long)nchunks != (nblocks + bpc - 1) / bpc) return fail(c, CZ_E_ARG, "chunk count does not match the field");
+    // decoded over the reference itself: the statistics are the decoded field's
+    // against itself, as they are where a row is written before it is compared
+    // (the kernel's rows are written by tile copies, in no order with its reads)
+    if (d_field == d_ref) {
+        CZ_TRY(cz_field_decompress(c, d_data, d_off, nchunks, nx, ny, nz, p, stream, d_field));
+        d_field = nullptr;
+    }
     if (!d_field) {
         CZ_TRY(grow(c, c->tmp_field, sizeof(float) * (size_t)nx * ny * nz));
         d_field = P<float>(c->tmp_field);

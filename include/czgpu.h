@@ -183,7 +183,8 @@ int cz_field_decompress(cz_ctx *ctx, const uint8_t *d_data, const long long *d_c
  * e = |decoded - ref|, n = |ref| (e_2 and n_2 are sums of squares). The
  * differences and maxima are exact; sums are compensated per thread and
  * binary64 beyond (the reference sums serially in binary64). d_field may be
- * NULL (decode into context scratch). */
+ * NULL (decode into context scratch), or d_ref: the field is then decoded over
+ * the reference, and the statistics are its own against itself. */
 int cz_field_diff(cz_ctx *ctx, const uint8_t *d_data, const long long *d_chunk_offsets, int nchunks, int nx, int ny,
                   int nz, const cz_params *p, const float *d_ref, void *stream, float *d_field, double *stats);
 /* cz2diff's RES line from those statistics and the compressed size
