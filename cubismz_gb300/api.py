@@ -297,6 +297,10 @@ class Plan:
         return data[int(o[0]):int(o[-1])], o - o[0]
 
     def info(self):
+        """The tuned shape and the times it was chosen by (cz_plan_shape). The
+        wavelet kernel's variants 0 and 1 are named by what they once were:
+        `split_prefetch` brings the next block into L2 ahead, `joint_prefetch`
+        does not."""
         w = C.c_int(0)
         t = (C.c_float * 3)()
         self.ctx.L.cz_plan_info(self.h, C.byref(w), t)

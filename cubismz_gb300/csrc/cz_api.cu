@@ -840,8 +840,9 @@ int cz_plan_create(cz_ctx *c, int nfields, const float *const *d_fields, const i
     }
     if ((rc = prepare(pl->c, f, total, &q, 0, pl->st, pl->job)) != CZ_OK) return bail(rc, "prepare");
     // autotuner, timed on this batch with CUDA events (best of the second
-    // and third run of each shape): first the LZ4 stage's CTA width (2, 4,
-    // 8 or 16 chunks per CTA) with the wavelet kernel's default variant,
+    // and third run of each shape that is a kernel of its own): first the LZ4
+    // stage's CTA width (2, 4, 8 or 16 chunks per CTA) with the wavelet kernel's
+    // default variant,
     // then the wavelet kernel with the next block brought into L2 ahead or
     // not, with that width. Every shape writes the same bytes.
     cz_stream tmp;
@@ -861,14 +862,21 @@ int cz_plan_create(cz_ctx *c, int nfields, const float *const *d_fields, const i
         };
         if (q.encoder == CZ_ENCODER_LZ4) {
             const int cand[4] = {2, 4, 8, 16};
+            // with few chunks the first three are one kernel, two warps and a
+            // CTA per chunk: timed once
+            const bool pairs = pl->job.nchunks <= kLzPairChunksPerSm * pl->c->sms;
             int pick = 4;
             float best = 1e30f;
             for (int k = 0; k < 4; ++k) {
-                pl->job.lz_warps = cand[k];
+                if (pairs && (k == 1 || k == 2)) {
+                    pl->lz_ms[k] = pl->lz_ms[0];
+                    continue;
+                }
+                pl->job.lz_warps = pairs && k == 0 ? 4 : cand[k];
                 if ((rc = time_stage(1, pl->lz_ms[k])) != CZ_OK) return bail(rc, "tune");
                 if (pl->lz_ms[k] < best) {
                     best = pl->lz_ms[k];
-                    pick = cand[k];
+                    pick = pl->job.lz_warps;
                 }
             }
             pl->job.lz_warps = pick;

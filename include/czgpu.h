@@ -256,7 +256,9 @@ int cz_plan_info(const cz_plan *plan, int *lz_warps, float *tune_ms /* 3: LZ4 ms
  * variant (0: the part of the next block that shared memory does not hold
  * yet is brought into L2 ahead, 1: it is not); ms[0..3] = LZ4 stage at
  * 2, 4, 8, 16 chunks per CTA, ms[4..5] = wavelet kernel in variant 0, 1
- * (-1 where not timed). No counterpart in the reference. */
+ * (-1 where not timed). Batches of at most 9 chunks per SM take a CTA with two
+ * warps per chunk for the widths 2, 4 and 8: one time, and the width is 4 or
+ * 16. No counterpart in the reference. */
 int cz_plan_shape(const cz_plan *plan, int *shape /* 2 */, float *ms /* 6 */);
 const char *cz_plan_last_error(const cz_plan *plan);
 int cz_plan_destroy(cz_plan *plan);
