@@ -284,7 +284,8 @@ def batch_report(cz, dev, steps):
            "autotune": {"space": "LZ4 chunks per CTA {2, 4, 8, 16} x next block into L2 ahead {yes, no}",
                         "chosen": info["shape"],
                         "lz4_stage_ms": {str(k): v for k, v in info["lz4_stage_ms"].items()},
-                        "wavelet_kernel_ms": info["wavelet_kernel_ms"]}}
+                        "wavelet_kernel_ms": dict(zip(("next_block_into_l2", "not"),
+                                                      info["wavelet_kernel_ms"].values()))}}
     plan.close()
     del fields
     torch.cuda.empty_cache()

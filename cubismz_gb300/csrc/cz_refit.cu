@@ -404,8 +404,7 @@ __global__ void __launch_bounds__(kNT, 1) iwt_adjoint_kernel(const float *in, fl
 // with the last part in one warp. A sum that binary64 holds exactly does not
 // depend on the order: where the exponents span 20 bits at most (24 + 20 + 9
 // bits for 512 values make 53), it is formed in integers; else as described.
-// meanwhile() runs in every warp after its part of the sum is out; then(sum)
-// in warp 0, before the closing barrier.
+// then(sum) runs in warp 0, before the closing barrier.
 struct SumPart {
     double d;              // a warp's sum
     unsigned long long s;  // the same in units of 2^(lo - 150), if exact
@@ -426,8 +425,8 @@ __device__ __forceinline__ double from_units(unsigned long long x, int lo)
     return x ? __longlong_as_double(__double_as_longlong((double)x) + ((long long)(lo - 150) << 52)) : 0.0;
 }
 
-template <class M, class F>
-__device__ __forceinline__ void block_sum(float v, SumPart *part, M &&meanwhile, F &&then)
+template <class F>
+__device__ __forceinline__ void block_sum(float v, SumPart *part, F &&then)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     {
@@ -466,7 +465,6 @@ __device__ __forceinline__ void block_sum(float v, SumPart *part, M &&meanwhile,
         }
         then(t);
     }
-    meanwhile();
     __syncthreads();
 }
 
@@ -683,7 +681,7 @@ refit_kernel(const CzField *fields, int nfields, long long total_blocks, int zer
             }
             // ---- alpha = gamma / ||q||^2
             if (it >= 0) {
-                block_sum(acc, part, [] {}, [&](double delta) {
+                block_sum(acc, part, [&](double delta) {
                     if (lane == 0) {
                         s_go = delta > 0.0;
                         s_ratio = delta > 0.0 ? (float)(s_gamma / delta) : 0.f;
@@ -743,7 +741,7 @@ refit_kernel(const CzField *fields, int nfields, long long total_blocks, int zer
                 const float v0 = sb[a], v1 = sb[a + 1], v2 = sb[a + 2], v3 = sb[a + 3];
                 acc = __fmaf_rn(v0, v0, __fmaf_rn(v1, v1, __fmaf_rn(v2, v2, __fmaf_rn(v3, v3, acc))));
             }
-            block_sum(acc, part, [] {}, [&](double gnew) {
+            block_sum(acc, part, [&](double gnew) {
                 if (lane == 0) {
                     s_ratio = it < 0 ? 0.f : (float)(gnew / s_gamma);
                     s_gamma = gnew;

@@ -276,7 +276,9 @@ int cz_plan_destroy(cz_plan *plan);
  * address and should come before any stream capture. Calls share the
  * scratch, so calls that overlap on the GPU race. Returns CZ_E_ARG for
  * nblocks beyond the maximum, and when d_blocks is not 16-byte aligned or
- * d_records or d_nbytes is not 4-byte aligned (checked before any launch). */
+ * d_records or d_nbytes is not 4-byte aligned (checked before any launch).
+ * d_nbytes[g] is -1 for every block where the kernel's tile copies did not
+ * complete in time. */
 #define CZ_NOALLOC_MAX_BLOCKS 16
 int cz_blocks_compress_noalloc(const float *d_blocks, int nblocks, float eps, int wtype, int zerobits, int shuffle,
                                uint8_t *d_records, int *d_nbytes, void *stream);
