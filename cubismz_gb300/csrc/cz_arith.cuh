@@ -32,7 +32,7 @@
 // where sources that are not zero cancel would their lo (+0) pass for a zero
 // source's; that takes two sources of one coefficient sign, so it concerns W1M
 // and W1L (see there). A line with a -0 thus needs no path of its own: a field with
-// a -0 background takes the encode kernel 62 us at 256^3; with such lines on the
+// a -0 background takes the encode kernel 61 us at 256^3; with such lines on the
 // out-of-line path below it took 172.
 //
 // What bounds a line on the GPU is instruction issue, so the main path keeps
@@ -40,9 +40,9 @@
 // arithmetic (two roundings per instruction, each as the scalar one's):
 // 5 instructions per 4-point stencil instead of 10; and it finds the line's
 // largest and smallest non-zero magnitude with three-input minima and maxima,
-// 2 instructions per source instead of 4. Encode kernel at 512^3: 0.516 -> 0.412
-// ms (wtype 1), 0.420 with the signs of cancelling zeros. The other paths are
-// rare and stay out of line, which keeps the kernels' code small.
+// 2 instructions per source instead of 4. Encode kernel at 512^3: 0.516 -> 0.416
+// ms (wtype 1). The other paths are rare and stay out of line, which keeps the
+// kernels' code small.
 //
 // All binary32 arithmetic goes through explicit round-to-nearest intrinsics so
 // the compiler cannot contract or reassociate it; host builds use

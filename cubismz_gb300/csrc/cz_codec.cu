@@ -34,8 +34,8 @@
 //   * corner -- levels 16 and 8 (an eighth of the block) stay in the first
 //     quarters of slabs 0..15 and are thresholded 8 positions per thread.
 // The decoder runs the same steps backwards. Measured at 512^3 (wtype 1,
-// threshold 1e-3 of the range): encode 0.664 -> 0.424 ms, decode 0.730 ->
-// 0.421 ms against one thread-block-wide pass per sweep with row loads into
+// threshold 1e-3 of the range): encode 0.664 -> 0.416 ms, decode 0.730 ->
+// 0.431 ms against one thread-block-wide pass per sweep with row loads into
 // registers (fourteen barriers a block, 16-byte loads and stores that touch
 // 32 rows each).
 #include "cz_block.cuh"
